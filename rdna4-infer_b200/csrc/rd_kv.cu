@@ -103,6 +103,8 @@ rope_kernel(float *__restrict__ x, int n_tok, int n_heads, int head_dim, int n_r
             float freq_base, const int32_t *__restrict__ pos, const __grid_constant__ RopeTable tab) {
   const int pairs = n_rot / 2;
   __shared__ float s_freq[kMaxRopePairs];
+  pdl_launch_dependents();
+  pdl_wait();
   for (int i = threadIdx.x; i < pairs; i += blockDim.x)
     s_freq[i] = i < kRopeTablePairs ? tab.f[i] : rope_freq(freq_base, i, n_rot);
   __syncthreads();
@@ -123,6 +125,8 @@ rope_kernel(float *__restrict__ x, int n_tok, int n_heads, int head_dim, int n_r
 __global__ void deinterleave_kernel(const float4 *__restrict__ yq, float4 *__restrict__ q,
                                     float4 *__restrict__ gate, int64_t n_rows, int hd4) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   if (i >= n_rows * hd4) return;
   const int64_t r = i / hd4;
   const int d = (int)(i % hd4);
@@ -132,6 +136,8 @@ __global__ void deinterleave_kernel(const float4 *__restrict__ yq, float4 *__res
 
 __global__ void sigmoid_gate_kernel(float *__restrict__ g, float *__restrict__ y, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   if (i >= n) return;
   const float s = __fdiv_rn(1.0f, 1.0f + expf(-g[i]));
   g[i] = s;
@@ -212,25 +218,28 @@ int launch_rope(float *x, int n_tok, int n_heads, int head_dim, int n_rot, float
                 const int32_t *pos, cudaStream_t st) {
   const int64_t total = (int64_t)n_tok * n_heads * (n_rot / 2);
   if (total == 0) return RD_OK;
-  rope_kernel<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(x, n_tok, n_heads, head_dim, n_rot,
-                                                               freq_base, pos,
-                                                               make_rope_table(n_rot, freq_base));
-  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_CUDA;
+  return launch_pdl(8, rope_kernel, dim3((unsigned)((total + 127) / 128)), dim3(128), 0, st, x, n_tok, n_heads,
+                    head_dim, n_rot, freq_base, pos, make_rope_table(n_rot, freq_base)) == cudaSuccess
+             ? RD_OK
+             : RD_ERR_CUDA;
 }
 
 int launch_deinterleave(const float *yq, float *q, float *gate, int64_t n_rows, int head_dim,
                         cudaStream_t st) {
   const int64_t n = n_rows * (head_dim / 4);
   if (n == 0) return RD_OK;
-  deinterleave_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-      (const float4 *)yq, (float4 *)q, (float4 *)gate, n_rows, head_dim / 4);
-  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_CUDA;
+  return launch_pdl(8, deinterleave_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (const float4 *)yq,
+                    (float4 *)q, (float4 *)gate, n_rows, head_dim / 4) == cudaSuccess
+             ? RD_OK
+             : RD_ERR_CUDA;
 }
 
 int launch_sigmoid_gate(float *g, float *y, int64_t n, cudaStream_t st) {
   if (n == 0) return RD_OK;
-  sigmoid_gate_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, y, n);
-  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_CUDA;
+  return launch_pdl(8, sigmoid_gate_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, g, y, n) ==
+                 cudaSuccess
+             ? RD_OK
+             : RD_ERR_CUDA;
 }
 
 // ---- stored rows -> f16 rows (the dequantizing loads of include/rdna4/kv.h:174-368) ------
@@ -329,6 +338,8 @@ kv_dequant_f16_kernel(const uint8_t *__restrict__ ksrc, uint4 *__restrict__ kdst
   const uint8_t *src = blockIdx.y == 0 ? ksrc : vsrc;
   uint4 *dst = blockIdx.y == 0 ? kdst : vdst;
   const int type = blockIdx.y == 0 ? kt : vt;
+  pdl_wait();
+  pdl_launch_dependents();   // after the wait: the tile kernel loads the caches without one
   if (src == nullptr) return;
   switch (type) {   // the same for the whole CTA
     case RD_KV_F32: dequant_tile<RD_KV_F32>(src, dst, n_blocks, blockIdx.x, stage); break;
@@ -350,9 +361,10 @@ int launch_kv_dequant_f16_pair(int kt, const void *k, void *kdst, int vt, const 
   const int64_t n_blocks = n_values / 32;
   if (n_blocks == 0 || (k == nullptr && v == nullptr)) return RD_OK;
   const dim3 grid((unsigned)((n_blocks + kDqTileBlocks - 1) / kDqTileBlocks), 2);
-  kv_dequant_f16_kernel<<<grid, 256, 0, st>>>((const uint8_t *)k, (uint4 *)kdst, kt, (const uint8_t *)v,
-                                              (uint4 *)vdst, vt, n_blocks);
-  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_CUDA;
+  return launch_pdl(8, kv_dequant_f16_kernel, grid, dim3(256), 0, st, (const uint8_t *)k, (uint4 *)kdst, kt,
+                    (const uint8_t *)v, (uint4 *)vdst, vt, n_blocks) == cudaSuccess
+             ? RD_OK
+             : RD_ERR_CUDA;
 }
 
 int launch_kv_dequant_f16(int type, const void *src, void *dst, int64_t n_values, cudaStream_t st) {

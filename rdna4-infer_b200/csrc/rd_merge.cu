@@ -205,7 +205,9 @@ int launch_merge_multi(const DecodeSeq *dev_seqs, const float *records, int n_se
   const int rows = n_seq * q_len * n_head;
   if (rows == 0) return RD_OK;
   const dim3 grid((unsigned)rows, kHeadDim / kMergeDims, 1);
-  return launch_pdl(4, merge_kernel<2>, grid, dim3(kMergeDims * kMergeGroups), 0, st, records, nullptr, 0, 1,
+  // not a dependent launch: thousands of CTAs that would take SM slots from the decode launch's
+  // last ones
+  return launch_pdl(0, merge_kernel<2>, grid, dim3(kMergeDims * kMergeGroups), 0, st, records, nullptr, 0, 1,
                     nullptr, dev_seqs, q_len * n_head, ExtraKey{}) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;

@@ -25,6 +25,8 @@ __global__ void __launch_bounds__(kRmsThreads)
 rms_norm_kernel(const float *__restrict__ x, const float *__restrict__ w, float *__restrict__ y,
                 int64_t ncols, float eps) {
   __shared__ float partial[kRmsThreads];
+  pdl_launch_dependents();
+  pdl_wait();
   const float *xr = x + (int64_t)blockIdx.x * ncols;
   float *yr = y + (int64_t)blockIdx.x * ncols;
   float acc = 0.0f;
@@ -47,8 +49,10 @@ rms_norm_kernel(const float *__restrict__ x, const float *__restrict__ w, float 
 int launch_rms_norm(const float *x, const float *w, float *y, int64_t nrows, int64_t ncols, float eps,
                     cudaStream_t st) {
   if (nrows == 0) return RD_OK;
-  rms_norm_kernel<<<(unsigned)nrows, kRmsThreads, 0, st>>>(x, w, y, ncols, eps);
-  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_CUDA;
+  return launch_pdl(8, rms_norm_kernel, dim3((unsigned)nrows), dim3(kRmsThreads), 0, st, x, w, y, ncols, eps) ==
+                 cudaSuccess
+             ? RD_OK
+             : RD_ERR_CUDA;
 }
 
 struct PreAttnArgs {
@@ -115,6 +119,8 @@ __global__ void __launch_bounds__(256) pre_attn_kernel(const __grid_constant__ P
   const int lane = threadIdx.x & 31;
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int per_tok = a.n_head + 2 * a.nkv;
+  pdl_launch_dependents();
+  pdl_wait();
   if (row >= (int64_t)a.n_tok * per_tok) return;
   const int tok = (int)(row / per_tok), r = (int)(row % per_tok);
   float x[8];
@@ -151,9 +157,10 @@ __global__ void __launch_bounds__(256) pre_attn_kernel(const __grid_constant__ P
 
 template <int KT>
 static int pre_attn_v(int vt, const PreAttnArgs &a, unsigned grid, cudaStream_t st) {
+  cudaError_t err = cudaSuccess;
 #define RD_V(VT)                                  \
   case VT:                                        \
-    pre_attn_kernel<KT, VT><<<grid, 256, 0, st>>>(a); \
+    err = launch_pdl(8, pre_attn_kernel<KT, VT>, dim3(grid), dim3(256), 0, st, a); \
     break;
   switch (vt) {
     RD_V(RD_KV_F32)
@@ -165,7 +172,7 @@ static int pre_attn_v(int vt, const PreAttnArgs &a, unsigned grid, cudaStream_t 
     default: return RD_ERR_TYPE;
   }
 #undef RD_V
-  return cudaGetLastError() == cudaSuccess ? RD_OK : RD_ERR_CUDA;
+  return err == cudaSuccess ? RD_OK : RD_ERR_CUDA;
 }
 
 int launch_pre_attn(int kt, int vt, const float *qg, const float *k_src, const float *v_src,

@@ -665,6 +665,7 @@ prefill_merge_kernel(const float *__restrict__ records, float *__restrict__ out,
                      int64_t n_rows, int n_splits) {
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 6);
   const int tx = threadIdx.x & 63;
+  pdl_launch_dependents();
   pdl_wait();   // launched under the tile kernel: its records are complete from here on
   if (row >= n_rows) return;
   const float *rec = records + (size_t)row * n_splits * kRec;
@@ -726,6 +727,9 @@ q_prep_kernel(const float *__restrict__ q, const int32_t *__restrict__ pos, int 
               uint4 *__restrict__ k_dst, uint4 *__restrict__ v_dst, int nkv,
               const __grid_constant__ RopeTable tab) {
   __shared__ float2 s_cs[32];
+  // the wait comes first: the tile kernel, launched under this pass, loads cache rows that
+  // earlier kernels wrote without waiting for this one
+  pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pairs = n_rot / 2;
@@ -882,10 +886,11 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   a.records = records;
   const dim3 grid((unsigned)((n_q + kPfM - 1) / kPfM), (unsigned)n_head, (unsigned)n_splits);
   if (prepass) {
-    q_prep_kernel<<<(unsigned)n_q, 256, 0, st>>>(q, pos, n_head, n_rot, a.qscale, (uint4 *)q16, k_new, v_new,
-                                                (uint4 *)k_dst, (uint4 *)v_dst, n_head_kv,
-                                                make_rope_table(n_rot, freq_base));
-    if (cudaGetLastError() != cudaSuccess) return RD_ERR_CUDA;
+    // (a pass of many waves gains nothing from starting early: measured 1.8 % slower at 8192 tokens)
+    if (launch_pdl(n_q <= 1024 ? 8 : 0, q_prep_kernel, dim3((unsigned)n_q), dim3(256), 0, st, q, pos, n_head, n_rot, a.qscale,
+                   (uint4 *)q16, k_new, v_new, (uint4 *)k_dst, (uint4 *)v_dst, n_head_kv,
+                   make_rope_table(n_rot, freq_base)) != cudaSuccess)
+      return RD_ERR_CUDA;
     // the tile kernel may start while that pass runs; it waits for it (griddepcontrol)
     // before it loads its Q tile
     cudaLaunchConfig_t cfg = {};
