@@ -71,8 +71,14 @@ struct PreAttnArgs {
   RopeTable rope;
 };
 
-// Normalise (optional) and rotate the 8 values a lane holds of one head row.
-__device__ __forceinline__ void norm_rope_row(float (&x)[8], const float *__restrict__ w, float eps,
+// Frequencies beyond the table (n_rot above 128): kept out of line, the common path stays short.
+__device__ __noinline__ float rope_freq_slow(float freq_base, int p, int n_rot) {
+  return (float)pow((double)freq_base, (double)(-2.0f * (float)p / (float)n_rot));
+}
+
+// Normalise (optional) and rotate the 8 values a lane holds of one head row; wv holds the
+// lane's norm weights.
+__device__ __forceinline__ void norm_rope_row(float (&x)[8], const float (&wv)[8], bool weighted, float eps,
                                               int n_rot, float fpos, const RopeTable &tab,
                                               float freq_base, int lane) {
   float p[8];
@@ -90,77 +96,110 @@ __device__ __forceinline__ void norm_rope_row(float (&x)[8], const float *__rest
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     x[k] = __fmul_rn(x[k], scale);
-    if (w != nullptr) x[k] = __fmul_rn(x[k], w[lane + 32 * k]);
+    if (weighted) x[k] = __fmul_rn(x[k], wv[k]);
   }
   const int hk = n_rot / 64;   // registers per half: pairs (k, k + hk), k < hk
+#pragma unroll 1
+  for (int k = 0; k < hk; ++k) {
+    const int pidx = lane + 32 * k;
+    const float freq = pidx < kRopeTablePairs ? tab.f[pidx] : rope_freq_slow(freq_base, pidx, n_rot);
+    float c, sn;
+    sincosf(fpos * freq, &sn, &c);
+    // x[k] and x[k + hk] by value: the loop stays rolled (one sincosf in the code) and x in registers
+    float x0 = 0.f, x1 = 0.f;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (k < hk) {
-      const int pidx = lane + 32 * k;
-      const float freq = pidx < kRopeTablePairs
-                             ? tab.f[pidx]
-                             : (float)pow((double)freq_base, (double)(-2.0f * (float)pidx / (float)n_rot));
-      float c, sn;
-      sincosf(fpos * freq, &sn, &c);
-#pragma unroll
-      for (int h = 1; h <= 4; ++h) {
-        if (h == hk && k + h < 8) {
-          const float x0 = x[k], x1 = x[k + h];
-          x[k] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, sn));
-          x[k + h] = __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, c));
-        }
-      }
+    for (int i = 0; i < 8; ++i) {
+      x0 = i == k ? x[i] : x0;
+      x1 = i == k + hk ? x[i] : x1;
     }
+    const float y0 = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, sn));
+    const float y1 = __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, c));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = i == k ? y0 : i == k + hk ? y1 : x[i];
   }
 }
 
-template <int KT, int VT>
+// SPLIT (a decode step or a verify block): latency-bound, so a warp quantizes ONE 32-value
+// block -- the eight blocks of a K row are eight warps that each load and normalise the whole
+// row (its sum of squares needs it; the loads hit L1 / L2) -- and everything a row needs is
+// requested before anything is used. At one token that is 88 short warps over 22 CTAs where one
+// warp per row ran eight quantizations in sequence on 4 SMs, in code eight times as long
+// (instruction fetch is a large part of a kernel that runs once): a 16-layer step over 137 f16
+// keys 253 -> 240 us, over 4096 keys 350 -> 294 us. Without SPLIT (prompt chunks) a warp owns a whole row.
+constexpr int kPreSplitTokens = 8;
+template <int KT, int VT, bool SPLIT>
 __global__ void __launch_bounds__(256) pre_attn_kernel(const __grid_constant__ PreAttnArgs a) {
   const int lane = threadIdx.x & 31;
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int per_tok = a.n_head + 2 * a.nkv;
+  const int kv_warps = SPLIT ? 8 * a.nkv : a.nkv;   // per tensor
+  const int per_tok = a.n_head + 2 * kv_warps;
   pdl_launch_dependents();
   pdl_wait();
   if (row >= (int64_t)a.n_tok * per_tok) return;
-  const int tok = (int)(row / per_tok), r = (int)(row % per_tok);
-  float x[8];
-  if (r < a.n_head) {
-    // a query head: split off the gate, normalise, rotate
-    const float *src = a.qg + ((size_t)tok * a.n_head + r) * (2 * kHeadDim);
+  const int tok = (int)(row / per_tok);
+  int r = (int)(row % per_tok);
+  if (r >= a.n_head + kv_warps) {   // a V row, or one block of it
+    r -= a.n_head + kv_warps;
+    const int kvh = SPLIT ? r >> 3 : r;
+    const float *src = a.v_src + ((size_t)tok * a.nkv + kvh) * kHeadDim;
+    uint8_t *dst = a.v_rows + ((size_t)tok * a.nkv + kvh) * row_bytes(VT);
+    if (SPLIT) {
+      store_block<VT>(src[lane + 32 * (r & 7)], dst, r & 7, lane);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) store_block<VT>(src[lane + 32 * k], dst, k, lane);
+    }
+    return;
+  }
+  const bool is_q = r < a.n_head;
+  const int kvh = SPLIT ? (r - a.n_head) >> 3 : r - a.n_head;
+  const float *src = is_q ? a.qg + ((size_t)tok * a.n_head + r) * (2 * kHeadDim)
+                          : a.k_src + ((size_t)tok * a.nkv + kvh) * kHeadDim;
+  const float *w = is_q ? a.q_w : a.k_w;
+  const float fpos = (float)a.pos[tok];
+  float x[8], wv[8], gv[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    x[k] = src[lane + 32 * k];
+    wv[k] = w != nullptr ? w[lane + 32 * k] : 1.f;
+    gv[k] = is_q ? src[kHeadDim + lane + 32 * k] : 0.f;
+  }
+  norm_rope_row(x, wv, w != nullptr, a.eps, a.n_rot, fpos, a.rope, a.freq_base, lane);
+  if (is_q) {
+    // a query head: the gate split off, the row normalised and rotated
     float *qo = a.q_out + ((size_t)tok * a.n_head + r) * kHeadDim;
     float *go = a.gate_out + ((size_t)tok * a.n_head + r) * kHeadDim;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      x[k] = src[lane + 32 * k];
-      go[lane + 32 * k] = src[kHeadDim + lane + 32 * k];
+      qo[lane + 32 * k] = x[k];
+      go[lane + 32 * k] = gv[k];
     }
-    norm_rope_row(x, a.q_w, a.eps, a.n_rot, (float)a.pos[tok], a.rope, a.freq_base, lane);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) qo[lane + 32 * k] = x[k];
-  } else if (r < a.n_head + a.nkv) {
-    const int kvh = r - a.n_head;
-    const float *src = a.k_src + ((size_t)tok * a.nkv + kvh) * kHeadDim;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = src[lane + 32 * k];
-    norm_rope_row(x, a.k_w, a.eps, a.n_rot, (float)a.pos[tok], a.rope, a.freq_base, lane);
-    uint8_t *dst = a.k_rows + ((size_t)tok * a.nkv + kvh) * row_bytes(KT);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) store_block<KT>(x[k], dst, k, lane);
   } else {
-    const int kvh = r - a.n_head - a.nkv;
-    const float *src = a.v_src + ((size_t)tok * a.nkv + kvh) * kHeadDim;
-    uint8_t *dst = a.v_rows + ((size_t)tok * a.nkv + kvh) * row_bytes(VT);
+    uint8_t *dst = a.k_rows + ((size_t)tok * a.nkv + kvh) * row_bytes(KT);
+    if (SPLIT) {
+      const int blk = (r - a.n_head) & 7;
+      float v = x[0];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) store_block<VT>(src[lane + 32 * k], dst, k, lane);
+      for (int k = 1; k < 8; ++k) v = k == blk ? x[k] : v;
+      store_block<KT>(v, dst, blk, lane);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) store_block<KT>(x[k], dst, k, lane);
+    }
   }
 }
 
 template <int KT>
-static int pre_attn_v(int vt, const PreAttnArgs &a, unsigned grid, cudaStream_t st) {
+static int pre_attn_v(int vt, const PreAttnArgs &a, cudaStream_t st) {
+  const bool split = a.n_tok <= kPreSplitTokens;
+  const int64_t warps = (int64_t)a.n_tok * (a.n_head + 2 * (split ? 8 : 1) * a.nkv);
+  const int per_cta = split ? 4 : 8;
+  const dim3 grid((unsigned)((warps + per_cta - 1) / per_cta)), block(32 * per_cta);
   cudaError_t err = cudaSuccess;
-#define RD_V(VT)                                  \
-  case VT:                                        \
-    err = launch_pdl(8, pre_attn_kernel<KT, VT>, dim3(grid), dim3(256), 0, st, a); \
+#define RD_V(VT)                                                                             \
+  case VT:                                                                                   \
+    err = split ? launch_pdl(8, pre_attn_kernel<KT, VT, true>, grid, block, 0, st, a)        \
+                : launch_pdl(8, pre_attn_kernel<KT, VT, false>, grid, block, 0, st, a);      \
     break;
   switch (vt) {
     RD_V(RD_KV_F32)
@@ -198,10 +237,8 @@ int launch_pre_attn(int kt, int vt, const float *qg, const float *k_src, const f
   a.eps = eps;
   a.freq_base = freq_base;
   a.rope = make_rope_table(n_rot, freq_base);
-  const int64_t warps = (int64_t)n_tok * (n_head + 2 * nkv);
-  const unsigned grid = (unsigned)((warps * 32 + 255) / 256);
 #define RD_K(KT) \
-  case KT: return pre_attn_v<KT>(vt, a, grid, st);
+  case KT: return pre_attn_v<KT>(vt, a, st);
   switch (kt) {
     RD_K(RD_KV_F32)
     RD_K(RD_KV_F16)
