@@ -104,12 +104,13 @@ int attn_core(const float *q, const void *k, const void *v, float *out, float *r
               float scale, int kt, int vt, float *gate, void *ws, size_t ws_bytes,
               DeviceStatus *status, int sms, cudaStream_t st) {
   const int tile = decode_tile_keys(kt, vt);
-  int64_t tiles = -1;
+  int64_t tiles = -1, n_keys = -1;
   if (pos == nullptr) {
-    const int64_t n_keys = t >= key_begin ? (int64_t)t - key_begin + 1 : 0;
+    n_keys = t >= key_begin ? (int64_t)t - key_begin + 1 : 0;
     tiles = (n_keys + tile - 1) / tile;
   }
-  int S = plan_splits(sms, n_tok, tiles);
+  const int direct = n_tok == 1 && out != nullptr ? step_splits(kt, vt, n_head_kv, n_keys) : 0;
+  int S = direct > 0 ? direct : plan_splits(sms, n_tok, tiles);
   if (out == nullptr) {
     // nest the internal splits inside the caller's: S = n_rec * r
     int r = S / n_rec;
@@ -136,7 +137,8 @@ int attn_core(const float *q, const void *k, const void *v, float *out, float *r
   const size_t need = partial_floats(n_tok, n_head, S) * sizeof(float);
   if (ws == nullptr || ws_bytes < need) return RD_ERR_WORKSPACE;
   a.partial = (float *)ws;
-  int rc = launch_decode(kt, vt, a, st);
+  if (direct > 0) return launch_step(kt, vt, a, out, gate, st);   // short context: one launch, no records
+  const int rc = launch_decode(kt, vt, a, st);
   if (rc != RD_OK) return rc;
   if (out != nullptr) return launch_merge((const float *)ws, out, n_tok * n_head, S, gate, st);
   return launch_merge_records((const float *)ws, records, n_tok * n_head, S, n_rec, st);
@@ -476,11 +478,13 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
   if ((rc = current_device(&dev)) != RD_OK) return rc;
   DeviceStatus *status = status_word(dev);   // every launch reports its bounded waits
   if (status == nullptr) return RD_ERR_CUDA;
-  // keys 0..t-1 through the split-KV kernel (whose first CTAs also store row t), then the
-  // merge with row t folded in
+  // Short contexts: one launch, row t quantized and stored by the CTAs that attend it. Otherwise
+  // keys 0..t-1 through the split-KV kernel (whose first CTAs also store row t), then the merge with
+  // row t folded in.
   const int tile = decode_tile_keys(k_type, v_type);
   const int64_t tiles = ((int64_t)t + tile - 1) / tile;
-  const int S = plan_splits(sm_count(dev), 1, tiles);
+  const int direct = step_splits(k_type, v_type, n_head_kv, (int64_t)t + 1);
+  const int S = direct > 0 ? direct : plan_splits(sm_count(dev), 1, tiles);
   if (workspace_bytes < partial_floats(1, n_head, S) * sizeof(float)) return RD_ERR_WORKSPACE;
   DecodeArgs a;
   a.q = q;
@@ -488,7 +492,7 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
   a.v = v_cache;
   a.partial = (float *)workspace;
   a.pos = nullptr;
-  a.t = t - 1;
+  a.t = direct > 0 ? t : t - 1;
   a.key_begin = 0;
   a.n_tok = 1;
   a.n_head = n_head;
@@ -500,6 +504,7 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
   a.v_new = v_new;
   a.new_row = t;
   cudaStream_t st = (cudaStream_t)stream;
+  if (direct > 0) return launch_step(k_type, v_type, a, out, gate, st);
   if ((rc = launch_decode(k_type, v_type, a, st)) != RD_OK) return rc;
   ExtraKey x;
   x.q = q;

@@ -82,6 +82,13 @@ struct DecodeArgs {
   float *push_gate = nullptr;   // optional
 };
 int launch_decode(int kt, int vt, const DecodeArgs &a, cudaStream_t st);
+// Short contexts, one token (rd_step.cuh): a cluster of n_splits CTAs per KV head attends keys
+// key_begin..t and writes the merged, optionally gated output itself (`partial` is not used). With
+// k_new / v_new the rows of key t are also quantized and stored as cache row t.
+int launch_step(int kt, int vt, const DecodeArgs &a, float *out, float *gate, cudaStream_t st);
+// CTAs per KV head of that launch for n_keys keys, or 0 where launch_decode is the faster one (or
+// n_keys < 0: not known on the host).
+int step_splits(int kt, int vt, int n_head_kv, int64_t n_keys);
 
 // One sequence of a multi-sequence launch, as the kernels read it from device memory.
 // The last of the q_len new tokens attends keys 0..t, token i keys 0..t-(q_len-1-i).
