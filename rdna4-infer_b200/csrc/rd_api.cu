@@ -92,6 +92,13 @@ int plan_splits(int sms, int n_tok, int64_t tiles_known) {
   return s;
 }
 
+// The same for a block of tokens: one CTA per (split, KV head, chunk of tokens). The key count is on the
+// device, so short contexts leave CTAs with empty records.
+int block_splits(int sms, int n_tok, int n_head_kv) {
+  const int per_split = n_head_kv * ((n_tok + block_chunk(n_tok) - 1) / block_chunk(n_tok));
+  return sms / per_split > 1 ? sms / per_split : 1;
+}
+
 size_t partial_floats(int n_tok, int n_head, int splits) {
   return (size_t)n_tok * n_head * splits * kRec;
 }
@@ -110,7 +117,7 @@ int attn_core(const float *q, const void *k, const void *v, float *out, float *r
     tiles = (n_keys + tile - 1) / tile;
   }
   const int direct = n_tok == 1 && out != nullptr ? step_splits(kt, vt, n_head_kv, n_keys) : 0;
-  int S = direct > 0 ? direct : plan_splits(sms, n_tok, tiles);
+  int S = direct > 0 ? direct : n_tok > 1 ? block_splits(sms, n_tok, n_head_kv) : plan_splits(sms, n_tok, tiles);
   if (out == nullptr) {
     // nest the internal splits inside the caller's: S = n_rec * r
     int r = S / n_rec;
@@ -130,24 +137,26 @@ int attn_core(const float *q, const void *k, const void *v, float *out, float *r
   a.scale = scale;
   a.n_splits = S;
   a.status = status;
+  // a block of tokens shares each dequantized key; one token has a warp per (head, key group)
+  auto launch = [&] { return n_tok > 1 ? launch_block(kt, vt, a, block_chunk(n_tok), st) : launch_decode(kt, vt, a, st); };
   if (out == nullptr && S == n_rec) {
     a.partial = records;
-    return launch_decode(kt, vt, a, st);
+    return launch();
   }
   const size_t need = partial_floats(n_tok, n_head, S) * sizeof(float);
   if (ws == nullptr || ws_bytes < need) return RD_ERR_WORKSPACE;
   a.partial = (float *)ws;
   if (direct > 0) return launch_step(kt, vt, a, out, gate, st);   // short context: one launch, no records
-  const int rc = launch_decode(kt, vt, a, st);
+  const int rc = launch();
   if (rc != RD_OK) return rc;
   if (out != nullptr) return launch_merge((const float *)ws, out, n_tok * n_head, S, gate, st);
   return launch_merge_records((const float *)ws, records, n_tok * n_head, S, n_rec, st);
 }
 
-size_t workspace_bytes_for(int sms, int n_tok, int n_head) {
+size_t workspace_bytes_for(int sms, int n_tok, int n_head, int n_head_kv) {
   // the largest split count attn_core can pick for this token count, plus slack for
   // the "nest inside the caller's splits" rounding
-  const int s = plan_splits(sms, n_tok, -1);
+  const int s = n_tok > 1 ? block_splits(sms, n_tok, n_head_kv) : plan_splits(sms, n_tok, -1);
   return partial_floats(n_tok, n_head, s) * sizeof(float) + 256;
 }
 
@@ -167,7 +176,7 @@ int attn_alloc(const float *q, const void *k, const void *v, float *out, float *
   DeviceStatus *status = status_word(dev);   // every launch reports its bounded waits
   if (status == nullptr) return RD_ERR_CUDA;
   const int sms = sm_count(dev);
-  size_t bytes = workspace_bytes_for(sms, n_tok, n_head);
+  size_t bytes = workspace_bytes_for(sms, n_tok, n_head, n_head_kv);
   if (out == nullptr) {
     const size_t nested = partial_floats(n_tok, n_head, sms + n_rec) * sizeof(float);
     if (nested > bytes) bytes = nested;
@@ -603,14 +612,18 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
 
   // Key split: chunks of equal length over all sequences, about four CTAs per SM in
   // total, so that a 32k-key sequence and a 1k-key one load the SMs evenly.
-  const int tile = decode_tile_keys(k_type, v_type);
+  // Blocks of tokens (q_len > 1) are CTAs per KV head: eight of those per SM, fewer where an item's
+  // records (one per token and head) would outgrow the workspace's 4 * sms + n_seq * q_len.
+  const int tok_chunk = block_chunk(q_len), n_chunks = (q_len + tok_chunk - 1) / tok_chunk;
+  const int tile = q_len > 1 ? 64 : decode_tile_keys(k_type, v_type);
+  const int target = q_len > 1 ? std::max(1, std::min(8 * sms / n_head_kv, 4 * sms / tok_chunk)) : 4 * sms;
   std::vector<int> tiles(n_seq);
   int64_t total = 0;
   for (int i = 0; i < n_seq; ++i) {
     tiles[i] = (seqs[i].t + tile) / tile;  // ceil((t + 1) / tile)
-    total += (int64_t)tiles[i] * q_len;
+    total += (int64_t)tiles[i] * n_chunks;
   }
-  int64_t chunk = (total + 4 * sms - 1) / (4 * sms);
+  int64_t chunk = (total + target - 1) / target;
   if (chunk < 4) chunk = 4;
   unsigned char *body = (unsigned char *)plan + kMultiPlanHeaderBytes;
   DecodeSeq *hs = reinterpret_cast<DecodeSeq *>(body);
@@ -637,7 +650,7 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
   for (int oi = 0; oi < n_seq; ++oi) {  // longest sequences first
     const int i = order[oi];
     for (int sp = 0; sp < hs[i].n_splits; ++sp)
-      for (int tok = 0; tok < q_len; ++tok) {
+      for (int tok = 0; tok < q_len; tok += tok_chunk) {
         if (n_items >= max_items) return RD_ERR_WORKSPACE;  // cannot happen by the bound above
         hi[n_items++] = make_int4(i, tok, sp, 0);
       }
@@ -653,7 +666,7 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
   a.host_seqs = hs;
   a.n_seq = n_seq;
   a.n_head_kv = n_head_kv;
-  if ((rc = launch_decode_multi(k_type, v_type, a, nullptr)) != RD_OK) return rc;
+  if ((rc = (q_len > 1 ? launch_block_multi : launch_decode_multi)(k_type, v_type, a, nullptr)) != RD_OK) return rc;
   MultiPlanHeader h;
   memset(&h, 0, sizeof(h));
   h.magic = kMultiPlanMagic;
@@ -706,7 +719,9 @@ int rd_attn_multi_launch(const void *plan, float scale, void *workspace, size_t 
   a.scale = scale;
   a.records = reinterpret_cast<float *>((unsigned char *)workspace + off_rec);
   a.status = status;
-  if ((rc = launch_decode_multi(h.k_type, h.v_type, a, (cudaStream_t)stream)) != RD_OK) return rc;
+  if ((rc = (h.q_len > 1 ? launch_block_multi : launch_decode_multi)(h.k_type, h.v_type, a, (cudaStream_t)stream)) !=
+      RD_OK)
+    return rc;
   return launch_merge_multi(a.dev_seqs, a.records, h.n_seq, h.q_len, h.n_head, (cudaStream_t)stream);
 }
 

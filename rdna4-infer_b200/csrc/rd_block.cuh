@@ -1,0 +1,536 @@
+// Attention of a BLOCK of query tokens (speculative verify, short chunks) over caches of any type:
+// up to eight tokens share every dequantized K and V value.
+//
+// Replaces attn_batch_kernel / attn_split_batch_kernel (include/rdna4/attn.cuh:268-424, 686-1049),
+// which re-read and re-expand the prefix for every token. Grid (n_splits, n_head_kv, token chunks) or
+// (work items, n_head_kv): a CTA owns a run of 64-key slots of one KV head and the 6 T <= 48 score
+// columns (token, query head) of its chunk, NT = 2, 3, 4 or 6 MMA tiles of 8 columns.
+//
+// The CTA's warps form teams of four; a team streams slots through its own ring (a tensor-map box of
+// [64 keys][one head's row] for quantized caches, a bulk copy per row for f16 / f32 rows, whose padded
+// boxes would fetch a cache line more than the row has). Per slot
+//   * warp w multiplies keys 16 w .. 16 w + 15 with all columns (K fragments dequantized in
+//     registers once, query fragments from shared memory);
+//   * one barrier (with the vote "does any score exceed the team's reference?") frees the K slot and
+//     the previous V slot, which the team's first warp refills;
+//   * the weights go to shared memory as MMA fragments, a second barrier, and warp w multiplies all 64
+//     keys with its quarter of the output dims: every V value is dequantized once, by one warp, and a
+//     warp holds 16 NT accumulators where a warp with all dims would hold 64 NT.
+// One record (m, l, acc[256]) per (token, head) and split, merged by merge_kernel.
+//
+// What bounds it: the 32 NT mma.sync of 16 keys (about 13 cycles each per scheduler) for 4-bit caches
+// from four tokens, the fetch of the narrow rows for 8-bit and f16 caches.
+#pragma once
+#include <string.h>
+
+#include <type_traits>
+
+#include "rd_frag.cuh"
+#include "rd_internal.h"
+
+namespace rd {
+
+constexpr int kBlkKeys = 64;       // keys per slot
+constexpr int kBlkSmem = 222 * 1024;   // dynamic; the static arrays take up to 4.5 KB
+constexpr int kBlkPlane = 268;     // floats per column in the epilogue planes (12 mod 32)
+constexpr float kBlkSlack = 8.0f;  // see kRefSlack
+constexpr float kBlkNone = -1.0e30f;
+
+// column tiles for a chunk of n tokens
+__host__ __device__ constexpr int block_tiles(int n) { return n <= 2 ? 2 : n <= 4 ? 3 : n == 5 ? 4 : 6; }
+
+template <int KT, int VT, int NT>
+struct BlockGeo {
+  static constexpr int kPK = slot_pitch(KT), kPV = slot_pitch(VT);
+  static constexpr int kSK = kBlkKeys * kPK, kSV = kBlkKeys * kPV;   // multiples of 128
+  static constexpr int kQBytes = NT * 4096;                          // query fragments
+  static constexpr int kPBytes = NT * 1024;                          // weight fragments of a slot, per team
+  static constexpr int kHead = 512 + 512 + kQBytes;                  // barriers, dim table, query fragments
+  static constexpr int budget(int teams) { return (kBlkSmem - kHead) / teams - kPBytes; }
+  // two teams where each gets at least one slot, and another K or V of the next
+  static constexpr int kTeams = budget(2) >= kSK + kSV + (kSK < kSV ? kSK : kSV) ? 2 : 1;
+  static constexpr int kRing = budget(kTeams) & ~127;
+  static constexpr int kBoth = min_i(4, kRing / (kSK + kSV));
+  // what is left takes one more V (K is refilled half a slot earlier than V)
+  static constexpr int DK = kBoth, DV = kBoth < 4 && kRing >= kBoth * (kSK + kSV) + kSV ? kBoth + 1 : kBoth;
+  static constexpr int kRingBytes = DK * kSK + DV * kSV;
+  static constexpr int kPlaneBytes = NT * 8 * kBlkPlane * 4;   // a team's ring doubles as its plane
+  static constexpr int kTeamBytes = kPBytes + (kRingBytes > kPlaneBytes ? kRingBytes : (kPlaneBytes + 127) & ~127);
+  static constexpr int kSmem = kHead + kTeams * kTeamBytes;
+  static constexpr int kThreads = kTeams * 128;
+  static_assert(kBoth >= 1 && kSK % 128 == 0 && kSV % 128 == 0 && kSmem <= kBlkSmem, "ring geometry");
+  static_assert(kTeams * (DK + DV) * 8 <= 512, "barriers");
+};
+
+struct BlockArgs {
+  alignas(64) CUtensorMap tm_k;   // single sequence: boxes of [64 keys][slot_pitch], quantized types only
+  alignas(64) CUtensorMap tm_v;
+  const float *q;                 // [n_tok][n_head][256]
+  const uint8_t *k;
+  const uint8_t *v;
+  float *partial;                 // [n_tok][n_head][n_splits][258]
+  const int32_t *pos;             // device: token i attends keys 0..pos[i]
+  int n_tok;
+  int chunk;                      // tokens per chunk
+  int n_head;
+  int nkv;
+  float qscale;                   // scale * log2(e)
+  DeviceStatus *status;
+  const DecodeSeq *seqs;          // many sequences: CTA x works on items[x] = (sequence, first token, split)
+  const int4 *items;
+};
+
+// Barrier of one team, and one that also ORs a predicate over it.
+__device__ __forceinline__ void team_sync(int team) {
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + team) : "memory");
+}
+__device__ __forceinline__ bool team_any(int team, bool x) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)x), "r"(1 + team)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+
+template <int KT, int VT, int NT>
+__global__ void __launch_bounds__(BlockGeo<KT, VT, NT>::kThreads, 1)
+block_kernel(const __grid_constant__ BlockArgs p) {
+  using Geo = BlockGeo<KT, VT, NT>;
+  using KL = KLoad<KT>;
+  using VL = VLoad<VT>;
+  constexpr int RK = row_bytes(KT), RV = row_bytes(VT), PK = Geo::kPK, PV = Geo::kPV, SK = Geo::kSK, SV = Geo::kSV;
+  constexpr int DK = Geo::DK, DV = Geo::DV, TEAMS = Geo::kTeams, COLS = NT * 8;
+  constexpr bool BOX_K = KT >= RD_KV_Q8_0, BOX_V = VT >= RD_KV_Q8_0;
+  constexpr unsigned FULL = 0xffffffffu;
+
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ int s_abort;
+  __shared__ int s_t[COLS];                                  // last key of the column's token (-1: padding)
+  __shared__ float s_max[TEAMS][4][COLS], s_sum[TEAMS][4][COLS], s_ref[TEAMS][COLS];
+  __shared__ float s_wt[TEAMS][COLS], s_ml[COLS][2];
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, tq = lane & 3;
+  const int team = warp >> 2, part = warp & 3;
+  const int kvh = blockIdx.y, nkv = p.nkv;
+  const uint32_t sbase = smem_u32(smem);
+  const uint32_t bar_k = sbase + team * (DK + DV) * 8, bar_v = bar_k + DK * 8;
+  unsigned short *inv = reinterpret_cast<unsigned short *>(smem + 512);
+  const uint32_t qfrag = sbase + 1024;
+  const uint32_t team0 = sbase + Geo::kHead + team * Geo::kTeamBytes;
+  const uint32_t ring_k = team0, ring_v = ring_k + DK * SK;
+  const uint32_t pfrag = team0 + (Geo::kTeamBytes - Geo::kPBytes);
+
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int i = 0; i < TEAMS * (DK + DV); ++i) mbar_init(sbase + 8 * i, 1);
+    fence_barrier_init();
+  }
+  // dim -> byte offset of the half in a column's query fragments (inverts KL::dim): 16 bytes per
+  // (pair of MMAs, quad lane)
+  for (int i = threadIdx.x; i < 256; i += Geo::kThreads) {
+    const int tq_i = i >> 6, n_i = (i >> 2) & 15, e_i = i & 3;
+    inv[KL::dim(tq_i, n_i, e_i)] =
+        (unsigned short)((n_i >> 1) * 512 + tq_i * 16 + (n_i & 1) * 8 + (e_i >> 1) * 4 + (e_i & 1) * 2);
+  }
+  __syncthreads();
+  pdl_wait();   // everything below reads what earlier kernels of the stream wrote
+
+  int s, S, tok0, n_tok;
+  const float *qsrc;
+  const uint8_t *khead, *vhead;
+  const CUtensorMap *tmk = &p.tm_k, *tmv = &p.tm_v;
+  float *rec0;
+  int t_seq = 0;
+  if (p.items != nullptr) {
+    const int4 item = p.items[blockIdx.x];
+    if (item.x < 0) return;   // padding of a plan with a fixed item count
+    const DecodeSeq &d = p.seqs[item.x];
+    tok0 = item.y;
+    s = item.z;
+    S = d.n_splits;
+    t_seq = d.t - (p.n_tok - 1);   // the first token's last key
+    qsrc = d.q;
+    khead = d.k;
+    vhead = d.v;
+    tmk = reinterpret_cast<const CUtensorMap *>(d.tm_k);
+    tmv = reinterpret_cast<const CUtensorMap *>(d.tm_v);
+    rec0 = p.partial + (size_t)d.rec_base * kRec;
+    // these descriptors were written by an ordinary copy and may have been rewritten since an earlier
+    // launch read them: make the copy visible to the tensor-map proxy of the issuing threads
+    if (part == 0 && lane == 0) {
+      if (BOX_K) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmk) : "memory");
+      if (BOX_V) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmv) : "memory");
+    }
+  } else {
+    tok0 = blockIdx.z * p.chunk;
+    s = blockIdx.x;
+    S = gridDim.x;
+    qsrc = p.q;
+    khead = p.k;
+    vhead = p.v;
+    rec0 = p.partial;
+  }
+  n_tok = min(p.chunk, p.n_tok - tok0);
+  khead += (size_t)kvh * RK;
+  vhead += (size_t)kvh * RV;
+  const size_t kb = (size_t)nkv * RK, vb = (size_t)nkv * RV;
+  for (int c = threadIdx.x; c < COLS; c += Geo::kThreads) {
+    const int j = c / kGroup;
+    s_t[c] = j < n_tok ? (p.items != nullptr ? t_seq + tok0 + j : p.pos[tok0 + j]) : -1;
+  }
+  // query fragments, pre-scaled into log2 units (and by the loader's fixed-point factor); the padding
+  // columns are zero
+  {
+    const float qmul = p.qscale * KL::kUnscale;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < COLS * 64; i += Geo::kThreads) {
+      const int c = i >> 6, j = c / kGroup, h = c % kGroup;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j < n_tok)
+        v = *reinterpret_cast<const float4 *>(qsrc + ((size_t)(tok0 + j) * p.n_head + kvh * kGroup + h) * kHeadDim +
+                                              4 * (i & 63));
+      const uint32_t cb = qfrag + (c >> 3) * 4096 + (c & 7) * 64;
+      const uint2 off = *reinterpret_cast<const uint2 *>(inv + 4 * (i & 63));
+      const float x[4] = {v.x, v.y, v.z, v.w};
+      const uint32_t o[4] = {off.x & 0xffffu, off.x >> 16, off.y & 0xffffu, off.y >> 16};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const unsigned short hbits = __half_as_ushort(__float2half_rn(x[e] * qmul));
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(cb + o[e]), "h"(hbits) : "memory");
+      }
+    }
+  }
+  __syncthreads();
+  // last and first "last key" of the chunk's tokens
+  int t_max = -1, t_min = 0x7fffffff;
+  for (int c = 0; c < n_tok * kGroup; c += kGroup) {
+    t_max = max(t_max, s_t[c]);
+    t_min = min(t_min, s_t[c]);
+  }
+  const int slots_total = (t_max + kBlkKeys) / kBlkKeys;   // ceil((t_max + 1) / 64)
+  const int c_b = (int)(((int64_t)slots_total * s) / S), c_e = (int)(((int64_t)slots_total * (s + 1)) / S);
+  // the team's slots: c_b + team + i * TEAMS
+  const int n_mine = c_e - c_b > team ? (c_e - c_b - team + TEAMS - 1) / TEAMS : 0;
+
+  // Loads the team's i-th slot (one tensor) into its ring; warp-collective, by the team's first warp.
+  // Whole slots are one box; f16 / f32 rows and the last, partial slot go row by row, rows
+  // behind the last key repeating it.
+  auto fill = [&](auto is_v_c, int i) {
+    constexpr bool is_v = decltype(is_v_c)::value;
+    constexpr int R = is_v ? RV : RK, P = is_v ? PV : PK, DD = is_v ? DV : DK;
+    if (i >= n_mine) return;
+    const int row0 = (c_b + team + i * TEAMS) * kBlkKeys;
+    const uint32_t bar = (is_v ? bar_v : bar_k) + 8 * (i % DD);
+    const uint32_t dst = (is_v ? ring_v : ring_k) + (i % DD) * (is_v ? SV : SK);
+    if ((is_v ? BOX_V : BOX_K) && row0 + kBlkKeys - 1 <= t_max) {
+      if (lane == 0) {
+        mbar_expect_tx(bar, kBlkKeys * P);
+        tma_load_2d(dst, is_v ? tmv : tmk, kvh * (R / 8), row0, bar);
+      }
+      return;
+    }
+    if (lane == 0) mbar_expect_tx(bar, kBlkKeys * R);
+    __syncwarp();
+    const uint8_t *head = is_v ? vhead : khead;
+    const size_t stride = is_v ? vb : kb;
+#pragma unroll
+    for (int r = lane; r < kBlkKeys; r += 32) {
+      const int key = row0 + r > t_max ? t_max : row0 + r;
+      bulk_g2s(dst + r * P, head + (size_t)key * stride, R, bar);
+    }
+  };
+  const std::integral_constant<bool, false> is_k;
+  const std::integral_constant<bool, true> is_v;
+  if (part == 0) {
+    for (int i = 0; i < DV; ++i) {
+      if (i < DK) fill(is_k, i);
+      fill(is_v, i);
+    }
+  }
+
+  float O[4][NT][4];                     // [M-tile of this warp's quarter of the dims][column tile]
+  float ref[NT][2], run[NT][2], l[NT][2];   // per lane column: team's reference, lane-local maximum and sum
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    ref[nt][0] = ref[nt][1] = run[nt][0] = run[nt][1] = kBlkNone;
+    l[nt][0] = l[nt][1] = 0.f;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) O[m][nt][0] = O[m][nt][1] = O[m][nt][2] = O[m][nt][3] = 0.f;
+  }
+  const uint32_t qlane = qfrag + lane * 16;
+  bool dead = false;   // a bounded wait ran out: go through the motions (barriers) without waiting
+#pragma unroll 1
+  for (int i = 0; i < n_mine; ++i) {
+    const int row0 = (c_b + team + i * TEAMS) * kBlkKeys;
+    if (!dead && !mbar_wait(bar_k + 8 * (i % DK), (i / DK) & 1, p.status, 3)) s_abort = 1;
+    // ---- S = K Q^T: this warp's 16 keys x all columns ----
+    float Sv[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) Sv[nt][0] = Sv[nt][1] = Sv[nt][2] = Sv[nt][3] = 0.f;
+    {
+      const uint32_t kr = ring_k + (i % DK) * SK + (16 * part + g) * PK;
+      uint4 qf[NT];
+      KL::run(kr, kr + 8 * PK, tq, [&](int n, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          if ((n & 1) == 0) qf[nt] = lds128(qlane + nt * 4096 + (n >> 1) * 512);
+          mma16816(Sv[nt], a0, a1, a2, a3, (n & 1) ? qf[nt].z : qf[nt].x, (n & 1) ? qf[nt].w : qf[nt].y);
+        }
+      });
+    }
+    if (row0 + kBlkKeys - 1 > t_min) {   // some column ends inside or before this slot
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (row0 + 16 * part + g + (e >> 1) * 8 > s_t[8 * nt + 2 * tq + (e & 1)]) Sv[nt][e] = -INFINITY;
+    }
+    bool grow = false;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        run[nt][e] = fmaxf(run[nt][e], fmaxf(Sv[nt][e], Sv[nt][e + 2]));
+        grow |= run[nt][e] > ref[nt][e] + kBlkSlack;
+      }
+    // every warp of the team is done with this K slot and with the V slot before it
+    const bool any = team_any(team, grow);
+    dead = *(volatile int *)&s_abort != 0;
+    if (part == 0 && !dead) {
+      fill(is_k, i + DK);
+      if (i > 0) fill(is_v, i - 1 + DV);
+    }
+    if (any) {
+      // the team's references move to the current maxima of the columns (over its 64 key rows)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float m = run[nt][e];
+#pragma unroll
+          for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
+          if (g == 0) s_max[team][part][8 * nt + 2 * tq + e] = m;
+        }
+      team_sync(team);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int c = 8 * nt + 2 * tq + e;
+          // a whole number: the rounding of the weights to f16 then does not depend on it, and results
+          // for different key splits differ in the order of f32 sums only
+          const float m = fmaxf(ceilf(fmaxf(fmaxf(s_max[team][0][c], s_max[team][1][c]),
+                                            fmaxf(s_max[team][2][c], s_max[team][3][c]))), ref[nt][e]);
+          const float f = ex2(ref[nt][e] - m);
+          ref[nt][e] = m;
+          l[nt][e] *= f;
+#pragma unroll
+          for (int mt = 0; mt < 4; ++mt) {
+            O[mt][nt][e] *= f;
+            O[mt][nt][e + 2] *= f;
+          }
+        }
+    }
+    // ---- P^T fragments of this warp's keys -> shared memory ----
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const float p0 = ex2(Sv[nt][0] - ref[nt][0]), p1 = ex2(Sv[nt][1] - ref[nt][1]);
+      const float p2 = ex2(Sv[nt][2] - ref[nt][0]), p3 = ex2(Sv[nt][3] - ref[nt][1]);
+      const uint32_t h01 = pack_h2(p0, p1), h23 = pack_h2(p2, p3);
+      // the sums take the weights as rounded for the tensor core: a common rounding error of a column
+      // then cancels in the quotient
+      const float2 r01 = unpack_h2(h01), r23 = unpack_h2(h23);
+      l[nt][0] += r01.x + r23.x;
+      l[nt][1] += r01.y + r23.y;
+      const uint32_t b0 = movmatrix_trans(h01), b1 = movmatrix_trans(h23);
+      asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(pfrag + (part * NT + nt) * 256 + lane * 8), "r"(b0), "r"(b1)
+                   : "memory");
+    }
+    team_sync(team);
+    // ---- O^T += V^T P^T: 64 keys x this warp's quarter of the dims ----
+    if (!dead && !mbar_wait(bar_v + 8 * (i % DV), (i / DV) & 1, p.status, 4)) s_abort = 1;
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      uint2 pb[NT];
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) pb[nt] = lds64(pfrag + (ks * NT + nt) * 256 + lane * 8);
+      const uint32_t r0 = ring_v + (i % DV) * SV + (16 * ks + 2 * tq) * PV;
+      const uint32_t rows[4] = {r0, r0 + PV, r0 + 8 * PV, r0 + 9 * PV};
+      VL::run_part(rows, g, part, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) mma16816(O[m][nt], a0, a1, a2, a3, pb[nt].x, pb[nt].y);
+      });
+    }
+  }
+  team_sync(team);   // the ring is free
+  if (*(volatile int *)&s_abort && part == 0 && lane == 0) {
+    // a bounded wait ran out: copies still in flight get one more bounded chance to land (later fills
+    // were not issued, so a barrier may stay open: the first that does ends the loop)
+    bool ok = true;
+    for (int i = 0; ok && i < DK; ++i) ok = i >= n_mine || mbar_wait(bar_k + 8 * i, 0, nullptr, 0);
+    for (int i = 0; ok && i < DV; ++i) ok = i >= n_mine || mbar_wait(bar_v + 8 * i, 0, nullptr, 0);
+  }
+
+  // ---- the teams meet ----
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float m = run[nt][e], ll = l[nt][e];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
+        ll += __shfl_xor_sync(FULL, ll, o);
+      }
+      if (g == 0) {
+        const int c = 8 * nt + 2 * tq + e;
+        s_max[team][part][c] = m;
+        s_sum[team][part][c] = ll;
+        if (part == 0) s_ref[team][c] = ref[nt][e];
+      }
+    }
+  // accumulators into the team's plane [column][dim] over its ring: dim d at 33 * (d >> 5) + (d & 31)
+  {
+    float *plane = reinterpret_cast<float *>(smem + Geo::kHead + team * Geo::kTeamBytes);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int d0 = VL::dim(g, 4 * part + m, 0), d1 = VL::dim(g, 4 * part + m, 1);
+      const int a0 = 33 * (d0 >> 5) + (d0 & 31), a1 = 33 * (d1 >> 5) + (d1 & 31);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        float *pc = plane + (8 * nt + 2 * tq) * kBlkPlane;
+        pc[a0] = O[m][nt][0];
+        pc[a0 + kBlkPlane] = O[m][nt][1];
+        pc[a1] = O[m][nt][2];
+        pc[a1 + kBlkPlane] = O[m][nt][3];
+      }
+    }
+  }
+  __syncthreads();
+  const bool aborted = s_abort != 0;
+  for (int c = threadIdx.x; c < n_tok * kGroup; c += Geo::kThreads) {
+    float mm = kBlkNone, ll = 0.f;
+#pragma unroll
+    for (int i = 0; i < TEAMS * 4; ++i) mm = fmaxf(mm, s_max[i >> 2][i & 3][c]);
+    const bool empty = aborted || mm <= 0.5f * kBlkNone;
+#pragma unroll
+    for (int i = 0; i < TEAMS; ++i) {
+      const float w = ex2(s_ref[i][c] - mm);   // a reference is at most 1 above the true maximum
+      s_wt[i][c] = empty ? 0.f : w * VL::kUnscale;
+      ll = fmaf((s_sum[i][0][c] + s_sum[i][1][c]) + (s_sum[i][2][c] + s_sum[i][3][c]), w, ll);
+    }
+    s_ml[c][0] = empty ? -INFINITY : mm * 0.6931471805599453f;   // natural log
+    s_ml[c][1] = empty ? 0.f : ll;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_tok * kGroup * (kHeadDim / 2); i += Geo::kThreads) {
+    const int c = i >> 7, dd = 2 * (i & 127);
+    const int off = c * kBlkPlane + 33 * (dd >> 5) + (dd & 31);
+    float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+    for (int w = 0; w < TEAMS; ++w) {
+      if (aborted) break;
+      const float *pl = reinterpret_cast<const float *>(smem + Geo::kHead + w * Geo::kTeamBytes) + off;
+      a0 = fmaf(pl[0], s_wt[w][c], a0);
+      a1 = fmaf(pl[1], s_wt[w][c], a1);
+    }
+    float *rec = rec0 + (((size_t)(tok0 + c / kGroup) * p.n_head + kvh * kGroup + c % kGroup) * S + s) * kRec;
+    if (dd == 0) {
+      rec[0] = s_ml[c][0];
+      rec[1] = s_ml[c][1];
+    }
+    if ((reinterpret_cast<uintptr_t>(rec) & 7) == 0) {   // always, for the library's workspace
+      *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a0, a1);
+    } else {
+      rec[2 + dd] = a0;
+      rec[3 + dd] = a1;
+    }
+  }
+}
+
+template <int KT, int VT, int NT>
+int launch_block_tiles(const BlockArgs &k, dim3 grid, cudaStream_t st) {
+  using Geo = BlockGeo<KT, VT, NT>;
+  static bool attr_set[32] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return RD_ERR_CUDA;
+  if (dev < 0 || dev >= 32 || !attr_set[dev]) {
+    if (cudaFuncSetAttribute(block_kernel<KT, VT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::kSmem) !=
+        cudaSuccess)
+      return RD_ERR_CUDA;
+    if (dev >= 0 && dev < 32) attr_set[dev] = true;
+  }
+  return launch_pdl(2, block_kernel<KT, VT, NT>, grid, dim3(Geo::kThreads), Geo::kSmem, st, k) == cudaSuccess
+             ? RD_OK
+             : RD_ERR_CUDA;
+}
+template <int KT, int VT>
+int launch_block_chunk(const BlockArgs &k, dim3 grid, cudaStream_t st) {
+  switch (block_tiles(k.chunk)) {
+    case 2: return launch_block_tiles<KT, VT, 2>(k, grid, st);
+    case 3: return launch_block_tiles<KT, VT, 3>(k, grid, st);
+    case 4: return launch_block_tiles<KT, VT, 4>(k, grid, st);
+    default: return launch_block_tiles<KT, VT, 6>(k, grid, st);
+  }
+}
+
+// One sequence: grid (n_splits, n_head_kv, chunks of a.chunk tokens).
+template <int KT, int VT>
+int launch_block_typed(const DecodeArgs &a, int chunk, cudaStream_t st) {
+  BlockArgs k;
+  memset(&k, 0, sizeof(k));
+  int rc;
+  if (KT >= RD_KV_Q8_0 && (rc = kv_slot_tmap(&k.tm_k, a.k, KT, a.n_head_kv, kBlkKeys, slot_pitch(KT))) != RD_OK) return rc;
+  if (VT >= RD_KV_Q8_0 && (rc = kv_slot_tmap(&k.tm_v, a.v, VT, a.n_head_kv, kBlkKeys, slot_pitch(VT))) != RD_OK) return rc;
+  k.q = a.q;
+  k.k = (const uint8_t *)a.k;
+  k.v = (const uint8_t *)a.v;
+  k.partial = a.partial;
+  k.pos = a.pos;
+  k.n_tok = a.n_tok;
+  k.chunk = chunk;
+  k.n_head = a.n_head;
+  k.nkv = a.n_head_kv;
+  k.qscale = a.scale * 1.4426950408889634f;
+  k.status = a.status;
+  return launch_block_chunk<KT, VT>(
+      k, dim3((unsigned)a.n_splits, (unsigned)a.n_head_kv, (unsigned)((a.n_tok + chunk - 1) / chunk)), st);
+}
+
+// Many sequences: with host_seqs set, the tensor maps into their descriptors; otherwise the launch.
+template <int KT, int VT>
+int launch_block_multi_typed(const MultiDecodeArgs &a, cudaStream_t st) {
+  if (a.host_seqs != nullptr) {
+    int rc;
+    for (int i = 0; i < a.n_seq; ++i) {
+      DecodeSeq &d = a.host_seqs[i];
+      if (KT >= RD_KV_Q8_0 && (rc = kv_slot_tmap(d.tm_k, d.k, KT, a.n_head_kv, kBlkKeys, slot_pitch(KT))) != RD_OK)
+        return rc;
+      if (VT >= RD_KV_Q8_0 && (rc = kv_slot_tmap(d.tm_v, d.v, VT, a.n_head_kv, kBlkKeys, slot_pitch(VT))) != RD_OK)
+        return rc;
+    }
+    return RD_OK;
+  }
+  BlockArgs k;
+  memset(&k, 0, sizeof(k));
+  k.partial = a.records;
+  k.n_tok = a.q_len;
+  k.chunk = block_chunk(a.q_len);
+  k.n_head = a.n_head;
+  k.nkv = a.n_head_kv;
+  k.qscale = a.scale * 1.4426950408889634f;
+  k.status = a.status;
+  k.seqs = a.dev_seqs;
+  k.items = a.dev_items;
+  return launch_block_chunk<KT, VT>(k, dim3((unsigned)a.n_items, (unsigned)a.n_head_kv), st);
+}
+
+}  // namespace rd

@@ -211,6 +211,9 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
   asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
+__device__ __forceinline__ float2 unpack_h2(uint32_t h) {
+  return __half22float2(*reinterpret_cast<const __half2 *>(&h));
+}
 __device__ __forceinline__ float ex2(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

@@ -1,5 +1,5 @@
-// Type dispatch of the split-KV decode kernel (instantiations live in
-// rd_decode_k_*.cu so that they compile in parallel).
+// Type dispatch of the decode-side attention kernels (instantiations live in rd_decode_k_*.cu and
+// rd_block_k_*.cu so that they compile in parallel).
 #include "rd_common.cuh"
 #include "rd_internal.h"
 #include "rd_step.cuh"
@@ -59,6 +59,44 @@ int launch_step(int kt, int vt, const DecodeArgs &a, float *out, float *gate, cu
     case RD_KV_Q4_0: return launch_step_k_q4_0(vt, a, out, gate, st);
     case RD_KV_Q5_0: return launch_step_k_q5_0(vt, a, out, gate, st);
     case RD_KV_Q4_1: return launch_step_k_q4_1(vt, a, out, gate, st);
+    default: return RD_ERR_UNSUPPORTED;
+  }
+}
+
+int launch_block_k_f32(int vt, const DecodeArgs &a, int chunk, cudaStream_t st);
+int launch_block_k_f16(int vt, const DecodeArgs &a, int chunk, cudaStream_t st);
+int launch_block_k_q8_0(int vt, const DecodeArgs &a, int chunk, cudaStream_t st);
+int launch_block_k_q4_0(int vt, const DecodeArgs &a, int chunk, cudaStream_t st);
+int launch_block_k_q5_0(int vt, const DecodeArgs &a, int chunk, cudaStream_t st);
+int launch_block_k_q4_1(int vt, const DecodeArgs &a, int chunk, cudaStream_t st);
+
+int launch_block(int kt, int vt, const DecodeArgs &a, int chunk, cudaStream_t st) {
+  switch (kt) {
+    case RD_KV_F32: return launch_block_k_f32(vt, a, chunk, st);
+    case RD_KV_F16: return launch_block_k_f16(vt, a, chunk, st);
+    case RD_KV_Q8_0: return launch_block_k_q8_0(vt, a, chunk, st);
+    case RD_KV_Q4_0: return launch_block_k_q4_0(vt, a, chunk, st);
+    case RD_KV_Q5_0: return launch_block_k_q5_0(vt, a, chunk, st);
+    case RD_KV_Q4_1: return launch_block_k_q4_1(vt, a, chunk, st);
+    default: return RD_ERR_UNSUPPORTED;
+  }
+}
+
+int launch_block_multi_k_f32(int vt, const MultiDecodeArgs &a, cudaStream_t st);
+int launch_block_multi_k_f16(int vt, const MultiDecodeArgs &a, cudaStream_t st);
+int launch_block_multi_k_q8_0(int vt, const MultiDecodeArgs &a, cudaStream_t st);
+int launch_block_multi_k_q4_0(int vt, const MultiDecodeArgs &a, cudaStream_t st);
+int launch_block_multi_k_q5_0(int vt, const MultiDecodeArgs &a, cudaStream_t st);
+int launch_block_multi_k_q4_1(int vt, const MultiDecodeArgs &a, cudaStream_t st);
+
+int launch_block_multi(int kt, int vt, const MultiDecodeArgs &a, cudaStream_t st) {
+  switch (kt) {
+    case RD_KV_F32: return launch_block_multi_k_f32(vt, a, st);
+    case RD_KV_F16: return launch_block_multi_k_f16(vt, a, st);
+    case RD_KV_Q8_0: return launch_block_multi_k_q8_0(vt, a, st);
+    case RD_KV_Q4_0: return launch_block_multi_k_q4_0(vt, a, st);
+    case RD_KV_Q5_0: return launch_block_multi_k_q5_0(vt, a, st);
+    case RD_KV_Q4_1: return launch_block_multi_k_q4_1(vt, a, st);
     default: return RD_ERR_UNSUPPORTED;
   }
 }

@@ -89,6 +89,13 @@ __device__ __forceinline__ void dq8(uint32_t u, const Q8Scale &s, uint32_t &lo, 
   hi = hfma2(prmt(u, 0u, 0x4342u), s.m, s.c);
 }
 
+// Bytes between the rows of a slot that holds ONE head's rows in shared memory. Every loader below is
+// free of bank conflicts when the pitch is 4 words mod 8: q8_0, q4_0 and q5_0 rows are already.
+__host__ __device__ constexpr int slot_pitch(int type) {
+  return row_bytes(type) + ((row_bytes(type) / 4) % 8 == 4 ? 0 : 16);
+}
+__host__ __device__ constexpr int min_i(int a, int b) { return a < b ? a : b; }
+
 // =============================== K loaders =======================================
 // A fragment of Q*K^T for MMA n (0..15): rows = keys g / g+8 of the 16-key group,
 // k-slots (2t, 2t+1, 2t+8, 2t+9) = four dims chosen by the loader. run() calls
@@ -310,6 +317,7 @@ struct KLoad<RD_KV_Q4_1> {
 // even m; false, dim(g, m, 1) = dim(g, m, 0) + 1. Either way the first dim is even.
 // rows[j] is the shared address of the stored row of key j of those four. run()
 // calls mma(m, a0, a1, a2, a3) for m = 0..15. Values come out multiplied by 1/kUnscale.
+// run_part() does the M-tiles 4 * part .. 4 * part + 3 alone and numbers them 0..3.
 template <int T>
 struct VLoad;
 
@@ -355,6 +363,32 @@ struct VLoad<RD_KV_Q4_0> {
       mma(2 * s + 1, l1a, h1a, l1c, h1c);
     }
   }
+  template <class F>
+  __device__ static void run_part(const uint32_t (&rows)[4], int g, int part, F &&mma) {
+    const uint32_t off = (18u * g) & ~3u;
+    const bool par = g & 1;
+    uint32_t w0[4], w1[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      w0[j] = lds32(rows[j] + off);
+      w1[j] = lds32(rows[j] + off + 4 + 4 * part);
+    }
+    const uint32_t seld = par ? 0x7632u : 0x5410u;
+    const Q4Scale sab(prmt(w0[0], w0[1], seld)), scd(prmt(w0[2], w0[3], seld));
+    const bool wrap = part == 3 && !par;   // slot 7 of an even block: the upper half of its first word
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const bool first = x == 1 && wrap;
+      const uint32_t sel = x ? 0x7632u : 0x5410u;
+      const uint32_t xab = prmt(first ? w0[0] : w1[0], first ? w0[1] : w1[1], sel);
+      const uint32_t xcd = prmt(first ? w0[2] : w1[2], first ? w0[3] : w1[3], sel);
+      uint32_t l0a, h0a, l1a, h1a, l0c, h0c, l1c, h1c;
+      dq4(xab, sab, l0a, h0a, l1a, h1a);
+      dq4(xcd, scd, l0c, h0c, l1c, h1c);
+      mma(2 * x, l0a, h0a, l0c, h0c);
+      mma(2 * x + 1, l1a, h1a, l1c, h1c);
+    }
+  }
 };
 
 template <>
@@ -397,6 +431,33 @@ struct VLoad<RD_KV_Q8_0> {
       mma(s, e0a, e1a, e0c, e1c);
     }
   }
+  template <class F>
+  __device__ static void run_part(const uint32_t (&rows)[4], int g, int part, F &&mma) {
+    const uint32_t off = (34u * g) & ~3u;
+    const bool par = g & 1;
+    uint32_t w0[4], w1[4], w2[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      w0[j] = lds32(rows[j] + off);
+      w1[j] = lds32(rows[j] + off + 4 + 8 * part);
+      w2[j] = lds32(rows[j] + off + 8 + 8 * part);
+    }
+    const uint32_t seld = par ? 0x7632u : 0x5410u;
+    const Q8Scale sab(prmt(w0[0], w0[1], seld)), scd(prmt(w0[2], w0[3], seld));
+    const bool wrap = part == 3 && !par;   // slot 15 of an even block: the upper half of its first word
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const bool first = x == 3 && wrap;
+      const uint32_t sel = (x & 1) ? 0x7362u : 0x5140u;
+      const uint32_t(&w)[4] = x < 2 ? w1 : w2;
+      const uint32_t tab = prmt(first ? w0[0] : w[0], first ? w0[1] : w[1], sel) ^ 0x80808080u;
+      const uint32_t tcd = prmt(first ? w0[2] : w[2], first ? w0[3] : w[3], sel) ^ 0x80808080u;
+      uint32_t e0a, e1a, e0c, e1c;
+      dq8(tab, sab, e0a, e1a);
+      dq8(tcd, scd, e0c, e1c);
+      mma(x, e0a, e1a, e0c, e1c);
+    }
+  }
 };
 
 template <>
@@ -422,6 +483,16 @@ struct VLoad<RD_KV_F16> {
           prmt(c.w, d.w, 0x7632u));
     }
   }
+  template <class F>
+  __device__ static void run_part(const uint32_t (&rows)[4], int g, int part, F &&mma) {
+    const uint32_t o = 16 * (g + 8 * part);
+    const uint4 a = lds128(rows[0] + o), b = lds128(rows[1] + o);
+    const uint4 c = lds128(rows[2] + o), d = lds128(rows[3] + o);
+    mma(0, prmt(a.x, b.x, 0x5410u), prmt(a.x, b.x, 0x7632u), prmt(c.x, d.x, 0x5410u), prmt(c.x, d.x, 0x7632u));
+    mma(1, prmt(a.y, b.y, 0x5410u), prmt(a.y, b.y, 0x7632u), prmt(c.y, d.y, 0x5410u), prmt(c.y, d.y, 0x7632u));
+    mma(2, prmt(a.z, b.z, 0x5410u), prmt(a.z, b.z, 0x7632u), prmt(c.z, d.z, 0x5410u), prmt(c.z, d.z, 0x7632u));
+    mma(3, prmt(a.w, b.w, 0x5410u), prmt(a.w, b.w, 0x7632u), prmt(c.w, d.w, 0x5410u), prmt(c.w, d.w, 0x7632u));
+  }
 };
 
 template <>
@@ -442,6 +513,21 @@ struct VLoad<RD_KV_F32> {
           pack_h2(RD_F(c.x), RD_F(d.x)), pack_h2(RD_F(c.y), RD_F(d.y)));
       mma(2 * ci + 1, pack_h2(RD_F(a.z), RD_F(b.z)), pack_h2(RD_F(a.w), RD_F(b.w)),
           pack_h2(RD_F(c.z), RD_F(d.z)), pack_h2(RD_F(c.w), RD_F(d.w)));
+#undef RD_F
+    }
+  }
+  template <class F>
+  __device__ static void run_part(const uint32_t (&rows)[4], int g, int part, F &&mma) {
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const uint32_t o = 16 * (g + 8 * (2 * part + x));
+      const uint4 a = lds128(rows[0] + o), b = lds128(rows[1] + o);
+      const uint4 c = lds128(rows[2] + o), d = lds128(rows[3] + o);
+#define RD_F(v) __uint_as_float(v)
+      mma(2 * x, pack_h2(RD_F(a.x), RD_F(b.x)), pack_h2(RD_F(a.y), RD_F(b.y)), pack_h2(RD_F(c.x), RD_F(d.x)),
+          pack_h2(RD_F(c.y), RD_F(d.y)));
+      mma(2 * x + 1, pack_h2(RD_F(a.z), RD_F(b.z)), pack_h2(RD_F(a.w), RD_F(b.w)), pack_h2(RD_F(c.z), RD_F(d.z)),
+          pack_h2(RD_F(c.w), RD_F(d.w)));
 #undef RD_F
     }
   }
@@ -492,6 +578,38 @@ struct VLoad<RD_KV_Q5_0> {
       mma(2 * s + 1, l1a, h1a, l1c, h1c);
     }
   }
+  template <class F>
+  __device__ static void run_part(const uint32_t (&rows)[4], int g, int part, F &&mma) {
+    const uint32_t off = (22u * g) & ~3u;
+    const bool par = g & 1;
+    const uint32_t sel = par ? 0x7654u : 0x5432u;   // odd g: the next word is already aligned
+    uint32_t dd[4], qh[4], qs[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w0 = lds32(rows[j] + off), w1 = lds32(rows[j] + off + 4);
+      const uint32_t a = lds32(rows[j] + off + 4 + 4 * part), b = lds32(rows[j] + off + 8 + 4 * part);
+      dd[j] = prmt(w0, w0, par ? 0x3232u : 0x1010u);
+      qh[j] = prmt(w0, w1, sel);
+      qs[j] = prmt(a, b, sel);
+    }
+    const Q5Scale sab(prmt(dd[0], dd[1], 0x5410u)), scd(prmt(dd[2], dd[3], 0x5410u));
+    const int sh = 4 * part;
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const uint32_t psel = x ? 0x7632u : 0x5410u;
+      const uint32_t xab = prmt(qs[0], qs[1], psel), xcd = prmt(qs[2], qs[3], psel);
+      // fifth bits of two elements, two keys side by side (see run)
+      const uint32_t bab = x ? ((qh[0] >> 2) & 0x33333333u) | (qh[1] & 0xCCCCCCCCu)
+                             : (qh[0] & 0x33333333u) | ((qh[1] & 0x33333333u) << 2);
+      const uint32_t bcd = x ? ((qh[2] >> 2) & 0x33333333u) | (qh[3] & 0xCCCCCCCCu)
+                             : (qh[2] & 0x33333333u) | ((qh[3] & 0x33333333u) << 2);
+      uint32_t l0a, h0a, l1a, h1a, l0c, h0c, l1c, h1c;
+      dq5(xab, (bab >> sh) & 0xFu, (bab >> (16 + sh)) & 0xFu, sab, l0a, h0a, l1a, h1a);
+      dq5(xcd, (bcd >> sh) & 0xFu, (bcd >> (16 + sh)) & 0xFu, scd, l0c, h0c, l1c, h1c);
+      mma(2 * x, l0a, h0a, l0c, h0c);
+      mma(2 * x + 1, l1a, h1a, l1c, h1c);
+    }
+  }
 };
 template <>
 struct VLoad<RD_KV_Q4_1> {
@@ -520,6 +638,26 @@ struct VLoad<RD_KV_Q4_1> {
       dq4(xcd, scd, l0c, h0c, l1c, h1c);
       mma(2 * s, l0a, h0a, l0c, h0c);
       mma(2 * s + 1, l1a, h1a, l1c, h1c);
+    }
+  }
+  template <class F>
+  __device__ static void run_part(const uint32_t (&rows)[4], int g, int part, F &&mma) {
+    uint32_t w0[4], w1[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      w0[j] = lds32(rows[j] + 20u * g);
+      w1[j] = lds32(rows[j] + 20u * g + 4 + 4 * part);
+    }
+    const Q41Scale sab(prmt(w0[0], w0[1], 0x5410u), prmt(w0[0], w0[1], 0x7632u));
+    const Q41Scale scd(prmt(w0[2], w0[3], 0x5410u), prmt(w0[2], w0[3], 0x7632u));
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const uint32_t sel = x ? 0x7632u : 0x5410u;
+      uint32_t l0a, h0a, l1a, h1a, l0c, h0c, l1c, h1c;
+      dq4(prmt(w1[0], w1[1], sel), sab, l0a, h0a, l1a, h1a);
+      dq4(prmt(w1[2], w1[3], sel), scd, l0c, h0c, l1c, h1c);
+      mma(2 * x, l0a, h0a, l0c, h0c);
+      mma(2 * x + 1, l1a, h1a, l1c, h1c);
     }
   }
 };

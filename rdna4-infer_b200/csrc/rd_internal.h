@@ -90,6 +90,15 @@ int launch_step(int kt, int vt, const DecodeArgs &a, float *out, float *gate, cu
 // n_keys < 0: not known on the host).
 int step_splits(int kt, int vt, int n_head_kv, int64_t n_keys);
 
+// Blocks of tokens (rd_block.cuh): token i attends keys 0..pos[i] (on the device); a CTA serves `chunk`
+// <= 8 tokens. Writes n_splits records per (token, head) like launch_decode.
+int launch_block(int kt, int vt, const DecodeArgs &a, int chunk, cudaStream_t st);
+// Tokens per CTA for a block of n_tok: as few chunks as possible, evenly filled.
+inline int block_chunk(int n_tok) {
+  const int chunks = (n_tok + 7) / 8;
+  return (n_tok + chunks - 1) / chunks;
+}
+
 // One sequence of a multi-sequence launch, as the kernels read it from device memory.
 // The last of the q_len new tokens attends keys 0..t, token i keys 0..t-(q_len-1-i).
 // Its records live at records[rec_base ...] as [q_len][n_head][n_splits][258].
@@ -117,7 +126,7 @@ struct MultiDecodeArgs {
   DecodeSeq *host_seqs;
   int n_seq;
   const DecodeSeq *dev_seqs;
-  const int4 *dev_items;  // (sequence, token, split, 0)
+  const int4 *dev_items;  // (sequence, first token, split, 0)
   int n_items;
   int q_len;
   int n_head;
@@ -126,7 +135,8 @@ struct MultiDecodeArgs {
   float *records;
   DeviceStatus *status;
 };
-int launch_decode_multi(int kt, int vt, const MultiDecodeArgs &a, cudaStream_t st);
+int launch_decode_multi(int kt, int vt, const MultiDecodeArgs &a, cudaStream_t st);   // q_len 1
+int launch_block_multi(int kt, int vt, const MultiDecodeArgs &a, cudaStream_t st);    // q_len > 1
 // Keys per tile of the (kt, vt) kernel: the granularity of the key split.
 int decode_tile_keys(int kt, int vt);
 
@@ -138,6 +148,10 @@ int decode_tile_keys(int kt, int vt);
 // driver entry point is unavailable, or the encoder refuses.
 int encode_kv_tmap(void *tmap_out, const void *base, int type, int n_head_kv, int64_t n_rows,
                    int tile_rows);
+
+// Tensor map over ONE head's rows of a KV cache (the head is chosen by the box's x): box of
+// [box_rows][pitch bytes]. The row count of the map is only a bound: callers load boxes whose rows exist.
+int kv_slot_tmap(void *tmap_out, const void *base, int type, int n_head_kv, int box_rows, int pitch);
 
 // Tensor map over an f16 KV cache [n_rows][n_head_kv * 256] with a box of
 // [tile_rows][64 dims] and the hardware 128-byte swizzle (what tcgen05.mma descriptors

@@ -28,11 +28,6 @@
 
 namespace rd {
 
-// Bytes between the rows of a slot in shared memory. Every fragment loader is free of bank
-// conflicts when the pitch is 4 words mod 8: q8_0, q4_0 and q5_0 rows are already.
-__host__ __device__ constexpr int slot_pitch(int type) {
-  return row_bytes(type) + ((row_bytes(type) / 4) % 8 == 4 ? 0 : 16);
-}
 // dim table (512), query fragments (3456), new row (2048), received sums (6144) and their (m, l) (768)
 constexpr int kStepRecv = 512 + 3456 + 2048;
 constexpr int kStepHeader = kStepRecv + 6144 + 768;
@@ -42,7 +37,6 @@ static_assert(kStepHeader % 16 == 0, "rings are 16-byte aligned");
 __host__ __device__ constexpr int step_pair_bytes(int kt, int vt) {
   return kSlotKeys * (slot_pitch(kt) + slot_pitch(vt));
 }
-__host__ __device__ constexpr int min_i(int a, int b) { return a < b ? a : b; }
 // Warps per CTA: as many as have two slots each in the ring budget, up to three per scheduler
 // (12 warps leave 168 registers each; the accumulators and query fragments alone are 96).
 __host__ __device__ constexpr int step_warps(int kt, int vt) {
