@@ -666,7 +666,7 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
   a.host_seqs = hs;
   a.n_seq = n_seq;
   a.n_head_kv = n_head_kv;
-  if ((rc = (q_len > 1 ? launch_block_multi : launch_decode_multi)(k_type, v_type, a, nullptr)) != RD_OK) return rc;
+  if (q_len == 1 && (rc = launch_decode_multi(k_type, v_type, a, nullptr)) != RD_OK) return rc;
   MultiPlanHeader h;
   memset(&h, 0, sizeof(h));
   h.magic = kMultiPlanMagic;

@@ -6,20 +6,24 @@
 // (work items, n_head_kv): a CTA owns a run of 64-key slots of one KV head and the 6 T <= 48 score
 // columns (token, query head) of its chunk, NT = 2, 3, 4 or 6 MMA tiles of 8 columns.
 //
-// The CTA's warps form teams of four; a team streams slots through its own ring (a tensor-map box of
-// [64 keys][one head's row] for quantized caches, a bulk copy per row for f16 / f32 rows, whose padded
-// boxes would fetch a cache line more than the row has). Per slot
-//   * warp w multiplies keys 16 w .. 16 w + 15 with all columns (K fragments dequantized in
-//     registers once, query fragments from shared memory);
-//   * one barrier (with the vote "does any score exceed the team's reference?") frees the K slot and
-//     the previous V slot, which the team's first warp refills;
-//   * the weights go to shared memory as MMA fragments, a second barrier, and warp w multiplies all 64
-//     keys with its quarter of the output dims: every V value is dequantized once, by one warp, and a
-//     warp holds 16 NT accumulators where a warp with all dims would hold 64 NT.
+// The CTA's warps form teams of four; a team streams slots through its own ring with 16-byte
+// asynchronous copies, every warp 16 of the 64 rows. Per slot
+//   * warp w multiplies keys 16 w .. 16 w + 15, the K rows it has copied itself, with all columns (K
+//     fragments dequantized in registers once, query fragments from shared memory), and requests
+//     its K rows of a later slot;
+//   * one barrier (with the vote "does any score exceed the team's reference?") frees the previous
+//     V slot, into which the warps request their V rows of a later one;
+//   * the weights go to shared memory as MMA fragments, a second barrier publishes them and the V
+//     rows, and warp w multiplies all 64 keys with its quarter of the output dims: every V value is
+//     dequantized once, by one warp, and a warp holds 16 NT accumulators where a warp with all dims
+//     would hold 64 NT.
+// (Tensor-map boxes of one head's rows were the slower copy: the TMA unit fetches whole cache lines,
+// and a 272-byte row of q8_0 lies in three of them. 64 sequences of config 5 verifying four tokens:
+// copies alone 817 us.)
 // One record (m, l, acc[256]) per (token, head) and split, merged by merge_kernel.
 //
 // What bounds it: the 32 NT mma.sync of 16 keys (about 13 cycles each per scheduler) for 4-bit caches
-// from four tokens, the fetch of the narrow rows for 8-bit and f16 caches.
+// from four tokens, HBM and the barriers for 8-bit and f16 caches.
 #pragma once
 #include <string.h>
 
@@ -45,7 +49,7 @@ struct BlockGeo {
   static constexpr int kSK = kBlkKeys * kPK, kSV = kBlkKeys * kPV;   // multiples of 128
   static constexpr int kQBytes = NT * 4096;                          // query fragments
   static constexpr int kPBytes = NT * 1024;                          // weight fragments of a slot, per team
-  static constexpr int kHead = 512 + 512 + kQBytes;                  // barriers, dim table, query fragments
+  static constexpr int kHead = 512 + kQBytes;                        // dim table, query fragments
   static constexpr int budget(int teams) { return (kBlkSmem - kHead) / teams - kPBytes; }
   // two teams where each gets at least one slot, and another K or V of the next
   static constexpr int kTeams = budget(2) >= kSK + kSV + (kSK < kSV ? kSK : kSV) ? 2 : 1;
@@ -59,12 +63,9 @@ struct BlockGeo {
   static constexpr int kSmem = kHead + kTeams * kTeamBytes;
   static constexpr int kThreads = kTeams * 128;
   static_assert(kBoth >= 1 && kSK % 128 == 0 && kSV % 128 == 0 && kSmem <= kBlkSmem, "ring geometry");
-  static_assert(kTeams * (DK + DV) * 8 <= 512, "barriers");
 };
 
 struct BlockArgs {
-  alignas(64) CUtensorMap tm_k;   // single sequence: boxes of [64 keys][slot_pitch], quantized types only
-  alignas(64) CUtensorMap tm_v;
   const float *q;                 // [n_tok][n_head][256]
   const uint8_t *k;
   const uint8_t *v;
@@ -75,7 +76,6 @@ struct BlockArgs {
   int n_head;
   int nkv;
   float qscale;                   // scale * log2(e)
-  DeviceStatus *status;
   const DecodeSeq *seqs;          // many sequences: CTA x works on items[x] = (sequence, first token, split)
   const int4 *items;
 };
@@ -107,11 +107,11 @@ block_kernel(const __grid_constant__ BlockArgs p) {
   using VL = VLoad<VT>;
   constexpr int RK = row_bytes(KT), RV = row_bytes(VT), PK = Geo::kPK, PV = Geo::kPV, SK = Geo::kSK, SV = Geo::kSV;
   constexpr int DK = Geo::DK, DV = Geo::DV, TEAMS = Geo::kTeams, COLS = NT * 8;
-  constexpr bool BOX_K = KT >= RD_KV_Q8_0, BOX_V = VT >= RD_KV_Q8_0;
+  // copies go out in the order K0 V0 K1 V1 ...; with a V slot more than K slots, V runs level with K
+  constexpr int WAIT_K = DV > DK ? 2 * DK - 1 : 2 * DK - 2, WAIT_V = DV > DK ? 2 * DK : 2 * DK - 2;
   constexpr unsigned FULL = 0xffffffffu;
 
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ int s_abort;
   __shared__ int s_t[COLS];                                  // last key of the column's token (-1: padding)
   __shared__ float s_max[TEAMS][4][COLS], s_sum[TEAMS][4][COLS], s_ref[TEAMS][COLS];
   __shared__ float s_wt[TEAMS][COLS], s_ml[COLS][2];
@@ -121,18 +121,12 @@ block_kernel(const __grid_constant__ BlockArgs p) {
   const int team = warp >> 2, part = warp & 3;
   const int kvh = blockIdx.y, nkv = p.nkv;
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t bar_k = sbase + team * (DK + DV) * 8, bar_v = bar_k + DK * 8;
-  unsigned short *inv = reinterpret_cast<unsigned short *>(smem + 512);
-  const uint32_t qfrag = sbase + 1024;
+  unsigned short *inv = reinterpret_cast<unsigned short *>(smem);
+  const uint32_t qfrag = sbase + 512;
   const uint32_t team0 = sbase + Geo::kHead + team * Geo::kTeamBytes;
   const uint32_t ring_k = team0, ring_v = ring_k + DK * SK;
   const uint32_t pfrag = team0 + (Geo::kTeamBytes - Geo::kPBytes);
 
-  if (threadIdx.x == 0) {
-    s_abort = 0;
-    for (int i = 0; i < TEAMS * (DK + DV); ++i) mbar_init(sbase + 8 * i, 1);
-    fence_barrier_init();
-  }
   // dim -> byte offset of the half in a column's query fragments (inverts KL::dim): 16 bytes per
   // (pair of MMAs, quad lane)
   for (int i = threadIdx.x; i < 256; i += Geo::kThreads) {
@@ -146,7 +140,6 @@ block_kernel(const __grid_constant__ BlockArgs p) {
   int s, S, tok0, n_tok;
   const float *qsrc;
   const uint8_t *khead, *vhead;
-  const CUtensorMap *tmk = &p.tm_k, *tmv = &p.tm_v;
   float *rec0;
   int t_seq = 0;
   if (p.items != nullptr) {
@@ -160,15 +153,7 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     qsrc = d.q;
     khead = d.k;
     vhead = d.v;
-    tmk = reinterpret_cast<const CUtensorMap *>(d.tm_k);
-    tmv = reinterpret_cast<const CUtensorMap *>(d.tm_v);
     rec0 = p.partial + (size_t)d.rec_base * kRec;
-    // these descriptors were written by an ordinary copy and may have been rewritten since an earlier
-    // launch read them: make the copy visible to the tensor-map proxy of the issuing threads
-    if (part == 0 && lane == 0) {
-      if (BOX_K) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmk) : "memory");
-      if (BOX_V) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmv) : "memory");
-    }
   } else {
     tok0 = blockIdx.z * p.chunk;
     s = blockIdx.x;
@@ -220,40 +205,23 @@ block_kernel(const __grid_constant__ BlockArgs p) {
   // the team's slots: c_b + team + i * TEAMS
   const int n_mine = c_e - c_b > team ? (c_e - c_b - team + TEAMS - 1) / TEAMS : 0;
 
-  // Loads the team's i-th slot (one tensor) into its ring; warp-collective, by the team's first warp.
-  // Whole slots are one box; f16 / f32 rows and the last, partial slot go row by row, rows
-  // behind the last key repeating it.
-  auto fill = [&](auto is_v_c, int i) {
-    constexpr bool is_v = decltype(is_v_c)::value;
-    constexpr int R = is_v ? RV : RK, P = is_v ? PV : PK, DD = is_v ? DV : DK;
-    if (i >= n_mine) return;
-    const int row0 = (c_b + team + i * TEAMS) * kBlkKeys;
-    const uint32_t bar = (is_v ? bar_v : bar_k) + 8 * (i % DD);
-    const uint32_t dst = (is_v ? ring_v : ring_k) + (i % DD) * (is_v ? SV : SK);
-    if ((is_v ? BOX_V : BOX_K) && row0 + kBlkKeys - 1 <= t_max) {
-      if (lane == 0) {
-        mbar_expect_tx(bar, kBlkKeys * P);
-        tma_load_2d(dst, is_v ? tmv : tmk, kvh * (R / 8), row0, bar);
-      }
-      return;
-    }
-    if (lane == 0) mbar_expect_tx(bar, kBlkKeys * R);
-    __syncwarp();
-    const uint8_t *head = is_v ? vhead : khead;
-    const size_t stride = is_v ? vb : kb;
-#pragma unroll
-    for (int r = lane; r < kBlkKeys; r += 32) {
-      const int key = row0 + r > t_max ? t_max : row0 + r;
-      bulk_g2s(dst + r * P, head + (size_t)key * stride, R, bar);
-    }
+  // This warp's 16 rows of the team's i-th slot; always one commit group, empty behind the end.
+  auto fill_k = [&](int i) {
+    if (i < n_mine)
+      copy_slot<KT>(ring_k + (i % DK) * SK + 16 * part * PK, khead, kb, (c_b + team + i * TEAMS) * kBlkKeys + 16 * part,
+                    t_max, lane);
+    cp_async_commit();
   };
-  const std::integral_constant<bool, false> is_k;
-  const std::integral_constant<bool, true> is_v;
-  if (part == 0) {
-    for (int i = 0; i < DV; ++i) {
-      if (i < DK) fill(is_k, i);
-      fill(is_v, i);
-    }
+  auto fill_v = [&](int i) {
+    if (i < n_mine)
+      copy_slot<VT>(ring_v + (i % DV) * SV + 16 * part * PV, vhead, vb, (c_b + team + i * TEAMS) * kBlkKeys + 16 * part,
+                    t_max, lane);
+    cp_async_commit();
+  };
+#pragma unroll 1
+  for (int i = 0; i < DK; ++i) {
+    fill_k(i);
+    if (i + 1 < DV) fill_v(i);
   }
 
   float O[4][NT][4];                     // [M-tile of this warp's quarter of the dims][column tile]
@@ -266,11 +234,11 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     for (int m = 0; m < 4; ++m) O[m][nt][0] = O[m][nt][1] = O[m][nt][2] = O[m][nt][3] = 0.f;
   }
   const uint32_t qlane = qfrag + lane * 16;
-  bool dead = false;   // a bounded wait ran out: go through the motions (barriers) without waiting
 #pragma unroll 1
   for (int i = 0; i < n_mine; ++i) {
     const int row0 = (c_b + team + i * TEAMS) * kBlkKeys;
-    if (!dead && !mbar_wait(bar_k + 8 * (i % DK), (i / DK) & 1, p.status, 3)) s_abort = 1;
+    cp_async_wait<WAIT_K>();
+    __syncwarp();
     // ---- S = K Q^T: this warp's 16 keys x all columns ----
     float Sv[NT][4];
 #pragma unroll
@@ -286,6 +254,8 @@ block_kernel(const __grid_constant__ BlockArgs p) {
         }
       });
     }
+    __syncwarp();
+    fill_k(i + DK);
     if (row0 + kBlkKeys - 1 > t_min) {   // some column ends inside or before this slot
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
@@ -301,13 +271,9 @@ block_kernel(const __grid_constant__ BlockArgs p) {
         run[nt][e] = fmaxf(run[nt][e], fmaxf(Sv[nt][e], Sv[nt][e + 2]));
         grow |= run[nt][e] > ref[nt][e] + kBlkSlack;
       }
-    // every warp of the team is done with this K slot and with the V slot before it
+    // every warp of the team is done with the V slot before this one
     const bool any = team_any(team, grow);
-    dead = *(volatile int *)&s_abort != 0;
-    if (part == 0 && !dead) {
-      fill(is_k, i + DK);
-      if (i > 0) fill(is_v, i - 1 + DV);
-    }
+    fill_v(i - 1 + DV);
     if (any) {
       // the team's references move to the current maxima of the columns (over its 64 key rows)
 #pragma unroll
@@ -354,9 +320,9 @@ block_kernel(const __grid_constant__ BlockArgs p) {
       asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(pfrag + (part * NT + nt) * 256 + lane * 8), "r"(b0), "r"(b1)
                    : "memory");
     }
+    cp_async_wait<WAIT_V>();
     team_sync(team);
     // ---- O^T += V^T P^T: 64 keys x this warp's quarter of the dims ----
-    if (!dead && !mbar_wait(bar_v + 8 * (i % DV), (i / DV) & 1, p.status, 4)) s_abort = 1;
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       uint2 pb[NT];
@@ -370,14 +336,8 @@ block_kernel(const __grid_constant__ BlockArgs p) {
       });
     }
   }
-  team_sync(team);   // the ring is free
-  if (*(volatile int *)&s_abort && part == 0 && lane == 0) {
-    // a bounded wait ran out: copies still in flight get one more bounded chance to land (later fills
-    // were not issued, so a barrier may stay open: the first that does ends the loop)
-    bool ok = true;
-    for (int i = 0; ok && i < DK; ++i) ok = i >= n_mine || mbar_wait(bar_k + 8 * i, 0, nullptr, 0);
-    for (int i = 0; ok && i < DV; ++i) ok = i >= n_mine || mbar_wait(bar_v + 8 * i, 0, nullptr, 0);
-  }
+  cp_async_wait<0>();   // (only empty groups are left)
+  team_sync(team);      // the ring is free
 
   // ---- the teams meet ----
 #pragma unroll
@@ -415,12 +375,11 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     }
   }
   __syncthreads();
-  const bool aborted = s_abort != 0;
   for (int c = threadIdx.x; c < n_tok * kGroup; c += Geo::kThreads) {
     float mm = kBlkNone, ll = 0.f;
 #pragma unroll
     for (int i = 0; i < TEAMS * 4; ++i) mm = fmaxf(mm, s_max[i >> 2][i & 3][c]);
-    const bool empty = aborted || mm <= 0.5f * kBlkNone;
+    const bool empty = mm <= 0.5f * kBlkNone;
 #pragma unroll
     for (int i = 0; i < TEAMS; ++i) {
       const float w = ex2(s_ref[i][c] - mm);   // a reference is at most 1 above the true maximum
@@ -437,7 +396,6 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     float a0 = 0.f, a1 = 0.f;
 #pragma unroll
     for (int w = 0; w < TEAMS; ++w) {
-      if (aborted) break;
       const float *pl = reinterpret_cast<const float *>(smem + Geo::kHead + w * Geo::kTeamBytes) + off;
       a0 = fmaf(pl[0], s_wt[w][c], a0);
       a1 = fmaf(pl[1], s_wt[w][c], a1);
@@ -487,9 +445,6 @@ template <int KT, int VT>
 int launch_block_typed(const DecodeArgs &a, int chunk, cudaStream_t st) {
   BlockArgs k;
   memset(&k, 0, sizeof(k));
-  int rc;
-  if (KT >= RD_KV_Q8_0 && (rc = kv_slot_tmap(&k.tm_k, a.k, KT, a.n_head_kv, kBlkKeys, slot_pitch(KT))) != RD_OK) return rc;
-  if (VT >= RD_KV_Q8_0 && (rc = kv_slot_tmap(&k.tm_v, a.v, VT, a.n_head_kv, kBlkKeys, slot_pitch(VT))) != RD_OK) return rc;
   k.q = a.q;
   k.k = (const uint8_t *)a.k;
   k.v = (const uint8_t *)a.v;
@@ -500,25 +455,13 @@ int launch_block_typed(const DecodeArgs &a, int chunk, cudaStream_t st) {
   k.n_head = a.n_head;
   k.nkv = a.n_head_kv;
   k.qscale = a.scale * 1.4426950408889634f;
-  k.status = a.status;
   return launch_block_chunk<KT, VT>(
       k, dim3((unsigned)a.n_splits, (unsigned)a.n_head_kv, (unsigned)((a.n_tok + chunk - 1) / chunk)), st);
 }
 
-// Many sequences: with host_seqs set, the tensor maps into their descriptors; otherwise the launch.
+// Many sequences: grid (work items, n_head_kv).
 template <int KT, int VT>
 int launch_block_multi_typed(const MultiDecodeArgs &a, cudaStream_t st) {
-  if (a.host_seqs != nullptr) {
-    int rc;
-    for (int i = 0; i < a.n_seq; ++i) {
-      DecodeSeq &d = a.host_seqs[i];
-      if (KT >= RD_KV_Q8_0 && (rc = kv_slot_tmap(d.tm_k, d.k, KT, a.n_head_kv, kBlkKeys, slot_pitch(KT))) != RD_OK)
-        return rc;
-      if (VT >= RD_KV_Q8_0 && (rc = kv_slot_tmap(d.tm_v, d.v, VT, a.n_head_kv, kBlkKeys, slot_pitch(VT))) != RD_OK)
-        return rc;
-    }
-    return RD_OK;
-  }
   BlockArgs k;
   memset(&k, 0, sizeof(k));
   k.partial = a.records;
@@ -527,7 +470,6 @@ int launch_block_multi_typed(const MultiDecodeArgs &a, cudaStream_t st) {
   k.n_head = a.n_head;
   k.nkv = a.n_head_kv;
   k.qscale = a.scale * 1.4426950408889634f;
-  k.status = a.status;
   k.seqs = a.dev_seqs;
   k.items = a.dev_items;
   return launch_block_chunk<KT, VT>(k, dim3((unsigned)a.n_items, (unsigned)a.n_head_kv), st);

@@ -149,10 +149,6 @@ int decode_tile_keys(int kt, int vt);
 int encode_kv_tmap(void *tmap_out, const void *base, int type, int n_head_kv, int64_t n_rows,
                    int tile_rows);
 
-// Tensor map over ONE head's rows of a KV cache (the head is chosen by the box's x): box of
-// [box_rows][pitch bytes]. The row count of the map is only a bound: callers load boxes whose rows exist.
-int kv_slot_tmap(void *tmap_out, const void *base, int type, int n_head_kv, int box_rows, int pitch);
-
 // Tensor map over an f16 KV cache [n_rows][n_head_kv * 256] with a box of
 // [tile_rows][64 dims] and the hardware 128-byte swizzle (what tcgen05.mma descriptors
 // with SWIZZLE_128B read).

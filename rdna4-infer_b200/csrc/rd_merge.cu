@@ -21,8 +21,9 @@ constexpr int kMergeGroups = 16;  // record groups per CTA
 // -- attended here as one more record (m = scale * q.k, l = 1, acc = v).
 // MODE 2: like 0, but row = (sequence, token, head) and the record block, split count,
 // output and gate come from the sequence's descriptor (rows_per_seq = q_len * n_head).
-template <int MODE>
-__global__ void __launch_bounds__(kMergeDims *kMergeGroups, MODE == 2 ? 2 : 1)
+// kBatch: records that a group requests at once (see below); up to four leave registers for two CTAs per SM.
+template <int MODE, int kBatch>
+__global__ void __launch_bounds__(kMergeDims *kMergeGroups, kBatch <= 4 ? 2 : 1)
 merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_in, int n_out,
              float *__restrict__ gate, const DecodeSeq *__restrict__ seqs, int rows_per_seq,
              const ExtraKey xk) {
@@ -52,13 +53,10 @@ merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_i
 
   // One pass: group ty walks records lo+ty, lo+ty+16, ... and keeps a local log-sum-exp
   // (m, l, acc); the 16 groups are then combined through shared memory. An empty record
-  // (m = -inf) weighs nothing and whatever its body holds is never used. A batch is ten
-  // records per group -- the 148 records of a full-GPU decode in ONE round trip to L2 (four
-  // per batch took three) -- and the first batch is requested before anything else, the
-  // gate value with it.
-  // (the many-sequence launch has thousands of CTAs with a handful of records each: there
-  // a small batch keeps the registers low enough for two CTAs per SM)
-  constexpr int kBatch = MODE == 2 ? 4 : 10;
+  // (m = -inf) weighs nothing and whatever its body holds is never used. The first batch is
+  // requested before anything else, the gate value with it. A batch of ten holds the 148 records
+  // of a full-GPU decode in ONE round trip to L2 (four per batch took three); rows with up to 64
+  // records (blocks of tokens, many sequences) have many CTAs and want two per SM.
   float mB[kBatch], aB[kBatch], lB[kBatch];
   auto request = [&](int s0) {
 #pragma unroll
@@ -174,8 +172,9 @@ int launch_merge(const float *partial, float *out, int n_rows, int n_splits, flo
                  cudaStream_t st) {
   if (n_rows == 0) return RD_OK;
   const dim3 grid((unsigned)n_rows, kHeadDim / kMergeDims, 1);
-  return launch_pdl(4, merge_kernel<0>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, out, n_splits,
-                    1, gate, nullptr, 1, ExtraKey{}) == cudaSuccess
+  const auto kernel = n_splits <= 4 * kMergeGroups ? merge_kernel<0, 4> : merge_kernel<0, 10>;
+  return launch_pdl(4, kernel, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, out, n_splits, 1, gate,
+                    nullptr, 1, ExtraKey{}) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
 }
@@ -184,7 +183,7 @@ int launch_merge_extra(const float *partial, float *out, int n_rows, int n_split
                        const ExtraKey &x, cudaStream_t st) {
   if (n_rows == 0) return RD_OK;
   const dim3 grid((unsigned)n_rows, kHeadDim / kMergeDims, 1);
-  return launch_pdl(4, merge_kernel<3>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, out, n_splits,
+  return launch_pdl(4, merge_kernel<3, 10>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, out, n_splits,
                     1, gate, nullptr, 1, x) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
@@ -194,7 +193,7 @@ int launch_merge_records(const float *partial, float *records, int n_rows, int n
                          cudaStream_t st) {
   if (n_rows == 0) return RD_OK;
   const dim3 grid((unsigned)n_rows, kHeadDim / kMergeDims, (unsigned)n_out);
-  return launch_pdl(4, merge_kernel<1>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, records, n_in,
+  return launch_pdl(4, merge_kernel<1, 10>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, records, n_in,
                     n_out, nullptr, nullptr, 1, ExtraKey{}) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
@@ -207,7 +206,7 @@ int launch_merge_multi(const DecodeSeq *dev_seqs, const float *records, int n_se
   const dim3 grid((unsigned)rows, kHeadDim / kMergeDims, 1);
   // not a dependent launch: thousands of CTAs that would take SM slots from the decode launch's
   // last ones
-  return launch_pdl(0, merge_kernel<2>, grid, dim3(kMergeDims * kMergeGroups), 0, st, records, nullptr, 0, 1,
+  return launch_pdl(0, merge_kernel<2, 4>, grid, dim3(kMergeDims * kMergeGroups), 0, st, records, nullptr, 0, 1,
                     nullptr, dev_seqs, q_len * n_head, ExtraKey{}) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;

@@ -76,56 +76,6 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void st_cluster_f32x2(uint32_t a, float x, float y) {
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(x), "f"(y) : "memory");
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const uint8_t *src) {
-  asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// One slot: rows row0 .. row0 + 15 of a head (`row_stride` bytes apart in the cache) to shared
-// memory, kSlotKeys rows slot_pitch apart. Warp-collective; rows behind t_load repeat it. Lanes
-// are dealt so that a copy instruction takes whole rows: the lane's part of the address is a constant.
-template <int T>
-__device__ __forceinline__ void copy_slot(uint32_t dst, const uint8_t *head_base, size_t row_stride, int row0,
-                                          int t_load, int lane) {
-  constexpr int R = row_bytes(T), P = slot_pitch(T), CH = R / 16;
-  if (row0 + kSlotKeys - 1 > t_load) {   // the ragged end: one slot of a launch
-#pragma unroll 1
-    for (int i = lane; i < CH * kSlotKeys; i += 32) {
-      const int r = i / CH, c = i % CH;
-      const int key = row0 + r > t_load ? t_load : row0 + r;
-      cp_async16(dst + r * P + 16 * c, head_base + (size_t)key * row_stride + 16 * c);
-    }
-    return;
-  }
-  const uint8_t *src = head_base + (size_t)row0 * row_stride;
-  if constexpr (CH == 17) {   // q8_0: two rows of 16 chunks per instruction, the 17th chunks in one
-    const uint8_t *s0 = src + (size_t)(lane >> 4) * row_stride + 16 * (lane & 15);
-    const uint32_t d0 = dst + (lane >> 4) * P + 16 * (lane & 15);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) cp_async16(d0 + 2 * j * P, s0 + (size_t)(2 * j) * row_stride);
-    if (lane < 16) cp_async16(dst + lane * P + 256, src + (size_t)lane * row_stride + 256);
-  } else if constexpr (CH >= 32) {
-#pragma unroll
-    for (int j = 0; j < kSlotKeys; ++j)
-#pragma unroll
-      for (int c = 0; c < CH / 32; ++c)
-        cp_async16(dst + j * P + 16 * (lane + 32 * c), src + (size_t)j * row_stride + 16 * (lane + 32 * c));
-  } else {
-    constexpr int RPI = 32 / CH;   // rows per instruction
-    const int r = lane / CH, c = lane % CH;
-    const uint8_t *s0 = src + (size_t)r * row_stride + 16 * c;
-    const uint32_t d0 = dst + r * P + 16 * c;
-#pragma unroll
-    for (int j = 0; j < kSlotKeys; j += RPI)
-      if (lane < RPI * CH && (j + RPI <= kSlotKeys || j + r < kSlotKeys))
-        cp_async16(d0 + j * P, s0 + (size_t)j * row_stride);
-  }
-}
-
 // Softmax reference: p = exp2(s - m) is taken against a reference m that is only moved (and the
 // accumulators rescaled) when a score exceeds it by more than kStepSlack, so p <= 2^8 -- exact
 // enough in f16 and far from overflow -- and the rescale runs once or twice per warp.

@@ -1,9 +1,6 @@
 // Host-side construction of TMA tensor maps for KV-cache tiles. The driver's encoder
 // is reached through cudaGetDriverEntryPoint, so the library links against the CUDA
 // runtime only.
-#include <string.h>
-
-#include <memory>
 #include <mutex>
 
 #include "rd_common.cuh"
@@ -52,47 +49,6 @@ int encode_kv_tmap(void *tmap_out, const void *base, int type, int n_head_kv, in
   return r == CUDA_SUCCESS ? RD_OK : RD_ERR_CUDA;
 }
 
-// Launches only read boxes whose rows all exist, so the row count need not be exact: a map is a
-// function of the cache's address and shape alone, and the last kTmapMemo maps of a host thread are
-// kept (encoding the two of a launch costs 0.7 us; a plan over 64 sequences has 128).
-namespace {
-struct TmapMemo {
-  const void *base;
-  int type, nkv, box_rows, pitch;
-  alignas(64) CUtensorMap map;
-};
-constexpr int kTmapMemo = 1024;
-constexpr cuuint64_t kAnyRows = (cuuint64_t)1 << 30;
-}  // namespace
-
-int kv_slot_tmap(void *tmap_out, const void *base, int type, int n_head_kv, int box_rows, int pitch) {
-  static thread_local std::unique_ptr<TmapMemo[]> memo;
-  if (!memo) memo.reset(new TmapMemo[kTmapMemo]());
-  const uint64_t h = ((uint64_t)(uintptr_t)base >> 4) * 0x9E3779B97F4A7C15ull;
-  TmapMemo &m = memo[(h ^ (h >> 29)) >> 54];
-  if (m.base != base || m.type != type || m.nkv != n_head_kv || m.box_rows != box_rows || m.pitch != pitch) {
-    std::call_once(g_once, resolve);
-    if (g_encode == nullptr) return RD_ERR_CUDA;
-    if (((uintptr_t)base & 15) != 0) return RD_ERR_ALIGN;
-    const int key_bytes = n_head_kv * row_bytes(type);
-    const cuuint64_t dims[2] = {(cuuint64_t)(key_bytes / 8), kAnyRows};
-    const cuuint64_t strides[1] = {(cuuint64_t)key_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)(pitch / 8), (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    m.base = nullptr;
-    if (g_encode(&m.map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void *>(base), dims, strides, box, estr,
-                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return RD_ERR_CUDA;
-    m.base = base;
-    m.type = type;
-    m.nkv = n_head_kv;
-    m.box_rows = box_rows;
-    m.pitch = pitch;
-  }
-  memcpy(tmap_out, &m.map, sizeof(CUtensorMap));
-  return RD_OK;
-}
 
 int encode_f16_tmap(void *tmap_out, const void *base, int n_head_kv, int64_t n_rows, int tile_rows) {
   std::call_once(g_once, resolve);
