@@ -4,9 +4,10 @@
 // for f16 K/V caches. One CTA owns a tile of 128 query tokens of ONE query head and walks
 // the keys in tiles of 128. Tensor memory (512 columns x 128 lanes, lane = query row):
 //   columns   0..255  O, the f32 output accumulator
-//   columns 256..511  two score buffers of 128 f32 columns; the f16 P of a tile is written
-//                     over the first 64 columns of its buffer (the A operand of O += P V,
-//                     read from TMEM)
+//   columns 256..383  the f32 scores of one tile: the next tile's can be computed as soon as
+//                     the softmax warps have these in registers
+//   columns 384..511  two buffers of 64 columns for the f16 P of a tile (the A operand of
+//                     O += P V, read from TMEM)
 // Shared memory (224 KB): Q as f16 in the K-major 128-byte-swizzled layout (64 KB), a ring
 // of three K units of [128 keys][128 dims] (96 KB) and a ring of two V units of 64 keys
 // (64 KB), all filled by TMA with the hardware 128B swizzle.
@@ -31,9 +32,9 @@
 // mbarrier.try_wait parks its whole warp). The two contractions have their own issuing
 // threads because issuing a tcgen05.mma costs the issuing thread tens of cycles.
 //
-// Scores are double-buffered: the tensor core computes S of tile j+1 while the softmax
-// warps work on tile j. S of tile j+2 waits for P V of tile j, which reads the P that
-// lives in its buffer.
+// What orders the tiles: S of tile j + 1 waits for the LOADS of tile j's scores only, P of tile j for
+// P V of tile j - 2. (With P written over its own scores, S of tile j + 2 waited for P V of tile j, a chain
+// S - softmax - P V - S of 6300 cycles per two tiles against 4096 of tensor-core work.)
 //
 // Synchronisation is mbarriers only (TMA transaction counts, tcgen05.commit); every wait
 // is bounded and a timeout unwinds the CTA (TMEM is always freed). No cluster launch, no
@@ -81,8 +82,8 @@ constexpr int kPfSmemBytes = kPfQBytes + kPfKSlots * kPfKUnitBytes + kPfVSlots *
 constexpr int kPfThreads = 384;           // 8 softmax warps, K TMA, S MMA, V TMA, PV MMA warps
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemO = 0;            // columns [0, 256): output accumulator
-constexpr uint32_t kTmemS = 256;          // columns [256, 512): two score buffers of 128; the
-                                          // f16 P of a tile overwrites its first 64 columns
+constexpr uint32_t kTmemS = 256;          // columns [256, 384): the scores of one tile
+constexpr uint32_t kTmemP = 384;          // columns [384, 512): two buffers of 64 for the f16 P
 constexpr float kLazyThreshold = 8.0f;    // log2 units
 constexpr int kPfMaxSplits = 8;           // key splits per (token tile, head) at most
 
@@ -111,8 +112,9 @@ struct PrefillArgs {
 
 // Barrier slots (8 bytes each).
 enum { kBarKFull = 0, kBarKFree = 6, kBarVFull = 12, kBarVFree = 14, kBarS = 16, kBarP = 18, kBarO = 22,
-       kBarQ = 24, kBarR = 25, kBarCount = 33 };   // kBarP: [score buffer][64-key half of P];
-                                                   // kBarR: [warp pair 0..3][tile parity]
+       kBarQ = 24, kBarR = 25, kBarL = 33, kBarCount = 34 };   // kBarP: [P buffer][64-key half of P];
+                                                   // kBarR: [warp pair 0..3][tile parity];
+                                                   // kBarL: the scores of a tile are in registers
 
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_constant__ PrefillArgs p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       mbar_init(bars + 8 * (kBarO + i), 1);
     }
     for (int i = 0; i < 8; ++i) mbar_init(bars + 8 * (kBarR + i), 1);
+    mbar_init(bars + 8 * kBarL, 4);
     mbar_init(bars + 8 * kBarQ, p.q16 ? 1 : 8);   // the TMA issuer, or one per converting warp
     fence_barrier_init();
   }
@@ -316,12 +319,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       for (int j = 0; j < nt && ok; ++j) {
         const int st = j & 1;
         RD_PF_TRACE(2, j, 0);
-        // score buffer st still holds P(j-2) until P V of tile j-2 has read it
-        if (j >= 2 && !mbar_wait(bars + 8 * (kBarO + st), ((j - 2) >> 1) & 1, p.status, 15)) {
+        // the softmax warps of tile j - 1 have its scores in registers
+        if (j >= 1 && !mbar_wait(bars + 8 * kBarL, (j - 1) & 1, p.status, 15)) {
           ok = false;
           break;
         }
-        const uint32_t d_s = tmem + kTmemS + 128 * st;
+        const uint32_t d_s = tmem + kTmemS;
         RD_PF_TRACE(2, j, 1);
         for (int u = 0; u < 2 && ok; ++u) {
           if (!mbar_wait(bars + 8 * (kBarKFull + slot), use & 1, p.status, 12)) {
@@ -383,7 +386,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
           // A = P(j) from TMEM (16 keys = 8 columns per step), B = V unit MN-major: 64-dim
           // groups 8 KB apart (LBO), 8-key groups 1 KB apart (SBO); 4 steps of 16 keys
           const uint64_t dvs = dv + (uint64_t)((slot * kPfVUnitBytes) >> 4);
-          const uint32_t a_p = tmem + kTmemS + 128 * st + 32 * u;
+          const uint32_t a_p = tmem + kTmemP + 64 * st + 32 * u;
           if (!(RD_PF_DEBUG(p) & 4)) {
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
@@ -392,7 +395,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
           }
           tc_commit(bars + 8 * (kBarVFree + slot));  // the V unit can be refilled
         }
-        tc_commit(bars + 8 * (kBarO + st));  // score buffer reusable, O settled
+        tc_commit(bars + 8 * (kBarO + st));  // P buffer reusable, O settled
         RD_PF_TRACE(3, j, 2);
       }
       if (!ok) s_abort = 1;
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const uint32_t bar_ref = bars + 8 * (kBarR + 2 * (warp & 3));
     bool ok = true;
     for (int j = set; j < nt && ok; j += 2) {
-      const int st = set;   // tile j's score buffer: j & 1
+      const int st = set;   // tile j's P buffer: j & 1
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 0);
       // the reference tile j - 1 left: its set published it right after its own maxima,
       // long before this tile's scores are ready -- fetched first, off the critical path
@@ -424,10 +427,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       tc_fence_after();
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 1);
       uint32_t sc[4][32];
-      const uint32_t scol = lane_addr + kTmemS + 128 * st;
+      const uint32_t scol = lane_addr + kTmemS, pcol = lane_addr + kTmemP + 64 * st;
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld32(scol + 32 * c, sc[c]);
       tmem_wait_ld();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + 8 * kBarL);   // S of tile j + 1 can be computed
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 2);
       const int key0 = (jt0 + j) * kPfN;
       // only tiles that reach past some row's last key need the causal mask
@@ -476,13 +482,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         }
         tmem_wait_st();
       }
-      // P = 2^(s - m_ref) as f16 pairs, written over the score buffer: key k of row r
-      // becomes half k & 1 of column k / 2 (the A operand of P V, read from TMEM); the
-      // columns a chunk overwrites hold scores that are already in registers
+      // P = 2^(s - m_ref) as f16 pairs: key k of row r becomes half k & 1 of column k / 2 (the A
+      // operand of P V, read from TMEM)
       // (s - m) and the row sum go through the packed f32x2 adds, two scores per
       // instruction: measured alone, one warp then needs ~1200 cycles per 128-score row
       // (the 128 exponentials alone are 1024 on the special-function unit) against ~1600
       // with scalar adds
+      // (P V of tile j - 2 has read this buffer)
+      if (j >= 2 && !mbar_wait(bars + 8 * (kBarO + st), ((j - 2) >> 1) & 1, p.status, 21)) { ok = false; break; }
+      tc_fence_after();
       unsigned long long neg_m = f2_pack(-m_new, -m_new);
       unsigned long long ls2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
@@ -499,7 +507,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
           ls2[i & 3] = f2_add(ls2[i & 3], f2_pack(x0, x1));
           pw[i] = (RD_PF_DEBUG(p) & 2) ? __float_as_uint(x0) : pack_h2(x0, x1);
         }
-        if (!(RD_PF_DEBUG(p) & 16)) tmem_st16(scol + 16 * c, pw);
+        if (!(RD_PF_DEBUG(p) & 16)) tmem_st16(pcol + 16 * c, pw);
         else if (pw[0] == 0x12345678u && pw[7] == 0x9abcdefu) l_run += 1.f;   // keeps the values live
         if (c == 1) {   // the first 64 keys of P are complete: hand them to the P V issuer
           tmem_wait_st();
