@@ -2,30 +2,30 @@
 //
 // Replaces attn_fa2_prefill_kernel (include/rdna4/attn_fa2.cuh:30-169 of the reference)
 // for f16 K/V caches. One CTA owns a tile of 128 query tokens of ONE query head and walks
-// the keys in tiles of 128. Tensor memory (512 columns x 128 lanes, lane = query row):
+// the keys in tiles of 128, in a pair (cta_group::2) with the CTA of the KV head's next query head:
+// each loads half of every K and V tile and the pair's MMAs (M = 256, issued by the leader) read
+// both halves. Alone, a CTA moves 320 KB through shared memory per tile (operands 192, copies
+// 128), 2500 cycles at 128 bytes a cycle against 2048 of tensor-core work; in a pair 192 KB. Tensor memory (512 columns x 128 lanes, lane = query row):
 //   columns   0..255  O, the f32 output accumulator
 //   columns 256..383  the f32 scores of one tile: the next tile's can be computed as soon as
 //                     the softmax warps have these in registers
 //   columns 384..511  two buffers of 64 columns for the f16 P of a tile (the A operand of
 //                     O += P V, read from TMEM)
 // Shared memory (224 KB): Q as f16 in the K-major 128-byte-swizzled layout (64 KB), a ring
-// of three K units of [128 keys][128 dims] (96 KB) and a ring of two V units of 64 keys
-// (64 KB), all filled by TMA with the hardware 128B swizzle.
+// of three half K tiles (96 KB) and a ring of two half V tiles (64 KB), filled by TMA with the
+// hardware 128B swizzle.
 //
 //   prologue   the 128 x 256 f32 query rows -> optional partial RoPE, scale*log2(e), f16,
 //              swizzled into shared memory (8 warps, 16 rows each);
 //   per 128-key tile j:
-//     warp 9     S = Q K_j^T        16 x tcgen05.mma M128 N128 K16, four per K chunk, each
-//                                   chunk handed back to the TMA producer as soon as its
-//                                   four MMAs are done (N = 128 keeps the tensor core busy
-//                                   for as long as the 128 x 16 A slice takes to fetch)
+//     warp 9     S = Q K_j^T        16 x tcgen05.mma M256 N128 K16
 //     warps 0-7  two threads per query row, 64 score columns each (row max exchanged
 //                through shared memory): tcgen05.ld the scores, causal mask
 //                (key <= pos[r]), running max with LAZY rescale (the reference point only
 //                moves when a row's max grows by more than 2^8, so P stays below 256 in
 //                f16 and O in TMEM is rarely touched), P -> f16 pairs, tcgen05.st
-//     warp 11    O += P V_j          8 x tcgen05.mma M128 N256 K16 (A = P from TMEM, B = V
-//                                   MN-major), four per V unit
+//     warp 11    O += P V_j          8 x tcgen05.mma M256 N256 K16 (A = P from TMEM, B = V
+//                                   MN-major)
 //   epilogue   O / l (times sigmoid(gate) if asked) through a swizzled staging tile to
 //              coalesced f32 stores.
 // Warps 8 and 10 are the K and V TMA producers (separate warps: a lane parked in
@@ -37,8 +37,7 @@
 // S - softmax - P V - S of 6300 cycles per two tiles against 4096 of tensor-core work.)
 //
 // Synchronisation is mbarriers only (TMA transaction counts, tcgen05.commit); every wait
-// is bounded and a timeout unwinds the CTA (TMEM is always freed). No cluster launch, no
-// multicast.
+// is bounded and a timeout unwinds the pair (TMEM is always freed). No multicast loads.
 #include <stdlib.h>
 #include <string.h>
 
@@ -71,14 +70,17 @@ namespace rd {
 constexpr int kPfM = 128;                 // query rows per CTA
 constexpr int kPfN = 128;                 // keys per tile
 constexpr int kPfQBytes = kPfM * kHeadDim * 2;             // 65536 (also the epilogue staging)
-constexpr int kPfKChunkBytes = kPfN * 128;                 // [128 keys][64 dims] f16: 16384
-constexpr int kPfKUnitBytes = 2 * kPfKChunkBytes;          // K unit: [128 keys][128 dims], two chunks
-constexpr int kPfKSlots = 3;                               // 1.5 tiles of K in flight
-constexpr int kPfVUnitKeys = 64;
-constexpr int kPfVUnitBytes = kPfVUnitKeys * kHeadDim * 2; // 32768
+// A CTA of the pair holds half of each K tile (64 of the 128 keys) and of each V tile (128 of the 256 dims).
+constexpr int kPfKKeys = kPfN / 2;
+constexpr int kPfKChunkBytes = kPfKKeys * 128;             // [64 keys][64 dims] f16: 8192
+constexpr int kPfKTileBytes = 4 * kPfKChunkBytes;          // 32768
+constexpr int kPfKSlots = 3;
+constexpr int kPfVDims = kHeadDim / 2;
+constexpr int kPfVChunkBytes = kPfN * 128;                 // [128 keys][64 dims]: 16384
+constexpr int kPfVTileBytes = 2 * kPfVChunkBytes;          // 32768
 constexpr int kPfVSlots = 2;
 // 224 KB of dynamic shared memory + < 3 KB static = the 227 KB an sm_100 CTA may use
-constexpr int kPfSmemBytes = kPfQBytes + kPfKSlots * kPfKUnitBytes + kPfVSlots * kPfVUnitBytes;
+constexpr int kPfSmemBytes = kPfQBytes + kPfKSlots * kPfKTileBytes + kPfVSlots * kPfVTileBytes;
 constexpr int kPfThreads = 384;           // 8 softmax warps, K TMA, S MMA, V TMA, PV MMA warps
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemO = 0;            // columns [0, 256): output accumulator
@@ -111,6 +113,8 @@ struct PrefillArgs {
 };
 
 // Barrier slots (8 bytes each).
+// In the leader (CTA 0 of the pair) alone: KFull, VFull, Q, P, L -- what its issuing threads wait for, from
+// both CTAs. In each CTA: KFree, VFree, S, O (tcgen05.commit arrives on both), R.
 enum { kBarKFull = 0, kBarKFree = 6, kBarVFull = 12, kBarVFree = 14, kBarS = 16, kBarP = 18, kBarO = 22,
        kBarQ = 24, kBarR = 25, kBarL = 33, kBarCount = 34 };   // kBarP: [P buffer][64-key half of P];
                                                    // kBarR: [warp pair 0..3][tile parity];
@@ -127,8 +131,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_launch_dependents();   // the merge pass of a key split may be scheduled under this kernel
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 0);   // kernel entry
-  const int tile = (int)gridDim.x - 1 - (int)blockIdx.x;  // heaviest (latest) tiles first
-  const int head = blockIdx.y;
+  const int tile = (int)gridDim.y - 1 - (int)blockIdx.y;  // heaviest (latest) tiles first
+  const int head = blockIdx.x;                            // heads 2 i and 2 i + 1 (one KV head) are a pair
+  const uint32_t rank = blockIdx.x & 1;
   const int kvh = head / kGroup;
   const int row0 = tile * kPfM;
 
@@ -141,9 +146,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   }
   const uint32_t sQ = base;
   const uint32_t sK = sQ + kPfQBytes;                       // slot s at + s * 32 KB
-  const uint32_t sV = sK + kPfKSlots * kPfKUnitBytes;       // slot s at + s * 32 KB
+  const uint32_t sV = sK + kPfKSlots * kPfKTileBytes;       // slot s at + s * 32 KB
   uint8_t *gQ = smem_raw;                                   // generic pointer to sQ
-  const uint32_t bars = smem_u32(s_bars);
+  const uint32_t bars = smem_u32(s_bars), lead = cluster_addr(bars, 0);   // this CTA's barriers, the leader's
 
   // Requested first, so that their latency runs under the set-up below: the positions of
   // this tile's rows and -- where the tile is converted here -- all 16 query rows of the
@@ -178,21 +183,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       mbar_init(bars + 8 * (kBarVFull + i), 1);
       mbar_init(bars + 8 * (kBarVFree + i), 1);
       mbar_init(bars + 8 * (kBarS + i), 1);
-      mbar_init(bars + 8 * (kBarP + 2 * i), 4);       // one elected lane per softmax warp of the
-      mbar_init(bars + 8 * (kBarP + 2 * i + 1), 4);   // tile's set, per 64-key half of P
+      mbar_init(bars + 8 * (kBarP + 2 * i), 8);       // one elected lane per softmax warp of the
+      mbar_init(bars + 8 * (kBarP + 2 * i + 1), 8);   // tile's set (both CTAs), per 64-key half of P
       mbar_init(bars + 8 * (kBarO + i), 1);
     }
     for (int i = 0; i < 8; ++i) mbar_init(bars + 8 * (kBarR + i), 1);
-    mbar_init(bars + 8 * kBarL, 4);
-    mbar_init(bars + 8 * kBarQ, p.q16 ? 1 : 8);   // the TMA issuer, or one per converting warp
+    mbar_init(bars + 8 * kBarL, 8);
+    mbar_init(bars + 8 * kBarQ, p.q16 ? 1 : 16);   // the TMA issuer, or one per converting warp
     fence_barrier_init();
   }
   if (warp == 9) {  // TMEM: 512 columns for this CTA (one CTA per SM: no contention)
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&s_tmem_base)),
                  "r"(kTmemCols)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   __syncthreads();
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 1);   // barriers + TMEM allocated
@@ -205,7 +210,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     if (lane == 0) atomicMax(&s_maxpos, mx);
   }
   tc_fence_before();
-  __syncthreads();
+  cluster_sync();   // the pair's barriers are initialised, its tensor memory allocated
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 2);   // positions known
   tc_fence_after();
   const uint32_t tmem = s_tmem_base;
@@ -221,11 +226,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     // and V producers are already loading.
     if (threadIdx.x == 0) {
       pdl_wait();   // that pass has completed (this launch may have started under it)
-      const uint32_t full = bars + 8 * kBarQ;
-      mbar_expect_tx(full, kPfQBytes);
+      if (rank == 0) mbar_expect_tx(bars + 8 * kBarQ, 2 * kPfQBytes);
 #pragma unroll
       for (int c = 0; c < 4; ++c)
-        tma_load_2d(sQ + c * (kPfM * 128), &p.tm_q, head * kHeadDim + 64 * c, row0, full);
+        tma_load_2d_pair(sQ + c * (kPfM * 128), &p.tm_q, head * kHeadDim + 64 * c, row0, lead + 8 * kBarQ);
     }
   } else if (warp < 8) {
     // f32 rows -> x scale * log2(e) -> f16, warps 0-7, 16 rows each
@@ -242,7 +246,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     }
     fence_proxy_async();  // generic-proxy writes -> visible to the tensor core's async proxy
     __syncwarp();
-    if (lane == 0) mbar_arrive(bars + 8 * kBarQ);  // the S MMAs wait for all 8 warps
+    if (lane == 0) mbar_arrive_cluster(lead + 8 * kBarQ);  // the S MMAs wait for all 16 warps
     if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 3);   // this warp's Q rows converted
   }
 
@@ -252,27 +256,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   if (warp >= 8) {
   if (warp == 8) {
     // =============================== K producer ====================================
-    // unit g = 2 j + u: keys of tile j, dims [128 u, 128 u + 128) as two 64-dim chunks, into
-    // slot g % 3 -- one barrier per unit: the issuing thread pays for every wait and commit
+    // this CTA's half of tile j (64 keys) into slot j % 3; both CTAs' copies complete on the leader's barrier
     if (lane == 0) {
       if (p.kv_wait) pdl_wait();   // the pre-pass of this call appended rows to the caches
       int slot = 0, use = 0;
-      for (int g = 0; g < 2 * nt; ++g) {
+      for (int j = 0; j < nt; ++j) {
         if (use > 0 && !mbar_wait(bars + 8 * (kBarKFree + slot), (use - 1) & 1, p.status, 11)) {
           s_abort = 1;
           break;
         }
         if (*(volatile int *)&s_abort) break;
-        const uint32_t full = bars + 8 * (kBarKFull + slot);
-        if (RD_PF_DEBUG(p) & 32) {
-          mbar_arrive(full);
-        } else {
-          mbar_expect_tx(full, kPfKUnitBytes);
+        if (rank == 0) mbar_expect_tx(bars + 8 * (kBarKFull + slot), 2 * kPfKTileBytes);
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
-            tma_load_2d(sK + slot * kPfKUnitBytes + h * kPfKChunkBytes, &p.tm_k,
-                        kvh * kHeadDim + 128 * (g & 1) + 64 * h, (jt0 + (g >> 1)) * kPfN, full);
-        }
+        for (int c = 0; c < 4; ++c)
+          tma_load_2d_pair(sK + slot * kPfKTileBytes + c * kPfKChunkBytes, &p.tm_k, kvh * kHeadDim + 64 * c,
+                           (jt0 + j) * kPfN + (int)rank * kPfKKeys, lead + 8 * (kBarKFull + slot));
         if (++slot == kPfKSlots) {
           slot = 0;
           ++use;
@@ -281,94 +279,85 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     }
   } else if (warp == 10) {
     // =============================== V producer ====================================
-    // unit g = 2 j + u: keys [128 j + 64 u, + 64) of all 256 dims, into slot g % 2
+    // this CTA's half of tile j (128 of the 256 dims) into slot j % 2
     if (lane == 0) {
-      bool ok = true;
       if (p.kv_wait) pdl_wait();
-      for (int g = 0; g < 2 * nt && ok; ++g) {
-        const int slot = g & 1;
-        if (g >= 2 && !mbar_wait(bars + 8 * (kBarVFree + slot), ((g >> 1) - 1) & 1, p.status, 22)) {
-          ok = false;
+      for (int j = 0; j < nt; ++j) {
+        const int slot = j & 1;
+        if (j >= 2 && !mbar_wait(bars + 8 * (kBarVFree + slot), ((j >> 1) - 1) & 1, p.status, 22)) {
+          s_abort = 1;
           break;
         }
         if (*(volatile int *)&s_abort) break;
-        const uint32_t full = bars + 8 * (kBarVFull + slot);
-        if (RD_PF_DEBUG(p) & 32) {
-          mbar_arrive(full);
-          continue;
-        }
-        mbar_expect_tx(full, kPfVUnitBytes);
+        if (rank == 0) mbar_expect_tx(bars + 8 * (kBarVFull + slot), 2 * kPfVTileBytes);
 #pragma unroll
-        for (int c = 0; c < 4; ++c)  // four [64 keys][64 dims] sub-tiles
-          tma_load_2d(sV + slot * kPfVUnitBytes + c * (kPfVUnitKeys * 128), &p.tm_v, kvh * kHeadDim + 64 * c,
-                      (2 * jt0 + g) * kPfVUnitKeys, full);
+        for (int c = 0; c < 2; ++c)
+          tma_load_2d_pair(sV + slot * kPfVTileBytes + c * kPfVChunkBytes, &p.tm_v,
+                           kvh * kHeadDim + (int)rank * kPfVDims + 64 * c, (jt0 + j) * kPfN, lead + 8 * (kBarVFull + slot));
       }
-      if (!ok) s_abort = 1;
     }
   } else if (warp == 9) {
     // ============================ MMA issuer: S = Q K^T =============================
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = idesc_f16(kPfM, kPfN, false);
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc_s = idesc_f16(2 * kPfM, kPfN, false);
       // Descriptors differ only in the 16-byte-granular start address (low 14 bits, and
       // every address here is below 256 KB), so each one is a base plus a constant.
       const uint64_t dq = smem_desc(sQ, 16, 1024);
       const uint64_t dk = smem_desc(sK, 16, 1024);
-      bool ok = mbar_wait(bars + 8 * kBarQ, 0, p.status, 18);  // Q tile written by warps 0-3
+      bool ok = mbar_wait_cluster(bars + 8 * kBarQ, 0, p.status, 18);  // both Q tiles are there
       tc_fence_after();
       int slot = 0, use = 0;
       for (int j = 0; j < nt && ok; ++j) {
-        const int st = j & 1;
         RD_PF_TRACE(2, j, 0);
-        // the softmax warps of tile j - 1 have its scores in registers
+        if (!mbar_wait(bars + 8 * (kBarKFull + slot), use & 1, p.status, 12)) {
+          ok = false;
+          break;
+        }
+        RD_PF_TRACE(2, j, 1);
+        // the softmax warps of tile j - 1 (both CTAs) have its scores in registers
         if (j >= 1 && !mbar_wait(bars + 8 * kBarL, (j - 1) & 1, p.status, 15)) {
           ok = false;
           break;
         }
-        const uint32_t d_s = tmem + kTmemS;
-        RD_PF_TRACE(2, j, 1);
-        for (int u = 0; u < 2 && ok; ++u) {
-          if (!mbar_wait(bars + 8 * (kBarKFull + slot), use & 1, p.status, 12)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          if (u == 0) RD_PF_TRACE(2, j, 3);
-          // per 64-dim chunk c = 2 u + h: A = Q sub-tile c ([128 rows][64 dims]), B = K chunk
-          // ([128 keys][64 dims]), both K-major with 8-row groups 1 KB apart; four steps of
-          // 16 dims = 32 bytes each
-          if (!(RD_PF_DEBUG(p) & 8)) {
+        tc_fence_after();
+        RD_PF_TRACE(2, j, 3);
+        // per 64-dim chunk c: A = Q sub-tile c ([128 rows][64 dims] in each CTA), B = K chunk c ([64
+        // keys][64 dims] in each), K-major with 8-row groups 1 KB apart; four steps of 16 dims
+        if (!(RD_PF_DEBUG(p) & 8)) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const uint64_t a0 = dq + (uint64_t)(((2 * u + h) * (kPfM * 128)) >> 4);
-              const uint64_t b0 = dk + (uint64_t)((slot * kPfKUnitBytes + h * kPfKChunkBytes) >> 4);
+          for (int c = 0; c < 4; ++c) {
+            const uint64_t a0 = dq + (uint64_t)((c * (kPfM * 128)) >> 4);
+            const uint64_t b0 = dk + (uint64_t)((slot * kPfKTileBytes + c * kPfKChunkBytes) >> 4);
 #pragma unroll
-              for (int kk = 0; kk < 4; ++kk)
-                tc_mma_f16(d_s, a0 + (uint64_t)(2 * kk), b0 + (uint64_t)(2 * kk), idesc_s,
-                           (u > 0 || h > 0 || kk > 0) ? 1u : 0u);
-            }
-          }
-          if (u == 0) RD_PF_TRACE(2, j, 4);
-          tc_commit(bars + 8 * (kBarKFree + slot));  // the unit can be refilled
-          if (u == 0) RD_PF_TRACE(2, j, 5);
-          if (++slot == kPfKSlots) {
-            slot = 0;
-            ++use;
+            for (int kk = 0; kk < 4; ++kk)
+              tc_mma2_f16(tmem + kTmemS, a0 + (uint64_t)(2 * kk), b0 + (uint64_t)(2 * kk), idesc_s,
+                          (c > 0 || kk > 0) ? 1u : 0u);
           }
         }
-        tc_commit(bars + 8 * (kBarS + st));
+        RD_PF_TRACE(2, j, 4);
+        tc_commit2(bars + 8 * (kBarS + (j & 1)));
+        tc_commit2(bars + 8 * (kBarKFree + slot));  // the tile can be refilled
+        if (++slot == kPfKSlots) {
+          slot = 0;
+          ++use;
+        }
         RD_PF_TRACE(2, j, 2);
       }
       if (!ok) s_abort = 1;
     }
   } else if (warp == 11) {
     // ============================ MMA issuer: O += P V ==============================
-    if (lane == 0) {
-      constexpr uint32_t idesc_o = idesc_f16(kPfM, kHeadDim, true);
-      const uint64_t dv = smem_desc(sV, kPfVUnitKeys * 128, 1024);
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc_o = idesc_f16(2 * kPfM, kHeadDim, true);
+      const uint64_t dv = smem_desc(sV, kPfVChunkBytes, 1024);
       bool ok = true;
       for (int j = 0; j < nt && ok; ++j) {
         const int st = j & 1;
         RD_PF_TRACE(3, j, 0);
+        if (!mbar_wait(bars + 8 * (kBarVFull + st), (j >> 1) & 1, p.status, 19)) {
+          ok = false;
+          break;
+        }
         for (int u = 0; u < 2 && ok; ++u) {
           // P arrives in two halves of 64 keys: P V of the first runs while the softmax
           // threads are still on the second
@@ -377,25 +366,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
             break;
           }
           if (u == 0) RD_PF_TRACE(3, j, 1);
-          const int g = 2 * j + u, slot = g & 1;
-          if (!mbar_wait(bars + 8 * (kBarVFull + slot), (g >> 1) & 1, p.status, 19)) {
-            ok = false;
-            break;
-          }
           tc_fence_after();
-          // A = P(j) from TMEM (16 keys = 8 columns per step), B = V unit MN-major: 64-dim
-          // groups 8 KB apart (LBO), 8-key groups 1 KB apart (SBO); 4 steps of 16 keys
-          const uint64_t dvs = dv + (uint64_t)((slot * kPfVUnitBytes) >> 4);
+          // A = P(j) from TMEM (16 keys = 8 columns per step), B = V MN-major, 128 of the 256 dims in each
+          // CTA: 64-dim groups 16 KB apart (LBO), 8-key groups 1 KB apart (SBO); 4 steps of 16 keys
+          const uint64_t dvs = dv + (uint64_t)((st * kPfVTileBytes + u * 8192) >> 4);
           const uint32_t a_p = tmem + kTmemP + 64 * st + 32 * u;
           if (!(RD_PF_DEBUG(p) & 4)) {
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-              tc_mma_f16_ts(tmem + kTmemO, a_p + 8 * kk, dvs + (uint64_t)((kk * 2048) >> 4), idesc_o,
-                            (j > 0 || u > 0 || kk > 0) ? 1u : 0u);
+              tc_mma2_f16_ts(tmem + kTmemO, a_p + 8 * kk, dvs + (uint64_t)((kk * 2048) >> 4), idesc_o,
+                             (j > 0 || u > 0 || kk > 0) ? 1u : 0u);
           }
-          tc_commit(bars + 8 * (kBarVFree + slot));  // the V unit can be refilled
         }
-        tc_commit(bars + 8 * (kBarO + st));  // P buffer reusable, O settled
+        if (!ok) break;
+        tc_commit2(bars + 8 * (kBarVFree + st));  // the V tile can be refilled
+        tc_commit2(bars + 8 * (kBarO + st));      // P buffer reusable, O settled
         RD_PF_TRACE(3, j, 2);
       }
       if (!ok) s_abort = 1;
@@ -433,7 +418,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bars + 8 * kBarL);   // S of tile j + 1 can be computed
+      if (lane == 0) mbar_arrive_peer(lead + 8 * kBarL);   // S of tile j + 1 can be computed
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 2);
       const int key0 = (jt0 + j) * kPfN;
       // only tiles that reach past some row's last key need the causal mask
@@ -513,7 +498,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bars + 8 * (kBarP + 2 * st));
+          if (lane == 0) mbar_arrive_peer(lead + 8 * (kBarP + 2 * st));
           // keeps the second half's arithmetic behind the hand-over (the compiler would
           // otherwise hoist all 128 exponentials above the first store)
           asm volatile("mov.b64 %0, %0;" : "+l"(neg_m)::"memory");
@@ -529,7 +514,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bars + 8 * (kBarP + 2 * st + 1));
+      if (lane == 0) mbar_arrive_peer(lead + 8 * (kBarP + 2 * st + 1));
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 5);
     }
     if (ok && nt > 0 && !mbar_wait(bars + 8 * (kBarO + ((nt - 1) & 1)), ((nt - 1) >> 1) & 1, p.status, 16))
@@ -542,8 +527,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   // completed: o may alias q, which it is still reading. A CTA with key tiles knows this from
   // its Q tile; one without (no row attends a key) waits for the tile here -- its TMA load was
   // issued behind the dependency wait all the same.
-  if (p.q16 && nt == 0 && threadIdx.x == 0 && !mbar_wait(bars + 8 * kBarQ, 0, p.status, 23)) s_abort = 1;
-  __syncthreads();
+  if (p.q16 && nt == 0 && threadIdx.x == 0 && rank == 0 && !mbar_wait_cluster(bars + 8 * kBarQ, 0, p.status, 23))
+    s_abort = 1;
+  cluster_sync();   // both CTAs are done with each other's barriers, shared and tensor memory
   const bool aborted = s_abort != 0;
   // the two sets' row sums, each with the reference it is expressed in: [set][sum,
   // reference][row], over the K ring (every load into it has been consumed by now)
@@ -657,10 +643,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     }
   }
   tc_fence_before();
-  __syncthreads();
+  cluster_sync();   // the pair frees its tensor memory together
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 5);   // epilogue stores done
   if (warp == 9) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols)
                  : "memory");
   }
 }
@@ -857,9 +843,9 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
                    cudaStream_t st) {
   PrefillArgs a;
   memset(&a, 0, sizeof(a));
-  int rc = encode_f16_tmap(&a.tm_k, k, n_head_kv, keys_total, kPfN);
+  int rc = encode_f16_tmap(&a.tm_k, k, n_head_kv, keys_total, kPfKKeys);
   if (rc != RD_OK) return rc;
-  rc = encode_f16_tmap(&a.tm_v, v, n_head_kv, keys_total, kPfVUnitKeys);
+  rc = encode_f16_tmap(&a.tm_v, v, n_head_kv, keys_total, kPfN);
   if (rc != RD_OK) return rc;
   a.q = q;
   a.out = out;
@@ -892,30 +878,30 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   }
   if (n_splits < 1 || records == nullptr) n_splits = 1;
   a.records = records;
-  const dim3 grid((unsigned)((n_q + kPfM - 1) / kPfM), (unsigned)n_head, (unsigned)n_splits);
   if (prepass) {
     // (a pass of many waves gains nothing from starting early: measured 1.8 % slower at 8192 tokens)
     if (launch_pdl(n_q <= 1024 ? 8 : 0, q_prep_kernel, dim3((unsigned)n_q), dim3(256), 0, st, q, pos, n_head, n_rot, a.qscale,
                    (uint4 *)q16, k_new, v_new, (uint4 *)k_dst, (uint4 *)v_dst, n_head_kv,
                    make_rope_table(n_rot, freq_base)) != cudaSuccess)
       return RD_ERR_CUDA;
-    // the tile kernel may start while that pass runs; it waits for it (griddepcontrol)
-    // before it loads its Q tile
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kPfThreads);
-    cfg.dynamicSmemBytes = kPfSmemBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, prefill_kernel, a) != cudaSuccess) return RD_ERR_CUDA;
-  } else {
-    prefill_kernel<<<grid, kPfThreads, kPfSmemBytes, st>>>(a);
-    if (cudaGetLastError() != cudaSuccess) return RD_ERR_CUDA;
   }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)n_head, (unsigned)((n_q + kPfM - 1) / kPfM), (unsigned)n_splits);
+  cfg.blockDim = dim3(kPfThreads);
+  cfg.dynamicSmemBytes = kPfSmemBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;   // a pair must lie along x
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  // under the pre-pass the tile kernel may start early: it waits for it (griddepcontrol)
+  // before it loads its Q tile
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = prepass ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, prefill_kernel, a) != cudaSuccess) return RD_ERR_CUDA;
   if (n_splits > 1) {
     const int64_t n_rows = (int64_t)n_q * n_head;
     if (n_splits > kPfMaxSplits) return RD_ERR_SHAPE;
