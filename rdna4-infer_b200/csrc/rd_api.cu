@@ -918,7 +918,7 @@ static int prefill_common(const float *q, const void *k, const void *v, float *o
                           const int32_t *pos, int n_q, int keys_total, int n_head, int n_head_kv,
                           int head_dim, float scale, int n_rot, float freq_base, void *stream,
                           void *records = nullptr, size_t record_bytes = 0, const float *k_new = nullptr,
-                          const float *v_new = nullptr, int row0 = 0) {
+                          const float *v_new = nullptr, int row0 = 0, bool kv_pending = false) {
   int rc = check_attn_shape(n_head, n_head_kv, head_dim, RD_KV_F16, RD_KV_F16);
   if (rc != RD_OK) return rc;
   if (n_q < 1 || keys_total <= 0) return RD_ERR_SHAPE;
@@ -930,24 +930,20 @@ static int prefill_common(const float *q, const void *k, const void *v, float *o
   if ((rc = current_device(&dev)) != RD_OK) return rc;
   DeviceStatus *status = status_word(dev);   // every launch reports its bounded waits
   if (status == nullptr) return RD_ERR_CUDA;
-  // scratch: [rotated f16 queries, if the call rotates][key-split records, if any]
   int splits = prefill_splits(n_q, keys_total, n_head, sm_count(dev));
-  const size_t rope_need = (n_rot > 0 || k_new != nullptr) ? align256(prefill_rope_bytes(n_q, n_head)) : 0;
   const size_t need = prefill_record_bytes(n_q, n_head, splits);
-  if (records == nullptr && rope_need + (splits > 1 ? need : 0) > 0) {
-    records = ensure_workspace(dev, rope_need + need);
-    record_bytes = records != nullptr ? rope_need + need : 0;
+  if (records == nullptr && splits > 1) {
+    records = ensure_workspace(dev, need);
+    if (records == nullptr) return RD_ERR_CUDA;
+    record_bytes = need;
   }
-  if (record_bytes < rope_need) return records == nullptr ? RD_ERR_CUDA : RD_ERR_WORKSPACE;
-  void *rope_cs = rope_need > 0 ? records : nullptr;
-  float *recs = (float *)((unsigned char *)records + rope_need);
-  if (splits > 1 && record_bytes - rope_need < need) splits = 1;   // no room: one CTA per (token tile, head) walks all keys
+  if (record_bytes < need) splits = 1;   // no room: one CTA per (token tile, head) walks all keys
   // a fused append stores rows row0 .. row0 + n_q - 1 of the (f16) caches
   const size_t row_bytes = (size_t)n_head_kv * kHeadDim * 2;
   void *k_dst = k_new != nullptr ? (void *)((unsigned char *)const_cast<void *>(k) + (size_t)row0 * row_bytes) : nullptr;
   void *v_dst = k_new != nullptr ? (void *)((unsigned char *)const_cast<void *>(v) + (size_t)row0 * row_bytes) : nullptr;
   return launch_prefill(q, k, v, o, gate, pos, n_q, keys_total, n_head, n_head_kv, scale, n_rot,
-                        freq_base, status, recs, splits, rope_cs, k_new, v_new, k_dst, v_dst,
+                        freq_base, status, (float *)records, splits, k_new, v_new, k_dst, v_dst, kv_pending,
                         (cudaStream_t)stream);
 }
 
@@ -988,7 +984,7 @@ size_t rd_attn_prefill_workspace_bytes(int k_type, int v_type, int n_q, int keys
   if (!known_type(k_type) || !known_type(v_type) || n_q < 1 || keys_total <= 0 || n_head < 1 ||
       n_head_kv < 1 || head_dim != kHeadDim || current_device(&dev) != RD_OK)
     return 0;
-  return prefill_copy_bytes(k_type, v_type, keys_total, n_head_kv) + align256(prefill_rope_bytes(n_q, n_head)) +
+  return prefill_copy_bytes(k_type, v_type, keys_total, n_head_kv) +
          align256(prefill_record_bytes(n_q, n_head, prefill_splits(n_q, keys_total, n_head, sm_count(dev))));
 }
 
@@ -1035,7 +1031,7 @@ int rd_attn_prefill_typed(const float *q, const void *k, const void *v, float *o
   static float s_dummy;   // non-null marker when no records are needed
   return prefill_common(q, k16, v16, o, gate, pos, n_q, keys_total, n_head, n_head_kv, head_dim, scale,
                         n_rot, freq_base, stream, rec != nullptr ? (void *)rec : (void *)&s_dummy,
-                        need > copies ? need - copies : 0);
+                        need > copies ? need - copies : 0, nullptr, nullptr, 0, kdst != nullptr || vdst != nullptr);
 }
 
 static int g_last_site = 0;   // `where` of the last time-out rd_device_status reported

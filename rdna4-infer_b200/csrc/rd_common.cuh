@@ -324,6 +324,10 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void *src, uin
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
+// Fetches `bytes` (a multiple of 16, 16-byte aligned) into L2.
+__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // global -> shared 2-D tile copy through a tensor map: box rows land densely in shared
 // memory (128-byte aligned), rows outside the tensor are filled with zeros. x is in
 // elements of the map's data type and must keep x * element size a multiple of 16.
@@ -334,6 +338,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap
       "{%2, %3}], [%4];" ::"r"(dst_smem),
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
+}
+// The same box to L2 only.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -154,6 +154,9 @@ int encode_kv_tmap(void *tmap_out, const void *base, int type, int n_head_kv, in
 // with SWIZZLE_128B read).
 int encode_f16_tmap(void *tmap_out, const void *base, int n_head_kv, int64_t n_rows, int tile_rows);
 
+// Tensor map over f32 activations [n_rows][n_head * 256] with a box of [tile_rows][one head], no swizzle.
+int encode_f32_tmap(void *tmap_out, const void *base, int n_head, int64_t n_rows, int tile_rows);
+
 // ---- rd_prefill.cu
 // Causal prefill attention over f16 caches on tcgen05: token i attends keys 0..pos[i]
 // (pos on the device), keys_total rows exist in the cache. gate (optional) fuses
@@ -162,9 +165,10 @@ int encode_f16_tmap(void *tmap_out, const void *base, int n_head_kv, int64_t n_r
 // over gridDim.z and a second launch merges the per-split records.
 int launch_prefill(const float *q, const void *k, const void *v, float *out, const float *gate,
                    const int32_t *pos, int n_q, int keys_total, int n_head, int n_head_kv, float scale,
-                   int n_rot, float freq_base, DeviceStatus *status, float *records, int n_splits, void *q16, const float *k_new, const float *v_new, void *k_dst, void *v_dst,
-                   cudaStream_t st);
-size_t prefill_rope_bytes(int n_q, int n_head);   // the f16 query copy launch_prefill needs when n_rot > 0
+                   int n_rot, float freq_base, DeviceStatus *status, float *records, int n_splits,
+                   const float *k_new, const float *v_new, void *k_dst, void *v_dst, bool kv_pending,
+                   cudaStream_t st);   // kv_pending: the launch before this one writes k and v, and has waited
+                                       // for everything before it (kv_dequant_f16_kernel)
 int prefill_splits(int n_q, int keys_total, int n_head, int sms);
 size_t prefill_record_bytes(int n_q, int n_head, int splits);
 

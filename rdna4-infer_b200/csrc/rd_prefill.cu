@@ -16,7 +16,7 @@
 // hardware 128B swizzle.
 //
 //   prologue   the 128 x 256 f32 query rows -> optional partial RoPE, scale*log2(e), f16,
-//              swizzled into shared memory (8 warps, 16 rows each);
+//              swizzled into shared memory;
 //   per 128-key tile j:
 //     warp 9     S = Q K_j^T        16 x tcgen05.mma M256 N128 K16
 //     warps 0-7  two threads per query row, 64 score columns each (row max exchanged
@@ -81,6 +81,7 @@ constexpr int kPfVTileBytes = 2 * kPfVChunkBytes;          // 32768
 constexpr int kPfVSlots = 2;
 // 224 KB of dynamic shared memory + < 3 KB static = the 227 KB an sm_100 CTA may use
 constexpr int kPfSmemBytes = kPfQBytes + kPfKSlots * kPfKTileBytes + kPfVSlots * kPfVTileBytes;
+constexpr int kPfRowsBytes = kPfM * kHeadDim * 4;          // a tile of f32 query or gate rows: 128 KB
 constexpr int kPfThreads = 384;           // 8 softmax warps, K TMA, S MMA, V TMA, PV MMA warps
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemO = 0;            // columns [0, 256): output accumulator
@@ -100,9 +101,12 @@ struct PrefillArgs {
   int n_head;
   int nkv;
   float qscale;          // scale * log2(e)
-  alignas(64) CUtensorMap tm_q;  // q16 != 0: the rotated, scaled f16 queries q_prep_kernel wrote
-  int q16;               // 1: Q tile by TMA from tm_q; 0: converted from `q` (f32, no rotation) here
-  int kv_wait;           // 1: that pre-pass also stored cache rows: the K / V loads wait for it too
+  alignas(64) CUtensorMap tm_q;  // f32 rows of `q` and `gate`: boxes of [128 tokens][one head]
+  alignas(64) CUtensorMap tm_g;
+  int n_rot;             // partial RoPE of the queries: dims [0, n_rot), pairs (d, d + n_rot / 2)
+  float freq[32];        // rotation frequencies of the pairs
+  int kv_wait;           // 1: the launch before this one (which waited for everything before it) stores cache
+                         // rows: only the K / V loads wait for it. 0: the whole kernel waits for its predecessor
   int debug;             // timing experiments only (bit mask), 0 in production
   DeviceStatus *status;
   // Split over the keys (gridDim.z > 1): CTA (tile, head, z) walks only its share of the
@@ -116,9 +120,12 @@ struct PrefillArgs {
 // In the leader (CTA 0 of the pair) alone: KFull, VFull, Q, P, L -- what its issuing threads wait for, from
 // both CTAs. In each CTA: KFree, VFree, S, O (tcgen05.commit arrives on both), R.
 enum { kBarKFull = 0, kBarKFree = 6, kBarVFull = 12, kBarVFree = 14, kBarS = 16, kBarP = 18, kBarO = 22,
-       kBarQ = 24, kBarR = 25, kBarL = 33, kBarCount = 34 };   // kBarP: [P buffer][64-key half of P];
+       kBarQ = 24, kBarR = 25, kBarL = 33, kBarC = 34, kBarF = 35, kBarG = 36, kBarCount = 37 };   // kBarP: [P buffer][64-key half of P];
                                                    // kBarR: [warp pair 0..3][tile parity];
-                                                   // kBarL: the scores of a tile are in registers
+                                                   // kBarL: the scores of a tile are in registers;
+                                                   // kBarF: the f32 query rows have arrived;
+                                                   // kBarC: they are converted (their staging is free);
+                                                   // kBarG: the gate rows are in shared memory
 
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_constant__ PrefillArgs p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -130,6 +137,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_launch_dependents();   // the merge pass of a key split may be scheduled under this kernel
+  if (!p.kv_wait) pdl_wait();
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 0);   // kernel entry
   const int tile = (int)gridDim.y - 1 - (int)blockIdx.y;  // heaviest (latest) tiles first
   const int head = blockIdx.x;                            // heads 2 i and 2 i + 1 (one KV head) are a pair
@@ -150,25 +158,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   uint8_t *gQ = smem_raw;                                   // generic pointer to sQ
   const uint32_t bars = smem_u32(s_bars), lead = cluster_addr(bars, 0);   // this CTA's barriers, the leader's
 
-  // Requested first, so that their latency runs under the set-up below: the positions of
-  // this tile's rows and -- where the tile is converted here -- all 16 query rows of the
-  // warp (32 float4 per lane; the conversion is bound by the latency of these loads).
+  // Requested first, so that their latency runs under the set-up below: the positions of this tile's
+  // rows and its f32 query rows, into K slots 1 and 2 and both V slots (128 KB that the pipeline needs
+  // last). One tensor-map box: a bulk copy per row took 57 cycles each to issue, 7300 for the tile.
   int my_pos = -1;
   if (threadIdx.x < 2 * kPfM) {
     const int r = row0 + (threadIdx.x & (kPfM - 1));
     if (r < p.n_q) my_pos = p.pos[r];
   }
-  float4 qa[16], qb[16];
-  if (!p.q16 && warp < 8) {
-#pragma unroll
-    for (int rr = 0; rr < 16; ++rr) {
-      const int gr = row0 + warp * 16 + rr;
-      qa[rr] = qb[rr] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (gr < p.n_q) {
-        const float4 *src = reinterpret_cast<const float4 *>(p.q + ((size_t)gr * p.n_head + head) * kHeadDim);
-        qa[rr] = src[2 * lane];
-        qb[rr] = src[2 * lane + 1];
-      }
+  const uint32_t sStage = sK + kPfKTileBytes;
+  if (warp == 10) {
+    if (lane == 0) {
+      mbar_init(bars + 8 * kBarF, 1);
+      fence_barrier_init();
+      mbar_expect_tx(bars + 8 * kBarF, kPfRowsBytes);   // (rows past n_q come as zeros)
+      tma_load_2d(sStage, &p.tm_q, head * kHeadDim, row0, bars + 8 * kBarF);
     }
   }
 
@@ -189,7 +193,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     }
     for (int i = 0; i < 8; ++i) mbar_init(bars + 8 * (kBarR + i), 1);
     mbar_init(bars + 8 * kBarL, 8);
-    mbar_init(bars + 8 * kBarQ, p.q16 ? 1 : 16);   // the TMA issuer, or one per converting warp
+    mbar_init(bars + 8 * kBarQ, 16);   // one per converting warp (both CTAs)
+    mbar_init(bars + 8 * kBarC, 8);
+    mbar_init(bars + 8 * kBarG, 1);
     fence_barrier_init();
   }
   if (warp == 9) {  // TMEM: 512 columns for this CTA (one CTA per SM: no contention)
@@ -220,36 +226,93 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   const int nt = (int)(((int64_t)nt_all * (blockIdx.z + 1)) / gridDim.z) - jt0;
 
   // ---- prologue: the Q tile as f16 in the swizzled K-major layout ----
-  if (p.q16) {
-    // rotated, scaled and rounded by q_prep_kernel: four TMA boxes of [128 rows][64 dims]
-    // (rows past n_q are filled with zeros). Only this thread waits for that pass: the K
-    // and V producers are already loading.
-    if (threadIdx.x == 0) {
-      pdl_wait();   // that pass has completed (this launch may have started under it)
-      if (rank == 0) mbar_expect_tx(bars + 8 * kBarQ, 2 * kPfQBytes);
+  // f32 rows -> partial RoPE -> x scale * log2(e) -> f16 in the swizzled layout, warps 0-7. (A pre-pass
+  // that wrote rotated f16 queries for all heads cost its own 6 us and a second trip to memory:
+  // 15400 cycles from entry to the first S where this takes about 9000.)
+  if (warp < 8) {
+    const float *stage = reinterpret_cast<const float *>(smem_raw + kPfQBytes + kPfKTileBytes);
+    const int r = threadIdx.x & (kPfM - 1), h = threadIdx.x >> 7;
+    const uint32_t qrow = sQ + r * 128, swz = (uint32_t)(r & 7) << 4;   // (sub-tile 0: dims 0..63)
+    bool ok = true;
+    if (p.n_rot == 64) {
+      // Thread (row r, h): pairs 16 h .. 16 h + 15. The (cos, sin) while the rows are on their way, kept
+      // in the last two sub-tiles of Q (thread-private; those dims are converted after a barrier).
+      float2 *cs = reinterpret_cast<float2 *>(gQ + 2 * (kPfM * 128)) + threadIdx.x;
+      const float fpos = (float)my_pos;
+#pragma unroll 1
+      for (int i = 0; i < 16; i += 4) {
+        float2 v[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        tma_load_2d_pair(sQ + c * (kPfM * 128), &p.tm_q, head * kHeadDim + 64 * c, row0, lead + 8 * kBarQ);
-    }
-  } else if (warp < 8) {
-    // f32 rows -> x scale * log2(e) -> f16, warps 0-7, 16 rows each
+        for (int e = 0; e < 4; ++e) sincosf(fpos * p.freq[16 * h + i + e], &v[e].y, &v[e].x);
 #pragma unroll
-    for (int rr = 0; rr < 16; ++rr) {
-      const int r = warp * 16 + rr;      // row inside the tile
-      const uint32_t w0 = pack_h2(qa[rr].x * p.qscale, qa[rr].y * p.qscale);
-      const uint32_t w1 = pack_h2(qa[rr].z * p.qscale, qa[rr].w * p.qscale);
-      const uint32_t w2 = pack_h2(qb[rr].x * p.qscale, qb[rr].y * p.qscale);
-      const uint32_t w3 = pack_h2(qb[rr].z * p.qscale, qb[rr].w * p.qscale);
-      // lane = 16-byte chunk of the row: sub-tile lane/8, chunk lane%8, swizzled by the row
-      const uint32_t dst = sQ + (lane >> 3) * (kPfM * 128) + r * 128 + (((lane & 7) ^ (r & 7)) << 4);
-      sts128(dst, w0, w1, w2, w3);
+        for (int e = 0; e < 4; ++e) cs[(i + e) * 256] = v[e];
+      }
+      ok = mbar_wait(bars + 8 * kBarF, 0, p.status, 24);
+      if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int kk = (k + lane) & 3;   // four pairs; the lanes of a warp take them in turn (rows are 1 KB apart)
+        const float4 a = *reinterpret_cast<const float4 *>(stage + r * kHeadDim + 16 * h + 4 * kk);
+        const float4 b = *reinterpret_cast<const float4 *>(stage + r * kHeadDim + 32 + 16 * h + 4 * kk);
+        const float x0[4] = {a.x, a.y, a.z, a.w}, x1[4] = {b.x, b.y, b.z, b.w};
+        float y0[4], y1[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 c = cs[(4 * kk + e) * 256];
+          y0[e] = __fsub_rn(__fmul_rn(x0[e], c.x), __fmul_rn(x1[e], c.y)) * p.qscale;
+          y1[e] = __fadd_rn(__fmul_rn(x0[e], c.y), __fmul_rn(x1[e], c.x)) * p.qscale;
+        }
+        const uint32_t lo = (uint32_t)(2 * h + (kk >> 1)) << 4, hi = lo + 64, half = (kk & 1) * 8;
+        sts64(qrow + (lo ^ swz) + half, pack_h2(y0[0], y0[1]), pack_h2(y0[2], y0[3]));
+        sts64(qrow + (hi ^ swz) + half, pack_h2(y1[0], y1[1]), pack_h2(y1[2], y1[3]));
+      }
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+    } else {
+      ok = mbar_wait(bars + 8 * kBarF, 0, p.status, 24);
+      if (p.n_rot > 0) {   // other rotary sizes: value by value
+        auto put = [&](int d, float x) {
+          const unsigned short hx = __half_as_ushort(__float2half_rn(x * p.qscale));
+          asm volatile("st.shared.u16 [%0], %1;" ::"r"(qrow + (((uint32_t)(d >> 3) << 4) ^ swz) + 2 * (d & 7)), "h"(hx)
+                       : "memory");
+        };
+        const int nh = p.n_rot / 2;
+#pragma unroll 1
+        for (int d = h; d < nh; d += 2) {
+          float c, sn;
+          sincosf((float)my_pos * p.freq[d], &sn, &c);
+          const float x0 = stage[r * kHeadDim + d], x1 = stage[r * kHeadDim + d + nh];
+          put(d, __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, sn)));
+          put(d + nh, __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, c)));
+        }
+#pragma unroll 1
+        for (int d = p.n_rot + h; d < 64; d += 2) put(d, stage[r * kHeadDim + d]);
+      }
     }
-    fence_proxy_async();  // generic-proxy writes -> visible to the tensor core's async proxy
+    // the dims without rotation, a row per warp, four dims per lane
+    const int first = p.n_rot > 0 ? 16 : 0;
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int q4 = first + lane + 32 * m;
+      if (q4 < kHeadDim / 4) {
+#pragma unroll 8
+        for (int rr = warp; rr < kPfM; rr += 8) {
+          const float4 x = *reinterpret_cast<const float4 *>(stage + rr * kHeadDim + 4 * q4);
+          sts64(sQ + (q4 >> 4) * (kPfM * 128) + rr * 128 + (((uint32_t)((q4 >> 1) & 7) ^ (rr & 7)) << 4) + (q4 & 1) * 8,
+                pack_h2(x.x * p.qscale, x.y * p.qscale), pack_h2(x.z * p.qscale, x.w * p.qscale));
+        }
+      }
+    }
+    if (!ok) s_abort = 1;
+    fence_proxy_async();  // generic-proxy accesses before those of the tensor core and the copies
     __syncwarp();
-    if (lane == 0) mbar_arrive_cluster(lead + 8 * kBarQ);  // the S MMAs wait for all 16 warps
+    if (lane == 0) {
+      mbar_arrive_cluster(lead + 8 * kBarQ);  // the S MMAs wait for all 16 warps
+      mbar_arrive(bars + 8 * kBarC);
+    }
     if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 3);   // this warp's Q rows converted
   }
 
+  const bool with_gate = p.gate != nullptr && gridDim.z == 1;
   float l_run = 0.f;                 // softmax threads: row sum
   float m_ref = -1.0e30f;            //                  reference maximum (log2 units)
 
@@ -261,7 +324,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       if (p.kv_wait) pdl_wait();   // the pre-pass of this call appended rows to the caches
       int slot = 0, use = 0;
       for (int j = 0; j < nt; ++j) {
-        if (use > 0 && !mbar_wait(bars + 8 * (kBarKFree + slot), (use - 1) & 1, p.status, 11)) {
+        if (j == 1 ? !mbar_wait(bars + 8 * kBarC, 0, p.status, 25)   // the query rows have left slots 1 and 2
+                   : use > 0 && !mbar_wait(bars + 8 * (kBarKFree + slot), (use - 1) & 1, p.status, 11)) {
           s_abort = 1;
           break;
         }
@@ -277,14 +341,40 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         }
       }
     }
+    if (with_gate) {
+      // Q and the K ring are free once the last S has been computed: the gate rows come into them (128
+      // KB) under the last tile's softmax and P V. (Loaded to registers between the epilogue's
+      // stores, a few at a time, their latency was most of it: 15000 of 18000 cycles.)
+      // (lane 0 has waited for every earlier use of that K slot: a parity two uses old cannot pass)
+      if (lane == 0) {
+        const bool ok =
+            mbar_wait(bars + 8 * kBarC, 0, p.status, 26) &&
+            (nt == 0 ||
+             mbar_wait(bars + 8 * (kBarKFree + (nt - 1) % kPfKSlots), ((nt - 1) / kPfKSlots) & 1, p.status, 27));
+        if (ok) {
+          mbar_expect_tx(bars + 8 * kBarG, kPfRowsBytes);
+          tma_load_2d(sQ, &p.tm_g, head * kHeadDim, row0, bars + 8 * kBarG);
+        } else {
+          s_abort = 1;
+          mbar_arrive(bars + 8 * kBarG);   // nobody waits for long
+        }
+      }
+    }
   } else if (warp == 10) {
     // =============================== V producer ====================================
     // this CTA's half of tile j (128 of the 256 dims) into slot j % 2
+    if (with_gate && lane == 1) {
+      // the gate rows that the epilogue multiplies with, on their way to L2 once the queries have arrived
+      // (before, the two would share the memory's bandwidth and the queries come first)
+      mbar_wait(bars + 8 * kBarC, 0, nullptr, 0);
+      tma_prefetch_2d(&p.tm_g, head * kHeadDim, row0);
+    }
     if (lane == 0) {
       if (p.kv_wait) pdl_wait();
       for (int j = 0; j < nt; ++j) {
         const int slot = j & 1;
-        if (j >= 2 && !mbar_wait(bars + 8 * (kBarVFree + slot), ((j >> 1) - 1) & 1, p.status, 22)) {
+        if (j == 0 ? !mbar_wait(bars + 8 * kBarC, 0, p.status, 23)   // the query rows have left the slots
+                   : j >= 2 && !mbar_wait(bars + 8 * (kBarVFree + slot), ((j >> 1) - 1) & 1, p.status, 22)) {
           s_abort = 1;
           break;
         }
@@ -523,17 +613,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     tc_fence_after();
   }
 
-  // With the queries coming from the pre-pass, nothing may be stored before that pass has
-  // completed: o may alias q, which it is still reading. A CTA with key tiles knows this from
-  // its Q tile; one without (no row attends a key) waits for the tile here -- its TMA load was
-  // issued behind the dependency wait all the same.
-  if (p.q16 && nt == 0 && threadIdx.x == 0 && rank == 0 && !mbar_wait_cluster(bars + 8 * kBarQ, 0, p.status, 23))
-    s_abort = 1;
+  // A CTA without key tiles has copies of its query rows to wait for (they were converted by warps 0-7).
   cluster_sync();   // both CTAs are done with each other's barriers, shared and tensor memory
   const bool aborted = s_abort != 0;
   // the two sets' row sums, each with the reference it is expressed in: [set][sum,
-  // reference][row], over the K ring (every load into it has been consumed by now)
-  float (*s_fin)[2][kPfM] = reinterpret_cast<float (*)[2][kPfM]>(smem_raw + kPfQBytes);
+  // reference][row], over the third K slot (the gate rows lie in Q and the first two)
+  float (*s_fin)[2][kPfM] = reinterpret_cast<float (*)[2][kPfM]>(smem_raw + kPfQBytes + 2 * kPfKTileBytes);
   if (warp < 8) {
     s_fin[threadIdx.x >> 7][0][threadIdx.x & (kPfM - 1)] = l_run;
     s_fin[threadIdx.x >> 7][1][threadIdx.x & (kPfM - 1)] = m_ref;
@@ -542,7 +627,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 4);   // main loop done, sums exchanged
 
   // ---- epilogue: O / l (x sigmoid(gate)) -> global, 64 columns at a time ----
-  // staging tile [128 rows][64 floats] aliases the Q region; 16-byte chunk q of row r is
+  // staging tiles [128 rows][64 floats] lie over the V ring; 16-byte chunk q of row r is
   // stored at q ^ (r & 15), so both the row-wise writes and the coalesced reads are
   // conflict-free.
   if (warp < 8) {
@@ -563,8 +648,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       rec[0] = some ? m_fin * 0.6931471805599453f : -INFINITY;
       rec[1] = some ? l_tot : 0.f;
     }
-    const uint32_t stg = sQ + ch * (kPfM * 256);
-    uint8_t *gstg = gQ + ch * (kPfM * 256);
+    const uint32_t stg = sV + ch * (kPfM * 256);
+    uint8_t *gstg = gQ + (sV - sQ) + ch * (kPfM * 256);
     for (int cc = 0; cc < 2; ++cc) {
       const int c = 2 * cc + ch;
       uint32_t o[2][32];
@@ -582,6 +667,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
           w[e] = have ? __float_as_uint(__uint_as_float(o[hq][iq + e]) * inv) : 0u;
         sts128(stg + r * 256 + ((q ^ (r & 15)) << 4), w[0], w[1], w[2], w[3]);
       }
+      if (with_gate && cc == 0) mbar_wait(bars + 8 * kBarG, 0, p.status, 28);
       asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
       if (threadIdx.x == 0) RD_PF_TRACE(1, 47, 2 + cc);   // round cc staged
       // 128 threads: 8 rows x 16 chunks per pass
@@ -609,32 +695,18 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
                 *reinterpret_cast<const float4 *>(gstg + rr * 256 + ((q ^ (rr & 15)) << 4));
         }
       } else {
-        // the gate values of 4 passes are requested together before any store (out and gate
-        // may alias as far as the compiler knows, so it would otherwise wait for every load
-        // behind the previous store)
-        for (int p0 = 0; p0 < kPfM / 8; p0 += 4) {
-          float4 gv[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int rr = (p0 + k) * 8 + (gt >> 4), gr = row0 + rr;
-            gv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (gr < p.n_q)
-              gv[k] = *reinterpret_cast<const float4 *>(p.gate + ((size_t)gr * p.n_head + head) * kHeadDim +
-                                                        64 * c + 4 * (gt & 15));
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int rr = (p0 + k) * 8 + (gt >> 4), q = gt & 15;
-            const int gr = row0 + rr;
-            if (gr < p.n_q) {
-              float4 v = *reinterpret_cast<const float4 *>(gstg + rr * 256 + ((q ^ (rr & 15)) << 4));
-              // fast exp/divide: ~1e-6 relative, far inside the attention tolerance
-              v.x *= __fdividef(1.0f, 1.0f + __expf(-gv[k].x));
-              v.y *= __fdividef(1.0f, 1.0f + __expf(-gv[k].y));
-              v.z *= __fdividef(1.0f, 1.0f + __expf(-gv[k].z));
-              v.w *= __fdividef(1.0f, 1.0f + __expf(-gv[k].w));
-              *reinterpret_cast<float4 *>(p.out + ((size_t)gr * p.n_head + head) * kHeadDim + 64 * c + 4 * q) = v;
-            }
+#pragma unroll 4
+        for (int k = 0; k < kPfM / 8; ++k) {
+          const int rr = k * 8 + (gt >> 4), q = gt & 15, gr = row0 + rr;
+          if (gr < p.n_q) {
+            float4 v = *reinterpret_cast<const float4 *>(gstg + rr * 256 + ((q ^ (rr & 15)) << 4));
+            const float4 g = *reinterpret_cast<const float4 *>(gQ + rr * (kHeadDim * 4) + 256 * c + 16 * q);
+            // fast exp/divide: ~1e-6 relative, far inside the attention tolerance
+            v.x *= __fdividef(1.0f, 1.0f + __expf(-g.x));
+            v.y *= __fdividef(1.0f, 1.0f + __expf(-g.y));
+            v.z *= __fdividef(1.0f, 1.0f + __expf(-g.z));
+            v.w *= __fdividef(1.0f, 1.0f + __expf(-g.w));
+            *reinterpret_cast<float4 *>(p.out + ((size_t)gr * p.n_head + head) * kHeadDim + 64 * c + 4 * q) = v;
           }
         }
       }
@@ -710,98 +782,57 @@ prefill_merge_kernel(const float *__restrict__ records, float *__restrict__ out,
   *reinterpret_cast<float4 *>(out + (size_t)row * kHeadDim + 4 * tx) = o;
 }
 
-// Query pre-pass of the rotating prefill: one block per token. (cos, sin) of pos[t] * freq[i]
-// once per rotated pair (24 heads share them), then every head row: partial RoPE in f32 with
-// the operation order of the K side, x scale * log2(e), rounded to f16 -- [n_q][n_head][256]
-// f16, the layout the tile kernel's TMA boxes read. The tile kernel is launched directly
-// after it as a programmatic dependent launch.
+// Fused append: one block per token, a warp per K or V row. The K rows are rotated with the operation
+// order of kv_append_kernel, both are rounded to f16 -- the bytes rd_kv_append stores for f16
+// caches. The tile kernel is launched under it as a programmatic dependent launch.
 __global__ void __launch_bounds__(256)
-q_prep_kernel(const float *__restrict__ q, const int32_t *__restrict__ pos, int n_head, int n_rot, float qscale,
-              uint4 *__restrict__ q16, const float *__restrict__ k_new, const float *__restrict__ v_new,
-              uint4 *__restrict__ k_dst, uint4 *__restrict__ v_dst, int nkv,
-              const __grid_constant__ RopeTable tab) {
+kv_prep_kernel(const int32_t *__restrict__ pos, int n_rot, const float *__restrict__ k_new,
+               const float *__restrict__ v_new, uint4 *__restrict__ k_dst, uint4 *__restrict__ v_dst, int nkv,
+               const float *q, const float *gate, int n_head, const __grid_constant__ RopeTable tab) {
   __shared__ float2 s_cs[32];
-  // the wait comes first: the tile kernel, launched under this pass, loads cache rows that
-  // earlier kernels wrote without waiting for this one
+  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // This launch starts under the one before it: the token's query and gate rows can be on their way to L2
+  // before that one is done (L2 is where its writes arrive, too; nothing is read here).
+  if (q != nullptr && threadIdx.x == 0) bulk_prefetch_l2(q + (size_t)t * n_head * kHeadDim, n_head * kHeadDim * 4);
+  if (q != nullptr && gate != nullptr && threadIdx.x == 32)
+    bulk_prefetch_l2(gate + (size_t)t * n_head * kHeadDim, n_head * kHeadDim * 4);
+  // the wait comes first: the tile kernel reads what earlier kernels wrote without waiting for this one
   pdl_wait();
   pdl_launch_dependents();
-  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pairs = n_rot / 2;
-  // a warp has at most three head rows (n_head <= 24): requested before the table is
-  // computed, so that their latency and the sincosf run side by side
-  float4 pa[3], pb[3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const int head = warp + 8 * j;
-    pa[j] = pb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (head < n_head) {
-      const float4 *src = reinterpret_cast<const float4 *>(q + ((size_t)t * n_head + head) * kHeadDim);
-      pa[j] = src[2 * lane];
-      pb[j] = src[2 * lane + 1];
-    }
+  const bool is_k = warp < nkv;
+  const size_t row = (size_t)t * nkv + (is_k ? warp : warp - nkv);
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+  if (warp < 2 * nkv) {   // requested before the table is computed
+    const float4 *src = reinterpret_cast<const float4 *>((is_k ? k_new : v_new) + row * kHeadDim);
+    a = src[2 * lane];
+    b = src[2 * lane + 1];
   }
-  // ... and, with a fused append, the warp's K or V row of the token (2 * nkv <= 8 rows)
-  float4 ka = make_float4(0.f, 0.f, 0.f, 0.f), kb = ka;
-  if (k_new != nullptr && warp < 2 * nkv) {
-    const float4 *src = reinterpret_cast<const float4 *>((warp < nkv ? k_new : v_new) +
-                                                         ((size_t)t * nkv + (warp < nkv ? warp : warp - nkv)) * kHeadDim);
-    ka = src[2 * lane];
-    kb = src[2 * lane + 1];
-  }
-  if ((int)threadIdx.x < pairs) {
+  if ((int)threadIdx.x < n_rot / 2) {
     float c, s;
     sincosf((float)pos[t] * tab.f[threadIdx.x], &s, &c);
     s_cs[threadIdx.x] = make_float2(c, s);
   }
   __syncthreads();
-  // lanes 0..(n_rot/8 - 1) hold the rotated dims; dims d and d + n_rot/2 sit in lanes l and
-  // l ^ (n_rot/16) at the same element index
-  const int half_lanes = n_rot / 16;
-  const bool rot = lane < 2 * half_lanes, lo = lane < half_lanes;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const int head = warp + 8 * j;
-    if (head >= n_head) break;
-    const size_t row = (size_t)t * n_head + head;
-    const float4 a = pa[j], b = pb[j];
-    float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  if (warp >= 2 * nkv) return;
+  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  if (is_k && n_rot > 0) {
+    // lanes 0 .. n_rot / 8 - 1 hold the rotated dims; dims d and d + n_rot / 2 sit n_rot / 16 lanes apart
+    const int half_lanes = n_rot / 16;
+    const bool rot = lane < 2 * half_lanes, lo = lane < half_lanes;
+    const int src = !rot ? lane : lo ? lane + half_lanes : lane - half_lanes;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float other = __shfl_xor_sync(0xffffffffu, v[i], half_lanes);
+      const float other = __shfl_sync(0xffffffffu, v[i], src);
       if (rot) {
         const float2 cs = s_cs[8 * (lo ? lane : lane - half_lanes) + i];
         v[i] = lo ? __fsub_rn(__fmul_rn(v[i], cs.x), __fmul_rn(other, cs.y))
                   : __fadd_rn(__fmul_rn(other, cs.y), __fmul_rn(v[i], cs.x));
       }
     }
-    q16[row * 32 + lane] = make_uint4(pack_h2(v[0] * qscale, v[1] * qscale), pack_h2(v[2] * qscale, v[3] * qscale),
-                                      pack_h2(v[4] * qscale, v[5] * qscale), pack_h2(v[6] * qscale, v[7] * qscale));
   }
-  // Fused append (k_new != nullptr): the token's K rows, rotated with the same (cos, sin) and
-  // the operation order of kv_append_kernel, and its V rows, rounded to f16 into cache row t
-  // -- the bytes rd_kv_append stores for f16 caches.
-  if (k_new == nullptr || warp >= 2 * nkv) return;
-  {
-    const int r = warp;
-    const bool is_k = r < nkv;
-    const size_t row = (size_t)t * nkv + (is_k ? r : r - nkv);
-    float v[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
-    if (is_k) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float other = __shfl_xor_sync(0xffffffffu, v[i], half_lanes);
-        if (rot) {
-          const float2 cs = s_cs[8 * (lo ? lane : lane - half_lanes) + i];
-          v[i] = lo ? __fsub_rn(__fmul_rn(v[i], cs.x), __fmul_rn(other, cs.y))
-                    : __fadd_rn(__fmul_rn(other, cs.y), __fmul_rn(v[i], cs.x));
-        }
-      }
-    }
-    (is_k ? k_dst : v_dst)[row * 32 + lane] =
-        make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
-  }
+  (is_k ? k_dst : v_dst)[row * 32 + lane] =
+      make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
 }
-size_t prefill_rope_bytes(int n_q, int n_head) { return (size_t)n_q * n_head * kHeadDim * 2; }
 
 // Key splits that fill the GPU, picked with a three-constant cost model measured on B200:
 // a key tile costs a CTA about 2 us, a CTA's prologue + epilogue about 9 us (the query
@@ -839,7 +870,7 @@ size_t prefill_record_bytes(int n_q, int n_head, int splits) {
 int launch_prefill(const float *q, const void *k, const void *v, float *out, const float *gate,
                    const int32_t *pos, int n_q, int keys_total, int n_head, int n_head_kv, float scale,
                    int n_rot, float freq_base, DeviceStatus *status, float *records, int n_splits,
-                   void *q16, const float *k_new, const float *v_new, void *k_dst, void *v_dst,
+                   const float *k_new, const float *v_new, void *k_dst, void *v_dst, bool kv_pending,
                    cudaStream_t st) {
   PrefillArgs a;
   memset(&a, 0, sizeof(a));
@@ -855,13 +886,11 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   a.n_head = n_head;
   a.nkv = n_head_kv;
   a.qscale = scale * 1.4426950408889634f;
-  const bool prepass = n_rot > 0 || k_new != nullptr;   // rotation and / or fused append
-  a.q16 = prepass ? 1 : 0;
-  a.kv_wait = k_new != nullptr ? 1 : 0;
-  if (prepass) {
-    if (q16 == nullptr) return RD_ERR_WORKSPACE;
-    if ((rc = encode_f16_tmap(&a.tm_q, q16, n_head, n_q, kPfM)) != RD_OK) return rc;
-  }
+  if ((rc = encode_f32_tmap(&a.tm_q, q, n_head, n_q, kPfM)) != RD_OK) return rc;
+  if (gate != nullptr && (rc = encode_f32_tmap(&a.tm_g, gate, n_head, n_q, kPfM)) != RD_OK) return rc;
+  a.n_rot = n_rot;
+  if (n_rot > 0) memcpy(a.freq, make_rope_table(n_rot, freq_base).f, sizeof(a.freq));
+  a.kv_wait = k_new != nullptr || kv_pending ? 1 : 0;
   a.status = status;
   a.debug = 0;
 #ifdef RD_TIMING_SWITCHES
@@ -878,10 +907,11 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   }
   if (n_splits < 1 || records == nullptr) n_splits = 1;
   a.records = records;
-  if (prepass) {
-    // (a pass of many waves gains nothing from starting early: measured 1.8 % slower at 8192 tokens)
-    if (launch_pdl(n_q <= 1024 ? 8 : 0, q_prep_kernel, dim3((unsigned)n_q), dim3(256), 0, st, q, pos, n_head, n_rot, a.qscale,
-                   (uint4 *)q16, k_new, v_new, (uint4 *)k_dst, (uint4 *)v_dst, n_head_kv,
+  if (k_new != nullptr) {
+    // (a pass of many waves gains nothing from starting early)
+    const bool early = n_q <= 1024;
+    if (launch_pdl(early ? 8 : 0, kv_prep_kernel, dim3((unsigned)n_q), dim3(256), 0, st, pos, n_rot, k_new, v_new,
+                   (uint4 *)k_dst, (uint4 *)v_dst, n_head_kv, early ? q : nullptr, gate, n_head,
                    make_rope_table(n_rot, freq_base)) != cudaSuccess)
       return RD_ERR_CUDA;
   }
@@ -895,12 +925,11 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  // under the pre-pass the tile kernel may start early: it waits for it (griddepcontrol)
-  // before it loads its Q tile
+  // starts under the launch before it, see PrefillArgs::kv_wait
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = prepass ? 2 : 1;
+  cfg.numAttrs = 2;
   if (cudaLaunchKernelEx(&cfg, prefill_kernel, a) != cudaSuccess) return RD_ERR_CUDA;
   if (n_splits > 1) {
     const int64_t n_rows = (int64_t)n_q * n_head;

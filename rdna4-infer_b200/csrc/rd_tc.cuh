@@ -161,6 +161,10 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, ui
                : "memory");
 }
 
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+
 // Shared-memory matrix descriptor without swizzle (descriptor version 1): core matrices of
 // 8 rows x 16 bytes, 128 contiguous bytes each. K-major operand: LBO = bytes between core
 // matrices adjacent along K, SBO = bytes between 8-row groups along M/N. MN-major operand:
