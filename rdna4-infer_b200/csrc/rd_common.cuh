@@ -219,6 +219,11 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 // Packed pairs of f32 (sm_100 add.f32x2 / fma.rn.f32x2: two lanes per instruction).
 __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
   unsigned long long r;
@@ -339,7 +344,13 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
-// The same box to L2 only.
+// shared -> global: rows and columns outside the tensor are not written; completion by bulk groups.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src_smem, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
+               "r"(src_smem), "r"(x), "r"(y)
+               : "memory");
+}
+// A box of global memory to L2 only.
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }

@@ -154,7 +154,8 @@ int encode_kv_tmap(void *tmap_out, const void *base, int type, int n_head_kv, in
 // with SWIZZLE_128B read).
 int encode_f16_tmap(void *tmap_out, const void *base, int n_head_kv, int64_t n_rows, int tile_rows);
 
-// Tensor map over f32 activations [n_rows][n_head * 256] with a box of [tile_rows][one head], no swizzle.
+// Tensor map over f32 activations [n_rows][n_head * 256] with a box of [tile_rows][32 dims] and the
+// hardware 128-byte swizzle.
 int encode_f32_tmap(void *tmap_out, const void *base, int n_head, int64_t n_rows, int tile_rows);
 
 // ---- rd_prefill.cu

@@ -26,8 +26,7 @@
 //                f16 and O in TMEM is rarely touched), P -> f16 pairs, tcgen05.st
 //     warp 11    O += P V_j          8 x tcgen05.mma M256 N256 K16 (A = P from TMEM, B = V
 //                                   MN-major)
-//   epilogue   O / l (times sigmoid(gate) if asked) through a swizzled staging tile to
-//              coalesced f32 stores.
+//   epilogue   O / l (times sigmoid(gate) if asked) through shared memory to TMA stores.
 // Warps 8 and 10 are the K and V TMA producers (separate warps: a lane parked in
 // mbarrier.try_wait parks its whole warp). The two contractions have their own issuing
 // threads because issuing a tcgen05.mma costs the issuing thread tens of cycles.
@@ -81,7 +80,8 @@ constexpr int kPfVTileBytes = 2 * kPfVChunkBytes;          // 32768
 constexpr int kPfVSlots = 2;
 // 224 KB of dynamic shared memory + < 3 KB static = the 227 KB an sm_100 CTA may use
 constexpr int kPfSmemBytes = kPfQBytes + kPfKSlots * kPfKTileBytes + kPfVSlots * kPfVTileBytes;
-constexpr int kPfRowsBytes = kPfM * kHeadDim * 4;          // a tile of f32 query or gate rows: 128 KB
+constexpr int kPfRowsBytes = kPfM * kHeadDim * 4;          // a tile of f32 gate or output rows: 128 KB
+constexpr int kPfBoxBytes = kPfM * 128;                    // [128 rows][32 dims] of it
 constexpr int kPfThreads = 384;           // 8 softmax warps, K TMA, S MMA, V TMA, PV MMA warps
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemO = 0;            // columns [0, 256): output accumulator
@@ -101,8 +101,8 @@ struct PrefillArgs {
   int n_head;
   int nkv;
   float qscale;          // scale * log2(e)
-  alignas(64) CUtensorMap tm_q;  // f32 rows of `q` and `gate`: boxes of [128 tokens][one head]
-  alignas(64) CUtensorMap tm_g;
+  alignas(64) CUtensorMap tm_g;  // f32 rows of `gate` and `out`: boxes of [128 tokens][32 dims], 128-byte swizzle
+  alignas(64) CUtensorMap tm_o;
   int n_rot;             // partial RoPE of the queries: dims [0, n_rot), pairs (d, d + n_rot / 2)
   float freq[32];        // rotation frequencies of the pairs
   int kv_wait;           // 1: the launch before this one (which waited for everything before it) stores cache
@@ -120,11 +120,11 @@ struct PrefillArgs {
 // In the leader (CTA 0 of the pair) alone: KFull, VFull, Q, P, L -- what its issuing threads wait for, from
 // both CTAs. In each CTA: KFree, VFree, S, O (tcgen05.commit arrives on both), R.
 enum { kBarKFull = 0, kBarKFree = 6, kBarVFull = 12, kBarVFree = 14, kBarS = 16, kBarP = 18, kBarO = 22,
-       kBarQ = 24, kBarR = 25, kBarL = 33, kBarC = 34, kBarF = 35, kBarG = 36, kBarCount = 37 };   // kBarP: [P buffer][64-key half of P];
+       kBarQ = 24, kBarR = 25, kBarL = 33, kBarC = 34, kBarG = 35, kBarT = 36, kBarCount = 37 };   // kBarP: [P buffer][64-key half of P];
                                                    // kBarR: [warp pair 0..3][tile parity];
                                                    // kBarL: the scores of a tile are in registers;
-                                                   // kBarF: the f32 query rows have arrived;
-                                                   // kBarC: they are converted (their staging is free);
+                                                   // kBarC: the queries are converted;
+                                                   // kBarT: the (cos, sin) of the tile's rows are there;
                                                    // kBarG: the gate rows are in shared memory
 
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_constant__ PrefillArgs p) {
@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_maxpos;
   __shared__ int s_abort;
+  __shared__ int s_pos[kPfM];
   __shared__ float s_ref[2][kPfM];     // [tile parity][row]: the reference maximum that tile left
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -159,20 +160,31 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   const uint32_t bars = smem_u32(s_bars), lead = cluster_addr(bars, 0);   // this CTA's barriers, the leader's
 
   // Requested first, so that their latency runs under the set-up below: the positions of this tile's
-  // rows and its f32 query rows, into K slots 1 and 2 and both V slots (128 KB that the pipeline needs
-  // last). One tensor-map box: a bulk copy per row took 57 cycles each to issue, 7300 for the tile.
+  // rows and half of the warp's 16 query rows (the other half: to L2).
   int my_pos = -1;
+  float4 xa[8], xb[8];   // dims 4 lane .. + 3 and 128 + 4 lane .. + 3 of a row
+  const float *qw = p.q + ((size_t)(row0 + warp * 16) * p.n_head + head) * kHeadDim;
+  const size_t q_row = (size_t)p.n_head * kHeadDim;
+  const int rows_w = p.n_q - row0 - warp * 16;   // of the warp's rows, how many exist
+  auto load_rows = [&](int first) {
+#pragma unroll
+    for (int rr = 0; rr < 8; ++rr) {
+      xa[rr] = xb[rr] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (first + rr < rows_w) {
+        const float4 *src = reinterpret_cast<const float4 *>(qw + (first + rr) * q_row);
+        xa[rr] = src[lane];
+        xb[rr] = src[lane + 32];
+      }
+    }
+  };
   if (threadIdx.x < 2 * kPfM) {
     const int r = row0 + (threadIdx.x & (kPfM - 1));
     if (r < p.n_q) my_pos = p.pos[r];
-  }
-  const uint32_t sStage = sK + kPfKTileBytes;
-  if (warp == 10) {
-    if (lane == 0) {
-      mbar_init(bars + 8 * kBarF, 1);
-      fence_barrier_init();
-      mbar_expect_tx(bars + 8 * kBarF, kPfRowsBytes);   // (rows past n_q come as zeros)
-      tma_load_2d(sStage, &p.tm_q, head * kHeadDim, row0, bars + 8 * kBarF);
+    load_rows(0);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {   // 8 rows x 8 lines of 128 bytes
+      const int rr = 8 + (lane >> 3) + 4 * e;
+      if (rr < rows_w) asm volatile("prefetch.global.L2 [%0];" ::"l"(qw + rr * q_row + 32 * (lane & 7)));
     }
   }
 
@@ -194,6 +206,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     for (int i = 0; i < 8; ++i) mbar_init(bars + 8 * (kBarR + i), 1);
     mbar_init(bars + 8 * kBarL, 8);
     mbar_init(bars + 8 * kBarQ, 16);   // one per converting warp (both CTAs)
+    mbar_init(bars + 8 * kBarT, 16);
     mbar_init(bars + 8 * kBarC, 8);
     mbar_init(bars + 8 * kBarG, 1);
     fence_barrier_init();
@@ -211,6 +224,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   // ---- the last key any row of this tile attends ----
   if (threadIdx.x < kPfM) {
     int mx = my_pos;
+    s_pos[threadIdx.x] = my_pos;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) atomicMax(&s_maxpos, mx);
@@ -227,49 +241,96 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
 
   // ---- prologue: the Q tile as f16 in the swizzled K-major layout ----
   // f32 rows -> partial RoPE -> x scale * log2(e) -> f16 in the swizzled layout, warps 0-7. (A pre-pass
-  // that wrote rotated f16 queries for all heads cost its own 6 us and a second trip to memory:
-  // 15400 cycles from entry to the first S where this takes about 9000.)
+  // that wrote rotated f16 queries for all heads cost its own 6 us and a second trip to memory: 15400
+  // cycles from entry to the first S; the f32 rows by bulk copies or a tensor-map box: 13300; here XX.)
   if (warp < 8) {
-    const float *stage = reinterpret_cast<const float *>(smem_raw + kPfQBytes + kPfKTileBytes);
+    // thread (row r, h) rotates dims 0..63 of its row; they pass through V slot 1 as f32, 16-byte chunk q of
+    // a row at q ^ (r & 15)
+    float *stage = reinterpret_cast<float *>(gQ + (sV - sQ) + kPfVTileBytes);
     const int r = threadIdx.x & (kPfM - 1), h = threadIdx.x >> 7;
     const uint32_t qrow = sQ + r * 128, swz = (uint32_t)(r & 7) << 4;   // (sub-tile 0: dims 0..63)
-    bool ok = true;
+    // four dims of a row: sub-tile q4 / 16, 16-byte chunk q4 / 2, half q4 & 1
+    auto put4 = [&](int rr, int q4, const float4 &x) {
+      sts64(sQ + (q4 >> 4) * (kPfM * 128) + rr * 128 + (((uint32_t)((q4 >> 1) & 7) ^ (rr & 7)) << 4) + (q4 & 1) * 8,
+            pack_h2(x.x * p.qscale, x.y * p.qscale), pack_h2(x.z * p.qscale, x.w * p.qscale));
+    };
+    auto convert = [&](int first) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) put4(warp * 16 + first + k, lane + 32, xb[k]);
+      if (p.n_rot > 0 && lane < 16) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int rr = warp * 16 + first + k;
+          *reinterpret_cast<float4 *>(stage + rr * 64 + ((lane ^ (rr & 15)) << 2)) = xa[k];
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) put4(warp * 16 + first + k, lane, xa[k]);
+      }
+    };
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 2);
+    convert(0);
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 3);
+    load_rows(8);
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 4);
+    // (cos, sin) of all rows and pairs, while those are on their way: the two CTAs of the pair serve the same
+    // tokens, each computes 64 rows for both (16 sincosf per thread took 4200 cycles). [pair][row] in V slot 0.
+    const uint32_t cs0 = sV;
+    const float *cs = reinterpret_cast<const float *>(gQ + (sV - sQ));
     if (p.n_rot == 64) {
-      // Thread (row r, h): pairs 16 h .. 16 h + 15. The (cos, sin) while the rows are on their way, kept
-      // in the last two sub-tiles of Q (thread-private; those dims are converted after a barrier).
-      float2 *cs = reinterpret_cast<float2 *>(gQ + 2 * (kPfM * 128)) + threadIdx.x;
-      const float fpos = (float)my_pos;
+      const int tr = (int)rank * 64 + (threadIdx.x & 63), tp = (threadIdx.x >> 6) * 8;   // row, first of 8 pairs
+      const float fpos = (float)s_pos[tr];
+      const uint32_t peer = cluster_addr(cs0, rank ^ 1);
 #pragma unroll 1
-      for (int i = 0; i < 16; i += 4) {
+      for (int i = 0; i < 8; i += 4) {
         float2 v[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sincosf(fpos * p.freq[16 * h + i + e], &v[e].y, &v[e].x);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) cs[(i + e) * 256] = v[e];
-      }
-      ok = mbar_wait(bars + 8 * kBarF, 0, p.status, 24);
-      if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 0);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int kk = (k + lane) & 3;   // four pairs; the lanes of a warp take them in turn (rows are 1 KB apart)
-        const float4 a = *reinterpret_cast<const float4 *>(stage + r * kHeadDim + 16 * h + 4 * kk);
-        const float4 b = *reinterpret_cast<const float4 *>(stage + r * kHeadDim + 32 + 16 * h + 4 * kk);
-        const float x0[4] = {a.x, a.y, a.z, a.w}, x1[4] = {b.x, b.y, b.z, b.w};
-        float y0[4], y1[4];
+        for (int e = 0; e < 4; ++e) sincosf(fpos * p.freq[tp + i + e], &v[e].y, &v[e].x);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 c = cs[(4 * kk + e) * 256];
-          y0[e] = __fsub_rn(__fmul_rn(x0[e], c.x), __fmul_rn(x1[e], c.y)) * p.qscale;
-          y1[e] = __fadd_rn(__fmul_rn(x0[e], c.y), __fmul_rn(x1[e], c.x)) * p.qscale;
+          const uint32_t at = 8u * ((tp + i + e) * kPfM + tr);
+          sts64(cs0 + at, __float_as_uint(v[e].x), __float_as_uint(v[e].y));
+          asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(peer + at), "f"(v[e].x), "f"(v[e].y) : "memory");
         }
-        const uint32_t lo = (uint32_t)(2 * h + (kk >> 1)) << 4, hi = lo + 64, half = (kk & 1) * 8;
-        sts64(qrow + (lo ^ swz) + half, pack_h2(y0[0], y0[1]), pack_h2(y0[2], y0[3]));
-        sts64(qrow + (hi ^ swz) + half, pack_h2(y1[0], y1[1]), pack_h2(y1[2], y1[3]));
       }
+      __syncwarp();
+      if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 5);
+      if (lane == 0) {
+        mbar_arrive_cluster(cluster_addr(bars + 8 * kBarT, 0));
+        mbar_arrive_cluster(cluster_addr(bars + 8 * kBarT, 1));
+      }
+    }
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 0);
+    convert(8);
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 1);
+    if (p.n_rot > 0) {
+      if (p.n_rot == 64 && !mbar_wait_cluster(bars + 8 * kBarT, 0, p.status, 24)) s_abort = 1;
       asm volatile("bar.sync 2, 256;" ::: "memory");
-    } else {
-      ok = mbar_wait(bars + 8 * kBarF, 0, p.status, 24);
-      if (p.n_rot > 0) {   // other rotary sizes: value by value
+      auto chunk = [&](int q) { return *reinterpret_cast<const float4 *>(stage + r * 64 + ((q ^ (r & 15)) << 2)); };
+      if (p.n_rot == 64) {
+        float4 ca[4], cb[4];
+        float2 cc[16];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ca[k] = chunk(4 * h + k), cb[k] = chunk(8 + 4 * h + k);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) cc[e] = reinterpret_cast<const float2 *>(cs)[(16 * h + e) * kPfM + r];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {   // four pairs
+          const float4 a = ca[k], b = cb[k];
+          const float x0[4] = {a.x, a.y, a.z, a.w}, x1[4] = {b.x, b.y, b.z, b.w};
+          float y0[4], y1[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 c = cc[4 * k + e];
+            y0[e] = __fsub_rn(__fmul_rn(x0[e], c.x), __fmul_rn(x1[e], c.y)) * p.qscale;
+            y1[e] = __fadd_rn(__fmul_rn(x0[e], c.y), __fmul_rn(x1[e], c.x)) * p.qscale;
+          }
+          const uint32_t lo = (uint32_t)(2 * h + (k >> 1)) << 4, hi = lo + 64, half = (k & 1) * 8;
+          sts64(qrow + (lo ^ swz) + half, pack_h2(y0[0], y0[1]), pack_h2(y0[2], y0[3]));
+          sts64(qrow + (hi ^ swz) + half, pack_h2(y1[0], y1[1]), pack_h2(y1[2], y1[3]));
+        }
+      } else {   // other rotary sizes: value by value
+        auto get = [&](int d) { return stage[r * 64 + (((d >> 2) ^ (r & 15)) << 2) + (d & 3)]; };
         auto put = [&](int d, float x) {
           const unsigned short hx = __half_as_ushort(__float2half_rn(x * p.qscale));
           asm volatile("st.shared.u16 [%0], %1;" ::"r"(qrow + (((uint32_t)(d >> 3) << 4) ^ swz) + 2 * (d & 7)), "h"(hx)
@@ -280,33 +341,18 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         for (int d = h; d < nh; d += 2) {
           float c, sn;
           sincosf((float)my_pos * p.freq[d], &sn, &c);
-          const float x0 = stage[r * kHeadDim + d], x1 = stage[r * kHeadDim + d + nh];
+          const float x0 = get(d), x1 = get(d + nh);
           put(d, __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, sn)));
           put(d + nh, __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, c)));
         }
 #pragma unroll 1
-        for (int d = p.n_rot + h; d < 64; d += 2) put(d, stage[r * kHeadDim + d]);
+        for (int d = p.n_rot + h; d < 64; d += 2) put(d, get(d));
       }
     }
-    // the dims without rotation, a row per warp, four dims per lane
-    const int first = p.n_rot > 0 ? 16 : 0;
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const int q4 = first + lane + 32 * m;
-      if (q4 < kHeadDim / 4) {
-#pragma unroll 8
-        for (int rr = warp; rr < kPfM; rr += 8) {
-          const float4 x = *reinterpret_cast<const float4 *>(stage + rr * kHeadDim + 4 * q4);
-          sts64(sQ + (q4 >> 4) * (kPfM * 128) + rr * 128 + (((uint32_t)((q4 >> 1) & 7) ^ (rr & 7)) << 4) + (q4 & 1) * 8,
-                pack_h2(x.x * p.qscale, x.y * p.qscale), pack_h2(x.z * p.qscale, x.w * p.qscale));
-        }
-      }
-    }
-    if (!ok) s_abort = 1;
     fence_proxy_async();  // generic-proxy accesses before those of the tensor core and the copies
     __syncwarp();
     if (lane == 0) {
-      mbar_arrive_cluster(lead + 8 * kBarQ);  // the S MMAs wait for all 16 warps
+      mbar_arrive_peer(lead + 8 * kBarQ);   // the S MMAs wait for all 16 warps
       mbar_arrive(bars + 8 * kBarC);
     }
     if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 3);   // this warp's Q rows converted
@@ -324,8 +370,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       if (p.kv_wait) pdl_wait();   // the pre-pass of this call appended rows to the caches
       int slot = 0, use = 0;
       for (int j = 0; j < nt; ++j) {
-        if (j == 1 ? !mbar_wait(bars + 8 * kBarC, 0, p.status, 25)   // the query rows have left slots 1 and 2
-                   : use > 0 && !mbar_wait(bars + 8 * (kBarKFree + slot), (use - 1) & 1, p.status, 11)) {
+        if (use > 0 && !mbar_wait(bars + 8 * (kBarKFree + slot), (use - 1) & 1, p.status, 11)) {
           s_abort = 1;
           break;
         }
@@ -353,7 +398,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
              mbar_wait(bars + 8 * (kBarKFree + (nt - 1) % kPfKSlots), ((nt - 1) / kPfKSlots) & 1, p.status, 27));
         if (ok) {
           mbar_expect_tx(bars + 8 * kBarG, kPfRowsBytes);
-          tma_load_2d(sQ, &p.tm_g, head * kHeadDim, row0, bars + 8 * kBarG);
+          for (int c = 0; c < 8; ++c)
+            tma_load_2d(sQ + c * kPfBoxBytes, &p.tm_g, head * kHeadDim + 32 * c, row0, bars + 8 * kBarG);
         } else {
           s_abort = 1;
           mbar_arrive(bars + 8 * kBarG);   // nobody waits for long
@@ -367,13 +413,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       // the gate rows that the epilogue multiplies with, on their way to L2 once the queries have arrived
       // (before, the two would share the memory's bandwidth and the queries come first)
       mbar_wait(bars + 8 * kBarC, 0, nullptr, 0);
-      tma_prefetch_2d(&p.tm_g, head * kHeadDim, row0);
+      for (int c = 0; c < 8; ++c) tma_prefetch_2d(&p.tm_g, head * kHeadDim + 32 * c, row0);
     }
     if (lane == 0) {
       if (p.kv_wait) pdl_wait();
       for (int j = 0; j < nt; ++j) {
         const int slot = j & 1;
-        if (j == 0 ? !mbar_wait(bars + 8 * kBarC, 0, p.status, 23)   // the query rows have left the slots
+        if (j == 0 ? !mbar_wait(bars + 8 * kBarC, 0, p.status, 23)   // the query conversion has left the slots
                    : j >= 2 && !mbar_wait(bars + 8 * (kBarVFree + slot), ((j >> 1) - 1) & 1, p.status, 22)) {
           s_abort = 1;
           break;
@@ -394,7 +440,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       // every address here is below 256 KB), so each one is a base plus a constant.
       const uint64_t dq = smem_desc(sQ, 16, 1024);
       const uint64_t dk = smem_desc(sK, 16, 1024);
-      bool ok = mbar_wait_cluster(bars + 8 * kBarQ, 0, p.status, 18);  // both Q tiles are there
+      bool ok = mbar_wait(bars + 8 * kBarQ, 0, p.status, 18);  // both Q tiles are there
       tc_fence_after();
       int slot = 0, use = 0;
       for (int j = 0; j < nt && ok; ++j) {
@@ -613,7 +659,6 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     tc_fence_after();
   }
 
-  // A CTA without key tiles has copies of its query rows to wait for (they were converted by warps 0-7).
   cluster_sync();   // both CTAs are done with each other's barriers, shared and tensor memory
   const bool aborted = s_abort != 0;
   // the two sets' row sums, each with the reference it is expressed in: [set][sum,
@@ -626,7 +671,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   __syncthreads();
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 4);   // main loop done, sums exchanged
 
-  // ---- epilogue: O / l (x sigmoid(gate)) -> global, 64 columns at a time ----
+  // ---- epilogue ----
+  // Key splits: un-normalised records -> global, 64 columns at a time.
   // staging tiles [128 rows][64 floats] lie over the V ring; 16-byte chunk q of row r is
   // stored at q ^ (r & 15), so both the row-wise writes and the coalesced reads are
   // conflict-free.
@@ -648,9 +694,62 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       rec[0] = some ? m_fin * 0.6931471805599453f : -INFINITY;
       rec[1] = some ? l_tot : 0.f;
     }
+    if (!rec_mode) {
+      // O / l (x sigmoid(gate)) in place over the gate rows, 32 columns (a box of 128-byte swizzled rows)
+      // at a time, each box stored by TMA while the next is computed. What bounds it: the 32 bytes a
+      // cycle that an SM writes (4096 cycles) and 1.5 special functions per gate value (3072).
+      if (with_gate) mbar_wait(bars + 8 * kBarG, 0, p.status, 28);
+#pragma unroll 1
+      for (int b = ch; b < 8; b += 2) {
+        uint32_t o[32];
+        if (have) {
+          tmem_ld32(lane_addr + kTmemO + 32 * b, o);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = 0u;
+        }
+        const uint32_t brow = sQ + b * kPfBoxBytes + r * 128;
+        if (with_gate) {
+          // (branch-free from here to the stores: 32 independent chains)
+          float g[32];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint4 x = lds128(brow + ((uint32_t)(q ^ (r & 7)) << 4));
+            g[4 * q] = __uint_as_float(x.x);
+            g[4 * q + 1] = __uint_as_float(x.y);
+            g[4 * q + 2] = __uint_as_float(x.z);
+            g[4 * q + 3] = __uint_as_float(x.w);
+          }
+          // one reciprocal for two values; e^-g is capped at 2^60. Approximate exp and reciprocal: ~1e-6 relative
+#pragma unroll
+          for (int e = 0; e < 32; ++e) g[e] = 1.0f + ex2(fminf(g[e] * -1.4426950408889634f, 60.f));
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            const float rr = rcp_approx(g[e] * g[e + 1]) * inv;
+            o[e] = __float_as_uint(__uint_as_float(o[e]) * (g[e + 1] * rr));
+            o[e + 1] = __float_as_uint(__uint_as_float(o[e + 1]) * (g[e] * rr));
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * inv);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          sts128(brow + ((uint32_t)(q ^ (r & 7)) << 4), o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+        fence_proxy_async();
+        asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
+        if (gt == 0) {
+          tma_store_2d(&p.tm_o, sQ + b * kPfBoxBytes, head * kHeadDim + 32 * b, row0);   // rows past n_q are clipped
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        if (threadIdx.x == 0) RD_PF_TRACE(1, 47, b >> 1);
+      }
+      if (gt == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory outlives the copies
+    }
     const uint32_t stg = sV + ch * (kPfM * 256);
     uint8_t *gstg = gQ + (sV - sQ) + ch * (kPfM * 256);
-    for (int cc = 0; cc < 2; ++cc) {
+    for (int cc = 0; cc < 2 && rec_mode; ++cc) {
       const int c = 2 * cc + ch;
       uint32_t o[2][32];
       if (have) {
@@ -667,51 +766,22 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
           w[e] = have ? __float_as_uint(__uint_as_float(o[hq][iq + e]) * inv) : 0u;
         sts128(stg + r * 256 + ((q ^ (r & 15)) << 4), w[0], w[1], w[2], w[3]);
       }
-      if (with_gate && cc == 0) mbar_wait(bars + 8 * kBarG, 0, p.status, 28);
       asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
-      if (threadIdx.x == 0) RD_PF_TRACE(1, 47, 2 + cc);   // round cc staged
       // 128 threads: 8 rows x 16 chunks per pass
-      if (rec_mode) {
 #pragma unroll 8
-        for (int pass = 0; pass < kPfM / 8; ++pass) {
-          const int rr = pass * 8 + (gt >> 4), q = gt & 15;
-          const int gr = row0 + rr;
-          if (gr < p.n_q) {
-            // a record's values start 8 bytes into a 16-byte line: two 8-byte stores
-            const float4 v = *reinterpret_cast<const float4 *>(gstg + rr * 256 + ((q ^ (rr & 15)) << 4));
-            float2 *dst = reinterpret_cast<float2 *>(
-                p.records + (((size_t)gr * p.n_head + head) * gridDim.z + blockIdx.z) * kRec + 2 + 64 * c + 4 * q);
-            dst[0] = make_float2(v.x, v.y);
-            dst[1] = make_float2(v.z, v.w);
-          }
-        }
-      } else if (p.gate == nullptr) {
-#pragma unroll 8
-        for (int pass = 0; pass < kPfM / 8; ++pass) {
-          const int rr = pass * 8 + (gt >> 4), q = gt & 15;
-          const int gr = row0 + rr;
-          if (gr < p.n_q)
-            *reinterpret_cast<float4 *>(p.out + ((size_t)gr * p.n_head + head) * kHeadDim + 64 * c + 4 * q) =
-                *reinterpret_cast<const float4 *>(gstg + rr * 256 + ((q ^ (rr & 15)) << 4));
-        }
-      } else {
-#pragma unroll 4
-        for (int k = 0; k < kPfM / 8; ++k) {
-          const int rr = k * 8 + (gt >> 4), q = gt & 15, gr = row0 + rr;
-          if (gr < p.n_q) {
-            float4 v = *reinterpret_cast<const float4 *>(gstg + rr * 256 + ((q ^ (rr & 15)) << 4));
-            const float4 g = *reinterpret_cast<const float4 *>(gQ + rr * (kHeadDim * 4) + 256 * c + 16 * q);
-            // fast exp/divide: ~1e-6 relative, far inside the attention tolerance
-            v.x *= __fdividef(1.0f, 1.0f + __expf(-g.x));
-            v.y *= __fdividef(1.0f, 1.0f + __expf(-g.y));
-            v.z *= __fdividef(1.0f, 1.0f + __expf(-g.z));
-            v.w *= __fdividef(1.0f, 1.0f + __expf(-g.w));
-            *reinterpret_cast<float4 *>(p.out + ((size_t)gr * p.n_head + head) * kHeadDim + 64 * c + 4 * q) = v;
-          }
+      for (int pass = 0; pass < kPfM / 8; ++pass) {
+        const int rr = pass * 8 + (gt >> 4), q = gt & 15;
+        const int gr = row0 + rr;
+        if (gr < p.n_q) {
+          // a record's values start 8 bytes into a 16-byte line: two 8-byte stores
+          const float4 v = *reinterpret_cast<const float4 *>(gstg + rr * 256 + ((q ^ (rr & 15)) << 4));
+          float2 *dst = reinterpret_cast<float2 *>(
+              p.records + (((size_t)gr * p.n_head + head) * gridDim.z + blockIdx.z) * kRec + 2 + 64 * c + 4 * q);
+          dst[0] = make_float2(v.x, v.y);
+          dst[1] = make_float2(v.z, v.w);
         }
       }
       asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
-      if (threadIdx.x == 0) RD_PF_TRACE(1, 47, cc);   // round cc stored
     }
   }
   tc_fence_before();
@@ -886,8 +956,11 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   a.n_head = n_head;
   a.nkv = n_head_kv;
   a.qscale = scale * 1.4426950408889634f;
-  if ((rc = encode_f32_tmap(&a.tm_q, q, n_head, n_q, kPfM)) != RD_OK) return rc;
-  if (gate != nullptr && (rc = encode_f32_tmap(&a.tm_g, gate, n_head, n_q, kPfM)) != RD_OK) return rc;
+  if (n_splits < 1 || records == nullptr) n_splits = 1;
+  if (n_splits == 1) {
+    if (gate != nullptr && (rc = encode_f32_tmap(&a.tm_g, gate, n_head, n_q, kPfM)) != RD_OK) return rc;
+    if ((rc = encode_f32_tmap(&a.tm_o, out, n_head, n_q, kPfM)) != RD_OK) return rc;
+  }
   a.n_rot = n_rot;
   if (n_rot > 0) memcpy(a.freq, make_rope_table(n_rot, freq_base).f, sizeof(a.freq));
   a.kv_wait = k_new != nullptr || kv_pending ? 1 : 0;
@@ -905,7 +978,6 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
       return RD_ERR_CUDA;
     if (dev >= 0 && dev < 32) attr_set[dev] = true;
   }
-  if (n_splits < 1 || records == nullptr) n_splits = 1;
   a.records = records;
   if (k_new != nullptr) {
     // (a pass of many waves gains nothing from starting early)

@@ -73,11 +73,11 @@ int encode_f32_tmap(void *tmap_out, const void *base, int n_head, int64_t n_rows
   if (((uintptr_t)base & 15) != 0) return RD_ERR_ALIGN;
   const cuuint64_t dims[2] = {(cuuint64_t)n_head * kHeadDim, (cuuint64_t)n_rows};
   const cuuint64_t strides[1] = {(cuuint64_t)n_head * kHeadDim * 4};
-  const cuuint32_t box[2] = {kHeadDim, (cuuint32_t)tile_rows};
+  const cuuint32_t box[2] = {32, (cuuint32_t)tile_rows};  // 32 floats = one 128-byte swizzle row
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = g_encode((CUtensorMap *)tmap_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
                               const_cast<void *>(base), dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? RD_OK : RD_ERR_CUDA;
 }
