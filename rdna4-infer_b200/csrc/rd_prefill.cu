@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   const uint32_t bars = smem_u32(s_bars), lead = cluster_addr(bars, 0);   // this CTA's barriers, the leader's
 
   // Requested first, so that their latency runs under the set-up below: the positions of this tile's
-  // rows and half of the warp's 16 query rows (the other half: to L2).
+  // rows and, to L2, the warp's 16 query rows. (Loaded to registers here they are spilled, and the spill
+  // waits for them.)
   int my_pos = -1;
   float4 xa[8], xb[8];   // dims 4 lane .. + 3 and 128 + 4 lane .. + 3 of a row
   const float *qw = p.q + ((size_t)(row0 + warp * 16) * p.n_head + head) * kHeadDim;
@@ -180,10 +181,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   if (threadIdx.x < 2 * kPfM) {
     const int r = row0 + (threadIdx.x & (kPfM - 1));
     if (r < p.n_q) my_pos = p.pos[r];
-    load_rows(0);
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {   // 8 rows x 8 lines of 128 bytes
-      const int rr = 8 + (lane >> 3) + 4 * e;
+    for (int e = 0; e < 4; ++e) {   // 16 rows x 8 lines of 128 bytes
+      const int rr = (lane >> 3) + 4 * e;
       if (rr < rows_w) asm volatile("prefetch.global.L2 [%0];" ::"l"(qw + rr * q_row + 32 * (lane & 7)));
     }
   }
@@ -206,10 +206,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     for (int i = 0; i < 8; ++i) mbar_init(bars + 8 * (kBarR + i), 1);
     mbar_init(bars + 8 * kBarL, 8);
     mbar_init(bars + 8 * kBarQ, 16);   // one per converting warp (both CTAs)
-    mbar_init(bars + 8 * kBarT, 16);
+    mbar_init(bars + 8 * kBarT, 9);    // the CTA's warps, and the bytes of the peer's half
     mbar_init(bars + 8 * kBarC, 8);
     mbar_init(bars + 8 * kBarG, 1);
     fence_barrier_init();
+    mbar_expect_tx(bars + 8 * kBarT, p.n_rot == 64 ? 64 * 32 * 8 : 0);
   }
   if (warp == 9) {  // TMEM: 512 columns for this CTA (one CTA per SM: no contention)
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -242,7 +243,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   // ---- prologue: the Q tile as f16 in the swizzled K-major layout ----
   // f32 rows -> partial RoPE -> x scale * log2(e) -> f16 in the swizzled layout, warps 0-7. (A pre-pass
   // that wrote rotated f16 queries for all heads cost its own 6 us and a second trip to memory: 15400
-  // cycles from entry to the first S; the f32 rows by bulk copies or a tensor-map box: 13300; here XX.)
+  // cycles from entry to the first S; the f32 rows by bulk copies or a tensor-map box: 13300; here 11000, of
+  // which the loads of 128 KB take 2600 to issue.)
   if (warp < 8) {
     // thread (row r, h) rotates dims 0..63 of its row; they pass through V slot 1 as f32, 16-byte chunk q of
     // a row at q ^ (r & 15)
@@ -269,10 +271,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       }
     };
     if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 2);
-    convert(0);
-    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 3);
-    load_rows(8);
-    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 4);
+    load_rows(0);
     // (cos, sin) of all rows and pairs, while those are on their way: the two CTAs of the pair serve the same
     // tokens, each computes 64 rows for both (16 sincosf per thread took 4200 cycles). [pair][row] in V slot 0.
     const uint32_t cs0 = sV;
@@ -280,7 +279,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     if (p.n_rot == 64) {
       const int tr = (int)rank * 64 + (threadIdx.x & 63), tp = (threadIdx.x >> 6) * 8;   // row, first of 8 pairs
       const float fpos = (float)s_pos[tr];
-      const uint32_t peer = cluster_addr(cs0, rank ^ 1);
+      const uint32_t peer = cluster_addr(cs0, rank ^ 1), peer_bar = cluster_addr(bars + 8 * kBarT, rank ^ 1);
 #pragma unroll 1
       for (int i = 0; i < 8; i += 4) {
         float2 v[4];
@@ -290,21 +289,26 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         for (int e = 0; e < 4; ++e) {
           const uint32_t at = 8u * ((tp + i + e) * kPfM + tr);
           sts64(cs0 + at, __float_as_uint(v[e].x), __float_as_uint(v[e].y));
-          asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(peer + at), "f"(v[e].x), "f"(v[e].y) : "memory");
+          // (completes on the peer's barrier by bytes: no fence, no remote arrive)
+          asm volatile(
+              "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(peer + at),
+              "r"(__float_as_uint(v[e].x)), "r"(__float_as_uint(v[e].y)), "r"(peer_bar)
+              : "memory");
         }
       }
       __syncwarp();
       if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 5);
-      if (lane == 0) {
-        mbar_arrive_cluster(cluster_addr(bars + 8 * kBarT, 0));
-        mbar_arrive_cluster(cluster_addr(bars + 8 * kBarT, 1));
-      }
+      if (lane == 0) mbar_arrive(bars + 8 * kBarT);
     }
-    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 0);
+    convert(0);
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 3);
+    load_rows(8);
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 4);
     convert(8);
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 0);
     if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 1);
     if (p.n_rot > 0) {
-      if (p.n_rot == 64 && !mbar_wait_cluster(bars + 8 * kBarT, 0, p.status, 24)) s_abort = 1;
+      if (p.n_rot == 64 && !mbar_wait(bars + 8 * kBarT, 0, p.status, 24)) s_abort = 1;
       asm volatile("bar.sync 2, 256;" ::: "memory");
       auto chunk = [&](int q) { return *reinterpret_cast<const float4 *>(stage + r * 64 + ((q ^ (r & 15)) << 2)); };
       if (p.n_rot == 64) {

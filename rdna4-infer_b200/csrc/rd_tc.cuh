@@ -80,21 +80,12 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
   return a;
 }
-// Arrive on a barrier of either CTA (cluster address), ordering this thread's memory accesses before it.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-// The same without ordering ordinary memory accesses across the pair (what tcgen05 has written is
-// ordered by tcgen05.fence): a release at cluster scope waits 500 to 1000 cycles for all the thread's
-// accesses (with it in the key loop a tile took 3600 cycles instead of 2370).
+// Arrive on a barrier of either CTA (cluster address) without ordering ordinary memory accesses across
+// the pair: what tcgen05 has written is ordered by tcgen05.fence, operands in shared memory by
+// fence.proxy.async. A release at cluster scope waits 500 to 1000 cycles for all the thread's accesses
+// (with it in the key loop a tile took 3600 cycles instead of 2370).
 __device__ __forceinline__ void mbar_arrive_peer(uint32_t bar_cluster) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-// mbar_wait that also acquires what the other CTA's threads released.
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, DeviceStatus *status, int site) {
-  if (!mbar_wait(bar, parity, status, site)) return false;
-  asm volatile("fence.acq_rel.cluster;" ::: "memory");
-  return true;
 }
 __device__ __forceinline__ void cluster_sync() {
   __syncwarp();
