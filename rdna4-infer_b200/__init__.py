@@ -1,8 +1,8 @@
 """Python-side loader of ``librd_attn_b200.so`` -- the sm_100a attention / KV-cache
 library that drops in under rdna4-infer's launch API (``include/rd_attn.h``).
 
-The product is the C-ABI library; this module only binds it with ctypes so that the
-tests and the benchmark can drive it with torch-owned device memory. There is no CPU
+The product is the C-ABI library; this module only binds it (ctypes, and a small extension for the
+calls of a layer loop) so that the tests and the benchmark can drive it with torch-owned device memory. There is no CPU
 fallback of any kind: if the library has not been built, importing raises.
 
 The directory name carries a hyphen, so import it with
@@ -16,6 +16,7 @@ import subprocess
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "librd_attn_b200.so")
+BIND_PATH = os.path.join(HERE, "_rd_bind.so")
 
 F32, F16, Q8_0, Q4_0, Q5_0, Q4_1 = range(6)
 TYPE_NAMES = ("f32", "f16", "q8_0", "q4_0", "q5_0", "q4_1")
@@ -128,6 +129,17 @@ def _load():
         fn = getattr(lib, name)  # AttributeError here = header and library disagree
         fn.restype = res
         fn.argtypes = args
+    if os.path.exists(BIND_PATH):   # the layer loop's entries, without ctypes' 4 us per call
+        import importlib.machinery
+        import importlib.util
+        loader = importlib.machinery.ExtensionFileLoader("_rd_bind", BIND_PATH)
+        bind = importlib.util.module_from_spec(importlib.util.spec_from_loader("_rd_bind", loader))
+        loader.exec_module(bind)
+        for name in SIGNATURES:
+            fn = getattr(lib, name)
+            fast = bind.install(name, C.cast(fn, C.c_void_p).value, fn)
+            if fast is not None:
+                setattr(lib, name, fast)
     return lib
 
 
