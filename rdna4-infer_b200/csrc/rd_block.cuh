@@ -167,38 +167,28 @@ block_kernel(const __grid_constant__ BlockArgs p) {
   khead += (size_t)kvh * RK;
   vhead += (size_t)kvh * RV;
   const size_t kb = (size_t)nkv * RK, vb = (size_t)nkv * RV;
-  for (int c = threadIdx.x; c < COLS; c += Geo::kThreads) {
-    const int j = c / kGroup;
-    s_t[c] = j < n_tok ? (p.items != nullptr ? t_seq + tok0 + j : p.pos[tok0 + j]) : -1;
-  }
-  // query fragments, pre-scaled into log2 units (and by the loader's fixed-point factor); the padding
-  // columns are zero
-  {
-    const float qmul = p.qscale * KL::kUnscale;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < COLS * 64; i += Geo::kThreads) {
-      const int c = i >> 6, j = c / kGroup, h = c % kGroup;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (j < n_tok)
-        v = *reinterpret_cast<const float4 *>(qsrc + ((size_t)(tok0 + j) * p.n_head + kvh * kGroup + h) * kHeadDim +
-                                              4 * (i & 63));
-      const uint32_t cb = qfrag + (c >> 3) * 4096 + (c & 7) * 64;
-      const uint2 off = *reinterpret_cast<const uint2 *>(inv + 4 * (i & 63));
-      const float x[4] = {v.x, v.y, v.z, v.w};
-      const uint32_t o[4] = {off.x & 0xffffu, off.x >> 16, off.y & 0xffffu, off.y >> 16};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const unsigned short hbits = __half_as_ushort(__float2half_rn(x[e] * qmul));
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(cb + o[e]), "h"(hbits) : "memory");
-      }
-    }
-  }
-  __syncthreads();
   // last and first "last key" of the chunk's tokens
   int t_max = -1, t_min = 0x7fffffff;
-  for (int c = 0; c < n_tok * kGroup; c += kGroup) {
-    t_max = max(t_max, s_t[c]);
-    t_min = min(t_min, s_t[c]);
+  if (p.items != nullptr) {
+    t_min = t_seq + tok0;
+    t_max = t_min + n_tok - 1;
+  } else {
+    for (int i = 0; i < n_tok; ++i) {
+      const int t = p.pos[tok0 + i];
+      t_max = max(t_max, t);
+      t_min = min(t_min, t);
+    }
+  }
+  // the query rows: requested before the first slots, so that they do not queue behind them
+  constexpr int NQ = (COLS * 64 + Geo::kThreads - 1) / Geo::kThreads;
+  float4 qv[NQ];
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    const int i = threadIdx.x + k * Geo::kThreads, c = i >> 6, j = c / kGroup, h = c % kGroup;
+    qv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < COLS * 64 && j < n_tok)
+      qv[k] = *reinterpret_cast<const float4 *>(qsrc + ((size_t)(tok0 + j) * p.n_head + kvh * kGroup + h) * kHeadDim +
+                                                4 * (i & 63));
   }
   const int slots_total = (t_max + kBlkKeys) / kBlkKeys;   // ceil((t_max + 1) / 64)
   const int c_b = (int)(((int64_t)slots_total * s) / S), c_e = (int)(((int64_t)slots_total * (s + 1)) / S);
@@ -223,6 +213,31 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     fill_k(i);
     if (i + 1 < DV) fill_v(i);
   }
+
+  for (int c = threadIdx.x; c < COLS; c += Geo::kThreads) {
+    const int j = c / kGroup;
+    s_t[c] = j < n_tok ? (p.items != nullptr ? t_seq + tok0 + j : p.pos[tok0 + j]) : -1;
+  }
+  // query fragments, pre-scaled into log2 units (and by the loader's fixed-point factor); the padding
+  // columns are zero
+  {
+    const float qmul = p.qscale * KL::kUnscale;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      const int i = threadIdx.x + k * Geo::kThreads, c = i >> 6;
+      if (i >= COLS * 64) break;
+      const uint32_t cb = qfrag + (c >> 3) * 4096 + (c & 7) * 64;
+      const uint2 off = *reinterpret_cast<const uint2 *>(inv + 4 * (i & 63));
+      const float x[4] = {qv[k].x, qv[k].y, qv[k].z, qv[k].w};
+      const uint32_t o[4] = {off.x & 0xffffu, off.x >> 16, off.y & 0xffffu, off.y >> 16};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const unsigned short hbits = __half_as_ushort(__float2half_rn(x[e] * qmul));
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(cb + o[e]), "h"(hbits) : "memory");
+      }
+    }
+  }
+  __syncthreads();
 
   float O[4][NT][4];                     // [M-tile of this warp's quarter of the dims][column tile]
   float ref[NT][2], run[NT][2], l[NT][2];   // per lane column: team's reference, lane-local maximum and sum

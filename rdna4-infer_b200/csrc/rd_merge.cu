@@ -19,14 +19,10 @@ constexpr int kMergeGroups = 16;  // record groups per CTA
 // MODE 0: normalised output (optionally gated). MODE 1: un-normalised record out.
 // MODE 3: like 0, plus one more key -- the newest position's row, still only in the cache
 // -- attended here as one more record (m = scale * q.k, l = 1, acc = v).
-// MODE 2: like 0, but row = (sequence, token, head) and the record block, split count,
-// output and gate come from the sequence's descriptor (rows_per_seq = q_len * n_head).
-// kBatch: records that a group requests at once (see below); up to four leave registers for two CTAs per SM.
-template <int MODE, int kBatch>
-__global__ void __launch_bounds__(kMergeDims *kMergeGroups, kBatch <= 4 ? 2 : 1)
+template <int MODE>
+__global__ void __launch_bounds__(kMergeDims *kMergeGroups, 1)
 merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_in, int n_out,
-             float *__restrict__ gate, const DecodeSeq *__restrict__ seqs, int rows_per_seq,
-             const ExtraKey xk) {
+             float *__restrict__ gate, const ExtraKey xk) {
   __shared__ float s_l[kMergeGroups];
   __shared__ float s_gm[kMergeGroups];
   __shared__ float s_acc[kMergeGroups][kMergeDims];
@@ -38,25 +34,14 @@ merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_i
   const int j = MODE == 1 ? blockIdx.z : 0;  // output record index
   const int tx = threadIdx.x % kMergeDims, ty = threadIdx.x / kMergeDims;
   const int lo = MODE == 1 ? (int)(((int64_t)n_in * j) / n_out) : 0;
-  int hi = MODE == 1 ? (int)(((int64_t)n_in * (j + 1)) / n_out) : n_in;
+  const int hi = MODE == 1 ? (int)(((int64_t)n_in * (j + 1)) / n_out) : n_in;
   const float *base = partial + (size_t)row * n_in * kRec;
-  int out_row = row;
-  if (MODE == 2) {
-    const DecodeSeq &d = seqs[row / rows_per_seq];
-    out_row = row % rows_per_seq;
-    n_in = d.n_splits;
-    base = partial + ((size_t)d.rec_base + (size_t)out_row * n_in) * kRec;
-    out = d.out;
-    gate = d.gate;
-    hi = n_in;
-  }
-
   // One pass: group ty walks records lo+ty, lo+ty+16, ... and keeps a local log-sum-exp
   // (m, l, acc); the 16 groups are then combined through shared memory. An empty record
   // (m = -inf) weighs nothing and whatever its body holds is never used. The first batch is
   // requested before anything else, the gate value with it. A batch of ten holds the 148 records
-  // of a full-GPU decode in ONE round trip to L2 (four per batch took three); rows with up to 64
-  // records (blocks of tokens, many sequences) have many CTAs and want two per SM.
+  // of a full-GPU decode in ONE round trip to L2 (four per batch took three).
+  constexpr int kBatch = 10;
   float mB[kBatch], aB[kBatch], lB[kBatch];
   auto request = [&](int s0) {
 #pragma unroll
@@ -74,7 +59,7 @@ merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_i
   };
   request(lo + ty);
   float gate_in = 0.f;
-  if (MODE != 1 && gate != nullptr && ty == 0) gate_in = gate[(size_t)out_row * kHeadDim + quarter * kMergeDims + tx];
+  if (MODE != 1 && gate != nullptr && ty == 0) gate_in = gate[(size_t)row * kHeadDim + quarter * kMergeDims + tx];
 
   // MODE 3: the score of the extra key, by the first 256 threads (one dim each)
   float x_score = -INFINITY;
@@ -149,9 +134,9 @@ merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_i
     }
     if (MODE != 1) {
       float o = (mm != -INFINITY && l > 0.f) ? a / l : 0.f;
-      float *op = out + (size_t)out_row * kHeadDim + d;
+      float *op = out + (size_t)row * kHeadDim + d;
       if (gate != nullptr) {
-        float *gp = gate + (size_t)out_row * kHeadDim + d;
+        float *gp = gate + (size_t)row * kHeadDim + d;
         const float sg = __fdiv_rn(1.0f, 1.0f + expf(-gate_in));
         *gp = sg;
         o *= sg;
@@ -168,13 +153,133 @@ merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_i
   }
 }
 
+// Rows with few records (blocks of tokens: up to 37, many sequences: about ten): 64 threads of four dims
+// walk a row's records, G such groups share a row, a CTA of 256 threads has 4 / G rows. Bound by the
+// latency of a row's loads, requested eight records at a time. With a 1024-thread CTA per row and 64
+// dims, as for the 148 records of a long decode, most threads had no record: 64 sequences x 4 tokens x 24
+// heads took 194 us, here XX; 120 rows of 37 records 7.6 us, here YY.
+// MULTI: row = (sequence, token, head), records, split count, output and gate from the descriptor.
+template <bool MULTI, int G>
+__global__ void __launch_bounds__(256)
+merge_rows_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_rows, int n_in,
+                  float *__restrict__ gate, const DecodeSeq *__restrict__ seqs, int rows_per_seq) {
+  __shared__ float s_m[4], s_l[4];
+  __shared__ float4 s_acc[4][64];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tx = threadIdx.x & 63, grp = threadIdx.x >> 6;
+  const int row = G == 1 ? (int)blockIdx.x * 4 + grp : (int)blockIdx.x;
+  if (row >= n_rows) return;   // (G > 1: one row per CTA)
+  const float *base = partial + (size_t)row * n_in * kRec;
+  int out_row = row;
+  if (MULTI) {
+    const DecodeSeq &d = seqs[row / rows_per_seq];
+    out_row = row % rows_per_seq;
+    n_in = d.n_splits;
+    base = partial + ((size_t)d.rec_base + (size_t)out_row * n_in) * kRec;
+    out = d.out;
+    gate = d.gate;
+  }
+  const size_t at = (size_t)out_row * kHeadDim + 4 * tx;
+  const bool last = G == 1 || grp == 0;
+  float gv[4] = {0.f, 0.f, 0.f, 0.f};
+  if (last && gate != nullptr) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) gv[e] = gate[at + e];
+  }
+  constexpr int kBatch = 8;
+  float m = -INFINITY, l = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = G == 1 ? 0 : grp; s0 < n_in; s0 += kBatch * G) {
+    float mB[kBatch], lB[kBatch];
+    float2 va[kBatch], vb[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const int s = s0 + k * G;
+      mB[k] = -INFINITY;
+      lB[k] = 0.f;
+      va[k] = vb[k] = make_float2(0.f, 0.f);
+      if (s < n_in) {
+        const float *rec = base + (size_t)s * kRec;
+        mB[k] = rec[0];
+        lB[k] = rec[1];
+        va[k] = *reinterpret_cast<const float2 *>(rec + 2 + 4 * tx);   // (a record is 8-byte aligned)
+        vb[k] = *reinterpret_cast<const float2 *>(rec + 4 + 4 * tx);
+      }
+    }
+    float mm = m;
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) mm = fmaxf(mm, mB[k]);
+    if (mm == -INFINITY) continue;
+    const float f = expf(m - mm);   // 0 while nothing has been accumulated
+    acc.x *= f, acc.y *= f, acc.z *= f, acc.w *= f;
+    l *= f;
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      if (mB[k] != -INFINITY) {   // (an empty record weighs nothing, whatever its body holds)
+        const float w = expf(mB[k] - mm);
+        l = fmaf(lB[k], w, l);
+        acc.x = fmaf(va[k].x, w, acc.x);
+        acc.y = fmaf(va[k].y, w, acc.y);
+        acc.z = fmaf(vb[k].x, w, acc.z);
+        acc.w = fmaf(vb[k].y, w, acc.w);
+      }
+    }
+    m = mm;
+  }
+  if (G > 1) {
+    s_acc[grp][tx] = acc;
+    if (tx == 0) s_m[grp] = m, s_l[grp] = l;
+    __syncthreads();
+    if (grp != 0) return;
+    float mm = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < G; ++i) mm = fmaxf(mm, s_m[i]);
+    acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    l = 0.f;
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      if (s_m[i] == -INFINITY) continue;
+      const float w = expf(s_m[i] - mm);
+      const float4 a = s_acc[i][tx];
+      l = fmaf(s_l[i], w, l);
+      acc.x = fmaf(a.x, w, acc.x);
+      acc.y = fmaf(a.y, w, acc.y);
+      acc.z = fmaf(a.z, w, acc.z);
+      acc.w = fmaf(a.w, w, acc.w);
+    }
+    m = mm;
+  }
+  float o[4] = {0.f, 0.f, 0.f, 0.f};
+  if (m != -INFINITY && l > 0.f) o[0] = acc.x / l, o[1] = acc.y / l, o[2] = acc.z / l, o[3] = acc.w / l;
+  if (gate != nullptr) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float sg = __fdiv_rn(1.0f, 1.0f + expf(-gv[e]));
+      gate[at + e] = sg;
+      o[e] *= sg;
+    }
+  }
+  if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    *reinterpret_cast<float4 *>(out + at) = make_float4(o[0], o[1], o[2], o[3]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) out[at + e] = o[e];
+  }
+}
+
 int launch_merge(const float *partial, float *out, int n_rows, int n_splits, float *gate,
                  cudaStream_t st) {
   if (n_rows == 0) return RD_OK;
   const dim3 grid((unsigned)n_rows, kHeadDim / kMergeDims, 1);
-  const auto kernel = n_splits <= 4 * kMergeGroups ? merge_kernel<0, 4> : merge_kernel<0, 10>;
-  return launch_pdl(4, kernel, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, out, n_splits, 1, gate,
-                    nullptr, 1, ExtraKey{}) == cudaSuccess
+  // up to 64 records: a few hundred rows of a block of tokens, each with 256 threads
+  if (n_splits <= 64 && n_rows > 24 && (reinterpret_cast<uintptr_t>(partial) & 7) == 0)
+    return launch_pdl(4, merge_rows_kernel<false, 4>, dim3((unsigned)n_rows), dim3(256), 0, st, partial, out, n_rows,
+                      n_splits, gate, nullptr, 1) == cudaSuccess
+               ? RD_OK
+               : RD_ERR_CUDA;
+  return launch_pdl(4, merge_kernel<0>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, out, n_splits, 1, gate,
+                    ExtraKey{}) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
 }
@@ -183,8 +288,8 @@ int launch_merge_extra(const float *partial, float *out, int n_rows, int n_split
                        const ExtraKey &x, cudaStream_t st) {
   if (n_rows == 0) return RD_OK;
   const dim3 grid((unsigned)n_rows, kHeadDim / kMergeDims, 1);
-  return launch_pdl(4, merge_kernel<3, 10>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, out, n_splits,
-                    1, gate, nullptr, 1, x) == cudaSuccess
+  return launch_pdl(4, merge_kernel<3>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, out, n_splits,
+                    1, gate, x) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
 }
@@ -193,8 +298,8 @@ int launch_merge_records(const float *partial, float *records, int n_rows, int n
                          cudaStream_t st) {
   if (n_rows == 0) return RD_OK;
   const dim3 grid((unsigned)n_rows, kHeadDim / kMergeDims, (unsigned)n_out);
-  return launch_pdl(4, merge_kernel<1, 10>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, records, n_in,
-                    n_out, nullptr, nullptr, 1, ExtraKey{}) == cudaSuccess
+  return launch_pdl(4, merge_kernel<1>, grid, dim3(kMergeDims * kMergeGroups), 0, st, partial, records, n_in,
+                    n_out, nullptr, ExtraKey{}) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
 }
@@ -203,11 +308,8 @@ int launch_merge_multi(const DecodeSeq *dev_seqs, const float *records, int n_se
                        int n_head, cudaStream_t st) {
   const int rows = n_seq * q_len * n_head;
   if (rows == 0) return RD_OK;
-  const dim3 grid((unsigned)rows, kHeadDim / kMergeDims, 1);
-  // not a dependent launch: thousands of CTAs that would take SM slots from the decode launch's
-  // last ones
-  return launch_pdl(0, merge_kernel<2, 4>, grid, dim3(kMergeDims * kMergeGroups), 0, st, records, nullptr, 0, 1,
-                    nullptr, dev_seqs, q_len * n_head, ExtraKey{}) == cudaSuccess
+  return launch_pdl(4, merge_rows_kernel<true, 1>, dim3((unsigned)((rows + 3) / 4)), dim3(256), 0, st, records,
+                    (float *)nullptr, rows, 0, (float *)nullptr, dev_seqs, q_len * n_head) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
 }
