@@ -113,7 +113,8 @@ struct PrefillArgs {
   // key tiles and writes an un-normalised record (m, l, acc) per row instead of the
   // output; prefill_merge_kernel combines the records. Fills the SMs when n_q * n_head /
   // 128 CTAs would leave many idle.
-  float *records;        // [n_q * n_head][gridDim.z][2 + 256]
+  // Records: accumulators [n_q][n_head][gridDim.z][256] behind tm_o, then (m, l) here.
+  float2 *rec_ml;        // [n_q][n_head][gridDim.z]
 };
 
 // Barrier slots (8 bytes each).
@@ -676,10 +677,6 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 4);   // main loop done, sums exchanged
 
   // ---- epilogue ----
-  // Key splits: un-normalised records -> global, 64 columns at a time.
-  // staging tiles [128 rows][64 floats] lie over the V ring; 16-byte chunk q of row r is
-  // stored at q ^ (r & 15), so both the row-wise writes and the coalesced reads are
-  // conflict-free.
   if (warp < 8) {
     // warpgroup ch stores output columns [64*(2c+ch), +64), c = 0..1, through its own
     // staging tile and named barrier
@@ -691,14 +688,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const bool rec_mode = gridDim.z > 1;   // un-normalised records for prefill_merge_kernel
     const float inv = (l_tot > 0.f && !aborted) ? (rec_mode ? 1.0f : 1.0f / l_tot) : 0.f;
     const bool have = nt > 0 && !aborted;
+    // column of the first value in the output, or in the accumulators of the records
+    const int col0 = (rec_mode ? head * (int)gridDim.z + (int)blockIdx.z : head) * kHeadDim;
     if (rec_mode && ch == 0 && row0 + r < p.n_q) {
-      // header of this row's record; natural-log units like every record of the library
-      float *rec = p.records + (((size_t)(row0 + r) * p.n_head + head) * gridDim.z + blockIdx.z) * kRec;
+      // (m, l) of this row's record, in natural-log units
       const bool some = have && l_tot > 0.f;
-      rec[0] = some ? m_fin * 0.6931471805599453f : -INFINITY;
-      rec[1] = some ? l_tot : 0.f;
+      p.rec_ml[((size_t)(row0 + r) * p.n_head + head) * gridDim.z + blockIdx.z] =
+          some ? make_float2(m_fin * 0.6931471805599453f, l_tot) : make_float2(-INFINITY, 0.f);
     }
-    if (!rec_mode) {
+    {
       // O / l (x sigmoid(gate)) in place over the gate rows, 32 columns (a box of 128-byte swizzled rows)
       // at a time, each box stored by TMA while the next is computed. What bounds it: the 32 bytes a
       // cycle that an SM writes (4096 cycles) and 1.5 special functions per gate value (3072).
@@ -744,48 +742,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         fence_proxy_async();
         asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
         if (gt == 0) {
-          tma_store_2d(&p.tm_o, sQ + b * kPfBoxBytes, head * kHeadDim + 32 * b, row0);   // rows past n_q are clipped
+          tma_store_2d(&p.tm_o, sQ + b * kPfBoxBytes, col0 + 32 * b, row0);   // rows past n_q are clipped
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
         if (threadIdx.x == 0) RD_PF_TRACE(1, 47, b >> 1);
       }
       if (gt == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory outlives the copies
-    }
-    const uint32_t stg = sV + ch * (kPfM * 256);
-    uint8_t *gstg = gQ + (sV - sQ) + ch * (kPfM * 256);
-    for (int cc = 0; cc < 2 && rec_mode; ++cc) {
-      const int c = 2 * cc + ch;
-      uint32_t o[2][32];
-      if (have) {
-        tmem_ld32(lane_addr + kTmemO + 64 * c, o[0]);
-        tmem_ld32(lane_addr + kTmemO + 64 * c + 32, o[1]);
-        tmem_wait_ld();
-      }
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int hq = q >> 3, iq = (q & 7) * 4;
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          w[e] = have ? __float_as_uint(__uint_as_float(o[hq][iq + e]) * inv) : 0u;
-        sts128(stg + r * 256 + ((q ^ (r & 15)) << 4), w[0], w[1], w[2], w[3]);
-      }
-      asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
-      // 128 threads: 8 rows x 16 chunks per pass
-#pragma unroll 8
-      for (int pass = 0; pass < kPfM / 8; ++pass) {
-        const int rr = pass * 8 + (gt >> 4), q = gt & 15;
-        const int gr = row0 + rr;
-        if (gr < p.n_q) {
-          // a record's values start 8 bytes into a 16-byte line: two 8-byte stores
-          const float4 v = *reinterpret_cast<const float4 *>(gstg + rr * 256 + ((q ^ (rr & 15)) << 4));
-          float2 *dst = reinterpret_cast<float2 *>(
-              p.records + (((size_t)gr * p.n_head + head) * gridDim.z + blockIdx.z) * kRec + 2 + 64 * c + 4 * q);
-          dst[0] = make_float2(v.x, v.y);
-          dst[1] = make_float2(v.z, v.w);
-        }
-      }
-      asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
     }
   }
   tc_fence_before();
@@ -801,29 +763,27 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
 // (token, head); out = sum_z acc_z e^(m_z - M) / sum_z l_z e^(m_z - M), times sigmoid(gate)
 // if given (the gate is only read). Rows whose records are all empty give zeros.
 __global__ void __launch_bounds__(256)
-prefill_merge_kernel(const float *__restrict__ records, float *__restrict__ out, const float *__restrict__ gate,
-                     int64_t n_rows, int n_splits) {
+prefill_merge_kernel(const float4 *__restrict__ rec_acc, const float2 *__restrict__ rec_ml, float *__restrict__ out,
+                     const float *__restrict__ gate, int64_t n_rows, int n_splits) {
   const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 6);
   const int tx = threadIdx.x & 63;
   pdl_launch_dependents();
   pdl_wait();   // launched under the tile kernel: its records are complete from here on
   if (row >= n_rows) return;
-  const float *rec = records + (size_t)row * n_splits * kRec;
   // every load of the row is requested before the first is used (at most kPfMaxSplits
   // records): one round trip to L2 instead of one for the maxima and one per record
   float m[kPfMaxSplits], lz[kPfMaxSplits];
-  float2 va[kPfMaxSplits], vb[kPfMaxSplits];
+  float4 va[kPfMaxSplits];
 #pragma unroll
   for (int z = 0; z < kPfMaxSplits; ++z) {
     m[z] = -INFINITY;
     lz[z] = 0.f;
-    va[z] = vb[z] = make_float2(0.f, 0.f);
+    va[z] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (z < n_splits) {
-      const float *r = rec + (size_t)z * kRec;
-      m[z] = __ldcg(r);
-      lz[z] = __ldcg(r + 1);
-      va[z] = __ldcg(reinterpret_cast<const float2 *>(r + 2 + 4 * tx));   // a record's values start 8 bytes
-      vb[z] = __ldcg(reinterpret_cast<const float2 *>(r + 4 + 4 * tx));   // into a 16-byte line
+      const float2 ml = __ldcg(rec_ml + row * n_splits + z);
+      m[z] = ml.x;
+      lz[z] = ml.y;
+      va[z] = __ldcg(rec_acc + (row * n_splits + z) * (kHeadDim / 4) + tx);
     }
   }
   float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -841,8 +801,8 @@ prefill_merge_kernel(const float *__restrict__ records, float *__restrict__ out,
       l = fmaf(lz[z], w, l);
       acc.x = fmaf(va[z].x, w, acc.x);
       acc.y = fmaf(va[z].y, w, acc.y);
-      acc.z = fmaf(vb[z].x, w, acc.z);
-      acc.w = fmaf(vb[z].y, w, acc.w);
+      acc.z = fmaf(va[z].z, w, acc.z);
+      acc.w = fmaf(va[z].w, w, acc.w);
     }
   }
   const float inv = l > 0.f ? 1.0f / l : 0.f;
@@ -961,7 +921,10 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   a.nkv = n_head_kv;
   a.qscale = scale * 1.4426950408889634f;
   if (n_splits < 1 || records == nullptr) n_splits = 1;
-  if (n_splits == 1) {
+  if (n_splits > 1) {
+    a.rec_ml = reinterpret_cast<float2 *>(records + (size_t)n_q * n_head * n_splits * kHeadDim);
+    if ((rc = encode_f32_tmap(&a.tm_o, records, n_head * n_splits, n_q, kPfM)) != RD_OK) return rc;
+  } else {
     if (gate != nullptr && (rc = encode_f32_tmap(&a.tm_g, gate, n_head, n_q, kPfM)) != RD_OK) return rc;
     if ((rc = encode_f32_tmap(&a.tm_o, out, n_head, n_q, kPfM)) != RD_OK) return rc;
   }
@@ -982,7 +945,6 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
       return RD_ERR_CUDA;
     if (dev >= 0 && dev < 32) attr_set[dev] = true;
   }
-  a.records = records;
   if (k_new != nullptr) {
     // (a pass of many waves gains nothing from starting early)
     const bool early = n_q <= 1024;
@@ -1019,7 +981,8 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, prefill_merge_kernel, (const float *)records, out, gate, n_rows, n_splits) !=
+    if (cudaLaunchKernelEx(&cfg, prefill_merge_kernel, (const float4 *)records, (const float2 *)a.rec_ml, out,
+                           gate, n_rows, n_splits) !=
         cudaSuccess)
       return RD_ERR_CUDA;
   }
