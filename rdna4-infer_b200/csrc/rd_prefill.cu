@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   }
   __syncthreads();
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 1);   // barriers + TMEM allocated
+  if (warp < 8) load_rows(0);
 
   // ---- the last key any row of this tile attends ----
   if (threadIdx.x < kPfM) {
@@ -272,7 +273,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       }
     };
     if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 2);
-    load_rows(0);
+    convert(0);
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 3);
+    load_rows(8);
+    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 4);
     // (cos, sin) of all rows and pairs, while those are on their way: the two CTAs of the pair serve the same
     // tokens, each computes 64 rows for both (16 sincosf per thread took 4200 cycles). [pair][row] in V slot 0.
     const uint32_t cs0 = sV;
@@ -301,10 +305,6 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 5);
       if (lane == 0) mbar_arrive(bars + 8 * kBarT);
     }
-    convert(0);
-    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 3);
-    load_rows(8);
-    if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 4);
     convert(8);
     if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 0);
     if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 1);
