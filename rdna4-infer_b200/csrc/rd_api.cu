@@ -117,7 +117,8 @@ int attn_core(const float *q, const void *k, const void *v, float *out, float *r
     tiles = (n_keys + tile - 1) / tile;
   }
   const int direct = n_tok == 1 && out != nullptr ? step_splits(kt, vt, n_head_kv, n_keys) : 0;
-  int S = direct > 0 ? direct : n_tok > 1 ? block_splits(sms, n_tok, n_head_kv) : plan_splits(sms, n_tok, tiles);
+  const int per_head = n_tok == 1 && out != nullptr && direct == 0 ? step_record_splits(kt, vt, n_head_kv, n_keys, sms) : 0;
+  int S = direct > 0 ? direct : per_head > 0 ? per_head : n_tok > 1 ? block_splits(sms, n_tok, n_head_kv) : plan_splits(sms, n_tok, tiles);
   if (out == nullptr) {
     // nest the internal splits inside the caller's: S = n_rec * r
     int r = S / n_rec;
@@ -138,7 +139,11 @@ int attn_core(const float *q, const void *k, const void *v, float *out, float *r
   a.n_splits = S;
   a.status = status;
   // a block of tokens shares each dequantized key; one token has a warp per (head, key group)
-  auto launch = [&] { return n_tok > 1 ? launch_block(kt, vt, a, block_chunk(n_tok), st) : launch_decode(kt, vt, a, st); };
+  auto launch = [&] {
+    return n_tok > 1      ? launch_block(kt, vt, a, block_chunk(n_tok), st)
+           : per_head > 0 ? launch_step(kt, vt, a, nullptr, nullptr, st)
+                          : launch_decode(kt, vt, a, st);
+  };
   if (out == nullptr && S == n_rec) {
     a.partial = records;
     return launch();
@@ -493,7 +498,8 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
   const int tile = decode_tile_keys(k_type, v_type);
   const int64_t tiles = ((int64_t)t + tile - 1) / tile;
   const int direct = step_splits(k_type, v_type, n_head_kv, (int64_t)t + 1);
-  const int S = direct > 0 ? direct : plan_splits(sm_count(dev), 1, tiles);
+  const int per_head = direct == 0 ? step_record_splits(k_type, v_type, n_head_kv, (int64_t)t + 1, sm_count(dev)) : 0;
+  const int S = direct > 0 ? direct : per_head > 0 ? per_head : plan_splits(sm_count(dev), 1, tiles);
   if (workspace_bytes < partial_floats(1, n_head, S) * sizeof(float)) return RD_ERR_WORKSPACE;
   DecodeArgs a;
   a.q = q;
@@ -501,7 +507,7 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
   a.v = v_cache;
   a.partial = (float *)workspace;
   a.pos = nullptr;
-  a.t = direct > 0 ? t : t - 1;
+  a.t = direct > 0 || per_head > 0 ? t : t - 1;
   a.key_begin = 0;
   a.n_tok = 1;
   a.n_head = n_head;
@@ -514,6 +520,10 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
   a.new_row = t;
   cudaStream_t st = (cudaStream_t)stream;
   if (direct > 0) return launch_step(k_type, v_type, a, out, gate, st);
+  if (per_head > 0) {
+    if ((rc = launch_step(k_type, v_type, a, nullptr, nullptr, st)) != RD_OK) return rc;
+    return launch_merge((const float *)workspace, out, n_head, S, gate, st);
+  }
   if ((rc = launch_decode(k_type, v_type, a, st)) != RD_OK) return rc;
   ExtraKey x;
   x.q = q;

@@ -116,6 +116,11 @@ int step_splits(int kt, int vt, int n_head_kv, int64_t n_keys) {
   return n_keys <= 16 * kSlotKeys ? 8 : 16;
 }
 
+int step_record_splits(int kt, int vt, int n_head_kv, int64_t n_keys, int sms) {
+  if (n_keys < 0 || key_groups(kt, vt) > 1) return 0;
+  return sms / n_head_kv;
+}
+
 int decode_tile_keys(int kt, int vt) { return 16 * key_groups(kt, vt); }
 
 }  // namespace rd

@@ -89,6 +89,9 @@ int launch_step(int kt, int vt, const DecodeArgs &a, float *out, float *gate, cu
 // CTAs per KV head of that launch for n_keys keys, or 0 where launch_decode is the faster one (or
 // n_keys < 0: not known on the host).
 int step_splits(int kt, int vt, int n_head_kv, int64_t n_keys);
+// The same kernel with records (out == nullptr: a.n_splits CTAs per KV head write a.partial), for the long
+// contexts where that is the faster one: CTAs per KV head, or 0.
+int step_record_splits(int kt, int vt, int n_head_kv, int64_t n_keys, int sms);
 
 // Blocks of tokens (rd_block.cuh): token i attends keys 0..pos[i] (on the device); a CTA serves `chunk`
 // <= 8 tokens. Writes n_splits records per (token, head) like launch_decode.

@@ -66,6 +66,7 @@ struct StepArgs {
   // fused append: the rows of key t, quantized into cache row t by the CTA that attends it
   const float *k_new;
   const float *v_new;
+  float *partial;       // records [head][gridDim.x][258] instead of the output, or null
 };
 
 __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
@@ -119,13 +120,16 @@ step_kernel(const __grid_constant__ StepArgs p) {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   pdl_wait();   // everything below reads what earlier kernels of the stream wrote
 
-  // the CTA's rank in its cluster, and the cluster's size: a power of two
-  const int s = blockIdx.x, S = gridDim.x, shift = 31 - __clz(S);
+  // the CTA's rank in its cluster, and the cluster's size: a power of two. With records there are no
+  // clusters: CTA x of gridDim.x.
+  const bool records = p.partial != nullptr;
+  const int s = records ? 0 : blockIdx.x, S = records ? 1 : gridDim.x, shift = 31 - __clz(S);
   const int t_last = p.t, key_begin = p.key_begin;
   const bool append = p.k_new != nullptr;
   const int n_keys = t_last >= key_begin ? t_last - key_begin + 1 : 0;
   const int slots_total = (n_keys + kSlotKeys - 1) / kSlotKeys;
-  const int c_b = slots_total * s >> shift, c_e = slots_total * (s + 1) >> shift;
+  const int c_b = (int)((unsigned)slots_total * blockIdx.x / gridDim.x);   // (below 2^31: 2^22 slots at most)
+  const int c_e = (int)((unsigned)slots_total * (blockIdx.x + 1) / gridDim.x);
   const int n_warps = c_e - c_b < W ? c_e - c_b : W;   // warps with slots
   const int n_mine = c_e - c_b > warp ? (c_e - c_b - warp + W - 1) / W : 0;   // slots c_b + warp + it * W
   const int t_load = append ? t_last - 1 : t_last;   // last key that is read from the cache
@@ -159,7 +163,7 @@ step_kernel(const __grid_constant__ StepArgs p) {
   }
   // Fused append: the CTA that attends key t quantizes its rows of this KV head, one 32-value block
   // per warp, into shared memory; from there into the cache and into the slot that attends them.
-  const bool owner = append && s == S - 1;
+  const bool owner = append && blockIdx.x == gridDim.x - 1;
   if (owner) {
 #pragma unroll 1
     for (int b = warp; b < 16; b += W) {
@@ -325,6 +329,36 @@ step_kernel(const __grid_constant__ StepArgs p) {
   }
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   __syncthreads();
+  if (records) {   // a CTA's record per head, for merge_kernel
+    __shared__ float s_ml[kGroup][2];
+    for (int i = threadIdx.x; i < W * kGroup; i += NT) {
+      const int w = i / kGroup, h = i % kGroup;
+      float mm = kStepNone, ll = 0.f;
+      for (int j = 0; j < n_warps; ++j) mm = fmaxf(mm, s_t[j][h]);
+      s_wt[w][h] = ex2(s_m[w][h] - mm) * VL::kUnscale;
+      if (w == 0) {
+        for (int j = 0; j < n_warps; ++j) ll = fmaf(s_l[j][h], ex2(s_m[j][h] - mm), ll);
+        s_ml[h][0] = mm > 0.5f * kStepNone ? mm * 0.6931471805599453f : -INFINITY;   // natural log
+        s_ml[h][1] = mm > 0.5f * kStepNone ? ll : 0.f;
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kGroup * (kHeadDim / 2); i += NT) {
+      const int h = i >> 7, dd = 2 * (i & 127);
+      const int off = h * kPlane + 33 * (dd >> 5) + (dd & 31);
+      float a0 = 0.f, a1 = 0.f;
+#pragma unroll 4
+      for (int w = 0; w < n_warps; ++w) {
+        const float *pl = reinterpret_cast<const float *>(smem + kStepHeader + w * kPlaneStride) + off;
+        a0 = fmaf(pl[0], s_wt[w][h], a0);
+        a1 = fmaf(pl[1], s_wt[w][h], a1);
+      }
+      float *rec = p.partial + ((size_t)(kvh * kGroup + h) * gridDim.x + blockIdx.x) * kRec;
+      if (dd == 0) rec[0] = s_ml[h][0], rec[1] = s_ml[h][1];
+      *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a0, a1);
+    }
+    return;
+  }
   const uint32_t recv = sbase + kStepRecv, recv_ml = recv + 6144;   // [src][1536 / S] and [src][head][2]
   for (int i = threadIdx.x; i < n_warps * kGroup; i += NT) {
     const int w = i / kGroup, h = i % kGroup;
@@ -412,8 +446,9 @@ int launch_step_typed(const DecodeArgs &a, float *out, float *gate, cudaStream_t
   k.gate = gate;
   k.k_new = a.k_new;
   k.v_new = a.v_new;
+  k.partial = out == nullptr ? a.partial : nullptr;
   return launch_pdl_cluster(step_kernel<KT, VT>, dim3((unsigned)a.n_splits, (unsigned)a.n_head_kv),
-                            dim3(Geo::W * 32), Geo::kSmem, (unsigned)a.n_splits, st, k) == cudaSuccess
+                            dim3(Geo::W * 32), Geo::kSmem, out == nullptr ? 1u : (unsigned)a.n_splits, st, k) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
 }
