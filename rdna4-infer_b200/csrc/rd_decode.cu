@@ -101,15 +101,18 @@ int launch_block_multi(int kt, int vt, const MultiDecodeArgs &a, cudaStream_t st
   }
 }
 
-// Where the line lies, measured (us per layer with its pre-attention stage, 4 KV heads, this kernel /
-// decode_kernel + merge): q8_0 4096 keys 12.9 / 14.5, 8192 16.7 / 16.9, 12288 20.8 / 18.7; q4_0 8192 14.6 /
-// 15.8, 12288 17.3 / 16.7; q8_0/f16 12288 19.7 / 19.9; f16 16384 22.8 / 27.6. 64 SMs fetch a long context
-// more slowly than 148, and the wider the rows the later that shows, as decode_kernel has fewer warps
-// then (key_groups). With fewer KV heads fewer SMs work here, not there.
+// Where the lines lie, measured (us per layer with its pre-attention stage, 4 KV heads: one cluster per KV
+// head / step_kernel with records + merge / decode_kernel + merge):
+//   keys       3000       4096               8192              16384            32768            65536
+//   f16        11.9 / -   12.2 / 12.8 / 18   16.1 / 15.6 / 22  22.8 / 20.8 / 28 -  / 32 / 39     -
+//   q8_0/f16   12.0 / -   12.9 / 12.4 / 16   16.5 / 15.0 / 18  -  / 18.7 / 22   -  / 28.0 / 30   -  / 44.3 / 45.2
+//   q8_0       12.2 / -   12.7 / 12.0 / 14   16.5 / 14.8 / 17  -  / 19.0 / 20   -  / 26.1 / 24.8 -  / 39.3 / 36.5
+//   q4_0       11.0 / -   11.7 / 11.8 / 14   14.4 / 13.3 / 16  -  / 16.4 / 18   -  / 21.4 / 21.9 -  / 30.9 / 30.5
+// The cluster form saves the merge launch but uses 64 SMs; records use all. decode_kernel copies all KV heads of
+// a key in one box, which costs a long launch fewer issue slots and a short one a larger prologue; with f16
+// rows it has shared memory for four or eight warps only.
 int step_splits(int kt, int vt, int n_head_kv, int64_t n_keys) {
-  const int groups = key_groups(kt, vt);
-  int64_t most = groups == 3 ? 8192 : groups == 2 ? 12288 : 24576;
-  if (n_head_kv < 4 && most > 6144) most = 6144;
+  const int most = (key_groups(kt, vt) == 1 ? 5632 : 3584) * n_head_kv / 4;
   if (n_keys < 0 || n_keys > most) return 0;
   // at least one slot for some of the warps of each CTA: more CTAs share out the copies, and the
   // latency of a CTA's instruction fetch, down to about two slots each
@@ -117,7 +120,7 @@ int step_splits(int kt, int vt, int n_head_kv, int64_t n_keys) {
 }
 
 int step_record_splits(int kt, int vt, int n_head_kv, int64_t n_keys, int sms) {
-  if (n_keys < 0 || key_groups(kt, vt) > 1) return 0;
+  if (n_keys < 0 || (key_groups(kt, vt) == 3 && n_keys > 24576)) return 0;
   return sms / n_head_kv;
 }
 
