@@ -145,6 +145,18 @@ step_kernel(const __grid_constant__ StepArgs p) {
   for (int j = 0; j < NQ; ++j)
     if ((int)threadIdx.x + j * NT < NQ4) qv[j] = q4[threadIdx.x + j * NT];
 
+  // ... and so are the values of an appended row, by the CTA that attends it
+  const bool owner = append && blockIdx.x == gridDim.x - 1;
+  constexpr int NA = (16 + W - 1) / W;   // its 32-value blocks (8 of K, 8 of V) per warp
+  float xa[NA];
+#pragma unroll
+  for (int k = 0; k < NA; ++k) {
+    const int b = warp + k * W;
+    xa[k] = !owner || b >= 16 ? 0.f
+            : b < 8           ? p.k_new[(size_t)kvh * kHeadDim + b * 32 + lane]
+                              : p.v_new[(size_t)kvh * kHeadDim + (b - 8) * 32 + lane];
+  }
+
   // The warp's it-th slot into ring position d = it % D; always one commit group, empty behind the end.
   auto fill_k = [&](int it, int d) {
     if (it < n_mine && t_load >= key_begin)
@@ -163,14 +175,14 @@ step_kernel(const __grid_constant__ StepArgs p) {
   }
   // Fused append: the CTA that attends key t quantizes its rows of this KV head, one 32-value block
   // per warp, into shared memory; from there into the cache and into the slot that attends them.
-  const bool owner = append && blockIdx.x == gridDim.x - 1;
   if (owner) {
-#pragma unroll 1
-    for (int b = warp; b < 16; b += W) {
+#pragma unroll
+    for (int k = 0; k < NA; ++k) {
+      const int b = warp + k * W;
       if (b < 8)
-        store_block<KT>(p.k_new[(size_t)kvh * kHeadDim + b * 32 + lane], stage, b, lane);
-      else
-        store_block<VT>(p.v_new[(size_t)kvh * kHeadDim + (b - 8) * 32 + lane], stage + RK, b - 8, lane);
+        store_block<KT>(xa[k], stage, b, lane);
+      else if (b < 16)
+        store_block<VT>(xa[k], stage + RK, b - 8, lane);
     }
   }
   {
@@ -198,14 +210,15 @@ step_kernel(const __grid_constant__ StepArgs p) {
     const uint32_t *st = reinterpret_cast<const uint32_t *>(stage);
     for (int i = threadIdx.x; i < (RK + RV) / 4; i += NT) (i < RK / 4 ? kd[i] : vd[i - RK / 4]) = st[i];
   }
-  // the appended row into the slot, and something finite behind it
+  // the appended row into the slot; the rows behind it repeat the last stored one -- or, where there is
+  // none (nothing was copied), the appended one: something finite
   auto patch = [&](uint32_t slot, int pitch, const uint8_t *row, int words, int row0) {
+    const int first = t_last - row0, last = t_load < key_begin ? kSlotKeys - 1 : first;
 #pragma unroll 1
-    for (int i = lane; i < words * kSlotKeys; i += 32) {
-      const int r = i / words, c = i % words;
-      if (row0 + r >= t_last)
+    for (int r = first; r <= last; ++r)
+#pragma unroll 4
+      for (int c = lane; c < words; c += 32)
         *reinterpret_cast<uint32_t *>(smem + (slot - sbase) + r * pitch + 4 * c) = reinterpret_cast<const uint32_t *>(row)[c];
-    }
     __syncwarp();
   };
 
