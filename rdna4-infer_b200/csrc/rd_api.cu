@@ -620,21 +620,40 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
     return RD_ERR_WORKSPACE;
   if (pad_items > max_items) return RD_ERR_LIMIT;
 
-  // Key split: chunks of equal length over all sequences, about four CTAs per SM in
-  // total, so that a 32k-key sequence and a 1k-key one load the SMs evenly.
-  // Blocks of tokens (q_len > 1) are CTAs per KV head: eight of those per SM, fewer where an item's
-  // records (one per token and head) would outgrow the workspace's 4 * sms + n_seq * q_len.
+  // Key split: chunks of equal length over all sequences, so that a 32k-key sequence and a 1k-key one load
+  // the SMs evenly. Blocks of tokens (q_len > 1) are CTAs per KV head: eight of those per SM, fewer where an
+  // item's records (one per token and head) would outgrow the workspace's 4 * sms + n_seq * q_len.
   const int tok_chunk = block_chunk(q_len), n_chunks = (q_len + tok_chunk - 1) / tok_chunk;
   const int tile = q_len > 1 ? 64 : decode_tile_keys(k_type, v_type);
-  const int target = q_len > 1 ? std::max(1, std::min(8 * sms / n_head_kv, 4 * sms / tok_chunk)) : 4 * sms;
   std::vector<int> tiles(n_seq);
   int64_t total = 0;
   for (int i = 0; i < n_seq; ++i) {
     tiles[i] = (seqs[i].t + tile) / tile;  // ceil((t + 1) / tile)
     total += (int64_t)tiles[i] * n_chunks;
   }
-  int64_t chunk = (total + target - 1) / target;
-  if (chunk < 4) chunk = 4;
+  auto chunk_for = [&](int target) { return std::max<int64_t>(4, (total + target - 1) / target); };
+  int64_t chunk = 0;
+  if (q_len > 1) {
+    chunk = chunk_for(std::max(1, std::min(8 * sms / n_head_kv, 4 * sms / tok_chunk)));
+  } else {
+    // One to four CTAs per SM, in whole waves: a wave costs about 10 us beside its tiles (prologue, epilogue,
+    // records). Fewer only where that is clearly less, since items of different lengths level out over
+    // more waves. Measured: 8 sequences of 4000 to 30000 keys, q8_0/f16, 2 / 3 / 4 per SM: 94 / 107 / 116 us;
+    // 64 of 1024 to 32768: 524 / 502 / 496.
+    const double tile_us = (double)tile * n_head_kv * (row_bytes(k_type) + row_bytes(v_type)) / 42e3;   // 42 GB/s an SM
+    const int longest = *std::max_element(tiles.begin(), tiles.end());
+    double best = 0;
+    for (int k = 4; k >= 1; --k) {
+      int64_t c = chunk_for(k * sms), items = 0;
+      for (;; c += 1 + c / 32) {   // the smallest chunk whose items fit into k waves
+        items = 0;
+        for (int i = 0; i < n_seq; ++i) items += (tiles[i] + (int)c - 1) / (int)c;
+        if (items <= (int64_t)k * sms || c >= longest) break;
+      }
+      const double cost = (double)((items + sms - 1) / sms) * (10.0 + tile_us * total / items);
+      if (chunk == 0 || cost < 0.92 * best) best = cost, chunk = c;
+    }
+  }
   unsigned char *body = (unsigned char *)plan + kMultiPlanHeaderBytes;
   DecodeSeq *hs = reinterpret_cast<DecodeSeq *>(body);
   int4 *hi = reinterpret_cast<int4 *>(body + off_items);
@@ -694,7 +713,9 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
   return RD_OK;
 }
 
-int rd_attn_multi_launch(const void *plan, float scale, void *workspace, size_t workspace_bytes, void *stream) {
+// by_value: the plan is read during the call (it travels in kernel parameters, see launch_upload).
+static int multi_launch(const void *plan, float scale, void *workspace, size_t workspace_bytes, void *stream,
+                        bool by_value) {
   if (plan == nullptr) return RD_ERR_NULL;
   MultiPlanHeader h;
   memcpy(&h, plan, sizeof(h));
@@ -714,7 +735,11 @@ int rd_attn_multi_launch(const void *plan, float scale, void *workspace, size_t 
   if (workspace_bytes < need) return RD_ERR_WORKSPACE;
   // From pageable memory the copy has left the plan when cudaMemcpyAsync returns; from
   // pinned memory it reads the plan when the stream (or a replayed graph) reaches it.
-  if (cudaMemcpyAsync(workspace, (const unsigned char *)plan + kMultiPlanHeaderBytes, h.copy_bytes,
+  if (by_value) {
+    if ((rc = launch_upload((const unsigned char *)plan + kMultiPlanHeaderBytes, workspace, h.copy_bytes,
+                            (cudaStream_t)stream)) != RD_OK)
+      return rc;
+  } else if (cudaMemcpyAsync(workspace, (const unsigned char *)plan + kMultiPlanHeaderBytes, h.copy_bytes,
                       cudaMemcpyHostToDevice, (cudaStream_t)stream) != cudaSuccess)
     return RD_ERR_CUDA;
   MultiDecodeArgs a;
@@ -732,7 +757,12 @@ int rd_attn_multi_launch(const void *plan, float scale, void *workspace, size_t 
   if ((rc = (h.q_len > 1 ? launch_block_multi : launch_decode_multi)(h.k_type, h.v_type, a, (cudaStream_t)stream)) !=
       RD_OK)
     return rc;
-  return launch_merge_multi(a.dev_seqs, a.records, h.n_seq, h.q_len, h.n_head, (cudaStream_t)stream);
+  const int per_row = h.n_items / (h.n_seq * ((h.q_len + block_chunk(h.q_len) - 1) / block_chunk(h.q_len)));
+  return launch_merge_multi(a.dev_seqs, a.records, h.n_seq, h.q_len, h.n_head, per_row, (cudaStream_t)stream);
+}
+
+int rd_attn_multi_launch(const void *plan, float scale, void *workspace, size_t workspace_bytes, void *stream) {
+  return multi_launch(plan, scale, workspace, workspace_bytes, stream, false);
 }
 
 int rd_attn_decode_multi(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head, int n_head_kv,
@@ -750,7 +780,7 @@ int rd_attn_decode_multi(const rd_attn_seq *seqs, int n_seq, int q_len, int n_he
   int rc = rd_attn_multi_plan(seqs, n_seq, q_len, n_head, n_head_kv, head_dim, k_type, v_type, 0, plan.data(),
                               plan_bytes);
   if (rc != RD_OK) return rc;
-  return rd_attn_multi_launch(plan.data(), scale, workspace, workspace_bytes, stream);
+  return multi_launch(plan.data(), scale, workspace, workspace_bytes, stream, true);
 }
 
 // ---- context-sharded decode with the exchange fused into the merge -------------------

@@ -200,7 +200,11 @@ int launch_merge_records(const float *partial, float *records, int n_rows, int n
 // Multi-sequence merge: row (sequence, token, head) reads its n_splits records from the
 // sequence's block of `records` and writes (optionally gated) into the sequence's out.
 int launch_merge_multi(const DecodeSeq *dev_seqs, const float *records, int n_seq, int q_len,
-                       int n_head, cudaStream_t st);
+                       int n_head, int records_per_row, cudaStream_t st);
+
+// Host bytes to the device in kernel parameters (a pageable copy beyond what fits in them): the bytes are
+// read during the call. dst 16-byte aligned.
+int launch_upload(const void *src, void *dst, size_t bytes, cudaStream_t st);
 
 // ---- rd_shard.cu (launchers)
 // partial [n_head][n_in][258] (this rank's split records) -> one record per head stored

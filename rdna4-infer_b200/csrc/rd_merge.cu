@@ -8,6 +8,8 @@
 // record per SM, so a CTA owns (row, 64-dim quarter) and spreads the records over 16
 // thread groups: 4 * n_rows CTAs of 1024 threads keep the read of the partial buffer
 // wide enough to stay off the critical path of a ~25 us decode step.
+#include <string.h>
+
 #include "rd_common.cuh"
 #include "rd_internal.h"
 
@@ -153,18 +155,18 @@ merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_i
   }
 }
 
-// Rows with few records (blocks of tokens: up to 37, many sequences: about ten): 64 threads of four dims
-// walk a row's records, G such groups share a row, a CTA of 256 threads has 4 / G rows. Bound by the
-// latency of a row's loads, requested eight records at a time. With a 1024-thread CTA per row and 64
-// dims, as for the 148 records of a long decode, most threads had no record: 64 sequences x 4 tokens x 24
-// heads took 194 us, here XX; 120 rows of 37 records 7.6 us, here YY.
+// Rows of blocks of tokens and of many sequences: 64 threads of four dims walk a row's records, G such
+// groups share a row, a CTA has max(4, G) groups. Bound by the latency of a row's loads, requested eight
+// records at a time: G follows the records per row. With a 1024-thread CTA per row and 64 dims, as for the
+// 148 records of a long decode, most threads had no record: 64 sequences x 4 tokens x 24 heads took 194
+// us, here (G = 1) 14; 120 rows of 37 records 7.6 us, here (G = 4) 5.4.
 // MULTI: row = (sequence, token, head), records, split count, output and gate from the descriptor.
 template <bool MULTI, int G>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(G > 4 ? 64 * G : 256)
 merge_rows_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_rows, int n_in,
                   float *__restrict__ gate, const DecodeSeq *__restrict__ seqs, int rows_per_seq) {
-  __shared__ float s_m[4], s_l[4];
-  __shared__ float4 s_acc[4][64];
+  __shared__ float s_m[G], s_l[G];
+  __shared__ float4 s_acc[G][64];
   pdl_launch_dependents();
   pdl_wait();
   const int tx = threadIdx.x & 63, grp = threadIdx.x >> 6;
@@ -305,13 +307,47 @@ int launch_merge_records(const float *partial, float *records, int n_rows, int n
 }
 
 int launch_merge_multi(const DecodeSeq *dev_seqs, const float *records, int n_seq, int q_len,
-                       int n_head, cudaStream_t st) {
+                       int n_head, int records_per_row, cudaStream_t st) {
   const int rows = n_seq * q_len * n_head;
   if (rows == 0) return RD_OK;
-  return launch_pdl(4, merge_rows_kernel<true, 1>, dim3((unsigned)((rows + 3) / 4)), dim3(256), 0, st, records,
-                    (float *)nullptr, rows, 0, (float *)nullptr, dev_seqs, q_len * n_head) == cudaSuccess
+  // (the average: a row's own count follows its sequence's length)
+  const auto kernel = records_per_row <= 12   ? merge_rows_kernel<true, 1>
+                      : records_per_row <= 40 ? merge_rows_kernel<true, 4>
+                                              : merge_rows_kernel<true, 16>;
+  const dim3 grid((unsigned)(records_per_row <= 12 ? (rows + 3) / 4 : rows));
+  return launch_pdl(4, kernel, grid, dim3(records_per_row <= 40 ? 256 : 1024), 0, st, records, (float *)nullptr, rows, 0,
+                    (float *)nullptr, dev_seqs, q_len * n_head) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
+}
+
+// A copy from pageable memory is a stop for the launches around it (the copy engine, about 5 us); up to 32 KB
+// fit into the parameters of a kernel that takes part in the dependent launches.
+template <int N>
+struct UploadArgs {
+  uint4 *dst;
+  int n;
+  alignas(16) uint4 data[N];
+};
+template <int N>
+__global__ void __launch_bounds__(256) upload_kernel(const __grid_constant__ UploadArgs<N> a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int i = threadIdx.x; i < a.n; i += blockDim.x) a.dst[i] = a.data[i];
+}
+template <int N>
+static int upload(const void *src, void *dst, size_t bytes, cudaStream_t st) {
+  static thread_local UploadArgs<N> a;
+  a.dst = (uint4 *)dst;
+  a.n = (int)((bytes + 15) / 16);
+  memcpy(a.data, src, bytes);
+  return launch_pdl(4, upload_kernel<N>, dim3(1), dim3(256), 0, st, a) == cudaSuccess ? RD_OK : RD_ERR_CUDA;
+}
+int launch_upload(const void *src, void *dst, size_t bytes, cudaStream_t st) {
+  if (bytes <= 2048) return upload<128>(src, dst, bytes, st);
+  if (bytes <= 8192) return upload<512>(src, dst, bytes, st);
+  if (bytes <= 32640) return upload<2040>(src, dst, bytes, st);
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess ? RD_OK : RD_ERR_CUDA;
 }
 
 }  // namespace rd
