@@ -621,38 +621,39 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
   if (pad_items > max_items) return RD_ERR_LIMIT;
 
   // Key split: chunks of equal length over all sequences, so that a 32k-key sequence and a 1k-key one load
-  // the SMs evenly. Blocks of tokens (q_len > 1) are CTAs per KV head: eight of those per SM, fewer where an
-  // item's records (one per token and head) would outgrow the workspace's 4 * sms + n_seq * q_len.
+  // the SMs evenly, and in whole waves of CTAs (blocks of tokens, q_len > 1, are CTAs per KV head). A wave
+  // costs about 10 us beside its tiles (prologue, epilogue, records). Fewer waves only where that is clearly
+  // less, since items of different lengths level out over more. Measured: 8 sequences of 4000 to 30000 keys,
+  // q8_0/f16, 2 / 3 / 4 per SM: 94 / 107 / 116 us; 64 of 1024 to 32768 about / in four waves: 496 / 449.
   const int tok_chunk = block_chunk(q_len), n_chunks = (q_len + tok_chunk - 1) / tok_chunk;
-  const int tile = q_len > 1 ? 64 : decode_tile_keys(k_type, v_type);
+  const bool block = q_len > 1;
+  const int tile = block ? 64 : decode_tile_keys(k_type, v_type);
+  const int wave = block ? std::max(1, sms / n_head_kv) : sms;
+  // (records: an item of a block has one per token and head, the workspace holds 4 * sms + n_seq * q_len items' worth
+  // of one token)
+  const int most_waves = block ? std::max(1, std::min(8, 4 * sms / tok_chunk / wave)) : 4;
+  // 42 GB/s an SM; a block's tile is bound by its MMAs
+  const double tile_us = block ? 0.11 * tok_chunk * kGroup / 8 * 4
+                               : (double)tile * n_head_kv * (row_bytes(k_type) + row_bytes(v_type)) / 42e3;
   std::vector<int> tiles(n_seq);
   int64_t total = 0;
+  int longest = 1;
   for (int i = 0; i < n_seq; ++i) {
     tiles[i] = (seqs[i].t + tile) / tile;  // ceil((t + 1) / tile)
     total += (int64_t)tiles[i] * n_chunks;
+    longest = std::max(longest, tiles[i]);
   }
-  auto chunk_for = [&](int target) { return std::max<int64_t>(4, (total + target - 1) / target); };
   int64_t chunk = 0;
-  if (q_len > 1) {
-    chunk = chunk_for(std::max(1, std::min(8 * sms / n_head_kv, 4 * sms / tok_chunk)));
-  } else {
-    // One to four CTAs per SM, in whole waves: a wave costs about 10 us beside its tiles (prologue, epilogue,
-    // records). Fewer only where that is clearly less, since items of different lengths level out over
-    // more waves. Measured: 8 sequences of 4000 to 30000 keys, q8_0/f16, 2 / 3 / 4 per SM: 94 / 107 / 116 us;
-    // 64 of 1024 to 32768: 524 / 502 / 496.
-    const double tile_us = (double)tile * n_head_kv * (row_bytes(k_type) + row_bytes(v_type)) / 42e3;   // 42 GB/s an SM
-    const int longest = *std::max_element(tiles.begin(), tiles.end());
-    double best = 0;
-    for (int k = 4; k >= 1; --k) {
-      int64_t c = chunk_for(k * sms), items = 0;
-      for (;; c += 1 + c / 32) {   // the smallest chunk whose items fit into k waves
-        items = 0;
-        for (int i = 0; i < n_seq; ++i) items += (tiles[i] + (int)c - 1) / (int)c;
-        if (items <= (int64_t)k * sms || c >= longest) break;
-      }
-      const double cost = (double)((items + sms - 1) / sms) * (10.0 + tile_us * total / items);
-      if (chunk == 0 || cost < 0.92 * best) best = cost, chunk = c;
+  double best = 0;
+  for (int k = most_waves; k >= 1; --k) {
+    int64_t c = std::max<int64_t>(4, (total + (int64_t)k * wave - 1) / ((int64_t)k * wave)), items = 0;
+    for (;; c += 1 + c / 32) {   // the smallest chunk whose items fit into k waves
+      items = 0;
+      for (int i = 0; i < n_seq; ++i) items += (int64_t)n_chunks * ((tiles[i] + (int)c - 1) / (int)c);
+      if (items <= (int64_t)k * wave || c >= longest) break;
     }
+    const double cost = (double)((items + wave - 1) / wave) * (10.0 + tile_us * total / items);
+    if (chunk == 0 || cost < 0.92 * best) best = cost, chunk = c;
   }
   unsigned char *body = (unsigned char *)plan + kMultiPlanHeaderBytes;
   DecodeSeq *hs = reinterpret_cast<DecodeSeq *>(body);
