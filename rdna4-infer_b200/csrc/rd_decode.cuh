@@ -3,7 +3,7 @@
 //
 // Shape of the computation (replaces attn_split_kernel, include/rdna4/attn.cuh:445-560,
 // and the unsplit attn_kernel, :95-185):
-//   * grid (n_splits, n_tok): CTA s owns a contiguous slice of the key tiles and
+//   * grid n_splits: CTA s owns a contiguous slice of the key tiles and
 //     writes one partial record (m, l, acc[256]) per query head;
 //   * the CTA's warps form key groups of four (one warp per kv head); every group streams
 //     16-key slots through its own ring in shared memory -- one tensor-map (TMA) copy per
@@ -61,7 +61,6 @@ struct DecodeKernelArgs {
   // everything per-sequence comes from the descriptor instead of the fields above.
   const DecodeSeq *seqs;
   const int4 *items;
-  int q_len;
   // Fused append (single-sequence launches): quantize k_new / v_new [nkv][256] into cache
   // row new_row; null = nothing to append.
   const float *k_new;
@@ -183,10 +182,10 @@ decode_kernel(const __grid_constant__ DecodeKernelArgs p) {
   pdl_wait();   // everything below reads what earlier kernels of the stream wrote
   RD_TRACE(1);
 
-  // What this CTA works on: token qt, split s of S, keys key_begin..t_last of the caches
+  // What this CTA works on: split s of S, keys key_begin..t_last of the caches
   // at kbase / vbase (or behind the tensor maps tmk / tmv), one record per head at
   // rec0 + head * S * kRec.
-  int qt, s, S, t_last, key_begin, use_tk, use_tv;
+  int s, S, t_last, key_begin, use_tk, use_tv;
   const float *qsrc;
   const uint8_t *kbase, *vbase;
   const CUtensorMap *tmk, *tmv;
@@ -195,19 +194,18 @@ decode_kernel(const __grid_constant__ DecodeKernelArgs p) {
     const int4 item = p.items[blockIdx.x];
     if (item.x < 0) return;   // padding of a plan with a fixed item count
     const DecodeSeq &d = p.seqs[item.x];
-    qt = item.y;
     s = item.z;
     S = d.n_splits;
-    t_last = d.t - (p.q_len - 1 - qt);  // causal inside the block of q_len new tokens
+    t_last = d.t;
     key_begin = 0;
     use_tk = d.k_tmap;
     use_tv = d.v_tmap;
-    qsrc = d.q + (size_t)qt * p.n_head * kHeadDim;
+    qsrc = d.q;
     kbase = d.k;
     vbase = d.v;
     tmk = reinterpret_cast<const CUtensorMap *>(d.tm_k);
     tmv = reinterpret_cast<const CUtensorMap *>(d.tm_v);
-    rec0 = p.partial + ((size_t)d.rec_base + (size_t)qt * p.n_head * S + s) * kRec;
+    rec0 = p.partial + ((size_t)d.rec_base + s) * kRec;
     // These descriptors were written to global memory by an ordinary copy and may have
     // been rewritten since an earlier launch read them: make the copy visible to the
     // tensor-map proxy of every thread that may issue a load through them.
@@ -218,19 +216,18 @@ decode_kernel(const __grid_constant__ DecodeKernelArgs p) {
         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmv) : "memory");
     }
   } else {
-    qt = blockIdx.y;
     s = blockIdx.x;
     S = gridDim.x;
-    t_last = p.pos != nullptr ? p.pos[qt] : p.t;
+    t_last = p.pos != nullptr ? p.pos[0] : p.t;
     key_begin = p.key_begin;
     use_tk = p.k_tmap;
     use_tv = p.v_tmap;
-    qsrc = p.q + (size_t)qt * p.n_head * kHeadDim;
+    qsrc = p.q;
     kbase = p.k;
     vbase = p.v;
     tmk = &p.tm_k;
     tmv = &p.tm_v;
-    rec0 = p.partial + ((size_t)qt * p.n_head * S + s) * kRec;
+    rec0 = p.partial + (size_t)s * kRec;
   }
   // Key split in 16-key slots: CTA s owns slots [c_b, c_e) of the attended range and
   // deals them round-robin to its key groups (group x: local slots x, x + G, ...), so the
@@ -325,7 +322,7 @@ decode_kernel(const __grid_constant__ DecodeKernelArgs p) {
   // Nobody in this launch reads that row: the keys attended end before it, and the merge
   // that follows folds it in from the cache.
   if constexpr (!MULTI) {
-    if (p.k_new != nullptr && blockIdx.y == 0) {
+    if (p.k_new != nullptr) {
       const int per_tensor = nkv * (kHeadDim / 32);
       for (int b = (int)blockIdx.x * NW + warp; b < 2 * per_tensor; b += (int)gridDim.x * NW) {
         if (b < per_tensor)
@@ -777,19 +774,19 @@ int launch_decode_typed(const DecodeArgs &a, cudaStream_t st) {
   k.k_new = a.k_new;
   k.v_new = a.v_new;
   k.new_row = a.new_row;
-  if (a.push != nullptr && a.n_tok == 1) {   // memset above: world 0 = no exchange
+  if (a.push != nullptr) {   // memset above: world 0 = no exchange
     k.push = *a.push;
     k.x_out = a.push_out;
     k.x_gate = a.push_gate;
   }
 #ifdef RD_TIMING_SWITCHES
   if constexpr (tc_decode_usable(KT, VT)) {
-    if (tc_decode_enabled() && a.n_head_kv == 4 && a.n_tok == 1 && k.k_tmap && k.v_tmap && a.push == nullptr &&
+    if (tc_decode_enabled() && a.n_head_kv == 4 && k.k_tmap && k.v_tmap && a.push == nullptr &&
         a.k_new == nullptr)
       return launch_decode_tc<KT, VT>(k, a.n_splits, st);
   }
 #endif
-  const dim3 grid((unsigned)a.n_splits, (unsigned)a.n_tok);
+  const dim3 grid((unsigned)a.n_splits);
   return launch_pdl(2, decode_kernel<KT, VT, false>, grid, dim3(4 * G * 32), smem, st, k) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
@@ -829,7 +826,6 @@ int multi_decode_typed(const MultiDecodeArgs &a, cudaStream_t st) {
   k.status = a.status;
   k.seqs = a.dev_seqs;
   k.items = a.dev_items;
-  k.q_len = a.q_len;
   return launch_pdl(2, decode_kernel<KT, VT, true>, dim3((unsigned)a.n_items), dim3(4 * G * 32), smem, st,
                     k) == cudaSuccess
              ? RD_OK

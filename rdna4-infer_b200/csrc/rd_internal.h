@@ -51,9 +51,8 @@ struct ShardPeers {
   unsigned long long wait_ns;  // how long the merge waits for the other ranks' records
 };
 // ---- rd_decode_*.cu
-// One launch of the split-KV decode kernel: grid (n_splits, n_tok). Token i attends
-// keys key_begin..(pos ? pos[i] : t). Writes n_splits records per (token, head) into
-// partial[n_tok][n_head][n_splits][258].
+// One launch of the split-KV decode kernel, one token: attends keys key_begin..(pos ? pos[0] : t), writes
+// n_splits records per head into partial[n_head][n_splits][258]. (n_tok > 1: launch_block.)
 struct DecodeArgs {
   const float *q;
   const void *k;

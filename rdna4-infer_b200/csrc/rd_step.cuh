@@ -1,4 +1,5 @@
-// Decode attention of one query token over a SHORT context: one cluster per KV head, one launch.
+// Decode attention of one query token, one KV head per CTA: a cluster per KV head in one launch over
+// short contexts, records for merge_kernel over longer ones (step_splits, step_record_splits).
 //
 // Replaces attn_split_kernel (include/rdna4/attn.cuh:445-560) and the unsplit attn_kernel
 // (:95-185). Grid (n_splits, n_head_kv): a CTA owns a contiguous run of 16-key slots of ONE KV
@@ -17,10 +18,11 @@
 // q4_0 layer where the arithmetic takes 31. Asynchronous 16-byte copies take any row, need no
 // descriptor (none to encode on the host) and clamp the ragged end for free.
 //
-// What bounds it: latency (launch, first slot, the two meetings), and from about 2000 keys the
-// rate at which 32 SMs can fetch. Long contexts go to decode_kernel, whose slots span all KV heads
-// of a key: wide rows for the TMA unit, no copy instructions in warps that are already bound by
-// the dequantize + mma.sync issue slots (131001 q4_0 keys: 49 us per layer here, 44 there).
+// What bounds it: latency (launch, first slot, the two meetings), with one cluster per KV head from about
+// 2000 keys the rate at which 64 SMs can fetch (35 bytes a cycle each). The longest contexts of 4- and 8-bit
+// caches go to decode_kernel, whose slots span all KV heads of a key: wide rows for the TMA unit, no copy
+// instructions in warps that are bound by the dequantize + mma.sync issue slots (131001 q4_0 keys: 49
+// us per layer here, 44 there).
 #pragma once
 #include "rd_frag.cuh"
 #include "rd_internal.h"

@@ -1,5 +1,5 @@
-"""Short-context decode (one cluster per KV head, one launch): slot and cluster edges, the line to the
-split-KV kernel, fewer KV heads, a first key behind 0, the fused append at slot edges; against the oracle."""
+"""Per-head decode (one cluster per KV head, or records): slot and cluster edges, the lines between the forms,
+fewer KV heads, a first key behind 0, the fused append at slot edges; against the oracle."""
 import numpy as np
 import pytest
 import torch
@@ -26,13 +26,13 @@ def make(oracle, seed, nkv, n, kt, vt):
 @pytest.mark.parametrize("kt,vt,nkv", [(1, 1, 4), (2, 2, 4), (3, 3, 2), (4, 5, 1), (5, 4, 4), (2, 1, 4), (0, 0, 1)])
 def test_short_context_edges(G, oracle, kt, vt, nkv):
     rd, lib = G.rd, G.lib
-    n_max = 8193 if kt == 2 and vt == 2 else 1100
+    n_max = {(2, 2): 8193, (1, 1): 5634, (2, 1): 3586}.get((kt, vt), 1100)
     rng, q, kc, vc = make(oracle, 10 * kt + vt, nkv, n_max, kt, vt)
     gate = rng.standard_normal(q.shape).astype(np.float32)
     dq, dk, dv = G.dev(q), G.dev(kc), G.dev(vc)
     nb = lib.rd_attn_workspace_bytes(1, 6 * nkv, HD)
     ws = torch.empty(nb, dtype=torch.uint8, device="cuda")
-    for begin, n in ((0, 1), (0, 15), (0, 16), (0, 17), (0, 255), (0, 256), (0, 257), (3, 300), (77, n_max - 1), (0, n_max)):
+    for begin, n in ((0, 1), (0, 15), (0, 16), (0, 17), (0, 255), (0, 256), (0, 257), (3, 300), (77, n_max - 1), (0, n_max - 2), (0, n_max)):
         want = oracle.attn(q[None], kc.reshape(n_max, -1)[begin:n], vc.reshape(n_max, -1)[begin:n], [n - begin - 1], nkv,
                            1 / 16, kt, vt)[0]
         sg, want = oracle.sigmoid_gate(gate, want)
@@ -46,7 +46,7 @@ def test_short_context_edges(G, oracle, kt, vt, nkv):
 
 
 @pytest.mark.parametrize("kt,vt", [(1, 1), (3, 3), (4, 5), (2, 1)])
-@pytest.mark.parametrize("t", [15, 16, 17, 255, 256, 511])
+@pytest.mark.parametrize("t", [15, 16, 17, 255, 256, 511, 5700])
 def test_short_context_append(G, oracle, kt, vt, t):
     rd, lib = G.rd, G.lib
     nkv = 4
