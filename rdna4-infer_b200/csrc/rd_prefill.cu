@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   // rows and, to L2, the warp's 16 query rows. (Loaded to registers here they are spilled, and the spill
   // waits for them.)
   int my_pos = -1;
+  const int rows_cta = p.n_q - row0;                                  // rows of the tile that exist
+  const int rows_cs = rows_cta > 64 ? 128 : rows_cta > 32 ? 64 : 32;   // and that the (cos, sin) table is made for
   float4 xa[8], xb[8];   // dims 4 lane .. + 3 and 128 + 4 lane .. + 3 of a row
   const float *qw = p.q + ((size_t)(row0 + warp * 16) * p.n_head + head) * kHeadDim;
   const size_t q_row = (size_t)p.n_head * kHeadDim;
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     mbar_init(bars + 8 * kBarC, 8);
     mbar_init(bars + 8 * kBarG, 1);
     fence_barrier_init();
-    mbar_expect_tx(bars + 8 * kBarT, p.n_rot == 64 ? 64 * 32 * 8 : 0);
+    mbar_expect_tx(bars + 8 * kBarT, p.n_rot == 64 ? rows_cs / 2 * 32 * 8 : 0);
   }
   if (warp == 9) {  // TMEM: 512 columns for this CTA (one CTA per SM: no contention)
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -259,6 +261,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
             pack_h2(x.x * p.qscale, x.y * p.qscale), pack_h2(x.z * p.qscale, x.w * p.qscale));
     };
     auto convert = [&](int first) {
+      if (rows_cta <= 32 * (warp >> 1)) return;   // (no row of a whole softmax warp exists: nobody reads the scores)
 #pragma unroll
       for (int k = 0; k < 8; ++k) put4(warp * 16 + first + k, lane + 32, xb[k]);
       if (p.n_rot > 0 && lane < 16) {
@@ -278,20 +281,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     load_rows(8);
     if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 4);
     // (cos, sin) of all rows and pairs, while those are on their way: the two CTAs of the pair serve the same
-    // tokens, each computes 64 rows for both (16 sincosf per thread took 4200 cycles). [pair][row] in V slot 0.
+    // tokens, each computes half for both (16 sincosf per thread took 4200 cycles). [pair][row] in V slot 0.
     const uint32_t cs0 = sV;
     const float *cs = reinterpret_cast<const float *>(gQ + (sV - sQ));
     if (p.n_rot == 64) {
-      const int tr = (int)rank * 64 + (threadIdx.x & 63), tp = (threadIdx.x >> 6) * 8;   // row, first of 8 pairs
+      const int id = (int)rank * 256 + threadIdx.x, tr = id & (rows_cs - 1);   // row, and rows_cs / 16 pairs of it
+      const int tp = id / rows_cs * (rows_cs / 16);
       const float fpos = (float)s_pos[tr];
       const uint32_t peer = cluster_addr(cs0, rank ^ 1), peer_bar = cluster_addr(bars + 8 * kBarT, rank ^ 1);
 #pragma unroll 1
-      for (int i = 0; i < 8; i += 4) {
-        float2 v[4];
+      for (int i = 0; i < rows_cs / 16; i += 2) {
+        float2 v[2];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sincosf(fpos * p.freq[tp + i + e], &v[e].y, &v[e].x);
+        for (int e = 0; e < 2; ++e) sincosf(fpos * p.freq[tp + i + e], &v[e].y, &v[e].x);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < 2; ++e) {
           const uint32_t at = 8u * ((tp + i + e) * kPfM + tr);
           sts64(cs0 + at, __float_as_uint(v[e].x), __float_as_uint(v[e].y));
           // (completes on the peer's barrier by bytes: no fence, no remote arrive)
@@ -539,8 +543,22 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t bar_ref = bars + 8 * (kBarR + 2 * (warp & 3));
     bool ok = true;
+    const bool live = row0 + 32 * (warp & 3) < p.n_q;
     for (int j = set; j < nt && ok; j += 2) {
       const int st = set;   // tile j's P buffer: j & 1
+      if (!live) {   // none of the warp's rows exists: hands the buffers on
+        if (!mbar_wait(bars + 8 * (kBarS + st), (j >> 1) & 1, p.status, 14) ||
+            (j >= 2 && !mbar_wait(bars + 8 * (kBarO + st), ((j - 2) >> 1) & 1, p.status, 21))) {
+          ok = false;
+          break;
+        }
+        if (lane == 0) {
+          mbar_arrive_peer(lead + 8 * kBarL);
+          mbar_arrive_peer(lead + 8 * (kBarP + 2 * st));
+          mbar_arrive_peer(lead + 8 * (kBarP + 2 * st + 1));
+        }
+        continue;
+      }
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 0);
       // the reference tile j - 1 left: its set published it right after its own maxima,
       // long before this tile's scores are ready -- fetched first, off the critical path
@@ -704,6 +722,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
 #pragma unroll 1
       for (int b = ch; b < 8; b += 2) {
         uint32_t o[32];
+        if (row0 + 32 * (warp & 3) >= p.n_q) {   // none of the warp's rows exists: only the barrier below
+          asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
+          continue;
+        }
         if (have) {
           tmem_ld32(lane_addr + kTmemO + 32 * b, o);
           tmem_wait_ld();
