@@ -544,6 +544,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const uint32_t bar_ref = bars + 8 * (kBarR + 2 * (warp & 3));
     bool ok = true;
     const bool live = row0 + 32 * (warp & 3) < p.n_q;
+    // Rows past the last query see every key: nobody reads what they give, and a mask on their account would
+    // be a mask on every tile (24 queries at 16000: 94 us a layer with it).
+    const int last_key = row0 + r < p.n_q ? my_pos : 0x7fffffff;
     for (int j = set; j < nt && ok; j += 2) {
       const int st = set;   // tile j's P buffer: j & 1
       if (!live) {   // none of the warp's rows exists: hands the buffers on
@@ -581,12 +584,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 2);
       const int key0 = (jt0 + j) * kPfN;
       // only tiles that reach past some row's last key need the causal mask
-      if (__any_sync(0xffffffffu, key0 + kPfN - 1 > my_pos)) {
+      if (__any_sync(0xffffffffu, key0 + kPfN - 1 > last_key)) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (key0 + 32 * c + i > my_pos) sc[c][i] = 0xff800000u;  // -inf
+            if (key0 + 32 * c + i > last_key) sc[c][i] = 0xff800000u;  // -inf
       }
       // eight independent chains of three-input maxima
       float mx[8];
