@@ -194,6 +194,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   if (threadIdx.x == 0) {
     s_maxpos = -1;
     s_abort = 0;
+    // Softmax warps, of both CTAs, that have a row at all: the others take no part in the loop. (Handing the
+    // buffers on instead, they poll barriers in the shared memory that the matrix unit reads its operands from:
+    // 24 queries at 24000 86 us a layer.)
+    const int live_warps = 2 * min((rows_cta + 31) / 32, 4);
     for (int i = 0; i < kPfKSlots; ++i) {
       mbar_init(bars + 8 * (kBarKFull + i), 1);
       mbar_init(bars + 8 * (kBarKFree + i), 1);
@@ -202,12 +206,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       mbar_init(bars + 8 * (kBarVFull + i), 1);
       mbar_init(bars + 8 * (kBarVFree + i), 1);
       mbar_init(bars + 8 * (kBarS + i), 1);
-      mbar_init(bars + 8 * (kBarP + 2 * i), 8);       // one elected lane per softmax warp of the
-      mbar_init(bars + 8 * (kBarP + 2 * i + 1), 8);   // tile's set (both CTAs), per 64-key half of P
+      mbar_init(bars + 8 * (kBarP + 2 * i), live_warps);       // one elected lane per softmax warp of the
+      mbar_init(bars + 8 * (kBarP + 2 * i + 1), live_warps);   // tile's set (both CTAs), per 64-key half of P
       mbar_init(bars + 8 * (kBarO + i), 1);
     }
     for (int i = 0; i < 8; ++i) mbar_init(bars + 8 * (kBarR + i), 1);
-    mbar_init(bars + 8 * kBarL, 8);
+    mbar_init(bars + 8 * kBarL, live_warps);
     mbar_init(bars + 8 * kBarQ, 16);   // one per converting warp (both CTAs)
     mbar_init(bars + 8 * kBarT, 9);    // the CTA's warps, and the bytes of the peer's half
     mbar_init(bars + 8 * kBarC, 8);
@@ -543,25 +547,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t bar_ref = bars + 8 * (kBarR + 2 * (warp & 3));
     bool ok = true;
-    const bool live = row0 + 32 * (warp & 3) < p.n_q;
+    const bool live = 32 * (warp & 3) < rows_cta;   // (the barriers count the warps that have a row)
     // Rows past the last query see every key: nobody reads what they give, and a mask on their account would
     // be a mask on every tile (24 queries at 16000: 94 us a layer with it).
     const int last_key = row0 + r < p.n_q ? my_pos : 0x7fffffff;
-    for (int j = set; j < nt && ok; j += 2) {
+    for (int j = set; live && j < nt && ok; j += 2) {
       const int st = set;   // tile j's P buffer: j & 1
-      if (!live) {   // none of the warp's rows exists: hands the buffers on
-        if (!mbar_wait(bars + 8 * (kBarS + st), (j >> 1) & 1, p.status, 14) ||
-            (j >= 2 && !mbar_wait(bars + 8 * (kBarO + st), ((j - 2) >> 1) & 1, p.status, 21))) {
-          ok = false;
-          break;
-        }
-        if (lane == 0) {
-          mbar_arrive_peer(lead + 8 * kBarL);
-          mbar_arrive_peer(lead + 8 * (kBarP + 2 * st));
-          mbar_arrive_peer(lead + 8 * (kBarP + 2 * st + 1));
-        }
-        continue;
-      }
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 0);
       // the reference tile j - 1 left: its set published it right after its own maxima,
       // long before this tile's scores are ready -- fetched first, off the critical path
@@ -679,7 +670,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       if (lane == 0) mbar_arrive_peer(lead + 8 * (kBarP + 2 * st + 1));
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 5);
     }
-    if (ok && nt > 0 && !mbar_wait(bars + 8 * (kBarO + ((nt - 1) & 1)), ((nt - 1) >> 1) & 1, p.status, 16))
+    if (live && ok && nt > 0 && !mbar_wait(bars + 8 * (kBarO + ((nt - 1) & 1)), ((nt - 1) >> 1) & 1, p.status, 16))
       ok = false;
     if (!ok) s_abort = 1;
     tc_fence_after();
