@@ -128,6 +128,14 @@ enum { kBarKFull = 0, kBarKFree = 6, kBarVFull = 12, kBarVFree = 14, kBarS = 16,
                                                    // kBarT: the (cos, sin) of the tile's rows are there;
                                                    // kBarG: the gate rows are in shared memory
 
+// The softmax warps' waits park at the barrier at once instead of polling first: eight warps that poll take
+// shared-memory cycles from the matrix unit, which reads Q, K and V there (512 tokens at 7680: 119.0 -> 117.5
+// us a layer, 128 at 24000: 84.1 -> 83.0). The issuers' waits are on the critical path and go on polling.
+__device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, DeviceStatus *status, int site) {
+  for (int i = 0; i < 12; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait(bar, parity, status, site);   // bounded
+}
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_constant__ PrefillArgs p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) unsigned long long s_bars[kBarCount];
@@ -558,10 +566,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       // long before this tile's scores are ready -- fetched first, off the critical path
       float m_prev = -1.0e30f;
       if (j > 0) {
-        if (!mbar_wait(bar_ref + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, p.status, 20)) { ok = false; break; }
+        if (!mbar_wait_parked(bar_ref + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, p.status, 20)) { ok = false; break; }
         m_prev = s_ref[(j - 1) & 1][r];
       }
-      if (!mbar_wait(bars + 8 * (kBarS + st), (j >> 1) & 1, p.status, 14)) { ok = false; break; }
+      if (!mbar_wait_parked(bars + 8 * (kBarS + st), (j >> 1) & 1, p.status, 14)) { ok = false; break; }
       tc_fence_after();
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 1);
       uint32_t sc[4][32];
@@ -604,7 +612,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         // O is rescaled in tensor memory: P V of tile j - 1 must be done, and no later one
         // can start before this tile's P arrives
         const float f = ex2(m_prev - m_new);   // 1 for rows that keep their reference
-        if (!mbar_wait(bars + 8 * (kBarO + ((j - 1) & 1)), ((j - 1) >> 1) & 1, p.status, 17)) {
+        if (!mbar_wait_parked(bars + 8 * (kBarO + ((j - 1) & 1)), ((j - 1) >> 1) & 1, p.status, 17)) {
           ok = false;
           break;
         }
@@ -627,7 +635,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       // (the 128 exponentials alone are 1024 on the special-function unit) against ~1600
       // with scalar adds
       // (P V of tile j - 2 has read this buffer)
-      if (j >= 2 && !mbar_wait(bars + 8 * (kBarO + st), ((j - 2) >> 1) & 1, p.status, 21)) { ok = false; break; }
+      if (j >= 2 && !mbar_wait_parked(bars + 8 * (kBarO + st), ((j - 2) >> 1) & 1, p.status, 21)) { ok = false; break; }
       tc_fence_after();
       unsigned long long neg_m = f2_pack(-m_new, -m_new);
       unsigned long long ls2[4] = {0ull, 0ull, 0ull, 0ull};
@@ -670,7 +678,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       if (lane == 0) mbar_arrive_peer(lead + 8 * (kBarP + 2 * st + 1));
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 5);
     }
-    if (live && ok && nt > 0 && !mbar_wait(bars + 8 * (kBarO + ((nt - 1) & 1)), ((nt - 1) >> 1) & 1, p.status, 16))
+    if (live && ok && nt > 0 && !mbar_wait_parked(bars + 8 * (kBarO + ((nt - 1) & 1)), ((nt - 1) >> 1) & 1, p.status, 16))
       ok = false;
     if (!ok) s_abort = 1;
     tc_fence_after();
