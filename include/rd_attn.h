@@ -142,7 +142,8 @@ int rd_pre_attn_fused(const float *q_gate, const float *k_src, const float *v_sr
  * min(16, n_keys / 512) for quantized ones; forced > 0 overrides (the RD_ATTN_SPLITS
  * knob), capped at 16. Host arithmetic only.
  *
- * rd_attn_plan reports what THIS library does with a decode launch on a GPU of sm_count
+ * rd_attn_plan reports what THIS library does with a decode launch whose CTAs each serve all
+ * heads (the form of long contexts and of records-only calls) on a GPU of sm_count
  * SMs (<= 0: the current device): keys per shared-memory tile (16, 32 or 48 by K / V type),
  * stages of the TMA ring, and the internal split count (about one CTA per SM, never more
  * splits than key tiles). Any output pointer may be NULL. Host arithmetic only when
@@ -194,8 +195,8 @@ int rd_attn_decode_ws(const float *q, const void *k, const void *v, float *out, 
  * kv_store_row_launch twice, then attn_launch_split, graph.cuh:1011-1035 and 958-977).
  * Stores k_new / v_new ([n_head_kv][head_dim] f32, K already normalised and rotated) as
  * row t of the caches and returns the attention of q over keys 0..t, the new one
- * included: the first CTAs of the split-KV launch quantize and store the row while the
- * launch attends keys 0..t-1, and the merge folds key t in from the cache. Cache bytes
+ * included: the CTA of the decode launch that attends key t quantizes the row, stores it and
+ * attends it from shared memory. Short contexts take one launch (no merge). Cache bytes
  * equal rd_kv_append's; the output equals rd_attn_decode_ws after rd_kv_append within
  * the attention tolerance. q must not alias out (RD_ERR_UNSUPPORTED). gate as in
  * rd_attn_decode_ws; workspace from rd_attn_workspace_bytes(1, ...). */
@@ -221,8 +222,9 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
  * The descriptor array is read on the host during the call; the workspace
  * (rd_attn_multi_workspace_bytes, 256-byte aligned, device memory) receives the device
  * copies, the work list and the partial records, and must stay untouched until the
- * stream has passed the call. The call enqueues a host-to-device copy from pageable
- * memory, so it cannot be part of a stream capture. */
+ * stream has passed the call. The call uploads a plan that holds for this step only (in
+ * kernel parameters, or by a copy from pageable memory when it is larger than those), so it
+ * must not be part of a stream capture. */
 typedef struct rd_attn_seq {
   const float *q;
   const void *k;
@@ -376,11 +378,9 @@ int rd_fa2_prefill(const float *q, const void *k, const void *v, float *o, const
 /* The same kernel with its fused edges (no single counterpart in the reference: it is
  * rope_launch on q, include/rdna4/attn.cuh:56-63, + the prefill attention + the sigmoid
  * gate of nn.cuh:405-420 in one launch). n_rot > 0 (a multiple of 16, <= 64) rotates
- * the first n_rot dims of every query row by its pos[] -- in a pre-pass that writes the
- * rotated, scaled queries as f16 into the library's grown workspace (512 bytes per token
- * and head; the tile kernel starts under it as a programmatic dependent launch and loads
- * its query tile by TMA), so q itself is not modified unless it aliases o; the K rows in
- * the cache must already be rotated (use rd_kv_append with pos). gate != NULL multiplies
+ * the first n_rot dims of every query row by its pos[] -- while the tile kernel brings its
+ * query tile to f16, so q itself is not modified unless it aliases o; the K rows in the
+ * cache must already be rotated (use rd_kv_append with pos). gate != NULL multiplies
  * the output by sigmoid(gate); the gate buffer is read only. q, o and gate must be 16-byte
  * aligned. */
 int rd_attn_prefill_fused(const float *q, const void *k, const void *v, float *o, const float *gate,
@@ -389,10 +389,10 @@ int rd_attn_prefill_fused(const float *q, const void *k, const void *v, float *o
 
 /* The chunk's cache append fused in as well (f16 caches): rd_kv_append(k_new, v_new -> rows
  * row0 .. row0 + n_q - 1, K rotated by pos[] when n_rot > 0; kv_store_row_launch,
- * include/rdna4/kv.h:673-694, + rope_launch on k) and rd_attn_prefill_fused in one call. The
- * pre-pass that rotates the queries stores the new rows too -- the (cos, sin) of a token
- * are computed once for its 24 query and 4 key rows -- and writes the bytes rd_kv_append
- * writes. k_new / v_new are [n_q][n_head_kv][head_dim] f32, 16-byte aligned;
+ * include/rdna4/kv.h:673-694, + rope_launch on k) and rd_attn_prefill_fused in one call. A
+ * pre-pass stores the new rows, with the bytes rd_kv_append writes, and the tile kernel
+ * starts under it as a programmatic dependent launch. k_new / v_new are
+ * [n_q][n_head_kv][head_dim] f32, 16-byte aligned;
  * row0 + n_q <= keys_total. */
 int rd_attn_prefill_append_fused(const float *q, const float *k_new, const float *v_new, void *k, void *v,
                                  float *o, const float *gate, const int32_t *pos, int n_q, int row0,
@@ -403,8 +403,8 @@ int rd_attn_prefill_append_fused(const float *q, const float *k_new, const float
  * serves with its chunk path, attn_split_batch_launch (include/rdna4/attn.cuh:958-1049, all
  * 6 x 6 K x V types; dispatch src/graph.cuh:1486-1527), where every one of the n_q tokens
  * re-streams and re-expands its prefix. Here the caches that are not f16 are expanded ONCE
- * into `workspace` (rd_attn_prefill_workspace_bytes, which also covers the rotated f16
- * queries of a call with n_rot > 0 and the records of the key split) with the exact values of the reference's dequantizing loads
+ * into `workspace` (rd_attn_prefill_workspace_bytes, which also covers the records of
+ * the key split) with the exact values of the reference's dequantizing loads
  * (kv.h:174-368) rounded to f16, and the tcgen05 prefill kernel runs over that copy. Arguments as rd_attn_prefill_fused; token i attends
  * keys 0..pos[i], keys_total rows must exist. No allocation, no host synchronisation. */
 size_t rd_attn_prefill_workspace_bytes(int k_type, int v_type, int n_q, int keys_total, int n_head,
