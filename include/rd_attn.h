@@ -255,6 +255,11 @@ int rd_attn_decode_multi(const rd_attn_seq *seqs, int n_seq, int q_len, int n_he
  *                         replay's copy has completed. From pageable memory it behaves as
  *                         rd_attn_decode_multi (which is these two calls in a row). */
 size_t rd_attn_multi_plan_bytes(int n_seq, int q_len);
+/* The key split of such a call on a GPU of sm_count SMs (<= 0: the current device): t[i] is the last
+ * key of sequence i, n_splits[i] receives the items that its keys are cut into, each with one record
+ * per token and head. Both arrays are host memory. Host arithmetic only when sm_count is given. */
+int rd_attn_multi_split(const int32_t *t, int n_seq, int q_len, int n_head_kv, int k_type, int v_type,
+                        int sm_count, int32_t *n_splits);
 int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head, int n_head_kv,
                        int head_dim, int k_type, int v_type, int pad_items, void *plan, size_t plan_bytes);
 int rd_attn_multi_launch(const void *plan, float scale, void *workspace, size_t workspace_bytes,

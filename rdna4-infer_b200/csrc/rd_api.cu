@@ -597,6 +597,68 @@ size_t rd_attn_multi_plan_bytes(int n_seq, int q_len) {
   return kMultiPlanHeaderBytes + align256((size_t)n_seq * sizeof(DecodeSeq)) + align256(items * sizeof(int4));
 }
 
+// Key split of a many-sequence call: sequence i attends keys 0..t[i], in n_splits[i] items per chunk of its
+// tokens. Chunks of equal length over all sequences, so that a 32k-key sequence and a 1k-key one load
+// the SMs evenly, and in whole waves of CTAs (blocks of tokens, q_len > 1, are CTAs per KV head). A wave
+// costs about 10 us beside its tiles (prologue, epilogue, records). Fewer waves only where that is clearly
+// less, since items of different lengths level out over more. Measured: 8 sequences of 4000 to 30000 keys,
+// q8_0/f16, 2 / 3 / 4 per SM: 94 / 107 / 116 us; 64 of 1024 to 32768 about / in four waves: 496 / 449.
+static void multi_splits(const int *t, int n_seq, int q_len, int n_head_kv, int k_type, int v_type, int sms,
+                         int *n_splits) {
+  const int tok_chunk = block_chunk(q_len), n_chunks = (q_len + tok_chunk - 1) / tok_chunk;
+  const bool block = q_len > 1;
+  const int tile = block ? 64 : decode_tile_keys(k_type, v_type);
+  const int wave = block ? std::max(1, sms / n_head_kv) : sms;
+  // An item writes a record per token and head, and the workspace holds 4 * sms + n_seq * q_len records per head:
+  // the items of split sequences take the first part, one item per sequence and chunk always fits the second.
+  // (With one KV head a wave of items of five tokens and more is already beyond that.)
+  const int64_t room = 4 * sms / tok_chunk;
+  const int most_waves = block ? std::max(1, std::min(8, 4 * sms / tok_chunk / wave)) : 4;
+  // 42 GB/s an SM; a block's tile is bound by its MMAs
+  const double tile_us = block ? 0.11 * tok_chunk * kGroup / 8 * 4
+                               : (double)tile * n_head_kv * (row_bytes(k_type) + row_bytes(v_type)) / 42e3;
+  std::vector<int> tiles(n_seq);
+  int64_t total = 0;
+  int longest = 1;
+  for (int i = 0; i < n_seq; ++i) {
+    tiles[i] = (t[i] + tile) / tile;  // ceil((t + 1) / tile)
+    total += (int64_t)tiles[i] * n_chunks;
+    longest = std::max(longest, tiles[i]);
+  }
+  int64_t chunk = 0;
+  double best = 0;
+  for (int k = most_waves; k >= 1; --k) {
+    const int64_t most = std::min((int64_t)k * wave, room);
+    int64_t c = std::max<int64_t>(4, (total + most - 1) / most), items = 0;
+    for (;; c += 1 + c / 32) {   // the smallest chunk whose items fit into k waves
+      items = 0;
+      for (int i = 0; i < n_seq; ++i) items += (int64_t)n_chunks * ((tiles[i] + (int)c - 1) / (int)c);
+      if (items <= most || c >= longest) break;
+    }
+    const double cost = (double)((items + wave - 1) / wave) * (10.0 + tile_us * total / items);
+    if (chunk == 0 || cost < 0.92 * best) best = cost, chunk = c;
+  }
+  for (int i = 0; i < n_seq; ++i) n_splits[i] = std::max(1, (int)((tiles[i] + chunk - 1) / chunk));
+}
+
+int rd_attn_multi_split(const int32_t *t, int n_seq, int q_len, int n_head_kv, int k_type, int v_type, int sm_count,
+                        int32_t *n_splits) {
+  if (!known_type(k_type) || !known_type(v_type)) return RD_ERR_TYPE;
+  if (n_head_kv != 1 && n_head_kv != 2 && n_head_kv != 4) return RD_ERR_UNSUPPORTED;
+  if (n_seq < 1 || q_len < 1) return RD_ERR_SHAPE;
+  if (t == nullptr || n_splits == nullptr) return RD_ERR_NULL;
+  for (int i = 0; i < n_seq; ++i)
+    if (t[i] < q_len - 1) return RD_ERR_SHAPE;
+  if (sm_count <= 0) {
+    int dev;
+    const int rc = current_device(&dev);
+    if (rc != RD_OK) return rc;
+    sm_count = ::sm_count(dev);
+  }
+  multi_splits(t, n_seq, q_len, n_head_kv, k_type, v_type, sm_count, n_splits);
+  return RD_OK;
+}
+
 int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head, int n_head_kv,
                        int head_dim, int k_type, int v_type, int pad_items, void *plan, size_t plan_bytes) {
   int rc = check_attn_shape(n_head, n_head_kv, head_dim, k_type, v_type);
@@ -620,47 +682,16 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
     return RD_ERR_WORKSPACE;
   if (pad_items > max_items) return RD_ERR_LIMIT;
 
-  // Key split: chunks of equal length over all sequences, so that a 32k-key sequence and a 1k-key one load
-  // the SMs evenly, and in whole waves of CTAs (blocks of tokens, q_len > 1, are CTAs per KV head). A wave
-  // costs about 10 us beside its tiles (prologue, epilogue, records). Fewer waves only where that is clearly
-  // less, since items of different lengths level out over more. Measured: 8 sequences of 4000 to 30000 keys,
-  // q8_0/f16, 2 / 3 / 4 per SM: 94 / 107 / 116 us; 64 of 1024 to 32768 about / in four waves: 496 / 449.
-  const int tok_chunk = block_chunk(q_len), n_chunks = (q_len + tok_chunk - 1) / tok_chunk;
-  const bool block = q_len > 1;
-  const int tile = block ? 64 : decode_tile_keys(k_type, v_type);
-  const int wave = block ? std::max(1, sms / n_head_kv) : sms;
-  // (records: an item of a block has one per token and head, the workspace holds 4 * sms + n_seq * q_len items' worth
-  // of one token)
-  const int most_waves = block ? std::max(1, std::min(8, 4 * sms / tok_chunk / wave)) : 4;
-  // 42 GB/s an SM; a block's tile is bound by its MMAs
-  const double tile_us = block ? 0.11 * tok_chunk * kGroup / 8 * 4
-                               : (double)tile * n_head_kv * (row_bytes(k_type) + row_bytes(v_type)) / 42e3;
-  std::vector<int> tiles(n_seq);
-  int64_t total = 0;
-  int longest = 1;
-  for (int i = 0; i < n_seq; ++i) {
-    tiles[i] = (seqs[i].t + tile) / tile;  // ceil((t + 1) / tile)
-    total += (int64_t)tiles[i] * n_chunks;
-    longest = std::max(longest, tiles[i]);
-  }
-  int64_t chunk = 0;
-  double best = 0;
-  for (int k = most_waves; k >= 1; --k) {
-    int64_t c = std::max<int64_t>(4, (total + (int64_t)k * wave - 1) / ((int64_t)k * wave)), items = 0;
-    for (;; c += 1 + c / 32) {   // the smallest chunk whose items fit into k waves
-      items = 0;
-      for (int i = 0; i < n_seq; ++i) items += (int64_t)n_chunks * ((tiles[i] + (int)c - 1) / (int)c);
-      if (items <= (int64_t)k * wave || c >= longest) break;
-    }
-    const double cost = (double)((items + wave - 1) / wave) * (10.0 + tile_us * total / items);
-    if (chunk == 0 || cost < 0.92 * best) best = cost, chunk = c;
-  }
+  std::vector<int> last(n_seq), splits(n_seq);
+  for (int i = 0; i < n_seq; ++i) last[i] = seqs[i].t;
+  multi_splits(last.data(), n_seq, q_len, n_head_kv, k_type, v_type, sms, splits.data());
+  const int tok_chunk = block_chunk(q_len);
   unsigned char *body = (unsigned char *)plan + kMultiPlanHeaderBytes;
   DecodeSeq *hs = reinterpret_cast<DecodeSeq *>(body);
   int4 *hi = reinterpret_cast<int4 *>(body + off_items);
   std::vector<int> order(n_seq);
   for (int i = 0; i < n_seq; ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return tiles[a] > tiles[b]; });
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return last[a] > last[b]; });
   int64_t rec_base = 0;
   int n_items = 0;
   for (int i = 0; i < n_seq; ++i) {
@@ -672,11 +703,11 @@ int rd_attn_multi_plan(const rd_attn_seq *seqs, int n_seq, int q_len, int n_head
     d.out = seqs[i].out;
     d.gate = seqs[i].gate;
     d.t = seqs[i].t;
-    int ns = (int)((tiles[i] + chunk - 1) / chunk);
-    d.n_splits = ns < 1 ? 1 : ns;
+    d.n_splits = splits[i];
     d.rec_base = (int)rec_base;
     rec_base += (int64_t)d.n_splits * q_len * n_head;
   }
+  if (rec_base > (int64_t)max_items * n_head) return RD_ERR_WORKSPACE;  // cannot happen, see multi_splits
   for (int oi = 0; oi < n_seq; ++oi) {  // longest sequences first
     const int i = order[oi];
     for (int sp = 0; sp < hs[i].n_splits; ++sp)

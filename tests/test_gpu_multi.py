@@ -210,3 +210,25 @@ def test_plan_and_launch_captured_with_a_growing_context(G, oracle):
     assert lib.rd_attn_multi_launch(None, 1 / 16, rd.ptr(ws), wbytes, G.st()) == rd.ERR_NULL
     bad = torch.zeros(pbytes, dtype=torch.uint8)
     assert lib.rd_attn_multi_launch(bad.data_ptr(), 1 / 16, rd.ptr(ws), wbytes, G.st()) == rd.ERR_SHAPE
+
+
+@pytest.mark.parametrize("q_len", [5, 8, 13])
+def test_one_kv_head_long_blocks(G, oracle, q_len):
+    """One KV head and blocks of five tokens and more: a wave of items would write more records than the
+    workspace holds, so the split is bounded by them. The bytes behind the workspace stay as they were."""
+    rd, lib = G.rd, G.lib
+    n, kt, vt = 14000, 3, 2
+    rng = np.random.default_rng(q_len)
+    K, V = (rng.standard_normal((n, 1, HD)).astype(np.float32) for _ in range(2))
+    q = rng.standard_normal((q_len, 6, HD)).astype(np.float32)
+    kc, vc = oracle.kv_store_rows(kt, K), oracle.kv_store_rows(vt, V)
+    dq, dk, dv, out = G.dev(q), G.dev(kc), G.dev(vc), G.poison(q.shape)
+    arr = (rd.AttnSeq * 1)()
+    arr[0].q, arr[0].k, arr[0].v, arr[0].out, arr[0].t = rd.ptr(dq), rd.ptr(dk), rd.ptr(dv), rd.ptr(out), n - 1
+    nb = lib.rd_attn_multi_workspace_bytes(1, q_len, 6, HD)
+    ws = torch.full((nb + 8 * 148 * 6 * 258 * 4,), 0x5A, dtype=torch.uint8, device="cuda")
+    rd.check(lib.rd_attn_decode_multi(C.addressof(arr), 1, q_len, 6, 1, HD, 1 / 16, kt, vt, rd.ptr(ws), nb, G.st()))
+    torch.cuda.synchronize()
+    assert bool((ws[nb:] == 0x5A).all())
+    check_attn(G.host(out), oracle.attn(q, kc, vc, np.arange(n - q_len, n, dtype=np.int32), 1, 1 / 16, kt, vt))
+    G.status_ok()
