@@ -17,6 +17,10 @@
 //     rows, and warp w multiplies all 64 keys with its quarter of the output dims: every V value is
 //     dequantized once, by one warp, and a warp holds 16 NT accumulators where a warp with all dims
 //     would hold 64 NT.
+// The columns of a slot share its V rows, also those behind the last key of a column's own token, with weight
+// 0. A non-finite value there (an f16 cache saturates to infinity) would make that 0 a NaN, so a launch whose
+// accumulators are not all finite runs the key loop once more, token by token (careful_pv). Any other launch pays
+// one check of its accumulators for that.
 // (Tensor-map boxes of one head's rows were the slower copy: the TMA unit fetches whole cache lines,
 // and a 272-byte row of q8_0 lies in three of them. 64 sequences of config 5 verifying four tokens:
 // copies alone 817 us.)
@@ -97,6 +101,34 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
   uint2 v;
   asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
   return v;
+}
+
+// The keys 2 tq, 2 tq + 1, 2 tq + 8 and 2 tq + 9 behind `first` that are at most t: masks of an A fragment's halves.
+__device__ __forceinline__ uint2 key_mask(int first, int t) {
+  const uint32_t lo = (first <= t ? 0xffffu : 0u) | (first + 1 <= t ? 0xffff0000u : 0u);
+  const uint32_t hi = (first + 8 <= t ? 0xffffu : 0u) | (first + 9 <= t ? 0xffff0000u : 0u);
+  return make_uint2(lo, hi);
+}
+// O += V^T P^T of 16 keys (from key0 on) and one M-tile, every token with its own keys only: rows behind its last
+// key count as zeros, and of a product only the token's six columns are taken.
+template <int NT>
+__device__ __forceinline__ void careful_pv(float (&O)[NT][4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                        const uint2 (&pb)[NT], const int *s_t, int n_tok, int key0, int tq) {
+#pragma unroll 1
+  for (int j = 0; j < n_tok; ++j) {
+    const uint2 mask = key_mask(key0 + 2 * tq, s_t[kGroup * j]);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      if (kGroup * j + kGroup <= 8 * nt || kGroup * j >= 8 * nt + 8) continue;   // no column of this token
+      float x[4] = {0.f, 0.f, 0.f, 0.f};
+      mma16816(x, a0 & mask.x, a1 & mask.x, a2 & mask.y, a3 & mask.y, pb[nt].x, pb[nt].y);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int c = 8 * nt + 2 * tq + (e & 1);
+        if (c >= kGroup * j && c < kGroup * j + kGroup) O[nt][e] += x[e];
+      }
+    }
+  }
 }
 
 template <int KT, int VT, int NT>
@@ -208,11 +240,14 @@ block_kernel(const __grid_constant__ BlockArgs p) {
                     t_max, lane);
     cp_async_commit();
   };
+  auto fill_first = [&] {
 #pragma unroll 1
-  for (int i = 0; i < DK; ++i) {
-    fill_k(i);
-    if (i + 1 < DV) fill_v(i);
-  }
+    for (int i = 0; i < DK; ++i) {
+      fill_k(i);
+      if (i + 1 < DV) fill_v(i);
+    }
+  };
+  fill_first();
 
   for (int c = threadIdx.x; c < COLS; c += Geo::kThreads) {
     const int j = c / kGroup;
@@ -241,118 +276,144 @@ block_kernel(const __grid_constant__ BlockArgs p) {
 
   float O[4][NT][4];                     // [M-tile of this warp's quarter of the dims][column tile]
   float ref[NT][2], run[NT][2], l[NT][2];   // per lane column: team's reference, lane-local maximum and sum
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
-    ref[nt][0] = ref[nt][1] = run[nt][0] = run[nt][1] = kBlkNone;
-    l[nt][0] = l[nt][1] = 0.f;
-#pragma unroll
-    for (int m = 0; m < 4; ++m) O[m][nt][0] = O[m][nt][1] = O[m][nt][2] = O[m][nt][3] = 0.f;
-  }
   const uint32_t qlane = qfrag + lane * 16;
+  bool careful = false;
 #pragma unroll 1
-  for (int i = 0; i < n_mine; ++i) {
-    const int row0 = (c_b + team + i * TEAMS) * kBlkKeys;
-    cp_async_wait<WAIT_K>();
-    __syncwarp();
-    // ---- S = K Q^T: this warp's 16 keys x all columns ----
-    float Sv[NT][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) Sv[nt][0] = Sv[nt][1] = Sv[nt][2] = Sv[nt][3] = 0.f;
-    {
-      const uint32_t kr = ring_k + (i % DK) * SK + (16 * part + g) * PK;
-      uint4 qf[NT];
-      KL::run(kr, kr + 8 * PK, tq, [&](int n, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          if ((n & 1) == 0) qf[nt] = lds128(qlane + nt * 4096 + (n >> 1) * 512);
-          mma16816(Sv[nt], a0, a1, a2, a3, (n & 1) ? qf[nt].z : qf[nt].x, (n & 1) ? qf[nt].w : qf[nt].y);
-        }
-      });
-    }
-    __syncwarp();
-    fill_k(i + DK);
-    if (row0 + kBlkKeys - 1 > t_min) {   // some column ends inside or before this slot
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (row0 + 16 * part + g + (e >> 1) * 8 > s_t[8 * nt + 2 * tq + (e & 1)]) Sv[nt][e] = -INFINITY;
-    }
-    bool grow = false;
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        run[nt][e] = fmaxf(run[nt][e], fmaxf(Sv[nt][e], Sv[nt][e + 2]));
-        grow |= run[nt][e] > ref[nt][e] + kBlkSlack;
-      }
-    // every warp of the team is done with the V slot before this one
-    const bool any = team_any(team, grow);
-    fill_v(i - 1 + DV);
-    if (any) {
-      // the team's references move to the current maxima of the columns (over its 64 key rows)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float m = run[nt][e];
-#pragma unroll
-          for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
-          if (g == 0) s_max[team][part][8 * nt + 2 * tq + e] = m;
-        }
-      team_sync(team);
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int c = 8 * nt + 2 * tq + e;
-          // a whole number: the rounding of the weights to f16 then does not depend on it, and results
-          // for different key splits differ in the order of f32 sums only
-          const float m = fmaxf(ceilf(fmaxf(fmaxf(s_max[team][0][c], s_max[team][1][c]),
-                                            fmaxf(s_max[team][2][c], s_max[team][3][c]))), ref[nt][e]);
-          const float f = ex2(ref[nt][e] - m);
-          ref[nt][e] = m;
-          l[nt][e] *= f;
-#pragma unroll
-          for (int mt = 0; mt < 4; ++mt) {
-            O[mt][nt][e] *= f;
-            O[mt][nt][e + 2] *= f;
-          }
-        }
-    }
-    // ---- P^T fragments of this warp's keys -> shared memory ----
+  for (;;) {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      const float p0 = ex2(Sv[nt][0] - ref[nt][0]), p1 = ex2(Sv[nt][1] - ref[nt][1]);
-      const float p2 = ex2(Sv[nt][2] - ref[nt][0]), p3 = ex2(Sv[nt][3] - ref[nt][1]);
-      const uint32_t h01 = pack_h2(p0, p1), h23 = pack_h2(p2, p3);
-      // the sums take the weights as rounded for the tensor core: a common rounding error of a column
-      // then cancels in the quotient
-      const float2 r01 = unpack_h2(h01), r23 = unpack_h2(h23);
-      l[nt][0] += r01.x + r23.x;
-      l[nt][1] += r01.y + r23.y;
-      const uint32_t b0 = movmatrix_trans(h01), b1 = movmatrix_trans(h23);
-      asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(pfrag + (part * NT + nt) * 256 + lane * 8), "r"(b0), "r"(b1)
-                   : "memory");
+      ref[nt][0] = ref[nt][1] = run[nt][0] = run[nt][1] = kBlkNone;
+      l[nt][0] = l[nt][1] = 0.f;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) O[m][nt][0] = O[m][nt][1] = O[m][nt][2] = O[m][nt][3] = 0.f;
     }
-    cp_async_wait<WAIT_V>();
-    team_sync(team);
-    // ---- O^T += V^T P^T: 64 keys x this warp's quarter of the dims ----
+#pragma unroll 1
+    for (int i = 0; i < n_mine; ++i) {
+      const int row0 = (c_b + team + i * TEAMS) * kBlkKeys;
+      cp_async_wait<WAIT_K>();
+      __syncwarp();
+      // ---- S = K Q^T: this warp's 16 keys x all columns ----
+      float Sv[NT][4];
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      uint2 pb[NT];
+      for (int nt = 0; nt < NT; ++nt) Sv[nt][0] = Sv[nt][1] = Sv[nt][2] = Sv[nt][3] = 0.f;
+      {
+        const uint32_t kr = ring_k + (i % DK) * SK + (16 * part + g) * PK;
+        uint4 qf[NT];
+        KL::run(kr, kr + 8 * PK, tq, [&](int n, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) pb[nt] = lds64(pfrag + (ks * NT + nt) * 256 + lane * 8);
-      const uint32_t r0 = ring_v + (i % DV) * SV + (16 * ks + 2 * tq) * PV;
-      const uint32_t rows[4] = {r0, r0 + PV, r0 + 8 * PV, r0 + 9 * PV};
-      VL::run_part(rows, g, part, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+          for (int nt = 0; nt < NT; ++nt) {
+            if ((n & 1) == 0) qf[nt] = lds128(qlane + nt * 4096 + (n >> 1) * 512);
+            mma16816(Sv[nt], a0, a1, a2, a3, (n & 1) ? qf[nt].z : qf[nt].x, (n & 1) ? qf[nt].w : qf[nt].y);
+          }
+        });
+      }
+      __syncwarp();
+      fill_k(i + DK);
+      if (row0 + kBlkKeys - 1 > t_min) {   // some column ends inside or before this slot
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) mma16816(O[m][nt], a0, a1, a2, a3, pb[nt].x, pb[nt].y);
-      });
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (row0 + 16 * part + g + (e >> 1) * 8 > s_t[8 * nt + 2 * tq + (e & 1)]) Sv[nt][e] = -INFINITY;
+      }
+      bool grow = false;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          run[nt][e] = fmaxf(run[nt][e], fmaxf(Sv[nt][e], Sv[nt][e + 2]));
+          grow |= run[nt][e] > ref[nt][e] + kBlkSlack;
+        }
+      // every warp of the team is done with the V slot before this one
+      const bool any = team_any(team, grow);
+      fill_v(i - 1 + DV);
+      if (any) {
+        // the team's references move to the current maxima of the columns (over its 64 key rows)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float m = run[nt][e];
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
+            if (g == 0) s_max[team][part][8 * nt + 2 * tq + e] = m;
+          }
+        team_sync(team);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int c = 8 * nt + 2 * tq + e;
+            // a whole number: the rounding of the weights to f16 then does not depend on it, and results
+            // for different key splits differ in the order of f32 sums only
+            const float m = fmaxf(ceilf(fmaxf(fmaxf(s_max[team][0][c], s_max[team][1][c]),
+                                              fmaxf(s_max[team][2][c], s_max[team][3][c]))), ref[nt][e]);
+            const float f = ex2(ref[nt][e] - m);
+            ref[nt][e] = m;
+            l[nt][e] *= f;
+#pragma unroll
+            for (int mt = 0; mt < 4; ++mt) {
+              O[mt][nt][e] *= f;
+              O[mt][nt][e + 2] *= f;
+            }
+          }
+      }
+      // ---- P^T fragments of this warp's keys -> shared memory ----
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const float p0 = ex2(Sv[nt][0] - ref[nt][0]), p1 = ex2(Sv[nt][1] - ref[nt][1]);
+        const float p2 = ex2(Sv[nt][2] - ref[nt][0]), p3 = ex2(Sv[nt][3] - ref[nt][1]);
+        const uint32_t h01 = pack_h2(p0, p1), h23 = pack_h2(p2, p3);
+        // the sums take the weights as rounded for the tensor core: a common rounding error of a column
+        // then cancels in the quotient
+        const float2 r01 = unpack_h2(h01), r23 = unpack_h2(h23);
+        l[nt][0] += r01.x + r23.x;
+        l[nt][1] += r01.y + r23.y;
+        const uint32_t b0 = movmatrix_trans(h01), b1 = movmatrix_trans(h23);
+        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(pfrag + (part * NT + nt) * 256 + lane * 8), "r"(b0), "r"(b1)
+                     : "memory");
+      }
+      cp_async_wait<WAIT_V>();
+      team_sync(team);
+      // ---- O^T += V^T P^T: 64 keys x this warp's quarter of the dims ----
+      auto pv = [&](int ks, auto &&mma) {
+        uint2 pb[NT];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) pb[nt] = lds64(pfrag + (ks * NT + nt) * 256 + lane * 8);
+        const uint32_t r0 = ring_v + (i % DV) * SV + (16 * ks + 2 * tq) * PV;
+        const uint32_t rows[4] = {r0, r0 + PV, r0 + 8 * PV, r0 + 9 * PV};
+        VL::run_part(rows, g, part, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+          mma(m, a0, a1, a2, a3, pb);
+        });
+      };
+      if (!careful) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          pv(ks, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const uint2(&pb)[NT]) {
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) mma16816(O[m][nt], a0, a1, a2, a3, pb[nt].x, pb[nt].y);
+          });
+      } else {
+#pragma unroll 1
+        for (int ks = 0; ks < 4; ++ks)
+          pv(ks, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const uint2(&pb)[NT]) {
+            careful_pv<NT>(O[m], a0, a1, a2, a3, pb, s_t, n_tok, row0 + 16 * ks, tq);
+          });
+      }
     }
+    cp_async_wait<0>();   // (only empty groups are left)
+    float finite = 0.f;   // 0, or NaN where an accumulator is not finite
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) finite = fmaf(O[m][nt][e], 0.f, finite);
+    // (also frees the rings)
+    if (!__syncthreads_or(!careful && finite != 0.f)) break;
+    careful = true;
+    fill_first();
   }
-  cp_async_wait<0>();   // (only empty groups are left)
-  team_sync(team);      // the ring is free
 
   // ---- the teams meet ----
 #pragma unroll

@@ -1,0 +1,84 @@
+"""Values that are not finite reach the outputs that they belong to, and no others; against the oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from tests.conftest import check_attn
+
+pytestmark = pytest.mark.gpu
+NKV, NH, HD = 4, 24, 256
+F16, Q4_1 = 1, 5
+ROW = {F16: 512, Q4_1: 160}
+
+
+@pytest.fixture(scope="module")
+def G(cuda):
+    from tests import gpu_util
+    return gpu_util
+
+
+def make(oracle, seed, n, kt, vt, n_tok):
+    rng = np.random.default_rng(seed)
+    K, V = (rng.standard_normal((n, NKV, HD)).astype(np.float32) for _ in range(2))
+    q = rng.standard_normal((n_tok, NH, HD)).astype(np.float32)
+    return q, oracle.kv_store_rows(kt, K), oracle.kv_store_rows(vt, V)
+
+
+def plant(vc, want, vt, row, kvh, pos):
+    """+inf as dim 37 of a V row (f16), or as the minimum of its second block (q4_1: 32 dims); and in what the
+    tokens that attend the row give. (The oracle itself widens the bytes of infinity to 65536, as the reference does.)"""
+    at, dims = (2 * 37, slice(37, 38)) if vt == F16 else (20 + 2, slice(32, 64))
+    vc.reshape(-1, NKV, ROW[vt])[row, kvh, at:at + 2] = (0x00, 0x7C)
+    want[np.asarray(pos) >= row, 6 * kvh:6 * kvh + 6, dims] = np.inf
+
+
+def same(got, want, what):
+    fin = np.isfinite(want)
+    assert not fin.all() and (np.isfinite(got) == fin).all(), what
+    assert np.array_equal(got[~fin], want[~fin], equal_nan=True), what
+    check_attn(np.where(fin, got, 0), np.where(fin, want, 0), what=what)
+
+
+@pytest.mark.parametrize("kt,vt", [(F16, F16), (2, F16), (Q4_1, Q4_1)])
+@pytest.mark.parametrize("n,n_tok", [(5, 5), (70, 3), (400, 2), (400, 8), (9000, 5), (300, 11)])
+def test_block_tokens_do_not_see_later_rows(G, oracle, kt, vt, n, n_tok):
+    q, kc, vc = make(oracle, n + n_tok, n, kt, vt, n_tok)
+    pos = np.arange(n - n_tok, n, dtype=np.int32)
+    want = oracle.attn(q, kc, vc, pos, NKV, 1 / 16, kt, vt)
+    plant(vc, want, vt, n - 1, 2, pos)
+    plant(vc, want, vt, n - 2, 0, pos)
+    same(G.attn_batch(q, kc, vc, pos, kt, vt, n_splits=4), want, f"{n_tok} tokens, {n} keys")
+    G.status_ok()
+
+
+def test_block_ragged_positions_and_inner_rows(G, oracle):
+    n, kt, vt = 500, 2, F16
+    q, kc, vc = make(oracle, 1, n, kt, vt, 7)
+    pos = np.array([499, 0, 64, 130, 129, 131, 320], dtype=np.int32)
+    want = oracle.attn(q, kc, vc, pos, NKV, 1 / 16, kt, vt)
+    for row, kvh in ((130, 1), (131, 2), (499, 3), (65, 0)):
+        plant(vc, want, vt, row, kvh, pos)
+    same(G.attn_batch(q, kc, vc, pos, kt, vt), want, "ragged")
+
+
+def test_block_of_many_sequences(G, oracle):
+    rd, lib = G.rd, G.lib
+    q_len, kt, vt, lens = 4, 2, F16, (4, 37, 900)
+    seqs, keep = (rd.AttnSeq * len(lens))(), []
+    for i, n in enumerate(lens):
+        q, kc, vc = make(oracle, n, n, kt, vt, q_len)
+        pos = np.arange(n - q_len, n, dtype=np.int32)
+        want = oracle.attn(q, kc, vc, pos, NKV, 1 / 16, kt, vt)
+        plant(vc, want, vt, n - 1, i, pos)
+        d = [G.dev(q), G.dev(kc), G.dev(vc), G.poison(q.shape)]
+        seqs[i].q, seqs[i].k, seqs[i].v, seqs[i].out = (rd.ptr(x) for x in d)
+        seqs[i].t = n - 1
+        keep.append((d, want, n))
+    nb = lib.rd_attn_multi_workspace_bytes(len(lens), q_len, NH, HD)
+    ws = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    rd.check(lib.rd_attn_decode_multi(C.addressof(seqs), len(lens), q_len, NH, NKV, HD, 1 / 16, kt, vt, rd.ptr(ws), nb, G.st()))
+    torch.cuda.synchronize()
+    for d, want, n in keep:
+        same(G.host(d[3]), want, f"{n} keys")
