@@ -736,8 +736,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
           for (int e = 0; e < 32; ++e) o[e] = 0u;
         }
         const uint32_t brow = sQ + b * kPfBoxBytes + r * 128;
+        uint32_t nan = 0;   // columns of the row with a NaN gate
+        auto box_at = [&](int e) { return ((uint32_t)((e >> 2) ^ (r & 7)) << 4) + 4 * (e & 3); };
         if (with_gate) {
-          // (branch-free from here to the stores: 32 independent chains)
           float g[32];
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
@@ -747,7 +748,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
             g[4 * q + 2] = __uint_as_float(x.z);
             g[4 * q + 3] = __uint_as_float(x.w);
           }
-          // one reciprocal for two values; e^-g is capped at 2^60. Approximate exp and reciprocal: ~1e-6 relative
+          // A NaN gate makes its output NaN, as in the merge of a key split. (The cap on e^-g below takes a NaN, and
+          // the pair's other value must not see it. Rolled loops: a kernel that runs once pays for every line of
+          // instructions it fetches; with these 32 values unrolled 512 tokens at 0 took 0.37 us a layer longer.)
+          unsigned long long sum[2] = {0ull, 0ull};   // NaN if one of the gates is
+#pragma unroll
+          for (int e = 0; e < 16; ++e) sum[e & 1] = f2_add(sum[e & 1], f2_pack(g[2 * e], g[2 * e + 1]));
+          float n0, n1;
+          f2_unpack(f2_add(sum[0], sum[1]), n0, n1);
+          if (n0 + n1 != n0 + n1) {
+#pragma unroll 1
+            for (int e = 0; e < 32; ++e)
+              nan |= (uint32_t)((lds32(brow + box_at(e)) & 0x7fffffffu) > 0x7f800000u) << e;
+          }
+          // Branch-free from here to the stores: 32 independent chains.
+          // One reciprocal for two values; e^-g is capped at 2^60. Approximate exp and reciprocal: ~1e-6 relative
 #pragma unroll
           for (int e = 0; e < 32; ++e) g[e] = 1.0f + ex2(fminf(g[e] * -1.4426950408889634f, 60.f));
 #pragma unroll
@@ -763,6 +778,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
 #pragma unroll
         for (int q = 0; q < 8; ++q)
           sts128(brow + ((uint32_t)(q ^ (r & 7)) << 4), o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+#pragma unroll 1
+        for (; nan != 0; nan &= nan - 1)
+          asm volatile("st.shared.u32 [%0], %1;" ::"r"(brow + box_at(__ffs(nan) - 1)), "r"(0x7fffffffu) : "memory");
         fence_proxy_async();
         asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
         if (gt == 0) {

@@ -82,3 +82,29 @@ def test_block_of_many_sequences(G, oracle):
     torch.cuda.synchronize()
     for d, want, n in keep:
         same(G.host(d[3]), want, f"{n} keys")
+
+
+@pytest.mark.parametrize("n_q,pos0,splits", [(5, 0, 1), (200, 0, 1), (130, 4000, 3)])
+def test_prefill_gate_nan(G, oracle, n_q, pos0, splits):
+    """A NaN gate makes its own output NaN, with and without a key split; infinite gates give 0 and the whole value."""
+    rd, lib = G.rd, G.lib
+    n = pos0 + n_q
+    z = C.c_int()
+    rd.check(lib.rd_attn_prefill_plan(n_q, n, NH, 148, C.addressof(z), None))
+    assert z.value == splits
+    q, kc, vc = make(oracle, n, n, F16, F16, n_q)
+    pos = np.arange(pos0, n, dtype=np.int32)
+    clean = oracle.attn(q, kc, vc, pos, NKV, 1 / 16, F16, F16)
+    gate = np.random.default_rng(2).standard_normal(q.shape).astype(np.float32)
+    at = ((0, 0, 0), (0, 3, 17), (n_q - 1, 23, 255), (n_q // 2, 7, 100), (n_q // 2, 7, 102))
+    for i in at:
+        gate[i] = np.nan
+    gate[0, 3, 16], gate[1, 5, 64], gate[1, 5, 65] = np.inf, -np.inf, np.inf
+    with np.errstate(over="ignore"):
+        want = clean * (1 / (1 + np.exp(-gate)))
+    dq, dk, dv, dg, dp, out = G.dev(q), G.dev(kc), G.dev(vc), G.dev(gate), G.dev(pos), G.poison(q.shape)
+    rd.check(lib.rd_attn_prefill_fused(rd.ptr(dq), rd.ptr(dk), rd.ptr(dv), rd.ptr(out), rd.ptr(dg), rd.ptr(dp), n_q, n, NH,
+                                       NKV, HD, 1 / 16, 0, 0.0, G.st()))
+    torch.cuda.synchronize()
+    same(G.host(out), want, f"{n_q} at {pos0}")
+    G.status_ok()
