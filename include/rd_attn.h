@@ -224,7 +224,7 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
  * copies, the work list and the partial records, and must stay untouched until the
  * stream has passed the call. The call uploads a plan that holds for this step only (in
  * kernel parameters, or by a copy from pageable memory when it is larger than those), so it
- * must not be part of a stream capture. */
+ * cannot be part of a stream capture: RD_ERR_CUDA, and nothing is launched. */
 typedef struct rd_attn_seq {
   const float *q;
   const void *k;

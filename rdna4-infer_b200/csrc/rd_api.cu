@@ -768,6 +768,10 @@ static int multi_launch(const void *plan, float scale, void *workspace, size_t w
   // From pageable memory the copy has left the plan when cudaMemcpyAsync returns; from
   // pinned memory it reads the plan when the stream (or a replayed graph) reaches it.
   if (by_value) {
+    // a graph would replay this step's plan
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing((cudaStream_t)stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
+      return RD_ERR_CUDA;
     if ((rc = launch_upload((const unsigned char *)plan + kMultiPlanHeaderBytes, workspace, h.copy_bytes,
                             (cudaStream_t)stream)) != RD_OK)
       return rc;

@@ -232,3 +232,28 @@ def test_one_kv_head_long_blocks(G, oracle, q_len):
     assert bool((ws[nb:] == 0x5A).all())
     check_attn(G.host(out), oracle.attn(q, kc, vc, np.arange(n - q_len, n, dtype=np.int32), 1, 1 / 16, kt, vt))
     G.status_ok()
+
+
+@pytest.mark.parametrize("n_seq", [1, 100])   # a plan in kernel parameters, and one that is copied
+def test_decode_multi_refuses_a_stream_capture(G, n_seq):
+    rd, lib = G.rd, G.lib
+    q, out = torch.zeros(1, NH, HD, device="cuda"), torch.zeros(1, NH, HD, device="cuda")
+    kc = torch.zeros(8 * NKV * 144, dtype=torch.uint8, device="cuda")
+    arr = (rd.AttnSeq * n_seq)()
+    for a in arr:
+        a.q, a.k, a.v, a.out, a.t = rd.ptr(q), rd.ptr(kc), rd.ptr(kc), rd.ptr(out), 7
+    nb = lib.rd_attn_multi_workspace_bytes(n_seq, 1, NH, HD)
+    ws = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    call = lambda: lib.rd_attn_decode_multi(C.addressof(arr), n_seq, 1, NH, NKV, HD, 1 / 16, 3, 3, rd.ptr(ws), nb,
+                                            rd.stream_ptr())
+    assert call() == rd.OK
+    torch.cuda.synchronize()
+    x, g = torch.zeros(1, device="cuda"), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        rc = call()
+        x += 1          # the capture itself goes on
+    assert rc == rd.ERR_CUDA
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x) == 1.0 and call() == rd.OK
+    G.status_ok()
