@@ -10,7 +10,9 @@
  *
  * Conventions kept from the reference:
  *   - all pointers are caller-owned DEVICE pointers unless a comment says host;
- *   - activations are f32; q and out may be the same buffer;
+ *   - activations are f32; q and out may be the same buffer; the attention entries read q in
+ *     16-byte pieces and the caches in 16-byte copies: a q or a cache that is not 16-byte aligned
+ *     is refused with RD_ERR_ALIGN, other f32 buffers need 4 bytes where nothing else is said;
  *   - K/V caches are rows [key][n_head_kv] of `row_bytes(type, head_dim)` bytes in
  *     GGUF 32-element blocks (fp16 scale first), key j / kv head h at
  *     (j*n_head_kv + h) * row_bytes;

@@ -174,7 +174,7 @@ int attn_alloc(const float *q, const void *k, const void *v, float *out, float *
   if (q == nullptr || k == nullptr || v == nullptr) return RD_ERR_NULL;
   if (out == nullptr && records == nullptr) return RD_ERR_NULL;
   if (n_tok < 1 || n_rec < 1) return RD_ERR_SHAPE;
-  if (!aligned(q, 4) || !aligned(out, 4) || !aligned(records, 4)) return RD_ERR_ALIGN;
+  if (!aligned(q, 16) || !aligned(out, 4) || !aligned(records, 4)) return RD_ERR_ALIGN;
   if (!aligned(k, 16) || !aligned(v, 16)) return RD_ERR_ALIGN;
   int dev;
   if ((rc = current_device(&dev)) != RD_OK) return rc;
@@ -461,7 +461,7 @@ int rd_attn_decode_ws(const float *q, const void *k, const void *v, float *out, 
   if (q == nullptr || k == nullptr || v == nullptr) return RD_ERR_NULL;
   if (out == nullptr && partial == nullptr) return RD_ERR_NULL;
   if (workspace == nullptr) return RD_ERR_WORKSPACE;
-  if (!aligned(q, 4) || !aligned(out, 4) || !aligned(partial, 4) || !aligned(gate, 4))
+  if (!aligned(q, 16) || !aligned(out, 4) || !aligned(partial, 4) || !aligned(gate, 4))
     return RD_ERR_ALIGN;
   if (!aligned(k, 16) || !aligned(v, 16) || !aligned(workspace, 256)) return RD_ERR_ALIGN;
   int dev;
@@ -485,7 +485,7 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
     return RD_ERR_NULL;
   if (q == out) return RD_ERR_UNSUPPORTED;  // the merge reads whole query rows while it writes out
   if (workspace == nullptr) return RD_ERR_WORKSPACE;
-  if (!aligned(q, 4) || !aligned(out, 4) || !aligned(gate, 4) || !aligned(k_new, 4) || !aligned(v_new, 4))
+  if (!aligned(q, 16) || !aligned(out, 4) || !aligned(gate, 4) || !aligned(k_new, 4) || !aligned(v_new, 4))
     return RD_ERR_ALIGN;
   if (!aligned(k_cache, 16) || !aligned(v_cache, 16) || !aligned(workspace, 256)) return RD_ERR_ALIGN;
   int dev;
@@ -545,7 +545,7 @@ int rd_attn_decode_noalloc(const float *q, const void *k, const void *v, float *
   int rc = check_attn_shape(n_head, n_head_kv, head_dim, k_type, v_type);
   if (rc != RD_OK) return rc;
   if (q == nullptr || k == nullptr || v == nullptr || out == nullptr) return RD_ERR_NULL;
-  if (!aligned(q, 4) || !aligned(out, 4) || !aligned(gate, 4)) return RD_ERR_ALIGN;
+  if (!aligned(q, 16) || !aligned(out, 4) || !aligned(gate, 4)) return RD_ERR_ALIGN;
   if (!aligned(k, 16) || !aligned(v, 16)) return RD_ERR_ALIGN;
   int dev;
   if ((rc = current_device(&dev)) != RD_OK) return rc;
@@ -913,7 +913,7 @@ static int decode_sharded(const float *q, const float *k_new, const float *v_new
   ShardPeers g;
   if ((rc = shard_peers(group, &g)) != RD_OK) return rc;
   if (workspace == nullptr) return RD_ERR_WORKSPACE;
-  if (!aligned(q, 4) || !aligned(out, 4) || !aligned(gate, 4)) return RD_ERR_ALIGN;
+  if (!aligned(q, 16) || !aligned(out, 4) || !aligned(gate, 4)) return RD_ERR_ALIGN;
   if (!aligned(k, 16) || !aligned(v, 16) || !aligned(workspace, 256)) return RD_ERR_ALIGN;
   int dev;
   if ((rc = current_device(&dev)) != RD_OK) return rc;

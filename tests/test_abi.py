@@ -105,3 +105,27 @@ def test_cpp_wrappers_compile_and_behave(rd, tmp_path):
                            "-L" + rd.HERE, "-lrd_attn_b200", "-Wl,-rpath," + rd.HERE])
     out = subprocess.run([exe], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout + out.stderr
+
+
+def test_misaligned_queries_are_refused(rd):
+    """The decode-side kernels read whole 16-byte pieces of a query row: refused on the host, before a device is asked."""
+    L = rd.lib
+    buf = np.zeros(8192, dtype=np.float32)
+    p = (buf.ctypes.data + 255) & ~255
+    for off in (4, 8, 12):
+        q = p + off
+        assert L.rd_attn_decode(q, p, p, p, 5, 24, 4, 256, 0.0625, 3, 3, None) == rd.ERR_ALIGN
+        assert L.rd_attn_decode_split(q, p, p, p, p, 5, 24, 4, 256, 0.0625, 3, 3, 4, None) == rd.ERR_ALIGN
+        assert L.rd_attn_decode_split(q, p, p, None, p, 5, 24, 4, 256, 0.0625, 3, 3, 4, None) == rd.ERR_ALIGN
+        assert L.rd_attn_decode_ws(q, p, p, p, None, 0, 5, 24, 4, 256, 0.0625, 3, 3, 1, None, p, 1 << 30,
+                                   None) == rd.ERR_ALIGN
+        assert L.rd_attn_decode_append_ws(q, p, p, p, p, p, 5, 24, 4, 256, 0.0625, 3, 3, None, p, 1 << 30,
+                                          None) == rd.ERR_ALIGN
+        assert L.rd_attn_decode_noalloc(q, p, p, p, 5, 24, 4, 256, 0.0625, 3, 3, None, None) == rd.ERR_ALIGN
+        assert L.rd_attn_batch(q, p, p, p, p, 2, 24, 4, 256, 0.0625, 3, 3, None) == rd.ERR_ALIGN
+        assert L.rd_attn_split_batch(q, p, p, p, p, p, 2, 24, 4, 256, 0.0625, 3, 3, 4, None) == rd.ERR_ALIGN
+        peers = rd.shard_group(0, [p])
+        assert L.rd_attn_decode_sharded(q, p, p, p, 5, 24, 4, 256, 0.0625, 3, 3, None, p, 1 << 30, C.addressof(peers),
+                                        None) == rd.ERR_ALIGN
+        assert L.rd_attn_decode_sharded_append(q, p, p, p, p, p, 5, 24, 4, 256, 0.0625, 3, 3, None, p, 1 << 30,
+                                               C.addressof(peers), None) == rd.ERR_ALIGN
