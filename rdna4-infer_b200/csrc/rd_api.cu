@@ -103,6 +103,26 @@ size_t partial_floats(int n_tok, int n_head, int splits) {
   return (size_t)n_tok * n_head * splits * kRec;
 }
 
+// What a decode call of one token that writes its output runs: one cluster of `splits` CTAs per KV head, `splits` CTAs
+// per KV head with records, or `splits` CTAs for all heads with records (step_splits, step_record_splits,
+// plan_splits). `all_heads` is the last one's count for the call; the records of the forms differ in number, and a
+// workspace that holds the records of that one is enough for every length: the per-head form is taken
+// where its own fit as well, and the cluster form has none.
+enum DecodeForm { kFormClusters, kFormHeadRecords, kFormAllHeads };
+struct DecodePlan {
+  DecodeForm form;
+  int splits;
+  size_t need;   // bytes of workspace without which the call is refused
+};
+DecodePlan plan_decode(int sms, int n_head, int n_head_kv, int kt, int vt, int64_t n_keys, int all_heads,
+                       size_t ws_bytes) {
+  const auto bytes = [&](int splits) { return partial_floats(1, n_head, splits) * sizeof(float); };
+  if (const int s = step_splits(kt, vt, n_head_kv, n_keys)) return {kFormClusters, s, bytes(std::min(s, all_heads))};
+  const int s = step_record_splits(kt, vt, n_head_kv, n_keys, sms);
+  if (s > 0 && ws_bytes >= bytes(s)) return {kFormHeadRecords, s, bytes(s)};
+  return {kFormAllHeads, all_heads, bytes(s > 0 ? std::min(s, all_heads) : all_heads)};
+}
+
 // Core: attention of n_tok tokens over keys key_begin..(pos ? pos[i] : t).
 //   out != null: merged (and optionally gated) output;
 //   out == null: exactly n_rec records per (token, head) into `records`.
@@ -116,9 +136,13 @@ int attn_core(const float *q, const void *k, const void *v, float *out, float *r
     n_keys = t >= key_begin ? (int64_t)t - key_begin + 1 : 0;
     tiles = (n_keys + tile - 1) / tile;
   }
-  const int direct = n_tok == 1 && out != nullptr ? step_splits(kt, vt, n_head_kv, n_keys) : 0;
-  const int per_head = n_tok == 1 && out != nullptr && direct == 0 ? step_record_splits(kt, vt, n_head_kv, n_keys, sms) : 0;
-  int S = direct > 0 ? direct : per_head > 0 ? per_head : n_tok > 1 ? block_splits(sms, n_tok, n_head_kv) : plan_splits(sms, n_tok, tiles);
+  const bool one = n_tok == 1 && out != nullptr;
+  int S = n_tok > 1 ? block_splits(sms, n_tok, n_head_kv) : plan_splits(sms, n_tok, tiles);
+  DecodePlan plan = {kFormAllHeads, S, 0};
+  if (one) {
+    plan = plan_decode(sms, n_head, n_head_kv, kt, vt, n_keys, S, ws_bytes);
+    S = plan.splits;
+  }
   if (out == nullptr) {
     // nest the internal splits inside the caller's: S = n_rec * r
     int r = S / n_rec;
@@ -140,18 +164,18 @@ int attn_core(const float *q, const void *k, const void *v, float *out, float *r
   a.status = status;
   // a block of tokens shares each dequantized key; one token has a warp per (head, key group)
   auto launch = [&] {
-    return n_tok > 1      ? launch_block(kt, vt, a, block_chunk(n_tok), st)
-           : per_head > 0 ? launch_step(kt, vt, a, nullptr, nullptr, st)
-                          : launch_decode(kt, vt, a, st);
+    return n_tok > 1                         ? launch_block(kt, vt, a, block_chunk(n_tok), st)
+           : plan.form == kFormHeadRecords ? launch_step(kt, vt, a, nullptr, nullptr, st)
+                                             : launch_decode(kt, vt, a, st);
   };
   if (out == nullptr && S == n_rec) {
     a.partial = records;
     return launch();
   }
-  const size_t need = partial_floats(n_tok, n_head, S) * sizeof(float);
+  const size_t need = one ? plan.need : partial_floats(n_tok, n_head, S) * sizeof(float);
   if (ws == nullptr || ws_bytes < need) return RD_ERR_WORKSPACE;
   a.partial = (float *)ws;
-  if (direct > 0) return launch_step(kt, vt, a, out, gate, st);   // short context: one launch, no records
+  if (plan.form == kFormClusters) return launch_step(kt, vt, a, out, gate, st);   // short context: one launch, no records
   const int rc = launch();
   if (rc != RD_OK) return rc;
   if (out != nullptr) return launch_merge((const float *)ws, out, n_tok * n_head, S, gate, st);
@@ -497,32 +521,31 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
   // row t folded in.
   const int tile = decode_tile_keys(k_type, v_type);
   const int64_t tiles = ((int64_t)t + tile - 1) / tile;
-  const int direct = step_splits(k_type, v_type, n_head_kv, (int64_t)t + 1);
-  const int per_head = direct == 0 ? step_record_splits(k_type, v_type, n_head_kv, (int64_t)t + 1, sm_count(dev)) : 0;
-  const int S = direct > 0 ? direct : per_head > 0 ? per_head : plan_splits(sm_count(dev), 1, tiles);
-  if (workspace_bytes < partial_floats(1, n_head, S) * sizeof(float)) return RD_ERR_WORKSPACE;
+  const DecodePlan plan = plan_decode(sm_count(dev), n_head, n_head_kv, k_type, v_type, (int64_t)t + 1,
+                                      plan_splits(sm_count(dev), 1, tiles), workspace_bytes);
+  if (workspace_bytes < plan.need) return RD_ERR_WORKSPACE;
   DecodeArgs a;
   a.q = q;
   a.k = k_cache;
   a.v = v_cache;
   a.partial = (float *)workspace;
   a.pos = nullptr;
-  a.t = direct > 0 || per_head > 0 ? t : t - 1;
+  a.t = plan.form == kFormAllHeads ? t - 1 : t;
   a.key_begin = 0;
   a.n_tok = 1;
   a.n_head = n_head;
   a.n_head_kv = n_head_kv;
   a.scale = scale;
-  a.n_splits = S;
+  a.n_splits = plan.splits;
   a.status = status;
   a.k_new = k_new;
   a.v_new = v_new;
   a.new_row = t;
   cudaStream_t st = (cudaStream_t)stream;
-  if (direct > 0) return launch_step(k_type, v_type, a, out, gate, st);
-  if (per_head > 0) {
+  if (plan.form == kFormClusters) return launch_step(k_type, v_type, a, out, gate, st);
+  if (plan.form == kFormHeadRecords) {
     if ((rc = launch_step(k_type, v_type, a, nullptr, nullptr, st)) != RD_OK) return rc;
-    return launch_merge((const float *)workspace, out, n_head, S, gate, st);
+    return launch_merge((const float *)workspace, out, n_head, plan.splits, gate, st);
   }
   if ((rc = launch_decode(k_type, v_type, a, st)) != RD_OK) return rc;
   ExtraKey x;
@@ -533,7 +556,7 @@ int rd_attn_decode_append_ws(const float *q, const float *k_new, const float *v_
   x.vt = v_type;
   x.nkv = n_head_kv;
   x.scale = scale;
-  return launch_merge_extra((const float *)workspace, out, n_head, S, gate, x, st);
+  return launch_merge_extra((const float *)workspace, out, n_head, plan.splits, gate, x, st);
 }
 
 int rd_attn_decode_noalloc(const float *q, const void *k, const void *v, float *out, int t,
