@@ -100,6 +100,11 @@ __host__ __device__ constexpr int min_i(int a, int b) { return a < b ? a : b; }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const uint8_t *src) {
   asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+// The same with zeros instead of the bytes at src where `have` is false.
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const uint8_t *src, bool have) {
+  asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(have ? 16 : 0)
+               : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -107,8 +112,8 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // One slot: rows row0 .. row0 + 15 of a head (`row_stride` bytes apart in the cache) to shared
-// memory, kSlotKeys rows slot_pitch apart. Warp-collective; rows behind t_load repeat it. Lanes
-// are dealt so that a copy instruction takes whole rows: the lane's part of the address is a constant.
+// memory, kSlotKeys rows slot_pitch apart. Warp-collective; rows behind t_load are zeros (a weight of 0 times
+// the last row again would be NaN where that row is infinite). Lanes are dealt so that a copy instruction takes whole rows: the lane's part of the address is a constant.
 template <int T>
 __device__ __forceinline__ void copy_slot(uint32_t dst, const uint8_t *head_base, size_t row_stride, int row0,
                                           int t_load, int lane) {
@@ -118,7 +123,7 @@ __device__ __forceinline__ void copy_slot(uint32_t dst, const uint8_t *head_base
     for (int i = lane; i < CH * kSlotKeys; i += 32) {
       const int r = i / CH, c = i % CH;
       const int key = row0 + r > t_load ? t_load : row0 + r;
-      cp_async16(dst + r * P + 16 * c, head_base + (size_t)key * row_stride + 16 * c);
+      cp_async16_or_zero(dst + r * P + 16 * c, head_base + (size_t)key * row_stride + 16 * c, row0 + r <= t_load);
     }
     return;
   }

@@ -212,15 +212,16 @@ step_kernel(const __grid_constant__ StepArgs p) {
     const uint32_t *st = reinterpret_cast<const uint32_t *>(stage);
     for (int i = threadIdx.x; i < (RK + RV) / 4; i += NT) (i < RK / 4 ? kd[i] : vd[i - RK / 4]) = st[i];
   }
-  // the appended row into the slot; the rows behind it repeat the last stored one -- or, where there is
-  // none (nothing was copied), the appended one: something finite
+  // the appended row into the slot; the rows behind it are zeros, by the slot's copy or, where nothing was
+  // copied, from here
   auto patch = [&](uint32_t slot, int pitch, const uint8_t *row, int words, int row0) {
     const int first = t_last - row0, last = t_load < key_begin ? kSlotKeys - 1 : first;
 #pragma unroll 1
     for (int r = first; r <= last; ++r)
 #pragma unroll 4
       for (int c = lane; c < words; c += 32)
-        *reinterpret_cast<uint32_t *>(smem + (slot - sbase) + r * pitch + 4 * c) = reinterpret_cast<const uint32_t *>(row)[c];
+        *reinterpret_cast<uint32_t *>(smem + (slot - sbase) + r * pitch + 4 * c) =
+            r == first ? reinterpret_cast<const uint32_t *>(row)[c] : 0u;
     __syncwarp();
   };
 

@@ -84,6 +84,38 @@ def test_block_of_many_sequences(G, oracle):
         same(G.host(d[3]), want, f"{n} keys")
 
 
+@pytest.mark.parametrize("append", [False, True])
+@pytest.mark.parametrize("kt,vt", [(F16, F16), (2, F16), (Q4_1, Q4_1)])
+@pytest.mark.parametrize("n", [1, 2, 17, 137, 255, 4100, 6000])
+def test_infinite_last_row_of_a_step(G, oracle, kt, vt, n, append):
+    """The slot of the last key has rows behind it, with weight 0: they must not turn an infinite last row into NaN."""
+    rd, lib = G.rd, G.lib
+    q, kc, vc = make(oracle, n, n, kt, vt, 1)
+    want = oracle.attn(q, kc, vc, [n - 1], NKV, 1 / 16, kt, vt)
+    dq, out = G.dev(q), G.poison(q.shape)
+    nb = lib.rd_attn_workspace_bytes(1, NH, HD)
+    ws = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    if append:   # f32 values that a new f16 row saturates; q4_1 blocks of one value have it as their minimum
+        kn, vn = (np.random.default_rng(n).standard_normal((NKV, HD)).astype(np.float32) for _ in range(2))
+        kc.reshape(n, -1)[n - 1] = oracle.kv_store_rows(kt, kn).reshape(-1)
+        vc.reshape(n, -1)[n - 1] = oracle.kv_store_rows(vt, vn).reshape(-1)
+        want = oracle.attn(q, kc, vc, [n - 1], NKV, 1 / 16, kt, vt)
+        dims = slice(37, 38) if vt == F16 else slice(32, 64)
+        vn[1, dims] = 1e6
+        want[0, 6:12, dims] = np.inf
+        dk, dv, dkn, dvn = G.dev(kc), G.dev(vc), G.dev(kn), G.dev(vn)
+        rd.check(lib.rd_attn_decode_append_ws(rd.ptr(dq), rd.ptr(dkn), rd.ptr(dvn), rd.ptr(dk), rd.ptr(dv), rd.ptr(out),
+                                              n - 1, NH, NKV, HD, 1 / 16, kt, vt, None, rd.ptr(ws), nb, G.st()))
+    else:
+        plant(vc, want, vt, n - 1, 1, [n - 1])
+        dk, dv = G.dev(kc), G.dev(vc)
+        rd.check(lib.rd_attn_decode_ws(rd.ptr(dq), rd.ptr(dk), rd.ptr(dv), rd.ptr(out), None, 0, n - 1, NH, NKV, HD,
+                                       1 / 16, kt, vt, 1, None, rd.ptr(ws), nb, G.st()))
+    torch.cuda.synchronize()
+    same(G.host(out), want, f"{n} keys")
+    G.status_ok()
+
+
 @pytest.mark.parametrize("n_q,pos0,splits", [(5, 0, 1), (200, 0, 1), (130, 4000, 3)])
 def test_prefill_gate_nan(G, oracle, n_q, pos0, splits):
     """A NaN gate makes its own output NaN, with and without a key split; infinite gates give 0 and the whole value."""
