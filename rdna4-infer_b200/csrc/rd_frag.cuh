@@ -100,11 +100,6 @@ __host__ __device__ constexpr int min_i(int a, int b) { return a < b ? a : b; }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const uint8_t *src) {
   asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-// The same with zeros instead of the bytes at src where `have` is false.
-__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const uint8_t *src, bool have) {
-  asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(have ? 16 : 0)
-               : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -118,13 +113,16 @@ template <int T>
 __device__ __forceinline__ void copy_slot(uint32_t dst, const uint8_t *head_base, size_t row_stride, int row0,
                                           int t_load, int lane) {
   constexpr int R = row_bytes(T), P = slot_pitch(T), CH = R / 16;
-  if (row0 + kSlotKeys - 1 > t_load) {   // the ragged end: one slot of a launch
+  // The ragged end: one slot of a launch, copies for the rows that exist and stores for the others (16 layers over
+  // 137 f16 keys: 130 us; with a zero-filling copy per row 135, unrolled further 131 and 4096 keys 196 instead of 194).
+  if (row0 + kSlotKeys - 1 > t_load) {
+    const int have = t_load - row0 + 1 > 0 ? t_load - row0 + 1 : 0;   // rows that exist
+#pragma unroll 2
+    for (int i = lane; i < CH * have; i += 32)
+      cp_async16(dst + (i / CH) * P + 16 * (i % CH), head_base + (size_t)(row0 + i / CH) * row_stride + 16 * (i % CH));
 #pragma unroll 1
-    for (int i = lane; i < CH * kSlotKeys; i += 32) {
-      const int r = i / CH, c = i % CH;
-      const int key = row0 + r > t_load ? t_load : row0 + r;
-      cp_async16_or_zero(dst + r * P + 16 * c, head_base + (size_t)key * row_stride + 16 * c, row0 + r <= t_load);
-    }
+    for (int i = CH * have + lane; i < CH * kSlotKeys; i += 32)
+      asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(dst + (i / CH) * P + 16 * (i % CH)), "r"(0) : "memory");
     return;
   }
   const uint8_t *src = head_base + (size_t)row0 * row_stride;
