@@ -21,6 +21,13 @@
 // 0. A non-finite value there (an f16 cache saturates to infinity) would make that 0 a NaN, so a launch whose
 // accumulators are not all finite runs the key loop once more, token by token (careful_pv). Any other launch pays
 // one check of its accumulators for that.
+// Precision: the weight of the key that is the reference is exactly 1 in f16, the others are rounded, and a reference
+// per team leaves fewer exact ones than one per 16 keys. The weights of a team's first slot therefore go to the tensor
+// cores in two f16 parts (a second pass of P V over the same slot), which makes up for it where the runs
+// are short; long runs never had much of it. Error against 64 bits, f16, with one reference per 16 keys / without the
+// second part / with it: 2 tokens over 100 keys 2.36 / 2.75 / 1.93e-4, 5 over 4096 2.87 / 2.97 / 2.52e-4, 5 over 20011
+// 2.94 / 2.96 / 2.87e-4. It costs 1.2 us a launch: 5 tokens over 20011 q4_0 keys 463 -> 483 us for 16 layers.
+// (Both parts for every slot: 511 us, 2.11e-4.)
 // (Tensor-map boxes of one head's rows were the slower copy: the TMA unit fetches whole cache lines,
 // and a 272-byte row of q8_0 lies in three of them. 64 sequences of config 5 verifying four tokens:
 // copies alone 817 us.)
@@ -52,7 +59,7 @@ struct BlockGeo {
   static constexpr int kPK = slot_pitch(KT), kPV = slot_pitch(VT);
   static constexpr int kSK = kBlkKeys * kPK, kSV = kBlkKeys * kPV;   // multiples of 128
   static constexpr int kQBytes = NT * 4096;                          // query fragments
-  static constexpr int kPBytes = NT * 1024;                          // weight fragments of a slot, per team
+  static constexpr int kPBytes = NT * 2048;                          // weight fragments of a slot, two parts, per team
   static constexpr int kHead = 512 + kQBytes;                        // dim table, query fragments
   static constexpr int budget(int teams) { return (kBlkSmem - kHead) / teams - kPBytes; }
   // two teams where each gets at least one slot, and another K or V of the next
@@ -102,7 +109,9 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
   asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
   return v;
 }
-
+__device__ __forceinline__ void st_frag(uint32_t addr, uint32_t a, uint32_t b) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
 // The keys 2 tq, 2 tq + 1, 2 tq + 8 and 2 tq + 9 behind `first` that are at most t: masks of an A fragment's halves.
 __device__ __forceinline__ uint2 key_mask(int first, int t) {
   const uint32_t lo = (first <= t ? 0xffffu : 0u) | (first + 1 <= t ? 0xffff0000u : 0u);
@@ -290,6 +299,7 @@ block_kernel(const __grid_constant__ BlockArgs p) {
 #pragma unroll 1
     for (int i = 0; i < n_mine; ++i) {
       const int row0 = (c_b + team + i * TEAMS) * kBlkKeys;
+      const bool fine = i == 0 && !careful;   // weights in two parts
       cp_async_wait<WAIT_K>();
       __syncwarp();
       // ---- S = K Q^T: this warp's 16 keys x all columns ----
@@ -344,10 +354,8 @@ block_kernel(const __grid_constant__ BlockArgs p) {
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int c = 8 * nt + 2 * tq + e;
-            // a whole number: the rounding of the weights to f16 then does not depend on it, and results
-            // for different key splits differ in the order of f32 sums only
-            const float m = fmaxf(ceilf(fmaxf(fmaxf(s_max[team][0][c], s_max[team][1][c]),
-                                              fmaxf(s_max[team][2][c], s_max[team][3][c]))), ref[nt][e]);
+            const float m = fmaxf(fmaxf(fmaxf(s_max[team][0][c], s_max[team][1][c]),
+                                        fmaxf(s_max[team][2][c], s_max[team][3][c])), ref[nt][e]);
             const float f = ex2(ref[nt][e] - m);
             ref[nt][e] = m;
             l[nt][e] *= f;
@@ -364,22 +372,26 @@ block_kernel(const __grid_constant__ BlockArgs p) {
         const float p0 = ex2(Sv[nt][0] - ref[nt][0]), p1 = ex2(Sv[nt][1] - ref[nt][1]);
         const float p2 = ex2(Sv[nt][2] - ref[nt][0]), p3 = ex2(Sv[nt][3] - ref[nt][1]);
         const uint32_t h01 = pack_h2(p0, p1), h23 = pack_h2(p2, p3);
-        // the sums take the weights as rounded for the tensor core: a common rounding error of a column
-        // then cancels in the quotient
         const float2 r01 = unpack_h2(h01), r23 = unpack_h2(h23);
-        l[nt][0] += r01.x + r23.x;
-        l[nt][1] += r01.y + r23.y;
-        const uint32_t b0 = movmatrix_trans(h01), b1 = movmatrix_trans(h23);
-        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(pfrag + (part * NT + nt) * 256 + lane * 8), "r"(b0), "r"(b1)
-                     : "memory");
+        const uint32_t at = pfrag + (part * NT + nt) * 256 + lane * 8;
+        st_frag(at, movmatrix_trans(h01), movmatrix_trans(h23));
+        if (fine) {
+          st_frag(at + NT * 1024, movmatrix_trans(pack_h2(p0 - r01.x, p1 - r01.y)),
+                  movmatrix_trans(pack_h2(p2 - r23.x, p3 - r23.y)));
+          l[nt][0] += p0 + p2;
+          l[nt][1] += p1 + p3;
+        } else {   // the sums take the weights as rounded: a common rounding error of a column cancels in the quotient
+          l[nt][0] += r01.x + r23.x;
+          l[nt][1] += r01.y + r23.y;
+        }
       }
       cp_async_wait<WAIT_V>();
       team_sync(team);
       // ---- O^T += V^T P^T: 64 keys x this warp's quarter of the dims ----
-      auto pv = [&](int ks, auto &&mma) {
+      auto pv = [&](int ks, uint32_t frag, auto &&mma) {
         uint2 pb[NT];
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) pb[nt] = lds64(pfrag + (ks * NT + nt) * 256 + lane * 8);
+        for (int nt = 0; nt < NT; ++nt) pb[nt] = lds64(frag + (ks * NT + nt) * 256 + lane * 8);
         const uint32_t r0 = ring_v + (i % DV) * SV + (16 * ks + 2 * tq) * PV;
         const uint32_t rows[4] = {r0, r0 + PV, r0 + 8 * PV, r0 + 9 * PV};
         VL::run_part(rows, g, part, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
@@ -389,14 +401,22 @@ block_kernel(const __grid_constant__ BlockArgs p) {
       if (!careful) {
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
-          pv(ks, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const uint2(&pb)[NT]) {
+          pv(ks, pfrag, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const uint2(&pb)[NT]) {
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) mma16816(O[m][nt], a0, a1, a2, a3, pb[nt].x, pb[nt].y);
           });
+        if (fine) {
+#pragma unroll 1
+          for (int ks = 0; ks < 4; ++ks)
+            pv(ks, pfrag + NT * 1024, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const uint2(&pb)[NT]) {
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) mma16816(O[m][nt], a0, a1, a2, a3, pb[nt].x, pb[nt].y);
+            });
+        }
       } else {
 #pragma unroll 1
         for (int ks = 0; ks < 4; ++ks)
-          pv(ks, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const uint2(&pb)[NT]) {
+          pv(ks, pfrag, [&](int m, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const uint2(&pb)[NT]) {
             careful_pv<NT>(O[m], a0, a1, a2, a3, pb, s_t, n_tok, row0 + 16 * ks, tq);
           });
       }
@@ -458,7 +478,7 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     const bool empty = mm <= 0.5f * kBlkNone;
 #pragma unroll
     for (int i = 0; i < TEAMS; ++i) {
-      const float w = ex2(s_ref[i][c] - mm);   // a reference is at most 1 above the true maximum
+      const float w = ex2(s_ref[i][c] - mm);   // references never exceed the true maximum
       s_wt[i][c] = empty ? 0.f : w * VL::kUnscale;
       ll = fmaf((s_sum[i][0][c] + s_sum[i][1][c]) + (s_sum[i][2][c] + s_sum[i][3][c]), w, ll);
     }

@@ -26,7 +26,9 @@ def exact(q, k, v, pos):
 
 
 # tokens, keys, bound, what it was with longer runs
-@pytest.mark.parametrize("n_tok,n,bound", [(1, 137, 2.52e-4), (1, 3000, 2.58e-4), (1, 4096, 2.60e-4)])   # 2.45 2.69 2.76e-4
+@pytest.mark.parametrize("n_tok,n,bound", [(1, 137, 2.52e-4), (1, 3000, 2.58e-4), (1, 4096, 2.60e-4),   # 2.45 2.69 2.76e-4
+                                           (2, 100, 2.36e-4), (4, 1000, 2.55e-4), (5, 4096, 2.88e-4),   # 2.75 2.99 2.97e-4
+                                           (5, 20011, 2.95e-4), (8, 20011, 2.96e-4)])                   # 2.96 2.96e-4
 def test_error_against_64_bits(G, n_tok, n, bound):
     rd, lib = G.rd, G.lib
     errs = []
