@@ -13,10 +13,12 @@ from __future__ import annotations
 import ctypes as C
 import os
 import subprocess
+import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "librd_attn_b200.so")
-BIND_PATH = os.path.join(HERE, "_rd_bind.so")
+BIND_PATH = os.path.join(HERE, "_rd_bind" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))   # this interpreter's
 
 F32, F16, Q8_0, Q4_0, Q5_0, Q4_1 = range(6)
 TYPE_NAMES = ("f32", "f16", "q8_0", "q4_0", "q5_0", "q4_1")
@@ -85,7 +87,7 @@ SIGNATURES = {
 
 def build(verbose: bool = False) -> str:
     """Compile the library in-tree with nvcc for sm_100a (needs no GPU)."""
-    cmd = ["make", "-C", HERE, "-j", str(os.cpu_count() or 4)]
+    cmd = ["make", "-C", HERE, "-j", str(os.cpu_count() or 4), "PYTHON=" + sys.executable]
     if not verbose:
         cmd.insert(1, "-s")
     subprocess.check_call(cmd)

@@ -22,3 +22,12 @@ def test_bound_callables_match_ctypes(rd):
     # what the converter does not take goes to ctypes
     x = C.c_float(1.0)
     assert rd.lib.rd_kv_store_rows(3, C.byref(x), 32, 33, 0) == rd.ERR_SHAPE
+
+
+def test_module_is_this_interpreters(rd):
+    """A module of another interpreter has another name: it is neither loaded nor taken for up to date by make."""
+    import os
+    import sysconfig
+    assert os.path.basename(rd.BIND_PATH) == "_rd_bind" + sysconfig.get_config_var("EXT_SUFFIX")
+    if os.path.exists(os.path.join(sysconfig.get_paths()["include"], "Python.h")):
+        assert os.path.exists(rd.BIND_PATH) and type(rd.lib.rd_kv_store_rows).__name__ == "builtin_function_or_method"
