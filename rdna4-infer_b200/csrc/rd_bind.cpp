@@ -5,7 +5,8 @@
 // argument is converted by the type that include/rd_attn.h declares for it: about 0.3 us. Anything but
 // plain numbers and None (a ctypes byref, an array, a wrong type) goes to the ctypes function.
 //
-// The module does not link the library: install(name, address, fallback) binds one entry point.
+// The module does not link the library: install(name, address, fallback) gives a callable for one entry point of
+// one library. What it is bound to belongs to the callable, so libraries loaded side by side keep their own.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -48,46 +49,45 @@ bool convert(PyObject *o, T &out) {
   }
 }
 
-// One entry point (told apart by N): its address, and the ctypes function for what this one does not take.
-template <int N, class F>
-struct Entry;
-template <int N, class R, class... A>
-struct Entry<N, R (*)(A...)> {
-  static inline R (*fn)(A...) = nullptr;
-  static inline PyObject *fallback = nullptr;
+// What a callable is bound to: the entry point, and the ctypes function for what convert does not take.
+struct Binding {
+  void *address;
+  PyObject *fallback;
+};
+constexpr const char *kBinding = "rd_bind.binding";
+void release(PyObject *self) {
+  Binding *b = static_cast<Binding *>(PyCapsule_GetPointer(self, kBinding));
+  Py_XDECREF(b->fallback);
+  delete b;
+}
 
+template <class F>
+struct Entry;
+template <class R, class... A>
+struct Entry<R (*)(A...)> {
   template <size_t... I>
   static bool take(PyObject *const *args, std::tuple<A...> &a, std::index_sequence<I...>) {
     return (convert(args[I], std::get<I>(a)) && ...);
   }
-  static PyObject *py(PyObject *, PyObject *const *args, Py_ssize_t n) {
+  static PyObject *py(PyObject *self, PyObject *const *args, Py_ssize_t n) {
+    const Binding *b = static_cast<const Binding *>(PyCapsule_GetPointer(self, kBinding));
+    if (b == nullptr) return nullptr;
     std::tuple<A...> a;
     if (n != (Py_ssize_t)sizeof...(A) || !take(args, a, std::index_sequence_for<A...>()))
-      return PyObject_Vectorcall(fallback, args, (size_t)n, nullptr);
+      return PyObject_Vectorcall(b->fallback, args, (size_t)n, nullptr);
     R r;
     Py_BEGIN_ALLOW_THREADS
-    r = std::apply(fn, a);
+    r = std::apply(reinterpret_cast<R (*)(A...)>(b->address), a);
     Py_END_ALLOW_THREADS
     return PyLong_FromLong((long)r);
   }
-  static void set(void *address, PyObject *ctypes_function) {
-    fn = reinterpret_cast<R (*)(A...)>(address);
-    Py_INCREF(ctypes_function);
-    Py_XSETREF(fallback, ctypes_function);
-  }
 };
 
-struct Bound {
-  void (*set)(void *, PyObject *);
-  PyMethodDef def;
-};
-#define RD_ENTRY(name)                                                                                  \
-  {&Entry<__LINE__, decltype(&::name)>::set,                                                            \
-   {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(                                  \
-               &Entry<__LINE__, decltype(&::name)>::py)),                                               \
-    METH_FASTCALL, "see include/rd_attn.h"}},
+#define RD_ENTRY(name)                                                                                             \
+  {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(Entry<decltype(&::name)>::py)), METH_FASTCALL, \
+   "see include/rd_attn.h"},
 
-Bound g_entries[] = {
+PyMethodDef g_entries[] = {
     RD_ENTRY(rd_kv_store_rows)
     RD_ENTRY(rd_kv_append)
     RD_ENTRY(rd_rope)
@@ -122,10 +122,18 @@ PyObject *install(PyObject *, PyObject *args) {
   unsigned long long address;
   PyObject *ctypes_function;
   if (!PyArg_ParseTuple(args, "sKO", &name, &address, &ctypes_function)) return nullptr;
-  for (Bound &b : g_entries)
-    if (std::strcmp(b.def.ml_name, name) == 0) {
-      b.set(reinterpret_cast<void *>(address), ctypes_function);
-      return PyCFunction_New(&b.def, nullptr);
+  for (PyMethodDef &def : g_entries)
+    if (std::strcmp(def.ml_name, name) == 0) {
+      Binding *b = new Binding{reinterpret_cast<void *>(address), Py_NewRef(ctypes_function)};
+      PyObject *self = PyCapsule_New(b, kBinding, release);
+      if (self == nullptr) {
+        Py_DECREF(b->fallback);
+        delete b;
+        return nullptr;
+      }
+      PyObject *callable = PyCFunction_New(&def, self);
+      Py_DECREF(self);
+      return callable;
     }
   Py_RETURN_NONE;
 }
