@@ -144,13 +144,25 @@ int rd_pre_attn_fused(const float *q_gate, const float *k_src, const float *v_sr
  * min(16, n_keys / 512) for quantized ones; forced > 0 overrides (the RD_ATTN_SPLITS
  * knob), capped at 16. Host arithmetic only.
  *
- * rd_attn_plan reports what THIS library does with a decode launch whose CTAs each serve all
- * heads (the form of long contexts and of records-only calls) on a GPU of sm_count
- * SMs (<= 0: the current device): keys per shared-memory tile (16, 32 or 48 by K / V type),
+ * rd_attn_plan reports the launch whose CTAs each serve all heads -- the one of long quantized contexts, of
+ * records-only calls and of small workspaces; rd_attn_launch_plan says which launch a call takes -- on a
+ * GPU of sm_count SMs (<= 0: the current device): keys per shared-memory tile (16, 32 or 48 by K / V type),
  * stages of the TMA ring, and the internal split count (about one CTA per SM, never more
  * splits than key tiles). Any output pointer may be NULL. Host arithmetic only when
  * sm_count is given. */
 int rd_attn_splits_for(int n_keys, int k_type, int v_type, int n_head, int forced);
+/* Which of its launches the library takes for an attention call that writes its output, with a workspace of
+ * rd_attn_workspace_bytes: n_tok 1 is a decode over n_keys keys (negative: the key count is on the
+ * device), n_tok above 1 a block of tokens.
+ *   RD_FORM_CLUSTERS       one launch: a cluster of n_splits CTAs per KV head writes the output itself
+ *   RD_FORM_HEAD_RECORDS   n_splits CTAs per KV head write records, a merge launch
+ *   RD_FORM_ALL_HEADS      n_splits CTAs for all heads write records, a merge launch (rd_attn_plan's launch)
+ *   RD_FORM_BLOCK          n_splits CTAs per KV head and chunk of up to eight tokens, a merge launch
+ * n_ctas is the grid of the first launch. rd_attn_multi_split reports the split of many sequences.
+ * Host arithmetic only when sm_count is given. */
+enum { RD_FORM_CLUSTERS = 0, RD_FORM_HEAD_RECORDS = 1, RD_FORM_ALL_HEADS = 2, RD_FORM_BLOCK = 3 };
+int rd_attn_launch_plan(int64_t n_keys, int n_tok, int n_head_kv, int k_type, int v_type, int sm_count,
+                        int *form, int *n_splits, int *n_ctas);
 /* What the prefill entries do with a chunk of n_q tokens over keys_total keys on a GPU of
  * sm_count SMs (<= 0: the current device): the key splits per (128-token tile, head) and
  * the CTAs of the tile-kernel launch. One split unless the cost model says that filling the

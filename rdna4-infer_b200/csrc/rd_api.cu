@@ -108,7 +108,7 @@ size_t partial_floats(int n_tok, int n_head, int splits) {
 // plan_splits). `all_heads` is the last one's count for the call; the records of the forms differ in number, and a
 // workspace that holds the records of that one is enough for every length: the per-head form is taken
 // where its own fit as well, and the cluster form has none.
-enum DecodeForm { kFormClusters, kFormHeadRecords, kFormAllHeads };
+enum DecodeForm { kFormClusters = RD_FORM_CLUSTERS, kFormHeadRecords = RD_FORM_HEAD_RECORDS, kFormAllHeads = RD_FORM_ALL_HEADS };
 struct DecodePlan {
   DecodeForm form;
   int splits;
@@ -429,6 +429,33 @@ int rd_attn_plan(int n_keys, int n_tok, int n_head_kv, int k_type, int v_type, i
   if (tile_keys != nullptr) *tile_keys = tile;
   if (ring_stages != nullptr) *ring_stages = stages;
   if (n_splits != nullptr) *n_splits = plan_splits(sm_count, n_tok, tiles);
+  return RD_OK;
+}
+
+int rd_attn_launch_plan(int64_t n_keys, int n_tok, int n_head_kv, int k_type, int v_type, int sm_count, int *form,
+                        int *n_splits, int *n_ctas) {
+  if (!known_type(k_type) || !known_type(v_type)) return RD_ERR_TYPE;
+  if (n_tok < 1) return RD_ERR_SHAPE;
+  if (n_head_kv != 1 && n_head_kv != 2 && n_head_kv != 4) return RD_ERR_UNSUPPORTED;
+  if (sm_count <= 0) {
+    int dev;
+    const int rc = current_device(&dev);
+    if (rc != RD_OK) return rc;
+    sm_count = ::sm_count(dev);
+  }
+  int f = RD_FORM_BLOCK, splits = block_splits(sm_count, n_tok, n_head_kv);
+  int ctas = splits * n_head_kv * ((n_tok + block_chunk(n_tok) - 1) / block_chunk(n_tok));
+  if (n_tok == 1) {
+    const int tile = decode_tile_keys(k_type, v_type);
+    const DecodePlan p = plan_decode(sm_count, kGroup * n_head_kv, n_head_kv, k_type, v_type, n_keys < 0 ? -1 : n_keys,
+                                     plan_splits(sm_count, 1, n_keys < 0 ? -1 : (n_keys + tile - 1) / tile), SIZE_MAX);
+    f = p.form;
+    splits = p.splits;
+    ctas = f == RD_FORM_ALL_HEADS ? splits : splits * n_head_kv;
+  }
+  if (form != nullptr) *form = f;
+  if (n_splits != nullptr) *n_splits = splits;
+  if (n_ctas != nullptr) *n_ctas = ctas;
   return RD_OK;
 }
 
