@@ -205,12 +205,14 @@ int rd_attn_decode_ws(const float *q, const void *k, const void *v, float *out, 
                       int k_type, int v_type, int n_splits, float *gate, void *workspace,
                       size_t workspace_bytes, void *stream);
 
-/* ---- append + decode in two launches (no counterpart: the reference runs
+/* ---- append + decode (no counterpart: the reference runs
  * kv_store_row_launch twice, then attn_launch_split, graph.cuh:1011-1035 and 958-977).
  * Stores k_new / v_new ([n_head_kv][head_dim] f32, K already normalised and rotated) as
  * row t of the caches and returns the attention of q over keys 0..t, the new one
- * included: the CTA of the decode launch that attends key t quantizes the row, stores it and
- * attends it from shared memory. Short contexts take one launch (no merge). Cache bytes
+ * included. In the per-head launches (rd_attn_launch_plan) the CTA that attends key t quantizes the row,
+ * stores it and attends it from shared memory; with RD_FORM_CLUSTERS that is the only launch. In the
+ * all-heads launch -- long quantized contexts -- the first CTAs store the row while keys 0..t-1 are
+ * attended, and the merge folds key t in from the cache. Cache bytes
  * equal rd_kv_append's; the output equals rd_attn_decode_ws after rd_kv_append within
  * the attention tolerance. q must not alias out (RD_ERR_UNSUPPORTED). gate as in
  * rd_attn_decode_ws; workspace from rd_attn_workspace_bytes(1, ...). */

@@ -29,12 +29,23 @@
 // 2.94 / 2.96 / 2.87e-4. It costs 1.2 us a launch: 5 tokens over 20011 q4_0 keys 463 -> 483 us for 16 layers.
 // (Both parts for every slot: 511 us, 2.11e-4.)
 // (Tensor-map boxes of one head's rows were the slower copy: the TMA unit fetches whole cache lines,
-// and a 272-byte row of q8_0 lies in three of them. 64 sequences of config 5 verifying four tokens:
-// copies alone 817 us.)
+// and a 272-byte row of q8_0 lies in three of them. 64 sequences of 1024 to 32768 keys
+// verifying four tokens: copies alone 817 us.)
 // One record (m, l, acc[256]) per (token, head) and split, merged by merge_kernel.
 //
-// What bounds it: the 32 NT mma.sync of 16 keys (about 13 cycles each per scheduler) for 4-bit caches
-// from four tokens, HBM and the barriers for 8-bit and f16 caches.
+// What bounds it: latency. Two warps per scheduler (registers), each a chain of shared-memory loads, dequantization,
+// mma.sync, vote, exponentials, fragment stores, barrier, mma.sync: 5 tokens over 20011 q4_0 keys issue in 35 % of the
+// active cycles, tensor pipe 22 %, DRAM 12 %; of the cycles between two issues of a warp (5.8) it waits 1.6 for fixed
+// latencies, 0.7 for shared memory, 0.7 for the tensor pipe, 0.4 for the first copies, 0.3 each at barriers and for
+// instructions. A launch takes about 9.8 us whatever the keys (prologue, ring fill, planes, records; the merge
+// launch 4 more) and 0.55 ns per key:
+//   us, records only       500      5000     20011     65536 keys
+//   q4_0, 2 tokens         6.3       8.4      14.4      32.0
+//   q4_0, 5                9.6      12.5      20.7      45.7
+//   q4_0, 8               13.1      17.0      27.1      57.0
+//   q8_0/f16, 4            8.4      12.0      20.4      46.1
+//   f16, 4                 8.4      13.3      24.5      57.1   (4.7 TB/s)
+//   q5_0/q4_1, 5           9.8      12.7      21.7      47.3
 #pragma once
 #include <string.h>
 
@@ -51,7 +62,8 @@ constexpr int kBlkPlane = 268;     // floats per column in the epilogue planes (
 constexpr float kBlkSlack = 8.0f;  // see kRefSlack
 constexpr float kBlkNone = -1.0e30f;
 
-// column tiles for a chunk of n tokens
+// Column tiles for a chunk of n tokens: the smallest of the four forms that holds them. Six tokens have no form of
+// their own (36 columns in 48); one of five tiles takes 23.5 instead of 26.1 us over 20011 q4_0 keys and is not built.
 __host__ __device__ constexpr int block_tiles(int n) { return n <= 2 ? 2 : n <= 4 ? 3 : n == 5 ? 4 : 6; }
 
 template <int KT, int VT, int NT>

@@ -108,6 +108,21 @@ int launch_block_multi(int kt, int vt, const MultiDecodeArgs &a, cudaStream_t st
 //   q8_0/f16   12.0 / -   12.9 / 12.4 / 16   16.5 / 15.0 / 18  -  / 18.7 / 22   -  / 28.0 / 30   -  / 44.3 / 45.2
 //   q8_0       12.2 / -   12.7 / 12.0 / 14   16.5 / 14.8 / 17  -  / 19.0 / 20   -  / 26.1 / 24.8 -  / 39.3 / 36.5
 //   q4_0       11.0 / -   11.7 / 11.8 / 14   14.4 / 13.3 / 16  -  / 16.4 / 18   -  / 21.4 / 21.9 -  / 30.9 / 30.5
+// The line at 24576 keys for the other three-group pairs (decode and merge alone, records per head / all heads):
+//   keys       4096        16384         24576         32768         65536
+//   q5_0/q4_1  8.4 / 11.5  14.2 / 14.8   17.6 / 17.5   20.1 / 19.5   31.3 / 29.1
+//   q4_1       7.9 / 11.0  12.7 / 13.9   15.7 / 16.3   17.6 / 17.9   26.1 / 25.6
+//   q8_0/q4_0  8.5 / 11.2  14.1 / 14.6   17.0 / 16.6   19.6 / 18.4   31.0 / 27.4
+// Fewer KV heads (one cluster per KV head / records per head / all heads). The first line scales with them, which
+// keeps clusters a little short of where they stop being faster for one head (8.4 against 8.0 at 4096 keys); the second was
+// taken over as it is, although all heads are the slower form there at every length:
+//   keys              896               1792              4096              24576          98304
+//   2, f16            5.6 / 7.1 / 9.8   7.3 / 7.4 / 9.9   9.4 / 8.2 / 12.5  - / 14.8 / 25  - / 40.1 / 77
+//   2, q4_0           5.6 / 7.4 / 9.5   6.4 / 7.5 / 9.5   8.4 / 7.6 / 9.8   - / 11.5 / 15  - / 22.4 / 31
+//   2, q5_0/q4_1      5.6 / 7.5 / 9.6   6.4 / 7.6 / 9.7   8.8 / 7.7 / 10.0  - / 12.4 / 16  - / 26.0 / 37
+//   1, f16            5.6 / 7.0 / 8.4   7.3 / 7.4 / 8.8   9.2 / 7.9 / 10.2  - / 11.4 / 20  - / 24.1 / 71
+//   1, q4_0           5.6 / 7.3 / 9.0   6.1 / 7.6 / 9.0   7.9 / 7.8 / 9.3   - / 9.4 / 14   - / 14.6 / 30
+//   1, q5_0/q4_1      5.6 / 7.5 / 9.3   6.2 / 7.9 / 9.3   8.4 / 8.0 / 9.6   - / 10.0 / 15  - / 17.3 / 36
 // The cluster form saves the merge launch but uses 64 SMs; records use all. decode_kernel copies all KV heads of
 // a key in one box, which costs a long launch fewer issue slots and a short one a larger prologue; with f16
 // rows it has shared memory for four or eight warps only.

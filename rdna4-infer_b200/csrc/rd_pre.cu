@@ -4,7 +4,7 @@
 // the attention call (include/rdna4/graph.cuh:915-954) --
 //   deinterleave [q | gate] per head, RMS-norm of every q and k head row with its weight,
 //   partial RoPE of q and k, quantize-and-store of the k and v rows into the caches --
-// in ONE launch, one warp per 256-wide head row.
+// in ONE launch, one warp per 256-wide head row (up to eight tokens: one per 32-value block of a K or V row).
 //
 // The sum of squares keeps the reference kernel's order (256 threads each squaring one
 // element, then a shared-memory tree over strides 128 .. 1), so it is bit-identical to

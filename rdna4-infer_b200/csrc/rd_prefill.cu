@@ -19,11 +19,11 @@
 //              swizzled into shared memory;
 //   per 128-key tile j:
 //     warp 9     S = Q K_j^T        16 x tcgen05.mma M256 N128 K16
-//     warps 0-7  two threads per query row, 64 score columns each (row max exchanged
-//                through shared memory): tcgen05.ld the scores, causal mask
-//                (key <= pos[r]), running max with LAZY rescale (the reference point only
-//                moves when a row's max grows by more than 2^8, so P stays below 256 in
-//                f16 and O in TMEM is rarely touched), P -> f16 pairs, tcgen05.st
+//     warps 0-7  one thread per query row and tile parity (warps 0-3 the even tiles, 4-7 the odd ones),
+//                all 128 scores of the row in its registers, the reference maximum handed from tile to
+//                tile through shared memory: tcgen05.ld the scores, causal mask (key <= pos[r]), LAZY
+//                rescale (the reference point only moves when a row's max grows by more than 2^8, so
+//                P stays below 256 in f16 and O in TMEM is rarely touched), P -> f16 pairs, tcgen05.st
 //     warp 11    O += P V_j          8 x tcgen05.mma M256 N256 K16 (A = P from TMEM, B = V
 //                                   MN-major)
 //   epilogue   O / l (times sigmoid(gate) if asked) through shared memory to TMA stores.
@@ -910,12 +910,25 @@ kv_prep_kernel(const int32_t *__restrict__ pos, int n_rot, const float *__restri
       make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
 }
 
-// Key splits that fill the GPU, picked with a three-constant cost model measured on B200:
-// a key tile costs a CTA about 2 us, a CTA's prologue + epilogue about 9 us (the query
-// tile is converted and the result written whatever the key count), and the records cost
-// about 0.5 ns each (written by the tile kernel, read by the merge pass). Splitting pays only when the waves it saves outweigh the fixed
-// costs it multiplies: 512 tokens x 24 heads gain from about 8192 keys upwards (3 splits:
-// 96 -> 288 CTAs = two full waves of 148 SMs), shorter prefixes do not.
+// Key splits that fill the GPU, picked with a cost model of three constants: a key tile, a CTA's prologue +
+// epilogue (the query tile is converted and the result written whatever the key count) and a record (written
+// by the tile kernel, read by the merge pass) in the ratio 2 : 9 : 0.0005. (In microseconds they are those of the kernel
+// before the pairs of CTAs; a tile now takes about 1.2 us and prologue + epilogue 11, but a split multiplies
+// both, and the counts it picks are still the best or next to it.) Splitting pays only when the waves it saves
+// outweigh the fixed costs it multiplies: 512 tokens x 24 heads gain from about 8192 keys upwards (3 splits:
+// 96 -> 288 CTAs = two full waves of 148 SMs), shorter prefixes do not. Measured, us a layer with gate and rotation,
+// by split count (chosen in brackets):
+//   tokens of keys     1        2        3        4        5        6        7       8
+//     24 of  4000    51.1     31.8     26.8    [23.7]    24.6     23.3     34.7    33.4
+//     60 of  9000    98.8     56.7     45.2     39.1     35.0    [32.2]    52.0    49.2
+//    130 of  4130    56.6     39.6    [33.2]    48.5     47.3     47.0     55.1    57.0
+//    200 of 12000   133.4     80.1    [65.1]    92.0     81.1     76.7     97.5    92.6
+//    389 of 12346   164.6    172.3   [135.1]   154.6    168.1    164.6    170.2   182.4
+//    512 of  4096   [62.9]    76.9     68.6     86.1    102.8    104.3    121.5   139.4
+//    512 of  8192   113.8    129.9    [99.4]   119.6    137.9    133.9    150.9   168.4
+//    512 of 16384   220.3    224.5   [169.4]   210.4    242.3    214.7    218.9   239.0
+//   1000 of  8192   211.7    215.1   [209.5]   251.9    260.2    271.5    297.8   320.5
+//   2048 of  8192  [329.2]   404.1    420.4    456.4    505.8    535.3    589.2   618.2
 int prefill_splits(int n_q, int keys_total, int n_head, int sms) {
   const int ctas = ((n_q + kPfM - 1) / kPfM) * n_head;
   const int tiles = (keys_total + kPfN - 1) / kPfN;
