@@ -15,8 +15,8 @@
 //
 // Copies: a head's row is a narrow piece (144 bytes of q4_0) of a key, and a tensor-map box of
 // such rows costs the TMA unit about 13 cycles per row whatever its width: 50 us for the 131001-key
-// q4_0 layer where the arithmetic takes 31. Asynchronous 16-byte copies take any row, need no
-// descriptor (none to encode on the host) and clamp the ragged end for free.
+// q4_0 layer where the arithmetic takes 31. Asynchronous 16-byte copies take any row and need no
+// descriptor (none to encode on the host).
 //
 // What bounds it: latency (launch, first slot, the two meetings), with one cluster per KV head from about
 // 2000 keys the rate at which 64 SMs can fetch (35 bytes a cycle each). The longest contexts of 4- and 8-bit
