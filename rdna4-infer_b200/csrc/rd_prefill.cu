@@ -24,16 +24,16 @@
 //                tile through shared memory: tcgen05.ld the scores, causal mask (key <= pos[r]), LAZY
 //                rescale (the reference point only moves when a row's max grows by more than 2^8, so
 //                P stays below 256 in f16 and O in TMEM is rarely touched), P -> f16 pairs, tcgen05.st
-//     warp 11    O += P V_j          8 x tcgen05.mma M256 N256 K16 (A = P from TMEM, B = V
+//                O += P V_j-2        8 x tcgen05.mma M256 N256 K16 (A = P from TMEM, B = V
 //                                   MN-major)
 //   epilogue   O / l (times sigmoid(gate) if asked) through shared memory to TMA stores.
 // Warps 8 and 10 are the K and V TMA producers (separate warps: a lane parked in
-// mbarrier.try_wait parks its whole warp). The two contractions have their own issuing
-// threads because issuing a tcgen05.mma costs the issuing thread tens of cycles.
+// mbarrier.try_wait parks its whole warp).
 //
 // What orders the tiles: S of tile j + 1 waits for the LOADS of tile j's scores only, P of tile j for
 // P V of tile j - 2. (With P written over its own scores, S of tile j + 2 waited for P V of tile j, a chain
-// S - softmax - P V - S of 6300 cycles per two tiles against 4096 of tensor-core work.)
+// S - softmax - P V - S of 6300 cycles per two tiles against 4096 of tensor-core work.) A tile takes 2060
+// cycles, the tensor core's own rate.
 //
 // Synchronisation is mbarriers only (TMA transaction counts, tcgen05.commit); every wait
 // is bounded and a timeout unwinds the pair (TMEM is always freed). No multicast loads.
@@ -82,7 +82,7 @@ constexpr int kPfVSlots = 2;
 constexpr int kPfSmemBytes = kPfQBytes + kPfKSlots * kPfKTileBytes + kPfVSlots * kPfVTileBytes;
 constexpr int kPfRowsBytes = kPfM * kHeadDim * 4;          // a tile of f32 gate or output rows: 128 KB
 constexpr int kPfBoxBytes = kPfM * 128;                    // [128 rows][32 dims] of it
-constexpr int kPfThreads = 384;           // 8 softmax warps, K TMA, S MMA, V TMA, PV MMA warps
+constexpr int kPfThreads = 352;           // 8 softmax warps, K TMA, MMA, V TMA warps
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemO = 0;            // columns [0, 256): output accumulator
 constexpr uint32_t kTmemS = 256;          // columns [256, 384): the scores of one tile
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   __shared__ int s_pos[kPfM];
   __shared__ float s_ref[2][kPfM];     // [tile parity][row]: the reference maximum that tile left
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (uniform)
   pdl_launch_dependents();   // the merge pass of a key split may be scheduled under this kernel
   if (!p.kv_wait) pdl_wait();
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 0);   // kernel entry
@@ -454,90 +454,101 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       }
     }
   } else if (warp == 9) {
-    // ============================ MMA issuer: S = Q K^T =============================
-    if (lane == 0 && rank == 0) {
+    // ============ MMA issuer: S = Q K^T of tile i, then O += P V of tile i - 2 ============
+    // One warp, one order: the tensor core works its queue off in order, so a tile's scores are ready after
+    // 1024 cycles and the softmax warps copy them to registers under the P V behind them. The warp stays
+    // converged and elect.sync picks the lane (see elect_one): issued by "lane 0" an instruction took 70 to
+    // 110 cycles of moves to uniform registers, as long as the tensor core runs it. Then each contraction
+    // needed a thread of its own, their instructions lay alternately in the queue, scores came 2300 to 2800 cycles
+    // after the request and the queue ran dry while they were copied: 2950 cycles a tile with all SMs at work,
+    // now 2060 (512 tokens at 7680: 1880 -> 1775 us for 16 layers, at the power cap; 8192 at 0: 825 -> 767).
+    if (rank == 0) {
       constexpr uint32_t idesc_s = idesc_f16(2 * kPfM, kPfN, false);
+      constexpr uint32_t idesc_o = idesc_f16(2 * kPfM, kHeadDim, true);
       // Descriptors differ only in the 16-byte-granular start address (low 14 bits, and
       // every address here is below 256 KB), so each one is a base plus a constant.
       const uint64_t dq = smem_desc(sQ, 16, 1024);
       const uint64_t dk = smem_desc(sK, 16, 1024);
-      bool ok = mbar_wait(bars + 8 * kBarQ, 0, p.status, 18);  // both Q tiles are there
+      const uint64_t dv = smem_desc(sV, kPfVChunkBytes, 1024);
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+      const int n = __shfl_sync(0xffffffffu, nt, 0);
+      auto wait = [&](int bar, int parity, int site) {
+        return __all_sync(0xffffffffu, mbar_wait(bars + 8 * bar, parity, p.status, site));
+      };
+      bool ok = wait(kBarQ, 0, 18);  // both Q tiles are there
       tc_fence_after();
       int slot = 0, use = 0;
-      for (int j = 0; j < nt && ok; ++j) {
-        RD_PF_TRACE(2, j, 0);
-        if (!mbar_wait(bars + 8 * (kBarKFull + slot), use & 1, p.status, 12)) {
-          ok = false;
-          break;
-        }
-        RD_PF_TRACE(2, j, 1);
-        // the softmax warps of tile j - 1 (both CTAs) have its scores in registers
-        if (j >= 1 && !mbar_wait(bars + 8 * kBarL, (j - 1) & 1, p.status, 15)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        RD_PF_TRACE(2, j, 3);
-        // per 64-dim chunk c: A = Q sub-tile c ([128 rows][64 dims] in each CTA), B = K chunk c ([64
-        // keys][64 dims] in each), K-major with 8-row groups 1 KB apart; four steps of 16 dims
-        if (!(RD_PF_DEBUG(p) & 8)) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint64_t a0 = dq + (uint64_t)((c * (kPfM * 128)) >> 4);
-            const uint64_t b0 = dk + (uint64_t)((slot * kPfKTileBytes + c * kPfKChunkBytes) >> 4);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              tc_mma2_f16(tmem + kTmemS, a0 + (uint64_t)(2 * kk), b0 + (uint64_t)(2 * kk), idesc_s,
-                          (c > 0 || kk > 0) ? 1u : 0u);
+      for (int i = 0; i < n + 2 && ok; ++i) {
+        if (i < n) {
+          RD_PF_TRACE(2, i, 0);
+          if (!wait(kBarKFull + slot, use & 1, 12)) {
+            ok = false;
+            break;
           }
+          RD_PF_TRACE(2, i, 1);
+          // the softmax warps of tile i - 1 (both CTAs) have its scores in registers
+          if (i >= 1 && !wait(kBarL, (i - 1) & 1, 15)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          RD_PF_TRACE(2, i, 3);
+          // per 64-dim chunk c: A = Q sub-tile c ([128 rows][64 dims] in each CTA), B = K chunk c ([64
+          // keys][64 dims] in each), K-major with 8-row groups 1 KB apart; four steps of 16 dims
+          if (elect_one()) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const uint64_t a0 = dq + (uint64_t)((c * (kPfM * 128)) >> 4);
+              const uint64_t b0 = dk + (uint64_t)((slot * kPfKTileBytes + c * kPfKChunkBytes) >> 4);
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk)
+                tc_mma2_f16(tm + kTmemS, a0 + (uint64_t)(2 * kk), b0 + (uint64_t)(2 * kk), idesc_s,
+                            (c > 0 || kk > 0) ? 1u : 0u);
+            }
+            tc_commit2(bars + 8 * (kBarS + (i & 1)));
+            tc_commit2(bars + 8 * (kBarKFree + slot));  // the tile can be refilled
+          }
+          __syncwarp();
+          RD_PF_TRACE(2, i, 4);
+          if (++slot == kPfKSlots) {
+            slot = 0;
+            ++use;
+          }
+          RD_PF_TRACE(2, i, 2);
         }
-        RD_PF_TRACE(2, j, 4);
-        tc_commit2(bars + 8 * (kBarS + (j & 1)));
-        tc_commit2(bars + 8 * (kBarKFree + slot));  // the tile can be refilled
-        if (++slot == kPfKSlots) {
-          slot = 0;
-          ++use;
-        }
-        RD_PF_TRACE(2, j, 2);
-      }
-      if (!ok) s_abort = 1;
-    }
-  } else if (warp == 11) {
-    // ============================ MMA issuer: O += P V ==============================
-    if (lane == 0 && rank == 0) {
-      constexpr uint32_t idesc_o = idesc_f16(2 * kPfM, kHeadDim, true);
-      const uint64_t dv = smem_desc(sV, kPfVChunkBytes, 1024);
-      bool ok = true;
-      for (int j = 0; j < nt && ok; ++j) {
-        const int st = j & 1;
+        if (i < 2) continue;
+        const int j = i - 2, st = j & 1;
         RD_PF_TRACE(3, j, 0);
-        if (!mbar_wait(bars + 8 * (kBarVFull + st), (j >> 1) & 1, p.status, 19)) {
+        if (!wait(kBarVFull + st, (j >> 1) & 1, 19)) {
           ok = false;
           break;
         }
         for (int u = 0; u < 2 && ok; ++u) {
           // P arrives in two halves of 64 keys: P V of the first runs while the softmax
           // threads are still on the second
-          if (!mbar_wait(bars + 8 * (kBarP + 2 * st + u), (j >> 1) & 1, p.status, 13)) {
+          if (!wait(kBarP + 2 * st + u, (j >> 1) & 1, 13)) {
             ok = false;
             break;
           }
-          if (u == 0) RD_PF_TRACE(3, j, 1);
+          RD_PF_TRACE(3, j, 1 + 2 * u);
           tc_fence_after();
           // A = P(j) from TMEM (16 keys = 8 columns per step), B = V MN-major, 128 of the 256 dims in each
           // CTA: 64-dim groups 16 KB apart (LBO), 8-key groups 1 KB apart (SBO); 4 steps of 16 keys
           const uint64_t dvs = dv + (uint64_t)((st * kPfVTileBytes + u * 8192) >> 4);
-          const uint32_t a_p = tmem + kTmemP + 64 * st + 32 * u;
-          if (!(RD_PF_DEBUG(p) & 4)) {
+          const uint32_t a_p = tm + kTmemP + 64 * st + 32 * u;
+          if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-              tc_mma2_f16_ts(tmem + kTmemO, a_p + 8 * kk, dvs + (uint64_t)((kk * 2048) >> 4), idesc_o,
+              tc_mma2_f16_ts(tm + kTmemO, a_p + 8 * kk, dvs + (uint64_t)((kk * 2048) >> 4), idesc_o,
                              (j > 0 || u > 0 || kk > 0) ? 1u : 0u);
+            if (u == 1) {
+              tc_commit2(bars + 8 * (kBarVFree + st));  // the V tile can be refilled
+              tc_commit2(bars + 8 * (kBarO + st));      // P buffer reusable, O settled
+            }
           }
+          __syncwarp();
         }
         if (!ok) break;
-        tc_commit2(bars + 8 * (kBarVFree + st));  // the V tile can be refilled
-        tc_commit2(bars + 8 * (kBarO + st));      // P buffer reusable, O settled
         RD_PF_TRACE(3, j, 2);
       }
       if (!ok) s_abort = 1;

@@ -12,6 +12,14 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
+// One lane of a converged warp. tcgen05.mma takes its descriptors from uniform registers: in a branch on the
+// lane number the compiler has to move every one of them there before each instruction, in a branch on
+// elect.sync it knows the warp's values to be uniform.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t x;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(x));
+  return x != 0;
+}
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
