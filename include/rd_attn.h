@@ -167,7 +167,11 @@ int rd_attn_launch_plan(int64_t n_keys, int n_tok, int n_head_kv, int k_type, in
  * sm_count SMs (<= 0: the current device): the key splits per (128-token tile, head) and
  * the CTAs of the tile-kernel launch. One split unless the cost model says that filling the
  * idle SMs outweighs a second wave of fixed costs and the records (from about 8192 keys for
- * 512 tokens x 24 heads on 148 SMs). Host arithmetic only when sm_count is given. */
+ * 512 tokens x 24 heads on 148 SMs). This is the plan of tiles of one head, whose records rd_attn_prefill_workspace_bytes
+ * has room for; rd_attn_prefill_launch_plan is what is launched, with the rows of a tile: tile_heads x tile_tokens.
+ * Host arithmetic only when sm_count is given. */
+int rd_attn_prefill_launch_plan(int n_q, int keys_total, int n_head, int sm_count, int *tile_heads, int *tile_tokens,
+                                int *n_splits, int *n_ctas);
 int rd_attn_prefill_plan(int n_q, int keys_total, int n_head, int sm_count, int *n_splits, int *n_ctas);
 int rd_attn_plan(int n_keys, int n_tok, int n_head_kv, int k_type, int v_type, int sm_count,
                  int *tile_keys, int *ring_stages, int *n_splits);

@@ -47,6 +47,7 @@ SIGNATURES = {
                                _F, _P]),
     "rd_attn_splits_for": (_I, [_I, _I, _I, _I, _I]),
     "rd_attn_prefill_plan": (_I, [_I, _I, _I, _I, _P, _P]),
+    "rd_attn_prefill_launch_plan": (_I, [_I, _I, _I, _I, _P, _P, _P, _P]),
     "rd_attn_launch_plan": (_I, [_L, _I, _I, _I, _I, _I, _P, _P, _P]),
     "rd_attn_plan": (_I, [_I, _I, _I, _I, _I, _I, _P, _P, _P]),
     "rd_attn_partial_bytes": (C.c_size_t, [_I, _I, _I]),

@@ -473,6 +473,26 @@ int rd_attn_prefill_plan(int n_q, int keys_total, int n_head, int sm_count, int 
   return RD_OK;
 }
 
+int rd_attn_prefill_launch_plan(int n_q, int keys_total, int n_head, int sm_count, int *tile_heads, int *tile_tokens,
+                                int *n_splits, int *n_ctas) {
+  if (n_q < 1 || keys_total < 1 || n_head < 1) return RD_ERR_SHAPE;
+  if (n_head % kGroup != 0) return RD_ERR_UNSUPPORTED;
+  if (sm_count <= 0) {
+    int dev;
+    const int rc = current_device(&dev);
+    if (rc != RD_OK) return rc;
+    sm_count = ::sm_count(dev);
+  }
+  const PrefillPlan p = prefill_plan(n_q, keys_total, n_head, sm_count,
+                                     prefill_splits(n_q, keys_total, n_head, sm_count) > 1 ? SIZE_MAX : 0);
+  const int tokens = prefill_tile_tokens(p.heads);
+  if (tile_heads != nullptr) *tile_heads = p.heads;
+  if (tile_tokens != nullptr) *tile_tokens = tokens;
+  if (n_splits != nullptr) *n_splits = p.splits;
+  if (n_ctas != nullptr) *n_ctas = (n_q + tokens - 1) / tokens * (n_head / p.heads) * p.splits;
+  return RD_OK;
+}
+
 size_t rd_attn_partial_bytes(int n_head, int head_dim, int n_splits) {
   if (n_head < 0 || head_dim < 0 || n_splits < 0) return 0;
   return (size_t)n_head * (size_t)n_splits * (2 + (size_t)head_dim) * sizeof(float);
@@ -1058,20 +1078,21 @@ static int prefill_common(const float *q, const void *k, const void *v, float *o
   if ((rc = current_device(&dev)) != RD_OK) return rc;
   DeviceStatus *status = status_word(dev);   // every launch reports its bounded waits
   if (status == nullptr) return RD_ERR_CUDA;
-  int splits = prefill_splits(n_q, keys_total, n_head, sm_count(dev));
-  const size_t need = prefill_record_bytes(n_q, n_head, splits);
-  if (records == nullptr && splits > 1) {
-    records = ensure_workspace(dev, need);
+  // Records of a key split: in the caller's memory as far as it goes, or in the library's workspace, which is
+  // used where the one-head form wants a split (an unsplit call needs none, and never allocates).
+  const int sms = sm_count(dev);
+  if (records == nullptr) record_bytes = prefill_splits(n_q, keys_total, n_head, sms) > 1 ? SIZE_MAX : 0;
+  const PrefillPlan plan = prefill_plan(n_q, keys_total, n_head, sms, record_bytes);
+  if (records == nullptr && plan.splits > 1) {
+    records = ensure_workspace(dev, prefill_record_bytes(n_q, n_head, plan.splits));
     if (records == nullptr) return RD_ERR_CUDA;
-    record_bytes = need;
   }
-  if (record_bytes < need) splits = 1;   // no room: one CTA per (token tile, head) walks all keys
   // a fused append stores rows row0 .. row0 + n_q - 1 of the (f16) caches
   const size_t row_bytes = (size_t)n_head_kv * kHeadDim * 2;
   void *k_dst = k_new != nullptr ? (void *)((unsigned char *)const_cast<void *>(k) + (size_t)row0 * row_bytes) : nullptr;
   void *v_dst = k_new != nullptr ? (void *)((unsigned char *)const_cast<void *>(v) + (size_t)row0 * row_bytes) : nullptr;
   return launch_prefill(q, k, v, o, gate, pos, n_q, keys_total, n_head, n_head_kv, scale, n_rot,
-                        freq_base, status, (float *)records, splits, k_new, v_new, k_dst, v_dst, kv_pending,
+                        freq_base, status, (float *)records, plan, k_new, v_new, k_dst, v_dst, kv_pending,
                         (cudaStream_t)stream);
 }
 
@@ -1106,14 +1127,23 @@ static size_t prefill_copy_bytes(int k_type, int v_type, int keys_total, int n_h
   const size_t one = align256((size_t)keys_total * n_head_kv * kHeadDim * 2);
   return (k_type != RD_KV_F16 ? one : 0) + (v_type != RD_KV_F16 ? one : 0);
 }
-size_t rd_attn_prefill_workspace_bytes(int k_type, int v_type, int n_q, int keys_total, int n_head,
-                                       int n_head_kv, int head_dim) {
+// What a call has to have, and what it makes use of: a chunk of up to 256 tokens is cut into more key ranges than
+// the one-head form's where its records find room.
+static size_t prefill_workspace(int k_type, int v_type, int n_q, int keys_total, int n_head, int n_head_kv,
+                                int head_dim, bool all) {
   int dev;
   if (!known_type(k_type) || !known_type(v_type) || n_q < 1 || keys_total <= 0 || n_head < 1 ||
       n_head_kv < 1 || head_dim != kHeadDim || current_device(&dev) != RD_OK)
     return 0;
+  const int sms = sm_count(dev);
+  int splits = prefill_splits(n_q, keys_total, n_head, sms);
+  if (all && n_q <= 256) splits = std::max(splits, prefill_plan(n_q, keys_total, n_head, sms, SIZE_MAX).splits);
   return prefill_copy_bytes(k_type, v_type, keys_total, n_head_kv) +
-         align256(prefill_record_bytes(n_q, n_head, prefill_splits(n_q, keys_total, n_head, sm_count(dev))));
+         align256(prefill_record_bytes(n_q, n_head, splits));
+}
+size_t rd_attn_prefill_workspace_bytes(int k_type, int v_type, int n_q, int keys_total, int n_head,
+                                       int n_head_kv, int head_dim) {
+  return prefill_workspace(k_type, v_type, n_q, keys_total, n_head, n_head_kv, head_dim, true);
 }
 
 int rd_attn_prefill_typed(const float *q, const void *k, const void *v, float *o, const float *gate,
@@ -1126,7 +1156,7 @@ int rd_attn_prefill_typed(const float *q, const void *k, const void *v, float *o
   if (k == nullptr || v == nullptr) return RD_ERR_NULL;
   if (!aligned(k, 16) || !aligned(v, 16)) return RD_ERR_ALIGN;
   const size_t copies = prefill_copy_bytes(k_type, v_type, keys_total, n_head_kv);
-  const size_t need = rd_attn_prefill_workspace_bytes(k_type, v_type, n_q, keys_total, n_head, n_head_kv, head_dim);
+  const size_t need = prefill_workspace(k_type, v_type, n_q, keys_total, n_head, n_head_kv, head_dim, false);
   if (need > 0) {
     if (workspace == nullptr || workspace_bytes < need) return RD_ERR_WORKSPACE;
     if (!aligned(workspace, 256)) return RD_ERR_ALIGN;
@@ -1159,7 +1189,8 @@ int rd_attn_prefill_typed(const float *q, const void *k, const void *v, float *o
   static float s_dummy;   // non-null marker when no records are needed
   return prefill_common(q, k16, v16, o, gate, pos, n_q, keys_total, n_head, n_head_kv, head_dim, scale,
                         n_rot, freq_base, stream, rec != nullptr ? (void *)rec : (void *)&s_dummy,
-                        need > copies ? need - copies : 0, nullptr, nullptr, 0, kdst != nullptr || vdst != nullptr);
+                        need > 0 ? workspace_bytes - copies : 0, nullptr, nullptr, 0,
+                        kdst != nullptr || vdst != nullptr);
 }
 
 static int g_last_site = 0;   // `where` of the last time-out rd_device_status reported

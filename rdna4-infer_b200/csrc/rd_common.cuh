@@ -344,15 +344,24 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
-// shared -> global: rows and columns outside the tensor are not written; completion by bulk groups.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src_smem, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
-               "r"(src_smem), "r"(x), "r"(y)
+__device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap *map, int x, int y, int z,
+                                            uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, "
+      "{%2, %3, %4}], [%5];" ::"r"(dst_smem),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+// shared -> global: what lies outside the tensor is not written; completion by bulk groups.
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, uint32_t src_smem, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map),
+               "r"(src_smem), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
 // A box of global memory to L2 only.
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int x, int y, int z) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(x), "r"(y), "r"(z)
+               : "memory");
 }
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

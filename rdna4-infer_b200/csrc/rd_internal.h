@@ -156,24 +156,30 @@ int encode_kv_tmap(void *tmap_out, const void *base, int type, int n_head_kv, in
 // with SWIZZLE_128B read).
 int encode_f16_tmap(void *tmap_out, const void *base, int n_head_kv, int64_t n_rows, int tile_rows);
 
-// Tensor map over f32 activations [n_rows][n_head * 256] with a box of [tile_rows][32 dims] and the
+// Tensor map over f32 activations [n_rows][n_head][width] with a box of [tokens][heads][32 dims] and the
 // hardware 128-byte swizzle.
-int encode_f32_tmap(void *tmap_out, const void *base, int n_head, int64_t n_rows, int tile_rows);
+int encode_f32_tmap(void *tmap_out, const void *base, int width, int n_head, int64_t n_rows, int heads, int tokens);
 
 // ---- rd_prefill.cu
 // Causal prefill attention over f16 caches on tcgen05: token i attends keys 0..pos[i]
 // (pos on the device), keys_total rows exist in the cache. gate (optional) fuses
 // out *= sigmoid(gate); n_rot > 0 applies the partial RoPE to the queries on load.
-// n_splits > 1 (with `records`, prefill_record_bytes(...) bytes): the keys are also split
+// splits > 1 (with `records`, prefill_record_bytes(...) bytes): the keys are also split
 // over gridDim.z and a second launch merges the per-split records.
+struct PrefillPlan {
+  int heads;    // of a CTA's rows: 1 (x 128 tokens) or 3 (x 42 tokens)
+  int splits;   // of the keys
+};
 int launch_prefill(const float *q, const void *k, const void *v, float *out, const float *gate,
                    const int32_t *pos, int n_q, int keys_total, int n_head, int n_head_kv, float scale,
-                   int n_rot, float freq_base, DeviceStatus *status, float *records, int n_splits,
+                   int n_rot, float freq_base, DeviceStatus *status, float *records, PrefillPlan plan,
                    const float *k_new, const float *v_new, void *k_dst, void *v_dst, bool kv_pending,
                    cudaStream_t st);   // kv_pending: the launch before this one writes k and v, and has waited
                                        // for everything before it (kv_dequant_f16_kernel)
 int prefill_splits(int n_q, int keys_total, int n_head, int sms);
 size_t prefill_record_bytes(int n_q, int n_head, int splits);
+int prefill_tile_tokens(int heads);
+PrefillPlan prefill_plan(int n_q, int keys_total, int n_head, int sms, size_t record_bytes);   // with that much memory
 
 // ---- rd_merge.cu
 // partial [n_rows][n_splits][258] -> out [n_rows][256]; optional fused sigmoid gate.

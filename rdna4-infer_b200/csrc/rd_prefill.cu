@@ -80,15 +80,18 @@ constexpr int kPfVTileBytes = 2 * kPfVChunkBytes;          // 32768
 constexpr int kPfVSlots = 2;
 // 224 KB of dynamic shared memory + < 3 KB static = the 227 KB an sm_100 CTA may use
 constexpr int kPfSmemBytes = kPfQBytes + kPfKSlots * kPfKTileBytes + kPfVSlots * kPfVTileBytes;
-constexpr int kPfRowsBytes = kPfM * kHeadDim * 4;          // a tile of f32 gate or output rows: 128 KB
-constexpr int kPfBoxBytes = kPfM * 128;                    // [128 rows][32 dims] of it
+constexpr int kPfBoxBytes = kPfM * 128;                    // [128 rows][32 dims] f32 of gate or output
 constexpr int kPfThreads = 352;           // 8 softmax warps, K TMA, MMA, V TMA warps
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemO = 0;            // columns [0, 256): output accumulator
 constexpr uint32_t kTmemS = 256;          // columns [256, 384): the scores of one tile
 constexpr uint32_t kTmemP = 384;          // columns [384, 512): two buffers of 64 for the f16 P
 constexpr float kLazyThreshold = 8.0f;    // log2 units
-constexpr int kPfMaxSplits = 8;           // key splits per (token tile, head) at most
+constexpr int kPfMaxSplits = 20;          // key splits of a tile at most
+// A CTA's 128 query rows: one head of 128 tokens (kHeads 1), or the three heads of half a KV head's group of 42
+// tokens, token by token (kHeads 3; two rows stay empty). The pair's CTAs serve the same tokens: two heads, or all
+// six of the group.
+constexpr int pf_tokens(int heads) { return heads == 1 ? kPfM : kPfM / heads; }
 
 struct PrefillArgs {
   alignas(64) CUtensorMap tm_k;
@@ -101,7 +104,7 @@ struct PrefillArgs {
   int n_head;
   int nkv;
   float qscale;          // scale * log2(e)
-  alignas(64) CUtensorMap tm_g;  // f32 rows of `gate` and `out`: boxes of [128 tokens][32 dims], 128-byte swizzle
+  alignas(64) CUtensorMap tm_g;  // f32 rows of `gate` and `out`: boxes of [tokens][heads][32 dims], 128-byte swizzle
   alignas(64) CUtensorMap tm_o;
   int n_rot;             // partial RoPE of the queries: dims [0, n_rot), pairs (d, d + n_rot / 2)
   float freq[32];        // rotation frequencies of the pairs
@@ -136,13 +139,15 @@ __device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, 
     if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait(bar, parity, status, site);   // bounded
 }
+template <int kHeads>
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_constant__ PrefillArgs p) {
+  constexpr int kTokens = pf_tokens(kHeads), kRows = kTokens * kHeads;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) unsigned long long s_bars[kBarCount];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_maxpos;
   __shared__ int s_abort;
-  __shared__ int s_pos[kPfM];
+  __shared__ int s_pos[kPfM];          // by token
   __shared__ float s_ref[2][kPfM];     // [tile parity][row]: the reference maximum that tile left
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (uniform)
@@ -150,10 +155,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   if (!p.kv_wait) pdl_wait();
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 0);   // kernel entry
   const int tile = (int)gridDim.y - 1 - (int)blockIdx.y;  // heaviest (latest) tiles first
-  const int head = blockIdx.x;                            // heads 2 i and 2 i + 1 (one KV head) are a pair
+  const int head = blockIdx.x * kHeads;                   // the CTA's first head; the pair's are of one KV head
   const uint32_t rank = blockIdx.x & 1;
   const int kvh = head / kGroup;
-  const int row0 = tile * kPfM;
+  const int tok0 = tile * kTokens;
 
   // carve-up of dynamic shared memory; 128B-swizzle atoms need the base 1 KB aligned
   const uint32_t base = smem_u32(smem_raw);
@@ -172,30 +177,32 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   // rows and, to L2, the warp's 16 query rows. (Loaded to registers here they are spilled, and the spill
   // waits for them.)
   int my_pos = -1;
-  const int rows_cta = p.n_q - row0;                                  // rows of the tile that exist
-  const int rows_cs = rows_cta > 64 ? 128 : rows_cta > 32 ? 64 : 32;   // and that the (cos, sin) table is made for
+  const int toks_cta = min(p.n_q - tok0, kTokens), rows_cta = toks_cta * kHeads;   // of the tile, how many exist
+  const int toks_cs = toks_cta > 64 ? 128 : toks_cta > 32 ? 64 : 32;   // and how many the (cos, sin) table is made for
   float4 xa[8], xb[8];   // dims 4 lane .. + 3 and 128 + 4 lane .. + 3 of a row
-  const float *qw = p.q + ((size_t)(row0 + warp * 16) * p.n_head + head) * kHeadDim;
-  const size_t q_row = (size_t)p.n_head * kHeadDim;
-  const int rows_w = p.n_q - row0 - warp * 16;   // of the warp's rows, how many exist
+  const int rows_w = rows_cta - warp * 16;   // of the warp's rows, how many exist
+  auto q_at = [&](int rr) {                  // its rr-th one
+    const int row = warp * 16 + rr;
+    return p.q + ((size_t)(tok0 + row / kHeads) * p.n_head + head + row % kHeads) * kHeadDim;
+  };
   auto load_rows = [&](int first) {
 #pragma unroll
     for (int rr = 0; rr < 8; ++rr) {
       xa[rr] = xb[rr] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (first + rr < rows_w) {
-        const float4 *src = reinterpret_cast<const float4 *>(qw + (first + rr) * q_row);
+        const float4 *src = reinterpret_cast<const float4 *>(q_at(first + rr));
         xa[rr] = src[lane];
         xb[rr] = src[lane + 32];
       }
     }
   };
   if (threadIdx.x < 2 * kPfM) {
-    const int r = row0 + (threadIdx.x & (kPfM - 1));
-    if (r < p.n_q) my_pos = p.pos[r];
+    const int r = threadIdx.x & (kPfM - 1);
+    if (r < rows_cta) my_pos = p.pos[tok0 + r / kHeads];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {   // 16 rows x 8 lines of 128 bytes
       const int rr = (lane >> 3) + 4 * e;
-      if (rr < rows_w) asm volatile("prefetch.global.L2 [%0];" ::"l"(qw + rr * q_row + 32 * (lane & 7)));
+      if (rr < rows_w) asm volatile("prefetch.global.L2 [%0];" ::"l"(q_at(rr) + 32 * (lane & 7)));
     }
   }
 
@@ -225,7 +232,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     mbar_init(bars + 8 * kBarC, 8);
     mbar_init(bars + 8 * kBarG, 1);
     fence_barrier_init();
-    mbar_expect_tx(bars + 8 * kBarT, p.n_rot == 64 ? rows_cs / 2 * 32 * 8 : 0);
+    mbar_expect_tx(bars + 8 * kBarT, p.n_rot == 64 ? toks_cs / 2 * 32 * 8 : 0);
   }
   if (warp == 9) {  // TMEM: 512 columns for this CTA (one CTA per SM: no contention)
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -241,7 +248,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   // ---- the last key any row of this tile attends ----
   if (threadIdx.x < kPfM) {
     int mx = my_pos;
-    s_pos[threadIdx.x] = my_pos;
+    if (kHeads == 1 || threadIdx.x % kHeads == 0) s_pos[threadIdx.x / kHeads] = my_pos;
+    if (kHeads > 1 && threadIdx.x > kTokens) s_pos[threadIdx.x] = -1;   // (the table is made for more tokens)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) atomicMax(&s_maxpos, mx);
@@ -293,16 +301,16 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     load_rows(8);
     if (threadIdx.x == 0) RD_PF_TRACE(0, 46, 4);
     // (cos, sin) of all rows and pairs, while those are on their way: the two CTAs of the pair serve the same
-    // tokens, each computes half for both (16 sincosf per thread took 4200 cycles). [pair][row] in V slot 0.
+    // tokens, each computes half for both (16 sincosf per thread took 4200 cycles). [pair][token] in V slot 0.
     const uint32_t cs0 = sV;
     const float *cs = reinterpret_cast<const float *>(gQ + (sV - sQ));
     if (p.n_rot == 64) {
-      const int id = (int)rank * 256 + threadIdx.x, tr = id & (rows_cs - 1);   // row, and rows_cs / 16 pairs of it
-      const int tp = id / rows_cs * (rows_cs / 16);
+      const int id = (int)rank * 256 + threadIdx.x, tr = id & (toks_cs - 1);   // token, and toks_cs / 16 pairs of it
+      const int tp = id / toks_cs * (toks_cs / 16);
       const float fpos = (float)s_pos[tr];
       const uint32_t peer = cluster_addr(cs0, rank ^ 1), peer_bar = cluster_addr(bars + 8 * kBarT, rank ^ 1);
 #pragma unroll 1
-      for (int i = 0; i < rows_cs / 16; i += 2) {
+      for (int i = 0; i < toks_cs / 16; i += 2) {
         float2 v[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) sincosf(fpos * p.freq[tp + i + e], &v[e].y, &v[e].x);
@@ -334,7 +342,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
 #pragma unroll
         for (int k = 0; k < 4; ++k) ca[k] = chunk(4 * h + k), cb[k] = chunk(8 + 4 * h + k);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) cc[e] = reinterpret_cast<const float2 *>(cs)[(16 * h + e) * kPfM + r];
+        for (int e = 0; e < 16; ++e) cc[e] = reinterpret_cast<const float2 *>(cs)[(16 * h + e) * kPfM + r / kHeads];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {   // four pairs
           const float4 a = ca[k], b = cb[k];
@@ -418,9 +426,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
             (nt == 0 ||
              mbar_wait(bars + 8 * (kBarKFree + (nt - 1) % kPfKSlots), ((nt - 1) / kPfKSlots) & 1, p.status, 27));
         if (ok) {
-          mbar_expect_tx(bars + 8 * kBarG, kPfRowsBytes);
+          mbar_expect_tx(bars + 8 * kBarG, kRows * kHeadDim * 4);
           for (int c = 0; c < 8; ++c)
-            tma_load_2d(sQ + c * kPfBoxBytes, &p.tm_g, head * kHeadDim + 32 * c, row0, bars + 8 * kBarG);
+            tma_load_3d(sQ + c * kPfBoxBytes, &p.tm_g, 32 * c, head, tok0, bars + 8 * kBarG);
         } else {
           s_abort = 1;
           mbar_arrive(bars + 8 * kBarG);   // nobody waits for long
@@ -434,7 +442,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       // the gate rows that the epilogue multiplies with, on their way to L2 once the queries have arrived
       // (before, the two would share the memory's bandwidth and the queries come first)
       mbar_wait(bars + 8 * kBarC, 0, nullptr, 0);
-      for (int c = 0; c < 8; ++c) tma_prefetch_2d(&p.tm_g, head * kHeadDim + 32 * c, row0);
+      for (int c = 0; c < 8; ++c) tma_prefetch_3d(&p.tm_g, 32 * c, head, tok0);
     }
     if (lane == 0) {
       if (p.kv_wait) pdl_wait();
@@ -569,7 +577,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const bool live = 32 * (warp & 3) < rows_cta;   // (the barriers count the warps that have a row)
     // Rows past the last query see every key: nobody reads what they give, and a mask on their account would
     // be a mask on every tile (24 queries at 16000: 94 us a layer with it).
-    const int last_key = row0 + r < p.n_q ? my_pos : 0x7fffffff;
+    const int last_key = r < rows_cta ? my_pos : 0x7fffffff;
     for (int j = set; live && j < nt && ok; j += 2) {
       const int st = set;   // tile j's P buffer: j & 1
       if ((threadIdx.x & 127) == 0) RD_PF_TRACE(set, j, 0);
@@ -719,12 +727,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const bool rec_mode = gridDim.z > 1;   // un-normalised records for prefill_merge_kernel
     const float inv = (l_tot > 0.f && !aborted) ? (rec_mode ? 1.0f : 1.0f / l_tot) : 0.f;
     const bool have = nt > 0 && !aborted;
-    // column of the first value in the output, or in the accumulators of the records
-    const int col0 = (rec_mode ? head * (int)gridDim.z + (int)blockIdx.z : head) * kHeadDim;
-    if (rec_mode && ch == 0 && row0 + r < p.n_q) {
+    // column of the first value in a head's output, or in the accumulators of its records
+    const int col0 = rec_mode ? (int)blockIdx.z * kHeadDim : 0;
+    if (rec_mode && ch == 0 && r < rows_cta) {
       // (m, l) of this row's record, in natural-log units
       const bool some = have && l_tot > 0.f;
-      p.rec_ml[((size_t)(row0 + r) * p.n_head + head) * gridDim.z + blockIdx.z] =
+      p.rec_ml[((size_t)(tok0 + r / kHeads) * p.n_head + head + r % kHeads) * gridDim.z + blockIdx.z] =
           some ? make_float2(m_fin * 0.6931471805599453f, l_tot) : make_float2(-INFINITY, 0.f);
     }
     {
@@ -735,7 +743,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
 #pragma unroll 1
       for (int b = ch; b < 8; b += 2) {
         uint32_t o[32];
-        if (row0 + 32 * (warp & 3) >= p.n_q) {   // none of the warp's rows exists: only the barrier below
+        if (32 * (warp & 3) >= rows_cta) {   // none of the warp's rows exists: only the barrier below
           asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
           continue;
         }
@@ -795,7 +803,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         fence_proxy_async();
         asm volatile("bar.sync %0, 128;" ::"r"(3 + ch) : "memory");
         if (gt == 0) {
-          tma_store_2d(&p.tm_o, sQ + b * kPfBoxBytes, col0 + 32 * b, row0);   // rows past n_q are clipped
+          tma_store_3d(&p.tm_o, sQ + b * kPfBoxBytes, col0 + 32 * b, head, tok0);   // tokens past n_q are clipped
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
         if (threadIdx.x == 0) RD_PF_TRACE(1, 47, b >> 1);
@@ -815,6 +823,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
 // Combines the key-split records of a row: one warp-pair (64 threads, 4 dims each) per row
 // (token, head); out = sum_z acc_z e^(m_z - M) / sum_z l_z e^(m_z - M), times sigmoid(gate)
 // if given (the gate is only read). Rows whose records are all empty give zeros.
+template <int kMax>   // records of a row at most
 __global__ void __launch_bounds__(256)
 prefill_merge_kernel(const float4 *__restrict__ rec_acc, const float2 *__restrict__ rec_ml, float *__restrict__ out,
                      const float *__restrict__ gate, int64_t n_rows, int n_splits) {
@@ -823,12 +832,12 @@ prefill_merge_kernel(const float4 *__restrict__ rec_acc, const float2 *__restric
   pdl_launch_dependents();
   pdl_wait();   // launched under the tile kernel: its records are complete from here on
   if (row >= n_rows) return;
-  // every load of the row is requested before the first is used (at most kPfMaxSplits
+  // every load of the row is requested before the first is used (at most kMax
   // records): one round trip to L2 instead of one for the maxima and one per record
-  float m[kPfMaxSplits], lz[kPfMaxSplits];
-  float4 va[kPfMaxSplits];
+  float m[kMax], lz[kMax];
+  float4 va[kMax];
 #pragma unroll
-  for (int z = 0; z < kPfMaxSplits; ++z) {
+  for (int z = 0; z < kMax; ++z) {
     m[z] = -INFINITY;
     lz[z] = 0.f;
     va[z] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -843,12 +852,12 @@ prefill_merge_kernel(const float4 *__restrict__ rec_acc, const float2 *__restric
   if (gate != nullptr) g = *reinterpret_cast<const float4 *>(gate + (size_t)row * kHeadDim + 4 * tx);
   float mm = -INFINITY;
 #pragma unroll
-  for (int z = 0; z < kPfMaxSplits; ++z) mm = fmaxf(mm, m[z]);
+  for (int z = 0; z < kMax; ++z) mm = fmaxf(mm, m[z]);
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float l = 0.f;
   if (mm != -INFINITY) {
 #pragma unroll
-    for (int z = 0; z < kPfMaxSplits; ++z) {
+    for (int z = 0; z < kMax; ++z) {
       if (m[z] == -INFINITY) continue;
       const float w = __expf(m[z] - mm);
       l = fmaf(lz[z], w, l);
@@ -955,7 +964,7 @@ int prefill_splits(int n_q, int keys_total, int n_head, int sms) {
   };
   int best = 1;
   double best_cost = cost(1) * 0.92;   // a split must win clearly to be worth its records
-  for (int z = 2; z <= kPfMaxSplits && tiles / z >= 8; ++z) {
+  for (int z = 2; z <= 8 && tiles / z >= 8; ++z) {
     if (cost(z) < best_cost) {
       best_cost = cost(z);
       best = z;
@@ -963,13 +972,49 @@ int prefill_splits(int n_q, int keys_total, int n_head, int sms) {
   }
   return best;
 }
+// The rows of a CTA and the key splits of a launch. In key tiles (1.05 us): a wave of CTAs takes its tiles and nine
+// more (prologue and epilogue, 19800 cycles), a record of a row 0.00045 (written, and read by the merge launch).
+// Three heads of 42 tokens leave fewer rows empty than one head of 128 where the tokens end soon behind a tile's
+// edge or do not fill a tile, and their smaller launch leaves room for more key ranges. Where both cost the same, the
+// smaller split launch is the faster one, of unsplit ones that with one head (its warps without a row do nothing).
+// us a layer, one head | three heads, best split in brackets:
+//     24 of 24024   58.6 (6) | 34.9 (18)       130 of  4130   33.3 (3) | 30.3 (4)       31 of   31   14.9 | 16.0
+//     60 of  9060   32.0 (6) | 30.1 (8)        200 of 12200   64.0 (3) | 60.4 (3)      450 of 4450   61.9 | 61.1
+//    700 of  5700   82.7     | 77.7            389 of 12346  123.5 (3) | 118.1 (3)    1500 of 4500  128.3 | 134.7
+PrefillPlan prefill_plan(int n_q, int keys_total, int n_head, int sms, size_t record_bytes) {
+  PrefillPlan best = {1, 1};
+  const int tiles = (keys_total + kPfN - 1) / kPfN;
+#ifdef RD_TIMING_SWITCHES
+  if (const char *e = getenv("RD_PF_FORM")) {   // timing builds: force heads and splits
+    best.heads = atoi(e);
+    if (const char *f = getenv("RD_PF_SPLITS")) best.splits = atoi(f);
+    return best;
+  }
+#endif
+  auto cost = [&](int heads, int z) {
+    const int ctas = (n_q + pf_tokens(heads) - 1) / pf_tokens(heads) * (n_head / heads) * z;
+    return (double)((ctas + sms - 1) / sms) * ((double)tiles / z + 9.0) + (z > 1 ? 0.00045 * n_q * n_head * z : 0.0) +
+           (heads == 3 && z > 1 ? -0.01 : 0.0);
+  };
+  double best_cost = cost(1, 1);
+  for (int heads = 1; heads <= 3; heads += 2)
+    for (int z = 1; z <= kPfMaxSplits && (z == 1 || tiles / z >= 4); ++z) {
+      if (prefill_record_bytes(n_q, n_head, z) > record_bytes) break;
+      if (cost(heads, z) < best_cost) {
+        best_cost = cost(heads, z);
+        best = {heads, z};
+      }
+    }
+  return best;
+}
+int prefill_tile_tokens(int heads) { return pf_tokens(heads); }
 size_t prefill_record_bytes(int n_q, int n_head, int splits) {
   return splits > 1 ? (size_t)n_q * n_head * splits * kRec * sizeof(float) : 0;
 }
 
 int launch_prefill(const float *q, const void *k, const void *v, float *out, const float *gate,
                    const int32_t *pos, int n_q, int keys_total, int n_head, int n_head_kv, float scale,
-                   int n_rot, float freq_base, DeviceStatus *status, float *records, int n_splits,
+                   int n_rot, float freq_base, DeviceStatus *status, float *records, PrefillPlan plan,
                    const float *k_new, const float *v_new, void *k_dst, void *v_dst, bool kv_pending,
                    cudaStream_t st) {
   PrefillArgs a;
@@ -986,13 +1031,14 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   a.n_head = n_head;
   a.nkv = n_head_kv;
   a.qscale = scale * 1.4426950408889634f;
-  if (n_splits < 1 || records == nullptr) n_splits = 1;
+  const int heads = plan.heads, tokens = pf_tokens(heads), n_splits = records == nullptr ? 1 : plan.splits;
+  if (n_splits < 1 || n_splits > kPfMaxSplits || (heads != 1 && heads != 3)) return RD_ERR_SHAPE;
   if (n_splits > 1) {
     a.rec_ml = reinterpret_cast<float2 *>(records + (size_t)n_q * n_head * n_splits * kHeadDim);
-    if ((rc = encode_f32_tmap(&a.tm_o, records, n_head * n_splits, n_q, kPfM)) != RD_OK) return rc;
+    if ((rc = encode_f32_tmap(&a.tm_o, records, kHeadDim * n_splits, n_head, n_q, heads, tokens)) != RD_OK) return rc;
   } else {
-    if (gate != nullptr && (rc = encode_f32_tmap(&a.tm_g, gate, n_head, n_q, kPfM)) != RD_OK) return rc;
-    if ((rc = encode_f32_tmap(&a.tm_o, out, n_head, n_q, kPfM)) != RD_OK) return rc;
+    if (gate != nullptr && (rc = encode_f32_tmap(&a.tm_g, gate, kHeadDim, n_head, n_q, heads, tokens)) != RD_OK) return rc;
+    if ((rc = encode_f32_tmap(&a.tm_o, out, kHeadDim, n_head, n_q, heads, tokens)) != RD_OK) return rc;
   }
   a.n_rot = n_rot;
   if (n_rot > 0) memcpy(a.freq, make_rope_table(n_rot, freq_base).f, sizeof(a.freq));
@@ -1006,9 +1052,9 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return RD_ERR_CUDA;
   if (dev < 0 || dev >= 32 || !attr_set[dev]) {
-    if (cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kPfSmemBytes) != cudaSuccess)
-      return RD_ERR_CUDA;
+    for (auto *f : {prefill_kernel<1>, prefill_kernel<3>})
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes) != cudaSuccess)
+        return RD_ERR_CUDA;
     if (dev >= 0 && dev < 32) attr_set[dev] = true;
   }
   if (k_new != nullptr) {
@@ -1020,7 +1066,7 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
       return RD_ERR_CUDA;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)n_head, (unsigned)((n_q + kPfM - 1) / kPfM), (unsigned)n_splits);
+  cfg.gridDim = dim3((unsigned)(n_head / heads), (unsigned)((n_q + tokens - 1) / tokens), (unsigned)n_splits);
   cfg.blockDim = dim3(kPfThreads);
   cfg.dynamicSmemBytes = kPfSmemBytes;
   cfg.stream = st;
@@ -1034,10 +1080,9 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  if (cudaLaunchKernelEx(&cfg, prefill_kernel, a) != cudaSuccess) return RD_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, heads == 1 ? prefill_kernel<1> : prefill_kernel<3>, a) != cudaSuccess) return RD_ERR_CUDA;
   if (n_splits > 1) {
     const int64_t n_rows = (int64_t)n_q * n_head;
-    if (n_splits > kPfMaxSplits) return RD_ERR_SHAPE;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((n_rows + 3) / 4));
     cfg.blockDim = dim3(256);
@@ -1047,7 +1092,10 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, prefill_merge_kernel, (const float4 *)records, (const float2 *)a.rec_ml, out,
+    if (cudaLaunchKernelEx(&cfg, n_splits <= 8    ? prefill_merge_kernel<8>
+                                 : n_splits <= 12 ? prefill_merge_kernel<12>
+                                                  : prefill_merge_kernel<kPfMaxSplits>,
+                           (const float4 *)records, (const float2 *)a.rec_ml, out,
                            gate, n_rows, n_splits) !=
         cudaSuccess)
       return RD_ERR_CUDA;

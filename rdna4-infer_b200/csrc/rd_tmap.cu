@@ -66,16 +66,16 @@ int encode_f16_tmap(void *tmap_out, const void *base, int n_head_kv, int64_t n_r
   return r == CUDA_SUCCESS ? RD_OK : RD_ERR_CUDA;
 }
 
-int encode_f32_tmap(void *tmap_out, const void *base, int n_head, int64_t n_rows, int tile_rows) {
+int encode_f32_tmap(void *tmap_out, const void *base, int width, int n_head, int64_t n_rows, int heads, int tokens) {
   std::call_once(g_once, resolve);
   if (g_encode == nullptr) return RD_ERR_CUDA;
-  if (n_rows < 1 || tile_rows > 256) return RD_ERR_SHAPE;
+  if (n_rows < 1 || tokens > 256 || heads > n_head) return RD_ERR_SHAPE;
   if (((uintptr_t)base & 15) != 0) return RD_ERR_ALIGN;
-  const cuuint64_t dims[2] = {(cuuint64_t)n_head * kHeadDim, (cuuint64_t)n_rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)n_head * kHeadDim * 4};
-  const cuuint32_t box[2] = {32, (cuuint32_t)tile_rows};  // 32 floats = one 128-byte swizzle row
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = g_encode((CUtensorMap *)tmap_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+  const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)n_head, (cuuint64_t)n_rows};
+  const cuuint64_t strides[2] = {(cuuint64_t)width * 4, (cuuint64_t)n_head * width * 4};
+  const cuuint32_t box[3] = {32, (cuuint32_t)heads, (cuuint32_t)tokens};  // 32 floats = one 128-byte swizzle row
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = g_encode((CUtensorMap *)tmap_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                               const_cast<void *>(base), dims, strides, box, estr,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

@@ -1,0 +1,79 @@
+"""Prefill tiles of three heads x 42 tokens: edges of a tile, rotation, gate, many key splits, a workspace with room
+for fewer records than the plan wants; against the oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from tests.conftest import check_attn
+from tests.test_gpu_prefill_edges import rotated
+
+pytestmark = pytest.mark.gpu
+HD, NKV, NH = 256, 1, 6
+
+
+@pytest.fixture(scope="module")
+def G(cuda):
+    from tests import gpu_util
+    return gpu_util
+
+
+def plan(lib, n_q, n):
+    heads, z = C.c_int(), C.c_int()
+    assert lib.rd_attn_prefill_launch_plan(n_q, n, NH, 148, C.addressof(heads), None, C.addressof(z), None) == 0
+    return heads.value, z.value
+
+
+@pytest.mark.parametrize("n_q,pos0,n_rot", [(1, 2100, 64), (31, 2100, 64), (42, 2100, 64), (43, 3000, 64), (64, 3000, 32),
+                                            (85, 2100, 64), (126, 2100, 0), (127, 2100, 64), (253, 6000, 64), (24, 9000, 64)])
+def test_three_head_tiles(G, oracle, n_q, pos0, n_rot):
+    rd, lib = G.rd, G.lib
+    n = pos0 + n_q
+    heads, z = plan(lib, n_q, n)
+    assert heads == 3 and (z > 12 if pos0 == 9000 else z > 1)
+    rng = np.random.default_rng(n_q)
+    K, V = (rng.standard_normal((n, NKV, HD)).astype(np.float32) for _ in range(2))
+    q, gate = (rng.standard_normal((n_q, NH, HD)).astype(np.float32) for _ in range(2))
+    pos = np.arange(pos0, n, dtype=np.int32)
+    kc, vc = oracle.kv_store_rows(1, K), oracle.kv_store_rows(1, V)
+    want = oracle.attn(rotated(oracle, q, n_rot, pos) if n_rot else q, kc, vc, pos, NKV, 1 / 16, 1, 1)
+    dq, dk, dv, dpos, dg = G.dev(q), G.dev(kc), G.dev(vc), G.dev(pos), G.dev(gate)
+    for g in (None, dg):
+        out = G.poison(q.shape)
+        rd.check(lib.rd_attn_prefill_fused(rd.ptr(dq), rd.ptr(dk), rd.ptr(dv), rd.ptr(out), rd.ptr(g), rd.ptr(dpos), n_q, n,
+                                           NH, NKV, HD, 1 / 16, n_rot, 1e7, G.st()))
+        torch.cuda.synchronize()
+        check_attn(G.host(out), want if g is None else want / (1 + np.exp(-gate)), what=f"gate {g is not None}")
+    G.status_ok()
+
+
+@pytest.mark.parametrize("n_q,pos0", [(24, 9000), (300, 7000)])
+def test_workspace_with_less_room_than_the_plan(G, oracle, n_q, pos0):
+    """The records of the plan, those of one-head tiles (what a call has to have), and what lies between."""
+    rd, lib = G.rd, G.lib
+    n, kt, vt = pos0 + n_q, 2, 2
+    rng = np.random.default_rng(n_q)
+    K, V = (rng.standard_normal((n, NKV, HD)).astype(np.float32) for _ in range(2))
+    q = rng.standard_normal((n_q, NH, HD)).astype(np.float32)
+    pos = np.arange(pos0, n, dtype=np.int32)
+    kc, vc = oracle.kv_store_rows(kt, K), oracle.kv_store_rows(vt, V)
+    want = oracle.attn(q, kc, vc, pos, NKV, 1 / 16, kt, vt)
+    dq, dk, dv, dpos = G.dev(q), G.dev(kc), G.dev(vc), G.dev(pos)
+    full = lib.rd_attn_prefill_workspace_bytes(kt, vt, n_q, n, NH, NKV, HD)
+    z = C.c_int()
+    rd.check(lib.rd_attn_prefill_plan(n_q, n, NH, 148, C.addressof(z), None))
+    align = lambda x: (x + 255) // 256 * 256
+    least = 2 * align(n * NKV * HD * 2) + align(n_q * NH * z.value * 1032)
+    assert full >= least
+    call = lambda out, nb: lib.rd_attn_prefill_typed(rd.ptr(dq), rd.ptr(dk), rd.ptr(dv), rd.ptr(out), None, rd.ptr(dpos), n_q,
+                                                     n, NH, NKV, HD, 1 / 16, kt, vt, 0, 0.0, rd.ptr(ws), nb, G.st())
+    for nb in sorted({full, (full + least) // 2, least}):
+        ws = torch.full((nb + 4096,), 0xA5, dtype=torch.uint8, device="cuda")
+        out = G.poison(q.shape)
+        rd.check(call(out, nb))
+        torch.cuda.synchronize()
+        check_attn(G.host(out), want, what=f"{nb} bytes")
+        assert (ws[nb:] == 0xA5).all()
+    assert call(out, least - 256) == rd.ERR_WORKSPACE
+    G.status_ok()
