@@ -168,7 +168,8 @@ int rd_attn_launch_plan(int64_t n_keys, int n_tok, int n_head_kv, int k_type, in
  * the CTAs of the tile-kernel launch. One split unless the cost model says that filling the
  * idle SMs outweighs a second wave of fixed costs and the records (from about 8192 keys for
  * 512 tokens x 24 heads on 148 SMs). This is the plan of tiles of one head, whose records rd_attn_prefill_workspace_bytes
- * has room for; rd_attn_prefill_launch_plan is what is launched, with the rows of a tile: tile_heads x tile_tokens.
+ * has room for; rd_attn_prefill_launch_plan is what is launched, with the rows of a tile: tile_heads x tile_tokens
+ * and, as n_splits, 0 for a launch whose tiles are cut into parts of uneven length.
  * Host arithmetic only when sm_count is given. */
 int rd_attn_prefill_launch_plan(int n_q, int keys_total, int n_head, int sm_count, int *tile_heads, int *tile_tokens,
                                 int *n_splits, int *n_ctas);

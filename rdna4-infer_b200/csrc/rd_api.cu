@@ -485,11 +485,10 @@ int rd_attn_prefill_launch_plan(int n_q, int keys_total, int n_head, int sm_coun
   }
   const PrefillPlan p = prefill_plan(n_q, keys_total, n_head, sm_count,
                                      prefill_splits(n_q, keys_total, n_head, sm_count) > 1 ? SIZE_MAX : 0);
-  const int tokens = prefill_tile_tokens(p.heads);
   if (tile_heads != nullptr) *tile_heads = p.heads;
-  if (tile_tokens != nullptr) *tile_tokens = tokens;
-  if (n_splits != nullptr) *n_splits = p.splits;
-  if (n_ctas != nullptr) *n_ctas = (n_q + tokens - 1) / tokens * (n_head / p.heads) * p.splits;
+  if (tile_tokens != nullptr) *tile_tokens = prefill_tile_tokens(p.heads);
+  if (n_splits != nullptr) *n_splits = p.pairs > 0 ? 0 : p.splits;
+  if (n_ctas != nullptr) *n_ctas = prefill_ctas(p, n_q, keys_total, n_head);
   return RD_OK;
 }
 
@@ -1066,7 +1065,7 @@ static int prefill_common(const float *q, const void *k, const void *v, float *o
                           const int32_t *pos, int n_q, int keys_total, int n_head, int n_head_kv,
                           int head_dim, float scale, int n_rot, float freq_base, void *stream,
                           void *records = nullptr, size_t record_bytes = 0, const float *k_new = nullptr,
-                          const float *v_new = nullptr, int row0 = 0, bool kv_pending = false) {
+                          const float *v_new = nullptr, int row0 = 0, const DequantJob *dequant = nullptr) {
   int rc = check_attn_shape(n_head, n_head_kv, head_dim, RD_KV_F16, RD_KV_F16);
   if (rc != RD_OK) return rc;
   if (n_q < 1 || keys_total <= 0) return RD_ERR_SHAPE;
@@ -1083,16 +1082,19 @@ static int prefill_common(const float *q, const void *k, const void *v, float *o
   const int sms = sm_count(dev);
   if (records == nullptr) record_bytes = prefill_splits(n_q, keys_total, n_head, sms) > 1 ? SIZE_MAX : 0;
   const PrefillPlan plan = prefill_plan(n_q, keys_total, n_head, sms, record_bytes);
-  if (records == nullptr && plan.splits > 1) {
-    records = ensure_workspace(dev, prefill_record_bytes(n_q, n_head, plan.splits));
+  if (records == nullptr && (plan.splits > 1 || plan.pairs > 0)) {
+    records = ensure_workspace(dev, prefill_record_bytes(n_q, n_head, plan));
     if (records == nullptr) return RD_ERR_CUDA;
   }
+  if (dequant != nullptr && (rc = launch_kv_dequant_f16_pair(*dequant, prefill_flags(records, plan), 2 * plan.pairs,
+                                                             (cudaStream_t)stream)) != RD_OK)
+    return rc;
   // a fused append stores rows row0 .. row0 + n_q - 1 of the (f16) caches
   const size_t row_bytes = (size_t)n_head_kv * kHeadDim * 2;
   void *k_dst = k_new != nullptr ? (void *)((unsigned char *)const_cast<void *>(k) + (size_t)row0 * row_bytes) : nullptr;
   void *v_dst = k_new != nullptr ? (void *)((unsigned char *)const_cast<void *>(v) + (size_t)row0 * row_bytes) : nullptr;
   return launch_prefill(q, k, v, o, gate, pos, n_q, keys_total, n_head, n_head_kv, scale, n_rot,
-                        freq_base, status, (float *)records, plan, k_new, v_new, k_dst, v_dst, kv_pending,
+                        freq_base, status, (float *)records, plan, k_new, v_new, k_dst, v_dst, dequant != nullptr,
                         (cudaStream_t)stream);
 }
 
@@ -1136,10 +1138,11 @@ static size_t prefill_workspace(int k_type, int v_type, int n_q, int keys_total,
       n_head_kv < 1 || head_dim != kHeadDim || current_device(&dev) != RD_OK)
     return 0;
   const int sms = sm_count(dev);
-  int splits = prefill_splits(n_q, keys_total, n_head, sms);
-  if (all && n_q <= 256) splits = std::max(splits, prefill_plan(n_q, keys_total, n_head, sms, SIZE_MAX).splits);
-  return prefill_copy_bytes(k_type, v_type, keys_total, n_head_kv) +
-         align256(prefill_record_bytes(n_q, n_head, splits));
+  const int splits = prefill_splits(n_q, keys_total, n_head, sms);
+  size_t records = prefill_record_bytes(n_q, n_head, splits);
+  if (all && n_q <= 256)
+    records = std::max(records, prefill_record_bytes(n_q, n_head, prefill_plan(n_q, keys_total, n_head, sms, SIZE_MAX)));
+  return prefill_copy_bytes(k_type, v_type, keys_total, n_head_kv) + align256(records);
 }
 size_t rd_attn_prefill_workspace_bytes(int k_type, int v_type, int n_q, int keys_total, int n_head,
                                        int n_head_kv, int head_dim) {
@@ -1167,7 +1170,6 @@ int rd_attn_prefill_typed(const float *q, const void *k, const void *v, float *o
   const int64_t n_values = (int64_t)keys_total * n_head_kv * kHeadDim;
   unsigned char *w = (unsigned char *)workspace;
   const void *k16 = k, *v16 = v;
-  cudaStream_t st = (cudaStream_t)stream;
   void *kdst = nullptr, *vdst = nullptr;
   if (k_type != RD_KV_F16) {
     kdst = w;
@@ -1178,11 +1180,7 @@ int rd_attn_prefill_typed(const float *q, const void *k, const void *v, float *o
     vdst = w;
     v16 = w;
   }
-  if (kdst != nullptr || vdst != nullptr) {   // one launch for both tensors
-    if ((rc = launch_kv_dequant_f16_pair(k_type, kdst != nullptr ? k : nullptr, kdst, v_type,
-                                         vdst != nullptr ? v : nullptr, vdst, n_values, st)) != RD_OK)
-      return rc;
-  }
+  const DequantJob job = {k_type, kdst != nullptr ? k : nullptr, kdst, v_type, vdst != nullptr ? v : nullptr, vdst, n_values};
   // what follows the copies holds the key-split records (never the library's own workspace:
   // this entry allocates nothing)
   unsigned char *rec = workspace != nullptr ? (unsigned char *)workspace + copies : nullptr;
@@ -1190,7 +1188,7 @@ int rd_attn_prefill_typed(const float *q, const void *k, const void *v, float *o
   return prefill_common(q, k16, v16, o, gate, pos, n_q, keys_total, n_head, n_head_kv, head_dim, scale,
                         n_rot, freq_base, stream, rec != nullptr ? (void *)rec : (void *)&s_dummy,
                         need > 0 ? workspace_bytes - copies : 0, nullptr, nullptr, 0,
-                        kdst != nullptr || vdst != nullptr);
+                        kdst != nullptr || vdst != nullptr ? &job : nullptr);
 }
 
 static int g_last_site = 0;   // `where` of the last time-out rd_device_status reported

@@ -22,8 +22,16 @@ int launch_sigmoid_gate(float *g, float *y, int64_t n, cudaStream_t st);
 // n_values stored values of `type` at src -> f16 at dst (the dequantizing loads of
 // include/rdna4/kv.h:174-368, rounded once).
 int launch_kv_dequant_f16(int type, const void *src, void *dst, int64_t n_values, cudaStream_t st);
-int launch_kv_dequant_f16_pair(int kt, const void *k, void *kdst, int vt, const void *v, void *vdst,
-                               int64_t n_values, cudaStream_t st);
+struct DequantJob {   // K and V, either with a null source: left out
+  int kt;
+  const void *k;
+  void *kdst;
+  int vt;
+  const void *v;
+  void *vdst;
+  int64_t n_values;
+};
+int launch_kv_dequant_f16_pair(const DequantJob &job, unsigned *flags, int n_flags, cudaStream_t st);   // zeroes flags, too
 
 // ---- rd_pre.cu
 int launch_rms_norm(const float *x, const float *w, float *y, int64_t nrows, int64_t ncols, float eps,
@@ -169,6 +177,7 @@ int encode_f32_tmap(void *tmap_out, const void *base, int width, int n_head, int
 struct PrefillPlan {
   int heads;    // of a CTA's rows: 1 (x 128 tokens) or 3 (x 42 tokens)
   int splits;   // of the keys
+  int pairs;    // above 0: a balanced launch of that many pairs of CTAs (splits 1)
 };
 int launch_prefill(const float *q, const void *k, const void *v, float *out, const float *gate,
                    const int32_t *pos, int n_q, int keys_total, int n_head, int n_head_kv, float scale,
@@ -178,7 +187,10 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
                                        // for everything before it (kv_dequant_f16_kernel)
 int prefill_splits(int n_q, int keys_total, int n_head, int sms);
 size_t prefill_record_bytes(int n_q, int n_head, int splits);
+size_t prefill_record_bytes(int n_q, int n_head, PrefillPlan plan);
+unsigned *prefill_flags(void *records, PrefillPlan plan);   // 2 pairs words that a launch finds zero, or null
 int prefill_tile_tokens(int heads);
+int prefill_ctas(PrefillPlan plan, int n_q, int keys_total, int n_head);
 PrefillPlan prefill_plan(int n_q, int keys_total, int n_head, int sms, size_t record_bytes);   // with that much memory
 
 // ---- rd_merge.cu

@@ -333,13 +333,15 @@ __device__ __forceinline__ void dequant_tile(const uint8_t *__restrict__ src, ui
 // (or absent) has src == nullptr and its CTAs leave at once.
 __global__ void __launch_bounds__(256)
 kv_dequant_f16_kernel(const uint8_t *__restrict__ ksrc, uint4 *__restrict__ kdst, int kt,
-                      const uint8_t *__restrict__ vsrc, uint4 *__restrict__ vdst, int vt, int64_t n_blocks) {
+                      const uint8_t *__restrict__ vsrc, uint4 *__restrict__ vdst, int vt, int64_t n_blocks, unsigned *flags,
+                      int n_flags) {
   __shared__ __align__(16) uint8_t stage[kDqTileBlocks * 34];
   const uint8_t *src = blockIdx.y == 0 ? ksrc : vsrc;
   uint4 *dst = blockIdx.y == 0 ? kdst : vdst;
   const int type = blockIdx.y == 0 ? kt : vt;
   pdl_wait();
   pdl_launch_dependents();   // after the wait: the tile kernel loads the caches without one
+  if (blockIdx.x == 0 && blockIdx.y == 0 && (int)threadIdx.x < n_flags) flags[threadIdx.x] = 0;   // (of a balanced tile launch)
   if (src == nullptr) return;
   switch (type) {   // the same for the whole CTA
     case RD_KV_F32: dequant_tile<RD_KV_F32>(src, dst, n_blocks, blockIdx.x, stage); break;
@@ -354,22 +356,22 @@ kv_dequant_f16_kernel(const uint8_t *__restrict__ ksrc, uint4 *__restrict__ kdst
 
 // Expands K (type kt) into kdst and V (type vt) into vdst as f16, one launch for both; a null
 // source skips that tensor. n_values per tensor.
-int launch_kv_dequant_f16_pair(int kt, const void *k, void *kdst, int vt, const void *v, void *vdst,
-                               int64_t n_values, cudaStream_t st) {
+int launch_kv_dequant_f16_pair(const DequantJob &job, unsigned *flags, int n_flags, cudaStream_t st) {
+  const auto [kt, k, kdst, vt, v, vdst, n_values] = job;
   if (n_values % 32 != 0) return RD_ERR_SHAPE;
   if ((k != nullptr && (kt < 0 || kt > RD_KV_Q4_1)) || (v != nullptr && (vt < 0 || vt > RD_KV_Q4_1))) return RD_ERR_TYPE;
   const int64_t n_blocks = n_values / 32;
   if (n_blocks == 0 || (k == nullptr && v == nullptr)) return RD_OK;
   const dim3 grid((unsigned)((n_blocks + kDqTileBlocks - 1) / kDqTileBlocks), 2);
   return launch_pdl(8, kv_dequant_f16_kernel, grid, dim3(256), 0, st, (const uint8_t *)k, (uint4 *)kdst, kt,
-                    (const uint8_t *)v, (uint4 *)vdst, vt, n_blocks) == cudaSuccess
+                    (const uint8_t *)v, (uint4 *)vdst, vt, n_blocks, flags, n_flags) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
 }
 
 int launch_kv_dequant_f16(int type, const void *src, void *dst, int64_t n_values, cudaStream_t st) {
   if (type < 0 || type > RD_KV_Q4_1) return RD_ERR_TYPE;
-  return launch_kv_dequant_f16_pair(type, src, dst, RD_KV_F16, nullptr, nullptr, n_values, st);
+  return launch_kv_dequant_f16_pair({type, src, dst, RD_KV_F16, nullptr, nullptr, n_values}, nullptr, 0, st);
 }
 
 }  // namespace rd

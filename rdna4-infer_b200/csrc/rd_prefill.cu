@@ -40,6 +40,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "rd_common.cuh"
 #include "rd_internal.h"
 #include "rd_tc.cuh"
@@ -88,6 +90,10 @@ constexpr uint32_t kTmemS = 256;          // columns [256, 384): the scores of o
 constexpr uint32_t kTmemP = 384;          // columns [384, 512): two buffers of 64 for the f16 P
 constexpr float kLazyThreshold = 8.0f;    // log2 units
 constexpr int kPfMaxSplits = 20;          // key splits of a tile at most
+constexpr int kPfMaxParts = 256;          // parts of a balanced launch at most
+constexpr int kPfMaxRecords = 7;          // of a unit there
+constexpr int kPfRecAcc = 8 * 8 * kPfM;   // a CTA's record there: float4 [32 dims][4 dims][row], then (m, l) [row]
+constexpr size_t kPfRecBytes = (size_t)kPfRecAcc * 16 + kPfM * 8;
 // A CTA's 128 query rows: one head of 128 tokens (kHeads 1), or the three heads of half a KV head's group of 42
 // tokens, token by token (kHeads 3; two rows stay empty). The pair's CTAs serve the same tokens: two heads, or all
 // six of the group.
@@ -118,7 +124,27 @@ struct PrefillArgs {
   // 128 CTAs would leave many idle.
   // Records: accumulators [n_q][n_head][gridDim.z][256] behind tm_o, then (m, l) here.
   float2 *rec_ml;        // [n_q][n_head][gridDim.z]
+  // Balanced launch: the units (token tile, pair of CTAs along the heads), laid one behind the other, are cut into
+  // as many equal runs of key tiles as pairs of CTAs fit the GPU, and every piece of a unit is a part for one pair.
+  // A unit's first part writes the output; its other parts leave records for it and set their flags. The parts that
+  // leave records come first in the grid, so a waiting CTA waits for CTAs that started before it, then the rest,
+  // longest first: as the first ones end, shortest first, each is followed by what was cut off it. A part covers
+  // [c0, c1) of the unit's key tiles counted from the tokens at the end of `keys`; where pos[] says otherwise, the
+  // same fractions of what it says.
+  float4 *rec;           // [record][CTA of the pair] of kPfRecBytes
+  unsigned *flags;       // [record][CTA of the pair], zero before the launch
+  int groups;            // units per token tile
+  int keys;
+  struct Part {
+    unsigned short unit, c0, c1, rec, n_rec;   // rec: its record, or the first of the n_rec that it collects
+  } parts[kPfMaxParts];
 };
+// Key tiles of a unit of token tile `tile`.
+__host__ __device__ inline int pf_unit_tiles(int tile, int tokens, int n_q, int keys) {
+  const int last = tile * tokens + tokens < n_q ? tile * tokens + tokens : n_q;
+  return (keys - n_q + last - 1) / kPfN + 1;
+}
+
 
 // Barrier slots (8 bytes each).
 // In the leader (CTA 0 of the pair) alone: KFull, VFull, Q, P, L -- what its issuing threads wait for, from
@@ -139,7 +165,24 @@ __device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, 
     if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait(bar, parity, status, site);   // bounded
 }
-template <int kHeads>
+// A word that says "the record is written": set behind a barrier of the threads that wrote it.
+__device__ __forceinline__ void flag_set(unsigned *flag) {
+  __threadfence();
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory");
+}
+__device__ __forceinline__ bool flag_wait(const unsigned *flag, DeviceStatus *status, int site) {
+  const unsigned long long t0 = global_ns();
+  for (uint32_t i = 1;; ++i) {
+    unsigned x;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(flag) : "memory");
+    if (x != 0) return true;
+    if ((i & 63u) == 0 && global_ns() - t0 > kWaitNs) break;
+  }
+  if (status != nullptr && atomicExch(&status->timeout_flag, 1) == 0) status->where = site;
+  return false;
+}
+
+template <int kHeads, bool kBalanced>
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_constant__ PrefillArgs p) {
   constexpr int kTokens = pf_tokens(kHeads), kRows = kTokens * kHeads;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -154,9 +197,19 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   pdl_launch_dependents();   // the merge pass of a key split may be scheduled under this kernel
   if (!p.kv_wait) pdl_wait();
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 0);   // kernel entry
-  const int tile = (int)gridDim.y - 1 - (int)blockIdx.y;  // heaviest (latest) tiles first
-  const int head = blockIdx.x * kHeads;                   // the CTA's first head; the pair's are of one KV head
   const uint32_t rank = blockIdx.x & 1;
+  int tile = (int)gridDim.y - 1 - (int)blockIdx.y;        // heaviest (latest) tiles first
+  int head = blockIdx.x * kHeads;                         // the CTA's first head; the pair's are of one KV head
+  int c0 = blockIdx.z, c1 = c0 + 1, n_cut = gridDim.z;    // parts [c0, c1) of n_cut of the keys
+  if (kBalanced) {
+    const PrefillArgs::Part &part = p.parts[blockIdx.x >> 1];
+    tile = part.unit / p.groups;
+    head = kHeads * (2 * (part.unit % p.groups) + (int)rank);
+    c0 = part.c0;
+    c1 = part.c1;
+    n_cut = pf_unit_tiles(tile, kTokens, p.n_q, p.keys);
+  }
+  const bool leaves = kBalanced && c0 > 0;                // a record
   const int kvh = head / kGroup;
   const int tok0 = tile * kTokens;
 
@@ -261,8 +314,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
   const uint32_t tmem = s_tmem_base;
   const int maxpos = s_maxpos;
   const int nt_all = maxpos >= 0 ? maxpos / kPfN + 1 : 0;  // key tiles the rows of this tile attend
-  const int jt0 = (int)(((int64_t)nt_all * blockIdx.z) / gridDim.z);        // this CTA's share of them
-  const int nt = (int)(((int64_t)nt_all * (blockIdx.z + 1)) / gridDim.z) - jt0;
+  const int jt0 = (int)(((int64_t)nt_all * c0) / n_cut);        // this CTA's share of them
+  const int nt = (int)(((int64_t)nt_all * c1) / n_cut) - jt0;
 
   // ---- prologue: the Q tile as f16 in the swizzled K-major layout ----
   // f32 rows -> partial RoPE -> x scale * log2(e) -> f16 in the swizzled layout, warps 0-7. (A pre-pass
@@ -387,7 +440,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 3);   // this warp's Q rows converted
   }
 
-  const bool with_gate = p.gate != nullptr && gridDim.z == 1;
+  const bool with_gate = p.gate != nullptr && gridDim.z == 1 && !leaves;
   float l_run = 0.f;                 // softmax threads: row sum
   float m_ref = -1.0e30f;            //                  reference maximum (log2 units)
 
@@ -725,8 +778,36 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const float m_fin = nt > 0 ? s_ref[(nt - 1) & 1][r] : -1.0e30f;
     const float l_tot = s_fin[0][0][r] * ex2(s_fin[0][1][r] - m_fin) + s_fin[1][0][r] * ex2(s_fin[1][1][r] - m_fin);
     const bool rec_mode = gridDim.z > 1;   // un-normalised records for prefill_merge_kernel
-    const float inv = (l_tot > 0.f && !aborted) ? (rec_mode ? 1.0f : 1.0f / l_tot) : 0.f;
     const bool have = nt > 0 && !aborted;
+    float l_sum = l_tot;   // of the unit's parts
+    // Weights of the parts: this one's, then [part][row] in the third K slot, behind the row sums.
+    float w_own = 1.f;
+    bool lost = false;
+    float (*s_w)[kPfM] = reinterpret_cast<float (*)[kPfM]>(smem_raw + kPfQBytes + 2 * kPfKTileBytes + 2048) + ch * kPfMaxRecords;
+    int n_other = 0;
+    const float4 *others = nullptr;   // records, 2 apart
+    if (kBalanced && !leaves) {
+      const PrefillArgs::Part &part = p.parts[blockIdx.x >> 1];
+      n_other = part.n_rec;
+      others = p.rec + (2 * (size_t)part.rec + rank) * (kPfRecBytes / 16) + r;
+    }
+    if (n_other > 0) {
+      pdl_wait();   // (the flags are zeroed by the launch before this one; its end was waited for long ago)
+      const bool there = lane >= n_other || flag_wait(p.flags + 2 * (p.parts[blockIdx.x >> 1].rec + lane) + rank, p.status, 29);
+      lost = !__all_sync(0xffffffffu, there);
+      float m_all = m_fin;
+      for (int i = 0; i < n_other; ++i)
+        m_all = fmaxf(m_all, __ldcg(reinterpret_cast<const float2 *>(others - r + 2 * i * (kPfRecBytes / 16) + kPfRecAcc) + r).x);
+      w_own = ex2(m_fin - m_all);
+      l_sum *= w_own;
+      for (int i = 0; i < n_other; ++i) {
+        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(others - r + 2 * i * (kPfRecBytes / 16) + kPfRecAcc) + r);
+        const float w = ex2(ml.x - m_all);
+        s_w[i][r] = w;   // (read by this thread only)
+        l_sum = fmaf(ml.y, w, l_sum);
+      }
+    }
+    const float inv = (l_sum > 0.f && !aborted && !lost) ? (rec_mode ? 1.0f : 1.0f / l_sum) : 0.f;
     // column of the first value in a head's output, or in the accumulators of its records
     const int col0 = rec_mode ? (int)blockIdx.z * kHeadDim : 0;
     if (rec_mode && ch == 0 && r < rows_cta) {
@@ -735,10 +816,37 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       p.rec_ml[((size_t)(tok0 + r / kHeads) * p.n_head + head + r % kHeads) * gridDim.z + blockIdx.z] =
           some ? make_float2(m_fin * 0.6931471805599453f, l_tot) : make_float2(-INFINITY, 0.f);
     }
-    {
+    if (leaves) {   // 512 contiguous bytes per store of a warp
+      const int slot = p.parts[blockIdx.x >> 1].rec;
+      float4 *rec = p.rec + (2 * (size_t)slot + rank) * (kPfRecBytes / 16) + r;
+      if (ch == 0) reinterpret_cast<float2 *>(rec - r + kPfRecAcc)[r] = have ? make_float2(m_fin, l_tot) : make_float2(-1.0e30f, 0.f);
+#pragma unroll 1
+      for (int b = ch; b < 8 && 32 * (warp & 3) < rows_cta; b += 2) {
+        uint32_t o[32];
+        if (have) {
+          tmem_ld32(lane_addr + kTmemO + 32 * b, o);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          __stcg(rec + (b * 8 + q) * kPfM, make_float4(__uint_as_float(o[4 * q]), __uint_as_float(o[4 * q + 1]),
+                                                       __uint_as_float(o[4 * q + 2]), __uint_as_float(o[4 * q + 3])));
+      }
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+      if (threadIdx.x == 0) flag_set(p.flags + 2 * slot + rank);
+    } else {
       // O / l (x sigmoid(gate)) in place over the gate rows, 32 columns (a box of 128-byte swizzled rows)
       // at a time, each box stored by TMA while the next is computed. What bounds it: the 32 bytes a
       // cycle that an SM writes (4096 cycles) and 1.5 special functions per gate value (3072).
+      float4 x[8];   // 32 values of a record
+      auto fetch = [&](int b, int i) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[q] = __ldcg(others + 2 * i * (kPfRecBytes / 16) + (b * 8 + q) * kPfM);
+      };
+      if (kBalanced && n_other > 0) fetch(ch, 0);
       if (with_gate) mbar_wait(bars + 8 * kBarG, 0, p.status, 28);
 #pragma unroll 1
       for (int b = ch; b < 8; b += 2) {
@@ -753,6 +861,27 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         } else {
 #pragma unroll
           for (int e = 0; e < 32; ++e) o[e] = 0u;
+        }
+        if (kBalanced && n_other > 0) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * w_own);
+#pragma unroll 1
+          for (int i = 0; i < n_other; ++i) {
+            const float w = s_w[i][r];
+            float4 y[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) y[q] = x[q];
+            // the next values are on their way while these, or the rest of the box, are worked on
+            if (i + 1 < n_other) fetch(b, i + 1);
+            else if (b + 2 < 8) fetch(b + 2, 0);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              o[4 * q] = __float_as_uint(fmaf(y[q].x, w, __uint_as_float(o[4 * q])));
+              o[4 * q + 1] = __float_as_uint(fmaf(y[q].y, w, __uint_as_float(o[4 * q + 1])));
+              o[4 * q + 2] = __float_as_uint(fmaf(y[q].z, w, __uint_as_float(o[4 * q + 2])));
+              o[4 * q + 3] = __float_as_uint(fmaf(y[q].w, w, __uint_as_float(o[4 * q + 3])));
+            }
+          }
         }
         const uint32_t brow = sQ + b * kPfBoxBytes + r * 128;
         uint32_t nan = 0;   // columns of the row with a NaN gate
@@ -811,6 +940,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       if (gt == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory outlives the copies
     }
   }
+  if (aborted && threadIdx.x == 0)   // whatever is still under way lands first
+    for (const unsigned long long t0 = global_ns(); global_ns() - t0 < 1000000ull;) {}
   tc_fence_before();
   cluster_sync();   // the pair frees its tensor memory together
   if (threadIdx.x == 0) RD_PF_TRACE(0, 47, 5);   // epilogue stores done
@@ -884,7 +1015,8 @@ prefill_merge_kernel(const float4 *__restrict__ rec_acc, const float2 *__restric
 __global__ void __launch_bounds__(256)
 kv_prep_kernel(const int32_t *__restrict__ pos, int n_rot, const float *__restrict__ k_new,
                const float *__restrict__ v_new, uint4 *__restrict__ k_dst, uint4 *__restrict__ v_dst, int nkv,
-               const float *q, const float *gate, int n_head, const __grid_constant__ RopeTable tab) {
+               const float *q, const float *gate, int n_head, const __grid_constant__ RopeTable tab, unsigned *flags,
+               int n_flags) {
   __shared__ float2 s_cs[32];
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // This launch starts under the one before it: the token's query and gate rows can be on their way to L2
@@ -895,6 +1027,7 @@ kv_prep_kernel(const int32_t *__restrict__ pos, int n_rot, const float *__restri
   // the wait comes first: the tile kernel reads what earlier kernels wrote without waiting for this one
   pdl_wait();
   pdl_launch_dependents();
+  if (t == 0 && (int)threadIdx.x < n_flags) flags[threadIdx.x] = 0;   // (of a balanced tile launch)
   const bool is_k = warp < nkv;
   const size_t row = (size_t)t * nkv + (is_k ? warp : warp - nkv);
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
@@ -981,13 +1114,20 @@ int prefill_splits(int n_q, int keys_total, int n_head, int sms) {
 //     24 of 24024   58.6 (6) | 34.9 (18)       130 of  4130   33.3 (3) | 30.3 (4)       31 of   31   14.9 | 16.0
 //     60 of  9060   32.0 (6) | 30.1 (8)        200 of 12200   64.0 (3) | 60.4 (3)      450 of 4450   61.9 | 61.1
 //    700 of  5700   82.7     | 77.7            389 of 12346  123.5 (3) | 118.1 (3)    1500 of 4500  128.3 | 134.7
+// A balanced launch has no empty SMs in its last wave and a fifth of the records, combined where they are wanted
+// instead of by a launch of their own; but most pairs of CTAs work on two parts, so it costs a run, the prologue (6) and
+// epilogue of both (a record 4, the output 5.5) and 1.5 per record read. It has to win by 5 %: long passes run at
+// the power cap, where idle SMs leave the others a higher clock. Best of the other two forms | balanced, one box:
+//    389 of 12346  131.7 | 108.2     450 of 9450  111.1 | 97.6     1000 of 8000  195.3 | 152.7    512 of 12512 154.5 | 135.5
+//    512 of  8192   94.3 | 93.4      640 of 9640  116.2 | 122.5     260 of 12260  87.4 | 90.5     200 of 12200  62.6 | 74.8
 PrefillPlan prefill_plan(int n_q, int keys_total, int n_head, int sms, size_t record_bytes) {
-  PrefillPlan best = {1, 1};
+  PrefillPlan best = {1, 1, 0};
   const int tiles = (keys_total + kPfN - 1) / kPfN;
 #ifdef RD_TIMING_SWITCHES
   if (const char *e = getenv("RD_PF_FORM")) {   // timing builds: force heads and splits
     best.heads = atoi(e);
     if (const char *f = getenv("RD_PF_SPLITS")) best.splits = atoi(f);
+    if (const char *f = getenv("RD_PF_PAIRS")) best.pairs = atoi(f);
     return best;
   }
 #endif
@@ -1002,14 +1142,80 @@ PrefillPlan prefill_plan(int n_q, int keys_total, int n_head, int sms, size_t re
       if (prefill_record_bytes(n_q, n_head, z) > record_bytes) break;
       if (cost(heads, z) < best_cost) {
         best_cost = cost(heads, z);
-        best = {heads, z};
+        best = {heads, z, 0};
       }
     }
-  return best;
+  PrefillPlan balanced = {1, 1, 0};
+  double balanced_cost = 0.0;
+  for (int heads = 1; heads <= 3; heads += 2) {
+    const int units = (n_q + pf_tokens(heads) - 1) / pf_tokens(heads) * (n_head / heads / 2);
+    if (keys_total < n_q || tiles > 60000) continue;
+    int pairs = sms / 2 < 120 ? sms / 2 : 120;   // (240 flags, zeroed by one block)
+    const size_t room = record_bytes / (2 * (kPfRecBytes + sizeof(unsigned)));
+    if ((size_t)pairs > room) pairs = (int)room;
+    if (pairs < 2 || units + pairs > kPfMaxParts) continue;
+    int64_t all = 0;
+    for (int t = 0; t * pf_tokens(heads) < n_q; ++t)
+      all += (int64_t)(n_head / heads / 2) * pf_unit_tiles(t, pf_tokens(heads), n_q, keys_total);
+    if (all / pairs < 4) continue;
+    const double run = (double)all / pairs, parts = tiles / run + 1;
+    if (parts > kPfMaxRecords - 1) continue;
+    const double c = run + 21.5 + 1.5 * tiles / run;
+    if (c < 0.95 * best_cost && (balanced.pairs == 0 || c < balanced_cost)) {
+      balanced_cost = c;
+      balanced = {heads, 1, pairs};
+    }
+  }
+  return balanced.pairs > 0 ? balanced : best;
 }
 int prefill_tile_tokens(int heads) { return pf_tokens(heads); }
+size_t prefill_record_bytes(int n_q, int n_head, PrefillPlan plan) {
+  return plan.pairs > 0 ? plan.pairs * 2 * (kPfRecBytes + sizeof(unsigned)) : prefill_record_bytes(n_q, n_head, plan.splits);
+}
+unsigned *prefill_flags(void *records, PrefillPlan plan) {
+  return plan.pairs > 0 ? (unsigned *)((char *)records + plan.pairs * 2 * kPfRecBytes) : nullptr;
+}
 size_t prefill_record_bytes(int n_q, int n_head, int splits) {
   return splits > 1 ? (size_t)n_q * n_head * splits * kRec * sizeof(float) : 0;
+}
+
+// The parts of a balanced launch in the order of its grid; their number, or 0 if they do not fit.
+static int balanced_parts(PrefillArgs::Part *out, int n_q, int keys, int groups, int tokens, int pairs) {
+  const int tiles = (n_q + tokens - 1) / tokens, units = tiles * groups;
+  int64_t all = 0;
+  for (int t = 0; t < tiles; ++t) all += (int64_t)groups * pf_unit_tiles(t, tokens, n_q, keys);
+  if (units + pairs > kPfMaxParts || all < pairs) return 0;
+  PrefillArgs::Part rest[kPfMaxParts];
+  int n_left = 0, n_rest = 0, run = 1;   // run: the next cut lies at all * run / pairs
+  int64_t before = 0;                    // key tiles of the units before this one
+  for (int unit = 0; unit < units; ++unit) {
+    const int n = pf_unit_tiles(unit / groups, tokens, n_q, keys);
+    PrefillArgs::Part first = {(unsigned short)unit, 0, (unsigned short)n, (unsigned short)n_left, 0};
+    for (; all * run / pairs < before + n; ++run) {
+      const int at = (int)(all * run / pairs - before);
+      if (at == 0) continue;   // (a cut between two units)
+      if (first.n_rec == 0) first.c1 = (unsigned short)at;
+      else out[n_left - 1].c1 = (unsigned short)at;
+      out[n_left] = {(unsigned short)unit, (unsigned short)at, (unsigned short)n, (unsigned short)n_left, 0};
+      ++n_left;
+      ++first.n_rec;
+    }
+    if (first.n_rec > kPfMaxRecords) return 0;
+    before += n;
+    rest[n_rest++] = first;
+  }
+  std::stable_sort(rest, rest + n_rest, [](const PrefillArgs::Part &x, const PrefillArgs::Part &y) {
+    return x.c1 - x.c0 > y.c1 - y.c0;
+  });
+  for (int i = 0; i < n_rest; ++i) out[n_left + i] = rest[i];
+  return n_left + n_rest;
+}
+
+int prefill_ctas(PrefillPlan plan, int n_q, int keys_total, int n_head) {
+  const int tokens = pf_tokens(plan.heads);
+  if (plan.pairs == 0) return (n_q + tokens - 1) / tokens * (n_head / plan.heads) * plan.splits;
+  PrefillArgs::Part parts[kPfMaxParts];
+  return 2 * balanced_parts(parts, n_q, keys_total, n_head / plan.heads / 2, tokens, plan.pairs);
 }
 
 int launch_prefill(const float *q, const void *k, const void *v, float *out, const float *gate,
@@ -1033,6 +1239,16 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   a.qscale = scale * 1.4426950408889634f;
   const int heads = plan.heads, tokens = pf_tokens(heads), n_splits = records == nullptr ? 1 : plan.splits;
   if (n_splits < 1 || n_splits > kPfMaxSplits || (heads != 1 && heads != 3)) return RD_ERR_SHAPE;
+  int n_parts = 0;
+  if (plan.pairs > 0) {
+    if (records == nullptr || n_splits != 1) return RD_ERR_SHAPE;
+    a.rec = (float4 *)records;
+    a.flags = prefill_flags(records, plan);
+    a.groups = n_head / heads / 2;
+    a.keys = keys_total;
+    n_parts = balanced_parts(a.parts, n_q, keys_total, a.groups, tokens, plan.pairs);
+    if (n_parts <= 0) return RD_ERR_SHAPE;
+  }
   if (n_splits > 1) {
     a.rec_ml = reinterpret_cast<float2 *>(records + (size_t)n_q * n_head * n_splits * kHeadDim);
     if ((rc = encode_f32_tmap(&a.tm_o, records, kHeadDim * n_splits, n_head, n_q, heads, tokens)) != RD_OK) return rc;
@@ -1052,7 +1268,7 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return RD_ERR_CUDA;
   if (dev < 0 || dev >= 32 || !attr_set[dev]) {
-    for (auto *f : {prefill_kernel<1>, prefill_kernel<3>})
+    for (auto *f : {prefill_kernel<1, false>, prefill_kernel<3, false>, prefill_kernel<1, true>, prefill_kernel<3, true>})
       if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes) != cudaSuccess)
         return RD_ERR_CUDA;
     if (dev >= 0 && dev < 32) attr_set[dev] = true;
@@ -1062,11 +1278,16 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
     const bool early = n_q <= 1024;
     if (launch_pdl(early ? 8 : 0, kv_prep_kernel, dim3((unsigned)n_q), dim3(256), 0, st, pos, n_rot, k_new, v_new,
                    (uint4 *)k_dst, (uint4 *)v_dst, n_head_kv, early ? q : nullptr, gate, n_head,
-                   make_rope_table(n_rot, freq_base)) != cudaSuccess)
+                   make_rope_table(n_rot, freq_base), a.flags, 2 * plan.pairs) != cudaSuccess)
       return RD_ERR_CUDA;
+  } else if (plan.pairs > 0 && !kv_pending) {   // (no launch of this call that zeroes the flags)
+    if (cudaMemsetAsync(a.flags, 0, 2 * plan.pairs * sizeof(unsigned), st) != cudaSuccess) return RD_ERR_CUDA;
   }
+  auto *kernel = plan.pairs > 0 ? (heads == 1 ? prefill_kernel<1, true> : prefill_kernel<3, true>)
+                                : (heads == 1 ? prefill_kernel<1, false> : prefill_kernel<3, false>);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(n_head / heads), (unsigned)((n_q + tokens - 1) / tokens), (unsigned)n_splits);
+  cfg.gridDim = plan.pairs > 0 ? dim3(2 * (unsigned)n_parts)
+                               : dim3((unsigned)(n_head / heads), (unsigned)((n_q + tokens - 1) / tokens), (unsigned)n_splits);
   cfg.blockDim = dim3(kPfThreads);
   cfg.dynamicSmemBytes = kPfSmemBytes;
   cfg.stream = st;
@@ -1080,7 +1301,7 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  if (cudaLaunchKernelEx(&cfg, heads == 1 ? prefill_kernel<1> : prefill_kernel<3>, a) != cudaSuccess) return RD_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, kernel, a) != cudaSuccess) return RD_ERR_CUDA;
   if (n_splits > 1) {
     const int64_t n_rows = (int64_t)n_q * n_head;
     cudaLaunchConfig_t cfg = {};

@@ -77,3 +77,35 @@ def test_workspace_with_less_room_than_the_plan(G, oracle, n_q, pos0):
         assert (ws[nb:] == 0xA5).all()
     assert call(out, least - 256) == rd.ERR_WORKSPACE
     G.status_ok()
+
+
+@pytest.mark.parametrize("n_q,pos0,heads,nh,ragged", [(389, 11957, 3, 24, False), (512, 7680, 1, 24, False), (1000, 7000, 3, 24, False),
+                                                      (450, 9000, 3, 24, True), (2000, 6000, 3, 12, False)])
+def test_balanced_launches(G, n_q, pos0, heads, nh, ragged):
+    """Parts of key ranges cut anywhere, records collected by the part that writes: against the same attention in f64,
+    with positions in order and with ones that the plan did not expect; twice, into the records of the first run."""
+    rd, lib = G.rd, G.lib
+    n, nkv = pos0 + n_q, nh // 6
+    got = [C.c_int() for _ in range(4)]
+    rd.check(lib.rd_attn_prefill_launch_plan(n_q, n, nh, 148, *[C.addressof(x) for x in got]))
+    assert [x.value for x in got[::2]] == [heads, 0]
+    g = torch.Generator(device="cuda").manual_seed(n_q)
+    q, gate = (torch.randn(n_q, nh, HD, device="cuda", generator=g) for _ in range(2))
+    K, V = (torch.randn(n, nkv, HD, device="cuda", generator=g).half() for _ in range(2))
+    pos = torch.arange(pos0, n, dtype=torch.int32, device="cuda")
+    if ragged:
+        pos = torch.randint(0, n, (n_q,), dtype=torch.int32, device="cuda", generator=g)
+        pos[7], pos[300:] = -1, pos[300:] // 8
+    out = torch.full_like(q, float("nan"))
+    for _ in range(2):
+        rd.check(lib.rd_attn_prefill_fused(rd.ptr(q), rd.ptr(K), rd.ptr(V), rd.ptr(out), rd.ptr(gate), rd.ptr(pos), n_q, n, nh,
+                                           nkv, HD, 1 / 16, 0, 0.0, G.st()))
+    torch.cuda.synchronize()
+    G.status_ok()
+    past = torch.arange(n, device="cuda")[None, :] > pos[:, None]
+    for h in range(0, nh, 5):
+        s = (q[:, h].double() @ K[:, h // 6].double().T / 16).masked_fill_(past, -torch.inf)
+        want = torch.nan_to_num(torch.softmax(s, 1)) @ V[:, h // 6].double() * torch.sigmoid(gate[:, h].double())
+        check_attn(out[:, h].cpu().numpy(), want.cpu().numpy(), what=f"head {h}")
+    if ragged:
+        assert (out[7] == 0).all()

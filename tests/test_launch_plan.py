@@ -21,3 +21,16 @@ def test_launch_plan_arguments(rd):
     assert f(8192, 1, 4, 2, 2, 148, None, None, None) == rd.OK
     assert f(10, 1, 4, 6, 3, 148, *out) == rd.ERR_TYPE and f(10, 0, 4, 3, 3, 148, *out) == rd.ERR_SHAPE
     assert f(10, 1, 3, 3, 3, 148, *out) == rd.ERR_UNSUPPORTED
+
+
+def test_prefill_launch_plan(rd):
+    """rd_attn_prefill_launch_plan: (tile heads, tile tokens, key splits, CTAs) on 148 SMs; argument errors."""
+    a = [C.c_int() for _ in range(4)]
+    f = rd.lib.rd_attn_prefill_launch_plan
+    plan = lambda n_q, keys, nh=24, sms=148: (f(n_q, keys, nh, sms, *[C.addressof(x) for x in a]), *[x.value for x in a])
+    assert plan(1, 1) == (0, 1, 128, 1, 24) and plan(512, 512) == (0, 1, 128, 1, 96)   # whole tiles, no records
+    assert plan(24, 24024) == (0, 3, 42, 18, 144) and plan(130, 4130) == (0, 3, 42, 4, 128)
+    assert plan(512, 4096) == (0, 1, 128, 1, 96) and plan(8192, 8192) == (0, 1, 128, 1, 1536)
+    assert plan(389, 12346) == (0, 3, 42, 0, 224) and plan(512, 8192) == (0, 1, 128, 0, 242)   # balanced: parts
+    assert f(0, 1, 24, 148, *[None] * 4) == rd.ERR_SHAPE and f(1, 0, 24, 148, *[None] * 4) == rd.ERR_SHAPE
+    assert f(1, 1, 5, 148, *[None] * 4) == rd.ERR_UNSUPPORTED and f(1, 1, 6, 148, *[None] * 4) == rd.OK
