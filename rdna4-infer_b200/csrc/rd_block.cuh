@@ -33,19 +33,15 @@
 // verifying four tokens: copies alone 817 us.)
 // One record (m, l, acc[256]) per (token, head) and split, merged by merge_kernel.
 //
-// What bounds it: latency. Two warps per scheduler (registers), each a chain of shared-memory loads, dequantization,
-// mma.sync, vote, exponentials, fragment stores, barrier, mma.sync: 5 tokens over 20011 q4_0 keys issue in 35 % of the
-// active cycles, tensor pipe 22 %, DRAM 12 %; of the cycles between two issues of a warp (5.8) it waits 1.6 for fixed
-// latencies, 0.7 for shared memory, 0.7 for the tensor pipe, 0.4 for the first copies, 0.3 each at barriers and for
-// instructions. A launch takes about 9.8 us whatever the keys (prologue, ring fill, planes, records; the merge
-// launch 4 more) and 0.55 ns per key:
-//   us, records only       500      5000     20011     65536 keys
-//   q4_0, 2 tokens         6.3       8.4      14.4      32.0
-//   q4_0, 5                9.6      12.5      20.7      45.7
-//   q4_0, 8               13.1      17.0      27.1      57.0
-//   q8_0/f16, 4            8.4      12.0      20.4      46.1
-//   f16, 4                 8.4      13.3      24.5      57.1   (4.7 TB/s)
-//   q5_0/q4_1, 5           9.8      12.7      21.7      47.3
+// What bounds it: latency. Two or three warps per scheduler (registers), each a chain of shared-memory loads,
+// dequantization, mma.sync, vote, exponentials, fragment stores, barrier, mma.sync (with two: issue in 35 % of the active
+// cycles, tensor pipe 22 %, DRAM 12 % over 20011 q4_0 keys). Of the 34500 cycles of a CTA there 10200 lie before the
+// first slot, 9700 in it (references, the second part of its weights, cold code), 8600 in the others, 5900 in the records.
+// A third team, where rings and registers allow it, pays where runs are long; the query rows are requested first and
+// converted under the first slot's copies, since a whole ring's copies take 4400 cycles to issue.
+//   us a layer with its pre-attention, merge and gate launches    two teams, ring first | now
+//   q4_0, 5 tokens over 20011 keys   30.4 | 29.6      q8_0, 4 over 20000   30.4 | 28.4      f16, 4 over 8000  24.2 | 21.9
+//   64 sequences, one layer: q4_0, 5 tokens    650 | 587     q8_0, 4    620 | 590     q8_0/f16, 4   606 | 581
 #pragma once
 #include <string.h>
 
@@ -58,6 +54,7 @@ namespace rd {
 
 constexpr int kBlkKeys = 64;       // keys per slot
 constexpr int kBlkSmem = 222 * 1024;   // dynamic; the static arrays take up to 4.5 KB
+constexpr int kBlkQPair = 576;     // bytes of a pair of MMAs in a tile's query fragments: 512, shifted by half the banks
 constexpr int kBlkPlane = 268;     // floats per column in the epilogue planes (12 mod 32)
 constexpr float kBlkSlack = 8.0f;  // see kRefSlack
 constexpr float kBlkNone = -1.0e30f;
@@ -70,18 +67,21 @@ template <int KT, int VT, int NT>
 struct BlockGeo {
   static constexpr int kPK = slot_pitch(KT), kPV = slot_pitch(VT);
   static constexpr int kSK = kBlkKeys * kPK, kSV = kBlkKeys * kPV;   // multiples of 128
-  static constexpr int kQBytes = NT * 4096;                          // query fragments
+  static constexpr int kQBytes = NT * 8 * kBlkQPair;                          // query fragments
   static constexpr int kPBytes = NT * 2048;                          // weight fragments of a slot, two parts, per team
   static constexpr int kHead = 512 + kQBytes;                        // dim table, query fragments
   static constexpr int budget(int teams) { return (kBlkSmem - kHead) / teams - kPBytes; }
-  // two teams where each gets at least one slot, and another K or V of the next
-  static constexpr int kTeams = budget(2) >= kSK + kSV + (kSK < kSV ? kSK : kSV) ? 2 : 1;
+  // Teams: three where each gets one slot and 168 registers hold its sums (up to four column tiles), two where each gets
+  // one and another K or V of the next
+  static constexpr int kPlaneBytes = NT * 8 * kBlkPlane * 4;   // a team's ring doubles as its plane
+  static constexpr int kTeams = NT <= 4 && budget(3) >= kSK + kSV && budget(3) >= kPlaneBytes   ? 3
+                                : budget(2) >= kSK + kSV + (kSK < kSV ? kSK : kSV) ? 2
+                                                                                   : 1;
   static constexpr int kRing = budget(kTeams) & ~127;
   static constexpr int kBoth = min_i(4, kRing / (kSK + kSV));
   // what is left takes one more V (K is refilled half a slot earlier than V)
   static constexpr int DK = kBoth, DV = kBoth < 4 && kRing >= kBoth * (kSK + kSV) + kSV ? kBoth + 1 : kBoth;
   static constexpr int kRingBytes = DK * kSK + DV * kSV;
-  static constexpr int kPlaneBytes = NT * 8 * kBlkPlane * 4;   // a team's ring doubles as its plane
   static constexpr int kTeamBytes = kPBytes + (kRingBytes > kPlaneBytes ? kRingBytes : (kPlaneBytes + 127) & ~127);
   static constexpr int kSmem = kHead + kTeams * kTeamBytes;
   static constexpr int kThreads = kTeams * 128;
@@ -185,7 +185,7 @@ block_kernel(const __grid_constant__ BlockArgs p) {
   for (int i = threadIdx.x; i < 256; i += Geo::kThreads) {
     const int tq_i = i >> 6, n_i = (i >> 2) & 15, e_i = i & 3;
     inv[KL::dim(tq_i, n_i, e_i)] =
-        (unsigned short)((n_i >> 1) * 512 + tq_i * 16 + (n_i & 1) * 8 + (e_i >> 1) * 4 + (e_i & 1) * 2);
+        (unsigned short)((n_i >> 1) * kBlkQPair + tq_i * 16 + (n_i & 1) * 8 + (e_i >> 1) * 4 + (e_i & 1) * 2);
   }
   __syncthreads();
   pdl_wait();   // everything below reads what earlier kernels of the stream wrote
@@ -220,6 +220,17 @@ block_kernel(const __grid_constant__ BlockArgs p) {
   khead += (size_t)kvh * RK;
   vhead += (size_t)kvh * RV;
   const size_t kb = (size_t)nkv * RK, vb = (size_t)nkv * RV;
+  // the query rows: requested before anything else, so that they do not queue behind the first slots
+  constexpr int NQ = (COLS * 64 + Geo::kThreads - 1) / Geo::kThreads;
+  float4 qv[NQ];
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    const int i = threadIdx.x + k * Geo::kThreads, c = i >> 6, j = c / kGroup, h = c % kGroup;
+    qv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < COLS * 64 && j < n_tok)
+      qv[k] = *reinterpret_cast<const float4 *>(qsrc + ((size_t)(tok0 + j) * p.n_head + kvh * kGroup + h) * kHeadDim +
+                                                4 * (i & 63));
+  }
   // last and first "last key" of the chunk's tokens
   int t_max = -1, t_min = 0x7fffffff;
   if (p.items != nullptr) {
@@ -231,17 +242,6 @@ block_kernel(const __grid_constant__ BlockArgs p) {
       t_max = max(t_max, t);
       t_min = min(t_min, t);
     }
-  }
-  // the query rows: requested before the first slots, so that they do not queue behind them
-  constexpr int NQ = (COLS * 64 + Geo::kThreads - 1) / Geo::kThreads;
-  float4 qv[NQ];
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) {
-    const int i = threadIdx.x + k * Geo::kThreads, c = i >> 6, j = c / kGroup, h = c % kGroup;
-    qv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < COLS * 64 && j < n_tok)
-      qv[k] = *reinterpret_cast<const float4 *>(qsrc + ((size_t)(tok0 + j) * p.n_head + kvh * kGroup + h) * kHeadDim +
-                                                4 * (i & 63));
   }
   const int slots_total = (t_max + kBlkKeys) / kBlkKeys;   // ceil((t_max + 1) / 64)
   const int c_b = (int)(((int64_t)slots_total * s) / S), c_e = (int)(((int64_t)slots_total * (s + 1)) / S);
@@ -261,14 +261,17 @@ block_kernel(const __grid_constant__ BlockArgs p) {
                     t_max, lane);
     cp_async_commit();
   };
-  auto fill_first = [&] {
+  auto fill_ring = [&](int first, int end) {
 #pragma unroll 1
-    for (int i = 0; i < DK; ++i) {
+    for (int i = first; i < end; ++i) {
       fill_k(i);
       if (i + 1 < DV) fill_v(i);
     }
   };
-  fill_first();
+  // the first slot now, the others behind the query fragments: the copies of a whole ring take thousands of cycles to issue
+  // (many sequences: other CTAs' copies are under way whenever these are not)
+  const bool early = p.items != nullptr;
+  fill_ring(0, early ? DK : 1);
 
   for (int c = threadIdx.x; c < COLS; c += Geo::kThreads) {
     const int j = c / kGroup;
@@ -282,7 +285,7 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     for (int k = 0; k < NQ; ++k) {
       const int i = threadIdx.x + k * Geo::kThreads, c = i >> 6;
       if (i >= COLS * 64) break;
-      const uint32_t cb = qfrag + (c >> 3) * 4096 + (c & 7) * 64;
+      const uint32_t cb = qfrag + (c >> 3) * (8 * kBlkQPair) + (c & 7) * 64;
       const uint2 off = *reinterpret_cast<const uint2 *>(inv + 4 * (i & 63));
       const float x[4] = {qv[k].x, qv[k].y, qv[k].z, qv[k].w};
       const uint32_t o[4] = {off.x & 0xffffu, off.x >> 16, off.y & 0xffffu, off.y >> 16};
@@ -293,6 +296,7 @@ block_kernel(const __grid_constant__ BlockArgs p) {
       }
     }
   }
+  if (!early) fill_ring(1, DK);
   __syncthreads();
 
   float O[4][NT][4];                     // [M-tile of this warp's quarter of the dims][column tile]
@@ -324,7 +328,7 @@ block_kernel(const __grid_constant__ BlockArgs p) {
         KL::run(kr, kr + 8 * PK, tq, [&](int n, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
-            if ((n & 1) == 0) qf[nt] = lds128(qlane + nt * 4096 + (n >> 1) * 512);
+            if ((n & 1) == 0) qf[nt] = lds128(qlane + nt * (8 * kBlkQPair) + (n >> 1) * kBlkQPair);
             mma16816(Sv[nt], a0, a1, a2, a3, (n & 1) ? qf[nt].z : qf[nt].x, (n & 1) ? qf[nt].w : qf[nt].y);
           }
         });
@@ -444,7 +448,7 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     // (also frees the rings)
     if (!__syncthreads_or(!careful && finite != 0.f)) break;
     careful = true;
-    fill_first();
+    fill_ring(0, DK);
   }
 
   // ---- the teams meet ----
