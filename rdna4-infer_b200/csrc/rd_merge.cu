@@ -156,10 +156,10 @@ merge_kernel(const float *__restrict__ partial, float *__restrict__ out, int n_i
 }
 
 // Rows of blocks of tokens and of many sequences: 64 threads of four dims walk a row's records, G such
-// groups share a row, a CTA has max(4, G) groups. Bound by the latency of a row's loads, requested eight
-// records at a time: G follows the records per row. With a 1024-thread CTA per row and 64 dims, as for the
+// groups share a row, a CTA has max(4, G) groups. Bound by the latency of a row's loads, requested eight to
+// ten records at a time: G follows the records per row. With a 1024-thread CTA per row and 64 dims, as for the
 // 148 records of a long decode, most threads had no record: 64 sequences x 4 tokens x 24 heads took 194
-// us, here (G = 1) 14; 120 rows of 37 records 7.6 us, here (G = 4) 5.4.
+// us, here (G = 1) 14; 120 rows of 37 records 7.6 us, here (G = 4) 5.4, and 4.3 with ten records at a time.
 // MULTI: row = (sequence, token, head), records, split count, output and gate from the descriptor.
 template <bool MULTI, int G>
 __global__ void __launch_bounds__(G > 4 ? 64 * G : 256)
@@ -189,7 +189,7 @@ merge_rows_kernel(const float *__restrict__ partial, float *__restrict__ out, in
 #pragma unroll
     for (int e = 0; e < 4; ++e) gv[e] = gate[at + e];
   }
-  constexpr int kBatch = 8;
+  constexpr int kBatch = G == 4 ? 10 : 8;   // (four groups take the 37 records of a quarter of the SMs in one round trip)
   float m = -INFINITY, l = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int s0 = G == 1 ? 0 : grp; s0 < n_in; s0 += kBatch * G) {
