@@ -329,10 +329,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void *src, uin
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
-// Fetches `bytes` (a multiple of 16, 16-byte aligned) into L2.
-__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
 // global -> shared 2-D tile copy through a tensor map: box rows land densely in shared
 // memory (128-byte aligned), rows outside the tensor are filled with zeros. x is in
 // elements of the map's data type and must keep x * element size a multiple of 16.
