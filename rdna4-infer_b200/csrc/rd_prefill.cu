@@ -1270,9 +1270,7 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
     if (dev >= 0 && dev < 32) attr_set[dev] = true;
   }
   if (k_new != nullptr) {
-    // (a pass of many waves gains nothing from starting early)
-    const bool early = n_q <= 1024;
-    if (launch_pdl(early ? 8 : 0, kv_prep_kernel, dim3((unsigned)n_q), dim3(256), 0, st, pos, n_rot, k_new, v_new,
+    if (launch_pdl(8, kv_prep_kernel, dim3((unsigned)n_q), dim3(256), 0, st, pos, n_rot, k_new, v_new,
                    (uint4 *)k_dst, (uint4 *)v_dst, n_head_kv, make_rope_table(n_rot, freq_base), a.flags, 2 * plan.pairs) != cudaSuccess)
       return RD_ERR_CUDA;
   } else if (plan.pairs > 0 && !kv_pending) {   // (no launch of this call that zeroes the flags)
