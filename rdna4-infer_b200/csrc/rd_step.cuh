@@ -10,7 +10,7 @@
 //
 // The warps' partial results meet once, in shared memory; then every CTA of the KV head's cluster
 // stores each part of its sums into the shared memory of the CTA that owns that part of the output,
-// and after one cluster barrier the owners combine them and write the (gated) output: no records,
+// which combines them as soon as all their bytes have arrived and writes the (gated) output: no records,
 // no second launch, no remote read.
 //
 // Copies: a head's row is a narrow piece (144 bytes of q4_0) of a key, and a tensor-map box of
@@ -69,6 +69,7 @@ struct StepArgs {
   const float *k_new;
   const float *v_new;
   float *partial;       // records [head][gridDim.x][258] instead of the output, or null
+  DeviceStatus *status;
 };
 
 __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
@@ -76,8 +77,16 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
   return a;
 }
-__device__ __forceinline__ void st_cluster_f32x2(uint32_t a, float x, float y) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(x), "f"(y) : "memory");
+// Stores into a CTA of the cluster that complete on its barrier by bytes.
+__device__ __forceinline__ void st_async_f32x2(uint32_t a, float x, float y, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(a), "f"(x),
+               "f"(y), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async_f32x4(uint32_t a, float x, float y, float z, float w, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(a),
+               "f"(x), "f"(y), "f"(z), "f"(w), "r"(bar)
+               : "memory");
 }
 // Softmax reference: p = exp2(s - m) is taken against a reference m that is only moved (and the
 // accumulators rescaled) when a score exceeds it by more than kStepSlack, so p <= 2^8 -- exact
@@ -103,6 +112,7 @@ step_kernel(const __grid_constant__ StepArgs p) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ float s_m[W][8], s_t[W][8], s_l[W][8];   // per (warp, head): reference, true maximum, sum
   __shared__ float s_wt[W][kGroup];                   // weight of a warp's plane
+  __shared__ __align__(8) unsigned long long s_bar;   // the other CTAs' sums
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;
@@ -120,9 +130,14 @@ step_kernel(const __grid_constant__ StepArgs p) {
     inv[KL::dim(tq_i, n_i, e_i)] =
         (unsigned short)(tq_i * kFragPitch + (2 * n_i + (e_i >> 1)) * 4 + (e_i & 1) * 2);
   }
+  if (threadIdx.x == 0 && p.partial == nullptr) {
+    mbar_init(smem_u32(&s_bar), 1);
+    fence_barrier_init();
+    mbar_expect_tx(smem_u32(&s_bar), kGroup * kHeadDim * 4 + gridDim.x * kGroup * 8);
+  }
   __syncthreads();
-  // every CTA of the cluster has started before another one stores into its shared memory (the
-  // matching wait is at the end of the key loop)
+  // every CTA of the cluster has started, and its barrier is set up, before another one stores into its shared memory
+  // (the matching wait is at the end of the key loop)
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   pdl_wait();   // everything below reads what earlier kernels of the stream wrote
 
@@ -357,19 +372,32 @@ step_kernel(const __grid_constant__ StepArgs p) {
   }
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   __syncthreads();
+  // A head per warp, the CTA's warps over its lanes: the CTA's maximum and sum, and the weights of the warps' planes.
+  // (references never exceed the true maximum)
+  auto combine = [&](auto &&emit) {
+    for (int h = warp; h < kGroup; h += W) {
+      const bool on = lane < n_warps;
+      float mm = on ? s_t[lane][h] : kStepNone;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(FULL, mm, o));
+      mm = __shfl_sync(FULL, mm, 0);
+      const float w = on ? ex2(s_m[lane][h] - mm) : 0.f;
+      float ll = on ? s_l[lane][h] * w : 0.f;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) ll += __shfl_xor_sync(FULL, ll, o);
+      ll = __shfl_sync(FULL, ll, 0);
+      if (lane < W) s_wt[lane][h] = w * VL::kUnscale;
+      emit(h, mm, ll);
+    }
+  };
   if (records) {   // a CTA's record per head, for merge_kernel
     __shared__ float s_ml[kGroup][2];
-    for (int i = threadIdx.x; i < W * kGroup; i += NT) {
-      const int w = i / kGroup, h = i % kGroup;
-      float mm = kStepNone, ll = 0.f;
-      for (int j = 0; j < n_warps; ++j) mm = fmaxf(mm, s_t[j][h]);
-      s_wt[w][h] = ex2(s_m[w][h] - mm) * VL::kUnscale;
-      if (w == 0) {
-        for (int j = 0; j < n_warps; ++j) ll = fmaf(s_l[j][h], ex2(s_m[j][h] - mm), ll);
+    combine([&](int h, float mm, float ll) {
+      if (lane == 0) {
         s_ml[h][0] = mm > 0.5f * kStepNone ? mm * 0.6931471805599453f : -INFINITY;   // natural log
         s_ml[h][1] = mm > 0.5f * kStepNone ? ll : 0.f;
       }
-    }
+    });
     __syncthreads();
     for (int i = threadIdx.x; i < kGroup * (kHeadDim / 2); i += NT) {
       const int h = i >> 7, dd = 2 * (i & 127);
@@ -388,55 +416,53 @@ step_kernel(const __grid_constant__ StepArgs p) {
     return;
   }
   const uint32_t recv = sbase + kStepRecv, recv_ml = recv + 6144;   // [src][1536 / S] and [src][head][2]
-  for (int i = threadIdx.x; i < n_warps * kGroup; i += NT) {
-    const int w = i / kGroup, h = i % kGroup;
-    float mm = kStepNone;
-    for (int j = 0; j < n_warps; ++j) mm = fmaxf(mm, s_t[j][h]);
-    s_wt[w][h] = ex2(s_m[w][h] - mm) * VL::kUnscale;   // references never exceed the true maximum
-  }
-  for (int i = threadIdx.x; i < S * kGroup; i += NT) {   // the CTA's maximum and sum, to every CTA
-    const int dst = i / kGroup, h = i % kGroup;
-    float mm = kStepNone, ll = 0.f;
-    for (int j = 0; j < n_warps; ++j) mm = fmaxf(mm, s_t[j][h]);
-    for (int j = 0; j < n_warps; ++j) ll = fmaf(s_l[j][h], ex2(s_m[j][h] - mm), ll);
-    st_cluster_f32x2(peer_addr(recv_ml + 8 * (s * kGroup + h), dst), mm, ll);
-  }
+  const uint32_t bar = smem_u32(&s_bar);
+  combine([&](int h, float mm, float ll) {   // to every CTA
+    if (lane < S) st_async_f32x2(peer_addr(recv_ml + 8 * (s * kGroup + h), lane), mm, ll, peer_addr(bar, lane));
+  });
   __syncthreads();
-  const int part = kGroup * kHeadDim >> shift;   // output values per CTA
-  for (int i = threadIdx.x; i < kGroup * (kHeadDim / 2); i += NT) {
-    const int h = i >> 7, dd = 2 * (i & 127);
+  const int part = kGroup * kHeadDim >> shift;   // output values per CTA: a multiple of 32
+  for (int i = threadIdx.x; i < kGroup * (kHeadDim / 4); i += NT) {
+    const int h = i >> 6, dd = 4 * (i & 63);
     const int off = h * kPlane + 33 * (dd >> 5) + (dd & 31);
-    float a0 = 0.f, a1 = 0.f;
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
     for (int w = 0; w < n_warps; ++w) {
       const float *pl = reinterpret_cast<const float *>(smem + kStepHeader + w * kPlaneStride) + off;
-      a0 = fmaf(pl[0], s_wt[w][h], a0);
-      a1 = fmaf(pl[1], s_wt[w][h], a1);
+      const float wt = s_wt[w][h];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] = fmaf(pl[e], wt, a[e]);
     }
-    const int owner_rank = 2 * i / part, at = 2 * i - owner_rank * part;
-    st_cluster_f32x2(peer_addr(recv + 4 * (s * part + at), owner_rank), a0, a1);
+    const int owner_rank = 4 * i / part, at = 4 * i - owner_rank * part;
+    st_async_f32x4(peer_addr(recv + 4 * (s * part + at), owner_rank), a[0], a[1], a[2], a[3], peer_addr(bar, owner_rank));
   }
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const int e = s * part + threadIdx.x;   // this CTA's part of the output: at most NQ passes
   float gate_in = 0.f;
   if (p.gate != nullptr && (int)threadIdx.x < part) gate_in = p.gate[(size_t)kvh * kGroup * kHeadDim + e];
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  for (int i = threadIdx.x; i < part; i += NT) {
+  // Every CTA waits for its own parts only, by bytes. (With a barrier of the whole cluster and the
+  // release of every thread's stores before it, and the combinations above thread by thread over all warps, the kernel
+  // spent 5700 of its 9300 cycles behind the key loop: 137 f16 keys 8.11 us a layer, now 7.46, 4096 12.41 and 11.47.)
+  const bool ok = mbar_wait(bar, 0, p.status, 40);
+  for (int i = threadIdx.x; i < part; i += NT) {   // (whole warps, each within one head)
     const int el = s * part + i, h = el >> 8;
     const size_t at = (size_t)kvh * kGroup * kHeadDim + el;
     if (i != (int)threadIdx.x && p.gate != nullptr) gate_in = p.gate[at];
-    const float2 *ml = reinterpret_cast<const float2 *>(smem + kStepRecv + 6144) + h;
+    // the sources' maxima and sums over the lanes
+    const float2 ml = lane < S ? reinterpret_cast<const float2 *>(smem + kStepRecv + 6144)[lane * kGroup + h]
+                               : make_float2(kStepNone, 0.f);
     const float *a = reinterpret_cast<const float *>(smem + kStepRecv) + i;
-    float mm = kStepNone, l = 0.f, o = 0.f;
-    for (int c = 0; c < S; ++c) mm = fmaxf(mm, ml[c * kGroup].x);
+    float mm = ml.x;
+#pragma unroll
+    for (int o2 = 8; o2 > 0; o2 >>= 1) mm = fmaxf(mm, __shfl_xor_sync(FULL, mm, o2));
+    mm = __shfl_sync(FULL, mm, 0);
+    const float w = lane < S ? ex2(ml.x - mm) : 0.f;
+    float l = ml.y * w, o = 0.f;
+#pragma unroll
+    for (int o2 = 8; o2 > 0; o2 >>= 1) l += __shfl_xor_sync(FULL, l, o2);
+    l = __shfl_sync(FULL, l, 0);
 #pragma unroll 4
-    for (int c = 0; c < S; ++c) {
-      const float w = ex2(ml[c * kGroup].x - mm);
-      l = fmaf(ml[c * kGroup].y, w, l);
-      o = fmaf(a[c * part], w, o);
-    }
-    o = mm > 0.5f * kStepNone && l > 0.f ? o / l : 0.f;
+    for (int c = 0; c < S; ++c) o = fmaf(a[c * part], __shfl_sync(FULL, w, c), o);
+    o = ok && mm > 0.5f * kStepNone && l > 0.f ? o / l : 0.f;
     if (p.gate != nullptr) {
       const float sg = __fdiv_rn(1.0f, 1.0f + expf(-gate_in));
       p.gate[at] = sg;
@@ -475,6 +501,7 @@ int launch_step_typed(const DecodeArgs &a, float *out, float *gate, cudaStream_t
   k.k_new = a.k_new;
   k.v_new = a.v_new;
   k.partial = out == nullptr ? a.partial : nullptr;
+  k.status = a.status;
   return launch_pdl_cluster(step_kernel<KT, VT>, dim3((unsigned)a.n_splits, (unsigned)a.n_head_kv),
                             dim3(Geo::W * 32), Geo::kSmem, out == nullptr ? 1u : (unsigned)a.n_splits, st, k) == cudaSuccess
              ? RD_OK
