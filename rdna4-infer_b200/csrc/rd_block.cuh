@@ -41,6 +41,7 @@
 // converted under the first slot's copies, since a whole ring's copies take 4400 cycles to issue.
 //   us a layer with its pre-attention, merge and gate launches    two teams, ring first | now
 //   q4_0, 5 tokens over 20011 keys   30.4 | 29.6      q8_0, 4 over 20000   30.4 | 28.4      f16, 4 over 8000  24.2 | 21.9
+// Records by four dims a thread: 5 q4_0 tokens over 20011 keys 28.8 -> 28.1, 8 35.7 -> 33.5 (with the merge of ten records).
 //   64 sequences, one layer: q4_0, 5 tokens    650 | 587     q8_0, 4    620 | 590     q8_0/f16, 4   606 | 581
 #pragma once
 #include <string.h>
@@ -502,15 +503,16 @@ block_kernel(const __grid_constant__ BlockArgs p) {
     s_ml[c][1] = empty ? 0.f : ll;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_tok * kGroup * (kHeadDim / 2); i += Geo::kThreads) {
-    const int c = i >> 7, dd = 2 * (i & 127);
+  for (int i = threadIdx.x; i < n_tok * kGroup * (kHeadDim / 4); i += Geo::kThreads) {   // four dims of a column
+    const int c = i >> 6, dd = 4 * (i & 63);
     const int off = c * kBlkPlane + 33 * (dd >> 5) + (dd & 31);
-    float a0 = 0.f, a1 = 0.f;
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int w = 0; w < TEAMS; ++w) {
       const float *pl = reinterpret_cast<const float *>(smem + Geo::kHead + w * Geo::kTeamBytes) + off;
-      a0 = fmaf(pl[0], s_wt[w][c], a0);
-      a1 = fmaf(pl[1], s_wt[w][c], a1);
+      const float wt = s_wt[w][c];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] = fmaf(pl[e], wt, a[e]);
     }
     float *rec = rec0 + (((size_t)(tok0 + c / kGroup) * p.n_head + kvh * kGroup + c % kGroup) * S + s) * kRec;
     if (dd == 0) {
@@ -518,10 +520,11 @@ block_kernel(const __grid_constant__ BlockArgs p) {
       rec[1] = s_ml[c][1];
     }
     if ((reinterpret_cast<uintptr_t>(rec) & 7) == 0) {   // always, for the library's workspace
-      *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a0, a1);
+      *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a[0], a[1]);
+      *reinterpret_cast<float2 *>(rec + 4 + dd) = make_float2(a[2], a[3]);
     } else {
-      rec[2 + dd] = a0;
-      rec[3 + dd] = a1;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) rec[2 + dd + e] = a[e];
     }
   }
 }
