@@ -399,19 +399,21 @@ step_kernel(const __grid_constant__ StepArgs p) {
       }
     });
     __syncthreads();
-    for (int i = threadIdx.x; i < kGroup * (kHeadDim / 2); i += NT) {
-      const int h = i >> 7, dd = 2 * (i & 127);
+    for (int i = threadIdx.x; i < kGroup * (kHeadDim / 4); i += NT) {
+      const int h = i >> 6, dd = 4 * (i & 63);
       const int off = h * kPlane + 33 * (dd >> 5) + (dd & 31);
-      float a0 = 0.f, a1 = 0.f;
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
       for (int w = 0; w < n_warps; ++w) {
         const float *pl = reinterpret_cast<const float *>(smem + kStepHeader + w * kPlaneStride) + off;
-        a0 = fmaf(pl[0], s_wt[w][h], a0);
-        a1 = fmaf(pl[1], s_wt[w][h], a1);
+        const float wt = s_wt[w][h];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a[e] = fmaf(pl[e], wt, a[e]);
       }
       float *rec = p.partial + ((size_t)(kvh * kGroup + h) * gridDim.x + blockIdx.x) * kRec;
       if (dd == 0) rec[0] = s_ml[h][0], rec[1] = s_ml[h][1];
-      *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a0, a1);
+      *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a[0], a[1]);
+      *reinterpret_cast<float2 *>(rec + 4 + dd) = make_float2(a[2], a[3]);
     }
     return;
   }
