@@ -563,36 +563,37 @@ decode_kernel(const __grid_constant__ DecodeKernelArgs p) {
     const bool wide = (reinterpret_cast<uintptr_t>(rec0) & 7) == 0;  // always true for the library's workspace
     const float *planes = reinterpret_cast<const float *>(smem + kRingOffset);
     const size_t plane_stride = group_bytes / sizeof(float);
-    for (int idx = threadIdx.x; idx < nkv * kGroup * (kHeadDim / 2); idx += NT) {
-      const int h = idx >> 7, dd = 2 * (idx & 127);
+    for (int idx = threadIdx.x; idx < nkv * kGroup * (kHeadDim / 4); idx += NT) {   // four dims of a head
+      const int h = idx >> 6, dd = 4 * (idx & 63);
       const int c = (h / kGroup) * 8 + h % kGroup;
       float mm = kNegBig;
 #pragma unroll
       for (int w = 0; w < G; ++w) mm = fmaxf(mm, s_t[w][c]);
       const bool empty = aborted || mm <= 0.5f * kNegBig;
       const int off = h * kPlaneHead + 33 * (dd >> 5) + (dd & 31);
-      float a0 = 0.f, a1 = 0.f, ll = 0.f;
+      float a[4] = {0.f, 0.f, 0.f, 0.f}, ll = 0.f;
 #pragma unroll
       for (int w = 0; w < G; ++w) {
         const float wg = ex2(s_m[w][c] - mm);   // references never exceed the true maximum
         ll += s_l[w][c] * wg;
         if (!empty) {
-          a0 += planes[w * plane_stride + off] * wg;
-          a1 += planes[w * plane_stride + off + 1] * wg;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] += planes[w * plane_stride + off + e] * wg;
         }
       }
-      a0 *= VL::kUnscale;
-      a1 *= VL::kUnscale;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] *= VL::kUnscale;
       float *rec = rec0 + h * head_stride;
       if (dd == 0) {
         rec[0] = empty ? -INFINITY : mm * 0.6931471805599453f;  // natural log
         rec[1] = empty ? 0.f : ll;
       }
       if (wide) {
-        *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a0, a1);
+        *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a[0], a[1]);
+        *reinterpret_cast<float2 *>(rec + 4 + dd) = make_float2(a[2], a[3]);
       } else {
-        rec[2 + dd] = a0;
-        rec[3 + dd] = a1;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) rec[2 + dd + e] = a[e];
       }
     }
   }
