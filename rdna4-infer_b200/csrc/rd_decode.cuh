@@ -563,30 +563,41 @@ decode_kernel(const __grid_constant__ DecodeKernelArgs p) {
     const bool wide = (reinterpret_cast<uintptr_t>(rec0) & 7) == 0;  // always true for the library's workspace
     const float *planes = reinterpret_cast<const float *>(smem + kRingOffset);
     const size_t plane_stride = group_bytes / sizeof(float);
-    for (int idx = threadIdx.x; idx < nkv * kGroup * (kHeadDim / 4); idx += NT) {   // four dims of a head
-      const int h = idx >> 6, dd = 4 * (idx & 63);
-      const int c = (h / kGroup) * 8 + h % kGroup;
-      float mm = kNegBig;
+    // a head's groups: their weights over their references, the record's m and l over the first group's
+    if ((int)threadIdx.x < nkv * kGroup) {
+      const int h = threadIdx.x, c = (h / kGroup) * 8 + h % kGroup;
+      float mm = kNegBig, ll = 0.f;
 #pragma unroll
       for (int w = 0; w < G; ++w) mm = fmaxf(mm, s_t[w][c]);
       const bool empty = aborted || mm <= 0.5f * kNegBig;
-      const int off = h * kPlaneHead + 33 * (dd >> 5) + (dd & 31);
-      float a[4] = {0.f, 0.f, 0.f, 0.f}, ll = 0.f;
 #pragma unroll
       for (int w = 0; w < G; ++w) {
         const float wg = ex2(s_m[w][c] - mm);   // references never exceed the true maximum
         ll += s_l[w][c] * wg;
-        if (!empty) {
+        s_m[w][c] = wg * VL::kUnscale;
+      }
+      s_t[0][c] = empty ? -INFINITY : mm * 0.6931471805599453f;  // natural log
+      s_l[0][c] = empty ? 0.f : ll;
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nkv * kGroup * (kHeadDim / 4); idx += NT) {   // four dims of a head
+      const int h = idx >> 6, dd = 4 * (idx & 63);
+      const int c = (h / kGroup) * 8 + h % kGroup;
+      const float mm = s_t[0][c];
+      const int off = h * kPlaneHead + 33 * (dd >> 5) + (dd & 31);
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+      if (mm != -INFINITY) {
+#pragma unroll
+        for (int w = 0; w < G; ++w) {
+          const float wg = s_m[w][c];
 #pragma unroll
           for (int e = 0; e < 4; ++e) a[e] += planes[w * plane_stride + off + e] * wg;
         }
       }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) a[e] *= VL::kUnscale;
       float *rec = rec0 + h * head_stride;
       if (dd == 0) {
-        rec[0] = empty ? -INFINITY : mm * 0.6931471805599453f;  // natural log
-        rec[1] = empty ? 0.f : ll;
+        rec[0] = mm;
+        rec[1] = s_l[0][c];
       }
       if (wide) {
         *reinterpret_cast<float2 *>(rec + 2 + dd) = make_float2(a[0], a[1]);
