@@ -390,8 +390,8 @@ int rd_attn_split_batch(const float *q, const void *k, const void *v, float *out
  * TMEM accumulators. The admission window is wider than the reference's (any n_q >= 1
  * and any key count), since the tensor-core kernel has no measured-only range to
  * protect. keys_total rows must exist in the caches; token i attends keys 0..pos[i].
- * When n_q * n_head / 128 CTAs would leave most SMs idle, the keys are split over more CTAs
- * and a second launch merges per-split records; rd_fa2_prefill and rd_attn_prefill_fused
+ * When the tiles alone would leave SMs idle, their keys are split over more CTAs, whose records a second
+ * launch merges or the tile's first CTA collects; rd_fa2_prefill and rd_attn_prefill_fused
  * keep those records in the library's own per-device workspace (grown on demand like that
  * of the allocating launchers above: warm up once before a stream capture), while
  * rd_attn_prefill_typed keeps them in the caller's workspace and never allocates. */
@@ -445,7 +445,7 @@ int rd_attn_prefill_typed(const float *q, const void *k, const void *v, float *o
  * Synchronises the device; meant for tests and debugging, not for the hot path. */
 int rd_device_status(void);
 /* Which wait gave up, for the last RD_ERR_DEVICE that rd_device_status returned: a small
- * site number from the kernel sources (prefill 11-23, decode 1-9 and 90, exchange 100 +
+ * site number from the kernel sources (prefill 11-29, decode 1-9, 40 and 90, exchange 100 +
  * rank); 0 if none was ever reported. For bug reports. */
 int rd_device_timeout_site(void);
 

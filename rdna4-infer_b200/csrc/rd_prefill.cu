@@ -1113,7 +1113,7 @@ int prefill_splits(int n_q, int keys_total, int n_head, int sms) {
 // A balanced launch has no empty SMs in its last wave and a fifth of the records, combined where they are wanted
 // instead of by a launch of their own; but most pairs of CTAs work on two parts, so it costs a run, the prologue (6) and
 // epilogue of both (a record 4, the output 5.5) and 1.5 per record read. It has to win by 5 %: long passes run at
-// the power cap, where idle SMs leave the others a higher clock. Best of the other two forms | balanced, one box:
+// the power cap, where idle SMs leave the others a higher clock. Best of the other two forms | balanced, on one GPU:
 //    389 of 12346  131.7 | 108.2     450 of 9450  111.1 | 97.6     1000 of 8000  195.3 | 152.7    512 of 12512 154.5 | 135.5
 //    512 of  8192   94.3 | 93.4      640 of 9640  116.2 | 122.5     260 of 12260  87.4 | 90.5     200 of 12200  62.6 | 74.8
 PrefillPlan prefill_plan(int n_q, int keys_total, int n_head, int sms, size_t record_bytes) {
