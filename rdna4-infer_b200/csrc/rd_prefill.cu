@@ -795,6 +795,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
       pdl_wait();   // (the flags are zeroed by the launch before this one; its end was waited for long ago)
       const bool there = lane >= n_other || flag_wait(p.flags + 2 * (p.parts[blockIdx.x >> 1].rec + lane) + rank, p.status, 29);
       lost = !__all_sync(0xffffffffu, there);
+      __syncwarp();   // what one lane's acquire has seen is seen by the others from here on (a vote orders no memory)
       float m_all = m_fin;
       for (int i = 0; i < n_other; ++i)
         m_all = fmaxf(m_all, __ldcg(reinterpret_cast<const float2 *>(others - r + 2 * i * (kPfRecBytes / 16) + kPfRecAcc) + r).x);

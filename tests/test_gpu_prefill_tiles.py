@@ -109,3 +109,31 @@ def test_balanced_launches(G, n_q, pos0, heads, nh, ragged):
         check_attn(out[:, h].cpu().numpy(), want.cpu().numpy(), what=f"head {h}")
     if ragged:
         assert (out[7] == 0).all()
+
+
+@pytest.mark.parametrize("n_q,pos0", [(512, 7680), (1000, 7000)])
+def test_balanced_launch_reads_the_records_of_its_own_pass(G, n_q, pos0):
+    """Two inputs in turn through the same record memory: a value collected before its part had written it is the other
+    input's, so every pass has to give the bits that the input gave the first time."""
+    rd, lib = G.rd, G.lib
+    n, nh, nkv = pos0 + n_q, 24, 4
+    z = C.c_int()
+    rd.check(lib.rd_attn_prefill_launch_plan(n_q, n, nh, 148, None, None, C.addressof(z), None))
+    assert z.value == 0
+    g = torch.Generator(device="cuda").manual_seed(n_q)
+    pos = torch.arange(pos0, n, dtype=torch.int32, device="cuda")
+    inputs = []
+    for _ in range(2):
+        q = torch.randn(n_q, nh, HD, device="cuda", generator=g)
+        K, V = (torch.randn(n, nkv, HD, device="cuda", generator=g).half() for _ in range(2))
+        inputs.append((q, K, V, *(torch.randn(n_q, nkv, HD, device="cuda", generator=g) for _ in range(2))))
+    out, first = torch.empty_like(inputs[0][0]), [None, None]
+    for i in range(24):
+        q, K, V, kn, vn = inputs[i & 1]
+        rd.check(lib.rd_attn_prefill_append_fused(rd.ptr(q), rd.ptr(kn), rd.ptr(vn), rd.ptr(K), rd.ptr(V), rd.ptr(out), None,
+                                                  rd.ptr(pos), n_q, pos0, n, nh, nkv, HD, 1 / 16, 64, 1e7, G.st()))
+        if first[i & 1] is None:
+            first[i & 1] = out.clone()
+        assert torch.equal(out, first[i & 1]), i
+    assert not torch.equal(*first)
+    G.status_ok()
