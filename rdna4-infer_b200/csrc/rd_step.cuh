@@ -88,6 +88,13 @@ __device__ __forceinline__ void st_async_f32x4(uint32_t a, float x, float y, flo
                "f"(x), "f"(y), "f"(z), "f"(w), "r"(bar)
                : "memory");
 }
+// Where a CTA's wait for the others' stores has run out: it stays until no store can reach its shared memory any more,
+// that is until every thread of the cluster has ended or has come here, and what those have sent has landed (a
+// millisecond is a thousand times what it takes). Every wait in the cluster is bounded, so this one is; whole warps.
+__device__ __forceinline__ void cluster_linger() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (const unsigned long long t0 = global_ns(); global_ns() - t0 < 1000000ull;) {}
+}
 // Softmax reference: p = exp2(s - m) is taken against a reference m that is only moved (and the
 // accumulators rescaled) when a score exceeds it by more than kStepSlack, so p <= 2^8 -- exact
 // enough in f16 and far from overflow -- and the rescale runs once or twice per warp.
@@ -472,6 +479,7 @@ step_kernel(const __grid_constant__ StepArgs p) {
     }
     p.out[at] = o;
   }
+  if (!__all_sync(FULL, ok)) cluster_linger();
 }
 
 // Grid (n_splits, n_head_kv), a cluster per KV head.

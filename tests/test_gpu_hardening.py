@@ -3,6 +3,7 @@ reported -- each case in a fresh process, so that the call under test is the fir
 library sees there."""
 import json
 import os
+import shutil
 import subprocess
 import sys
 
@@ -73,3 +74,15 @@ def test_multi_twice_on_one_workspace_with_growing_context(cuda, oracle):
         want = oracle.attn(q, kc, vc, np.array([n - 1], dtype=np.int32), NKV, 1 / 16, 2, 3)
         check_attn(G.host(out), want, what=f"{n} keys")
     G.status_ok()
+
+
+def test_timed_out_cluster_cta_stays_for_late_stores(cuda, tmp_path):
+    """A CTA that gives up on its cluster must not leave while a peer still stores into its shared memory."""
+    if shutil.which("nvcc") is None:
+        pytest.skip("no nvcc")
+    root, exe = os.path.dirname(HERE), str(tmp_path / "cluster_linger")
+    subprocess.check_call(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "--expt-relaxed-constexpr",
+                           "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "rdna4-infer_b200", "csrc"),
+                           "-o", exe, os.path.join(HERE, "cpp", "cluster_linger.cu")])
+    out = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0 and out.stdout.split() == ["gave", "up", "1,", "value", "42"], out.stdout + out.stderr
