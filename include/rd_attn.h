@@ -163,14 +163,17 @@ int rd_attn_splits_for(int n_keys, int k_type, int v_type, int n_head, int force
 enum { RD_FORM_CLUSTERS = 0, RD_FORM_HEAD_RECORDS = 1, RD_FORM_ALL_HEADS = 2, RD_FORM_BLOCK = 3 };
 int rd_attn_launch_plan(int64_t n_keys, int n_tok, int n_head_kv, int k_type, int v_type, int sm_count,
                         int *form, int *n_splits, int *n_ctas);
-/* What the prefill entries do with a chunk of n_q tokens over keys_total keys on a GPU of
- * sm_count SMs (<= 0: the current device): the key splits per (128-token tile, head) and
- * the CTAs of the tile-kernel launch. One split unless the cost model says that filling the
- * idle SMs outweighs a second wave of fixed costs and the records (from about 8192 keys for
- * 512 tokens x 24 heads on 148 SMs). This is the plan of tiles of one head, whose records rd_attn_prefill_workspace_bytes
- * has room for; rd_attn_prefill_launch_plan is what is launched, with the rows of a tile: tile_heads x tile_tokens
- * and, as n_splits, 0 for a launch whose tiles are cut into parts of uneven length.
- * Host arithmetic only when sm_count is given. */
+/* How a prefill chunk of n_q tokens over keys_total keys is cut on a GPU of sm_count SMs (<= 0: the current device).
+ * Host arithmetic only when sm_count is given; any output pointer may be NULL.
+ * rd_attn_prefill_launch_plan: the launch of rd_fa2_prefill, rd_attn_prefill_fused and rd_attn_prefill_append_fused:
+ * the rows of a CTA's tile (tile_heads x tile_tokens), the key splits of a tile (0: the tiles are cut into parts of
+ * uneven length) and the CTAs. rd_attn_prefill_typed takes the same rule with the record memory of its workspace (what
+ * lies behind the f16 copies), so over quantized caches it splits short chunks that are reported, and over f16 caches
+ * run, as one split.
+ * rd_attn_prefill_plan: the rule of tiles of one head and 128 tokens, which decides whether a call over f16 caches uses
+ * records at all and how many rd_attn_prefill_typed has to have room for: the key splits of a (128-token tile, head)
+ * and the CTAs that they make. One split unless the cost model says that filling the idle SMs outweighs a second wave
+ * of fixed costs and the records (from about 8192 keys for 512 tokens x 24 heads on 148 SMs). */
 int rd_attn_prefill_launch_plan(int n_q, int keys_total, int n_head, int sm_count, int *tile_heads, int *tile_tokens,
                                 int *n_splits, int *n_ctas);
 int rd_attn_prefill_plan(int n_q, int keys_total, int n_head, int sm_count, int *n_splits, int *n_ctas);
@@ -430,7 +433,7 @@ int rd_attn_prefill_append_fused(const float *q, const float *k_new, const float
  * 6 x 6 K x V types; dispatch src/graph.cuh:1486-1527), where every one of the n_q tokens
  * re-streams and re-expands its prefix. Here the caches that are not f16 are expanded ONCE
  * into `workspace` (rd_attn_prefill_workspace_bytes, which also covers the records of
- * the key split) with the exact values of the reference's dequantizing loads
+ * a key split that the call makes use of; none for f16 caches whose keys are not split) with the exact values of the reference's dequantizing loads
  * (kv.h:174-368) rounded to f16, and the tcgen05 prefill kernel runs over that copy. Arguments as rd_attn_prefill_fused; token i attends
  * keys 0..pos[i], keys_total rows must exist. No allocation, no host synchronisation. */
 size_t rd_attn_prefill_workspace_bytes(int k_type, int v_type, int n_q, int keys_total, int n_head,

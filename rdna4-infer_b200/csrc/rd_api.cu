@@ -1129,8 +1129,8 @@ static size_t prefill_copy_bytes(int k_type, int v_type, int keys_total, int n_h
   const size_t one = align256((size_t)keys_total * n_head_kv * kHeadDim * 2);
   return (k_type != RD_KV_F16 ? one : 0) + (v_type != RD_KV_F16 ? one : 0);
 }
-// What a call has to have, and what it makes use of: a chunk of up to 256 tokens is cut into more key ranges than
-// the one-head form's where its records find room.
+// What a call has to have, and (`all`) what it makes use of: a chunk of up to 256 tokens is cut into more key ranges
+// than the one-head form's where its records find room. A call that has to have nothing uses nothing.
 static size_t prefill_workspace(int k_type, int v_type, int n_q, int keys_total, int n_head, int n_head_kv,
                                 int head_dim, bool all) {
   int dev;
@@ -1139,10 +1139,11 @@ static size_t prefill_workspace(int k_type, int v_type, int n_q, int keys_total,
     return 0;
   const int sms = sm_count(dev);
   const int splits = prefill_splits(n_q, keys_total, n_head, sms);
+  const size_t copies = prefill_copy_bytes(k_type, v_type, keys_total, n_head_kv);
   size_t records = prefill_record_bytes(n_q, n_head, splits);
-  if (all && n_q <= 256)
+  if (all && n_q <= 256 && copies + records > 0)
     records = std::max(records, prefill_record_bytes(n_q, n_head, prefill_plan(n_q, keys_total, n_head, sms, SIZE_MAX)));
-  return prefill_copy_bytes(k_type, v_type, keys_total, n_head_kv) + align256(records);
+  return copies + align256(records);
 }
 size_t rd_attn_prefill_workspace_bytes(int k_type, int v_type, int n_q, int keys_total, int n_head,
                                        int n_head_kv, int head_dim) {

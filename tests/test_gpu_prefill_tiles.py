@@ -79,6 +79,18 @@ def test_workspace_with_less_room_than_the_plan(G, oracle, n_q, pos0):
     G.status_ok()
 
 
+@pytest.mark.parametrize("n_q,n", [(24, 1224), (64, 1864), (200, 1400), (8, 8)])
+def test_no_workspace_is_asked_for_that_is_not_used(G, n_q, n):
+    """f16 caches whose keys are not split need no workspace, so none is asked for and none is written."""
+    rd, lib = G.rd, G.lib
+    z = C.c_int()
+    rd.check(lib.rd_attn_prefill_plan(n_q, n, 24, 148, C.addressof(z), None))
+    assert z.value == 1
+    assert lib.rd_attn_prefill_workspace_bytes(1, 1, n_q, n, 24, 4, HD) == 0
+    copies = 2 * ((n * 4 * HD * 2 + 255) // 256 * 256)
+    assert lib.rd_attn_prefill_workspace_bytes(2, 2, n_q, n, 24, 4, HD) >= copies
+
+
 @pytest.mark.parametrize("n_q,pos0,heads,nh,ragged", [(389, 11957, 3, 24, False), (512, 7680, 1, 24, False), (1000, 7000, 3, 24, False),
                                                       (450, 9000, 3, 24, True), (2000, 6000, 3, 12, False)])
 def test_balanced_launches(G, n_q, pos0, heads, nh, ragged):
