@@ -70,6 +70,18 @@ void *ensure_workspace(int dev, size_t bytes) {
   return d.ws;
 }
 
+size_t workspace_room(int dev) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  return g_dev[dev].ws_bytes;
+}
+// Nothing can be allocated for a launch on `st` now (a capture is under way, there or in a way that reaches it).
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s;
+  if (cudaStreamIsCapturing(st, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 bool known_type(int t) { return t >= RD_KV_F32 && t <= RD_KV_Q4_1; }
 bool aligned(const void *p, size_t a) { return ((uintptr_t)p & (a - 1)) == 0; }
 
@@ -1080,10 +1092,19 @@ static int prefill_common(const float *q, const void *k, const void *v, float *o
   // Records of a key split: in the caller's memory as far as it goes, or in the library's workspace, which is
   // used where the one-head form wants a split (an unsplit call needs none, and never allocates).
   const int sms = sm_count(dev);
-  if (records == nullptr) record_bytes = prefill_splits(n_q, keys_total, n_head, sms) > 1 ? SIZE_MAX : 0;
-  const PrefillPlan plan = prefill_plan(n_q, keys_total, n_head, sms, record_bytes);
+  const int one_head = prefill_splits(n_q, keys_total, n_head, sms);
+  if (records == nullptr) record_bytes = one_head > 1 ? SIZE_MAX : 0;
+  PrefillPlan plan = prefill_plan(n_q, keys_total, n_head, sms, record_bytes);
   if (records == nullptr && (plan.splits > 1 || plan.pairs > 0)) {
-    records = ensure_workspace(dev, prefill_record_bytes(n_q, n_head, plan));
+    // A capture cannot grow the workspace: there, room for the one-head form's records is enough, so eager calls
+    // leave at least that much.
+    const size_t least = prefill_record_bytes(n_q, n_head, one_head), room = workspace_room(dev);
+    size_t need = std::max(least, prefill_record_bytes(n_q, n_head, plan));
+    if (need > room && least <= room && capturing((cudaStream_t)stream)) {
+      plan = prefill_plan(n_q, keys_total, n_head, sms, room);
+      need = room;
+    }
+    records = ensure_workspace(dev, need);
     if (records == nullptr) return RD_ERR_CUDA;
   }
   if (dequant != nullptr && (rc = launch_kv_dequant_f16_pair(*dequant, prefill_flags(records, plan), 2 * plan.pairs,

@@ -81,6 +81,44 @@ def mode_first_call_timeout():
     return {"rc": rc, "status_first": first, "status_second": second, "zeros": bool((out == 0).all())}
 
 
+def mode_capture_after_another_warm_up():
+    """The workspace was grown by eager prefill calls; what is captured then needs at most what the records of one-head
+    tiles took there: a longer prefix (whose own plan would want more), and a block of tokens. Replayed and checked."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    worst, rcs = 0.0, []
+
+    def case(n_q, pos0):
+        n = n_q + pos0
+        q, K, V = (torch.randn(*s, device="cuda", generator=g) for s in ((n_q, NH, HD), (n, NKV, HD), (n, NKV, HD)))
+        return n_q, n, q, K.half(), V.half(), torch.empty_like(q), torch.arange(pos0, n, dtype=torch.int32, device="cuda")
+
+    def prefill(n_q, n, q, K, V, out, pos):
+        rcs.append(lib.rd_attn_prefill_fused(rd.ptr(q), rd.ptr(K), rd.ptr(V), rd.ptr(out), None, rd.ptr(pos), n_q, n, NH,
+                                             NKV, HD, 1 / 16, 0, 0.0, rd.stream_ptr()))
+
+    def block(n_q, n, q, K, V, out, pos):
+        rcs.append(lib.rd_attn_split_batch(rd.ptr(q), rd.ptr(K), rd.ptr(V), rd.ptr(out), None, rd.ptr(pos), n_q, NH, NKV, HD,
+                                           1 / 16, 1, 1, 1, rd.stream_ptr()))
+
+    for warm, call, shape in (((64, 6000), prefill, (64, 8000)), ((512, 7680), block, (1000, 200))):
+        prefill(*case(*warm))
+        n_q, n, q, K, V, out, pos = case(*shape)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call(n_q, n, q, K, V, out, pos)
+        past = torch.arange(n, device="cuda")[None, :] > pos[:, None]
+        for _ in range(2):
+            out.fill_(float("nan"))
+            graph.replay()
+            torch.cuda.synchronize()
+            for h in (0, 7, 23):
+                s = (q[:, h].double() @ K[:, h // 6].double().T / 16).masked_fill_(past, -torch.inf)
+                worst = max(worst, float((out[:, h] - torch.softmax(s, 1) @ V[:, h // 6].double()).abs().nan_to_num(1e9).max()))
+    return {"rcs": rcs, "max_abs": worst, "status": lib.rd_device_status()}
+
+
 if __name__ == "__main__":
-    res = {"env_switches": mode_env_switches, "first_call_timeout": mode_first_call_timeout}[sys.argv[1]]()
+    res = {"capture_after_another_warm_up": mode_capture_after_another_warm_up,
+           "env_switches": mode_env_switches, "first_call_timeout": mode_first_call_timeout}[sys.argv[1]]()
     print("RESULT " + json.dumps(res))

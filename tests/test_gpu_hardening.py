@@ -47,6 +47,12 @@ def test_first_call_time_out_is_reported(cuda):
     assert res["zeros"]
 
 
+def test_prefill_capture_after_the_warm_up_of_another_shape(cuda):
+    """What could be captured with the one-head records' room can be captured still."""
+    res = run_child("capture_after_another_warm_up")
+    assert res["rcs"] == [0] * 4 and res["status"] == 0 and res["max_abs"] <= 2e-3, res
+
+
 def test_multi_twice_on_one_workspace_with_growing_context(cuda, oracle):
     """The per-sequence tensor maps are rewritten at the same workspace address by the
     second call: the kernel must read the new ones (newest keys attended)."""
