@@ -779,6 +779,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
     const float l_tot = s_fin[0][0][r] * ex2(s_fin[0][1][r] - m_fin) + s_fin[1][0][r] * ex2(s_fin[1][1][r] - m_fin);
     const bool rec_mode = gridDim.z > 1;   // un-normalised records for prefill_merge_kernel
     const bool have = nt > 0 && !aborted;
+    // Where a unit's parts are added up, a row without a key in this one gives nothing: its accumulators may be
+    // 0 x infinity, from values behind the row's last key.
+    const bool empty = !have || (kBalanced && l_tot == 0.f);
     float l_sum = l_tot;   // of the unit's parts
     // Weights of the parts: this one's, then [part][row] in the third K slot, behind the row sums.
     float w_own = 1.f;
@@ -827,7 +830,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         if (have) {
           tmem_ld32(lane_addr + kTmemO + 32 * b, o);
           tmem_wait_ld();
-        } else {
+        }
+        if (empty) {
 #pragma unroll
           for (int e = 0; e < 32; ++e) o[e] = 0u;
         }
@@ -859,7 +863,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_kernel(const __grid_con
         if (have) {
           tmem_ld32(lane_addr + kTmemO + 32 * b, o);
           tmem_wait_ld();
-        } else {
+        }
+        if (empty) {
 #pragma unroll
           for (int e = 0; e < 32; ++e) o[e] = 0u;
         }

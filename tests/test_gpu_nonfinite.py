@@ -140,3 +140,30 @@ def test_prefill_gate_nan(G, oracle, n_q, pos0, splits):
     torch.cuda.synchronize()
     same(G.host(out), want, f"{n_q} at {pos0}")
     G.status_ok()
+
+
+def test_balanced_prefill_parts_without_keys_of_a_row(G):
+    """A tile's first token attends all keys, the others the first 100 at most: an infinite row behind those lies in parts
+    of the tile's keys that they have nothing in, and is added to no output of theirs. Against f64."""
+    rd, lib = G.rd, G.lib
+    n_q, n = 450, 9450
+    tokens, z = C.c_int(), C.c_int()
+    rd.check(lib.rd_attn_prefill_launch_plan(n_q, n, NH, 148, None, C.addressof(tokens), C.addressof(z), None))
+    assert (tokens.value, z.value) == (42, 0)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q = torch.randn(n_q, NH, HD, device="cuda", generator=g)
+    K, V = (torch.randn(n, NKV, HD, device="cuda", generator=g).half() for _ in range(2))
+    V[n - 3, :, 5] = torch.inf
+    pos = torch.randint(0, 100, (n_q,), dtype=torch.int32, device="cuda", generator=g)
+    pos[::42], pos[7] = n - 1, -1
+    out = torch.full_like(q, float("nan"))
+    rd.check(lib.rd_fa2_prefill(rd.ptr(q), rd.ptr(K), rd.ptr(V), rd.ptr(out), rd.ptr(pos), n_q, n - 1, n, NH, NKV, HD, 1 / 16,
+                                G.st()))
+    torch.cuda.synchronize()
+    G.status_ok()
+    past, V[n - 3, :, 5] = torch.arange(n, device="cuda")[None, :] > pos[:, None], 0
+    for h in range(NH):
+        s = (q[:, h].double() @ K[:, h // 6].double().T / 16).masked_fill_(past, -torch.inf)
+        want = torch.nan_to_num(torch.softmax(s, 1)) @ V[:, h // 6].double()
+        want[::42, 5] = torch.inf
+        same(out[:, h].cpu().numpy(), want.cpu().numpy(), f"head {h}")
