@@ -19,10 +19,9 @@ int launch_rope(float *x, int n_tok, int n_heads, int head_dim, int n_rot, float
 int launch_deinterleave(const float *yq, float *q, float *gate, int64_t n_rows, int head_dim,
                         cudaStream_t st);
 int launch_sigmoid_gate(float *g, float *y, int64_t n, cudaStream_t st);
-// n_values stored values of `type` at src -> f16 at dst (the dequantizing loads of
-// include/rdna4/kv.h:174-368, rounded once).
-int launch_kv_dequant_f16(int type, const void *src, void *dst, int64_t n_values, cudaStream_t st);
-struct DequantJob {   // K and V, either with a null source: left out
+// n_values stored values of K (type kt) and V (type vt) -> f16 (the dequantizing loads of
+// include/rdna4/kv.h:174-368, rounded once); either with a null source: left out.
+struct DequantJob {
   int kt;
   const void *k;
   void *kdst;

@@ -369,9 +369,4 @@ int launch_kv_dequant_f16_pair(const DequantJob &job, unsigned *flags, int n_fla
              : RD_ERR_CUDA;
 }
 
-int launch_kv_dequant_f16(int type, const void *src, void *dst, int64_t n_values, cudaStream_t st) {
-  if (type < 0 || type > RD_KV_Q4_1) return RD_ERR_TYPE;
-  return launch_kv_dequant_f16_pair({type, src, dst, RD_KV_F16, nullptr, nullptr, n_values}, nullptr, 0, st);
-}
-
 }  // namespace rd

@@ -103,14 +103,12 @@ struct PrefillArgs {
   alignas(64) CUtensorMap tm_k;
   alignas(64) CUtensorMap tm_v;
   const float *q;
-  float *out;
   const float *gate;     // optional [n_q][n_head][256]
   const int32_t *pos;    // device, one per query token
   int n_q;
   int n_head;
-  int nkv;
   float qscale;          // scale * log2(e)
-  alignas(64) CUtensorMap tm_g;  // f32 rows of `gate` and `out`: boxes of [tokens][heads][32 dims], 128-byte swizzle
+  alignas(64) CUtensorMap tm_g;  // f32 rows of the gate and the output: boxes of [tokens][heads][32 dims], 128-byte swizzle
   alignas(64) CUtensorMap tm_o;
   int n_rot;             // partial RoPE of the queries: dims [0, n_rot), pairs (d, d + n_rot / 2)
   float freq[32];        // rotation frequencies of the pairs
@@ -127,10 +125,11 @@ struct PrefillArgs {
   // Balanced launch: the units (token tile, pair of CTAs along the heads), laid one behind the other, are cut into
   // as many equal runs of key tiles as pairs of CTAs fit the GPU, and every piece of a unit is a part for one pair.
   // A unit's first part writes the output; its other parts leave records for it and set their flags. The parts that
-  // leave records come first in the grid, so a waiting CTA waits for CTAs that started before it, then the rest,
-  // longest first: as the first ones end, shortest first, each is followed by what was cut off it. A part covers
-  // [c0, c1) of the unit's key tiles counted from the tokens at the end of `keys`; where pos[] says otherwise, the
-  // same fractions of what it says.
+  // leave records come first in the grid, then the rest, longest first: as the first ones end, shortest first, each is
+  // followed by what was cut off it. So a waiting CTA waits for CTAs that started before it, as long as the GPU starts
+  // blocks in the order of their numbers. CUDA does not promise that; where it were otherwise, the wait's limit of two
+  // seconds ends the launch, with zeros and a status word. A part covers [c0, c1) of the unit's key tiles counted from
+  // the tokens at the end of `keys`; where pos[] says otherwise, the same fractions of what it says.
   float4 *rec;           // [record][CTA of the pair] of kPfRecBytes
   unsigned *flags;       // [record][CTA of the pair], zero before the launch
   int groups;            // units per token tile
@@ -1232,12 +1231,10 @@ int launch_prefill(const float *q, const void *k, const void *v, float *out, con
   rc = encode_f16_tmap(&a.tm_v, v, n_head_kv, keys_total, kPfN);
   if (rc != RD_OK) return rc;
   a.q = q;
-  a.out = out;
   a.gate = gate;
   a.pos = pos;
   a.n_q = n_q;
   a.n_head = n_head;
-  a.nkv = n_head_kv;
   a.qscale = scale * 1.4426950408889634f;
   const int heads = plan.heads, tokens = pf_tokens(heads), n_splits = records == nullptr ? 1 : plan.splits;
   if (n_splits < 1 || n_splits > kPfMaxSplits || (heads != 1 && heads != 3)) return RD_ERR_SHAPE;
