@@ -116,13 +116,13 @@ def test_infinite_last_row_of_a_step(G, oracle, kt, vt, n, append):
     G.status_ok()
 
 
-@pytest.mark.parametrize("n_q,pos0,splits", [(5, 0, 1), (200, 0, 1), (130, 4000, 3)])
+@pytest.mark.parametrize("n_q,pos0,splits", [(5, 0, 1), (200, 0, 1), (130, 4000, 4)])
 def test_prefill_gate_nan(G, oracle, n_q, pos0, splits):
     """A NaN gate makes its own output NaN, with and without a key split; infinite gates give 0 and the whole value."""
     rd, lib = G.rd, G.lib
     n = pos0 + n_q
     z = C.c_int()
-    rd.check(lib.rd_attn_prefill_plan(n_q, n, NH, 148, C.addressof(z), None))
+    rd.check(lib.rd_attn_prefill_launch_plan(n_q, n, NH, 148, None, None, C.addressof(z), None))
     assert z.value == splits
     q, kc, vc = make(oracle, n, n, F16, F16, n_q)
     pos = np.arange(pos0, n, dtype=np.int32)
