@@ -1064,14 +1064,14 @@ kv_prep_kernel(const int32_t *__restrict__ pos, int n_rot, const float *__restri
       make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
 }
 
-// Key splits that fill the GPU, picked with a cost model of three constants: a key tile, a CTA's prologue +
-// epilogue (the query tile is converted and the result written whatever the key count) and a record (written
-// by the tile kernel, read by the merge pass) in the ratio 2 : 9 : 0.0005. (In microseconds they are those of the kernel
-// before the pairs of CTAs; a tile now takes about 1.2 us and prologue + epilogue 11, but a split multiplies
-// both, and the counts it picks are still the best or next to it.) Splitting pays only when the waves it saves
-// outweigh the fixed costs it multiplies: 512 tokens x 24 heads gain from about 8192 keys upwards (3 splits:
-// 96 -> 288 CTAs = two full waves of 148 SMs), shorter prefixes do not. Measured, us a layer with gate and rotation,
-// by split count (chosen in brackets):
+// The key split of tiles of one head and 128 tokens: whether a call over f16 caches uses records at all, and how many
+// rd_attn_prefill_typed has to have room for; what is launched is prefill_plan's choice below. A cost model of three
+// constants: a key tile, a CTA's prologue + epilogue (the query tile is converted and the result written whatever the key
+// count) and a record (written by the tile kernel, read by the merge pass) in the ratio 2 : 9 : 0.0005, those of the kernel
+// before the pairs of CTAs. Splitting pays only when the waves it saves outweigh the fixed costs it multiplies: 512
+// tokens x 24 heads gain from about 8192 keys upwards (3 splits: 96 -> 288 CTAs = two full waves of 148 SMs), shorter
+// prefixes do not. Measured at commit 430ed0c, which launched this split, us a layer with gate and rotation, by split
+// count (this rule's in brackets):
 //   tokens of keys     1        2        3        4        5        6        7       8
 //     24 of  4000    51.1     31.8     26.8    [23.7]    24.6     23.3     34.7    33.4
 //     60 of  9000    98.8     56.7     45.2     39.1     35.0    [32.2]    52.0    49.2
