@@ -868,6 +868,17 @@ static int multi_launch(const void *plan, float scale, void *workspace, size_t w
   a.dev_seqs = reinterpret_cast<const DecodeSeq *>(workspace);
   a.dev_items = reinterpret_cast<const int4 *>((const unsigned char *)workspace + h.off_items);
   a.n_items = h.n_items;
+  if (h.q_len > 1) {
+    int64_t slots = 0, runs = 0;
+    for (int i = 0; i < h.n_seq; ++i) {
+      DecodeSeq d;   // (a plan may lie anywhere in host memory)
+      memcpy(&d, (const unsigned char *)plan + kMultiPlanHeaderBytes + i * sizeof(d), sizeof(d));
+      slots += d.t / 64 + 1;
+      runs += d.n_splits;
+    }
+    a.item_slots = (int)(slots / std::max<int64_t>(1, runs));
+    a.waves = runs * ((h.q_len + block_chunk(h.q_len) - 1) / block_chunk(h.q_len)) * h.n_head_kv > sm_count(dev);
+  }
   a.q_len = h.q_len;
   a.n_head = h.n_head;
   a.scale = scale;

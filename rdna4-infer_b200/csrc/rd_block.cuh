@@ -37,12 +37,16 @@
 // dequantization, mma.sync, vote, exponentials, fragment stores, barrier, mma.sync (with two: issue in 35 % of the active
 // cycles, tensor pipe 22 %, DRAM 12 % over 20011 q4_0 keys). Of the 34500 cycles of a CTA there 10200 lie before the
 // first slot, 9700 in it (references, the second part of its weights, cold code), 8600 in the others, 5900 in the records.
-// A third team, where rings and registers allow it, pays where runs are long; the query rows are requested first and
-// converted under the first slot's copies, since a whole ring's copies take 4400 cycles to issue.
-//   us a layer with its pre-attention, merge and gate launches    two teams, ring first | now
-//   q4_0, 5 tokens over 20011 keys   30.4 | 29.6      q8_0, 4 over 20000   30.4 | 28.4      f16, 4 over 8000  24.2 | 21.9
-// Records by four dims a thread: 5 q4_0 tokens over 20011 keys 28.8 -> 28.1, 8 35.7 -> 33.5 (with the merge of ten records).
-//   64 sequences, one layer: q4_0, 5 tokens    650 | 587     q8_0, 4    620 | 590     q8_0/f16, 4   606 | 581
+// A third team, where rings and registers allow it, pays where runs are long (launch_block_tiles); the query rows are
+// requested first and converted under the first slot's copies, since a whole ring's copies take 4400 cycles to issue.
+//   us a layer with its pre-attention, merge and gate launches, commit 430ed0c (two teams, ring first, records by two dims a
+//   thread, merge of eight records at a time) | now (two teams; many sequences, without those launches, three):
+//                        5000 keys     20011 keys    32 sequences of 4096 to 16384
+//   q4_0, 5 tokens       22.5 | 20.1   31.5 | 28.1   319.7 | 292.1
+//   q8_0, 4              22.3 | 19.8   31.4 | 28.0   302.3 | 290.0
+//   q8_0/f16, 4          21.6 | 19.6   30.5 | 28.1   298.2 | 271.6
+//   q5_0/q4_1, 5         23.3 | 21.2   33.1 | 29.6   330.0 | 312.5
+//   f16, 4               22.8 | 19.4   34.5 | 31.0   (one team: two want 1 KB more than there is)
 #pragma once
 #include <string.h>
 
@@ -64,7 +68,7 @@ constexpr float kBlkNone = -1.0e30f;
 // their own (36 columns in 48); one of five tiles takes 23.5 instead of 26.1 us over 20011 q4_0 keys and is not built.
 __host__ __device__ constexpr int block_tiles(int n) { return n <= 2 ? 2 : n <= 4 ? 3 : n == 5 ? 4 : 6; }
 
-template <int KT, int VT, int NT>
+template <int KT, int VT, int NT, int MOST>
 struct BlockGeo {
   static constexpr int kPK = slot_pitch(KT), kPV = slot_pitch(VT);
   static constexpr int kSK = kBlkKeys * kPK, kSV = kBlkKeys * kPV;   // multiples of 128
@@ -72,10 +76,10 @@ struct BlockGeo {
   static constexpr int kPBytes = NT * 2048;                          // weight fragments of a slot, two parts, per team
   static constexpr int kHead = 512 + kQBytes;                        // dim table, query fragments
   static constexpr int budget(int teams) { return (kBlkSmem - kHead) / teams - kPBytes; }
-  // Teams: three where each gets one slot and 168 registers hold its sums (up to four column tiles), two where each gets
-  // one and another K or V of the next
+  // Teams, MOST at most (launch_block_tiles): three where each gets one slot and 168 registers hold its sums (up to four
+  // column tiles), two where each gets one and another K or V of the next
   static constexpr int kPlaneBytes = NT * 8 * kBlkPlane * 4;   // a team's ring doubles as its plane
-  static constexpr int kTeams = NT <= 4 && budget(3) >= kSK + kSV && budget(3) >= kPlaneBytes   ? 3
+  static constexpr int kTeams = MOST >= 3 && NT <= 4 && budget(3) >= kSK + kSV && budget(3) >= kPlaneBytes   ? 3
                                 : budget(2) >= kSK + kSV + (kSK < kSV ? kSK : kSV) ? 2
                                                                                    : 1;
   static constexpr int kRing = budget(kTeams) & ~127;
@@ -153,10 +157,10 @@ __device__ __forceinline__ void careful_pv(float (&O)[NT][4], uint32_t a0, uint3
   }
 }
 
-template <int KT, int VT, int NT>
-__global__ void __launch_bounds__(BlockGeo<KT, VT, NT>::kThreads, 1)
+template <int KT, int VT, int NT, int MOST>
+__global__ void __launch_bounds__(BlockGeo<KT, VT, NT, MOST>::kThreads, 1)
 block_kernel(const __grid_constant__ BlockArgs p) {
-  using Geo = BlockGeo<KT, VT, NT>;
+  using Geo = BlockGeo<KT, VT, NT, MOST>;
   using KL = KLoad<KT>;
   using VL = VLoad<VT>;
   constexpr int RK = row_bytes(KT), RV = row_bytes(VT), PK = Geo::kPK, PV = Geo::kPV, SK = Geo::kSK, SV = Geo::kSV;
@@ -529,29 +533,55 @@ block_kernel(const __grid_constant__ BlockArgs p) {
   }
 }
 
-template <int KT, int VT, int NT>
-int launch_block_tiles(const BlockArgs &k, dim3 grid, cudaStream_t st) {
-  using Geo = BlockGeo<KT, VT, NT>;
+template <int KT, int VT, int NT, int MOST>
+int launch_block_teams(const BlockArgs &k, dim3 grid, cudaStream_t st) {
+  using Geo = BlockGeo<KT, VT, NT, MOST>;
   static bool attr_set[32] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return RD_ERR_CUDA;
   if (dev < 0 || dev >= 32 || !attr_set[dev]) {
-    if (cudaFuncSetAttribute(block_kernel<KT, VT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::kSmem) !=
+    if (cudaFuncSetAttribute(block_kernel<KT, VT, NT, MOST>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::kSmem) !=
         cudaSuccess)
       return RD_ERR_CUDA;
     if (dev >= 0 && dev < 32) attr_set[dev] = true;
   }
-  return launch_pdl(2, block_kernel<KT, VT, NT>, grid, dim3(Geo::kThreads), Geo::kSmem, st, k) == cudaSuccess
+  return launch_pdl(2, block_kernel<KT, VT, NT, MOST>, grid, dim3(Geo::kThreads), Geo::kSmem, st, k) == cudaSuccess
              ? RD_OK
              : RD_ERR_CUDA;
 }
+// Two teams or three, by the 64-key slots of a CTA's run: `slots`, the mean over the items of many sequences (0: unknown,
+// the key count of one sequence is on the device), and whether the CTAs make more than a wave.
+// A third team shortens the run, but leaves each team a shallower ring (f16 values: one slot) and adds to the prologue and
+// to the planes that meet at the end. Measured, speed against commit 430ed0c, three teams | two:
+//   slots (items of a KV head)   8 (32)       16 (32)      24 (32)      24 (64)      32 (32)      34 (72)      64 (32)    147 (37)
+//   q8_0/f16, 2 tokens           0.91 | 1.03  0.91 | 1.02  0.91 | 1.00  0.96 | 1.00  0.94 | 1.00  1.04 | 1.00  0.99 | 1.01  1.11 | 0.99
+//   f16, 2                       0.95 | 1.01  0.94 | 1.00  0.95 | 1.00  1.00 | 1.02  0.96 | 1.00  1.06 | 1.00  0.99 | 1.00  1.11 | 1.00
+//   q4_0, 3                      0.97 | 1.00  1.03 | 1.03  1.02 | 1.02  1.02 | 1.02  1.02 | 1.02  1.03 | 1.00
+//   q5_0/q4_1, 4                 1.03 | 1.03  1.08 | 1.02  1.08 | 1.02  1.06 | 1.02  1.09 | 1.03  1.10 | 1.03
+// One sequence, 4 tokens         500 keys      5000          20011         40000
+//   q8_0/f16                     1.06 | 1.13   1.03 | 1.10   1.01 | 1.10   1.01 | 1.07
+//   q4_0                         1.06 | 1.13   1.08 | 1.11   1.04 | 1.10   1.06 | 1.07
+//   q5_0/q4_1                    1.12 | 1.12   1.08 | 1.08   1.16 | 1.14   1.14 | 1.09
+// (37 CTAs a KV head: 40000 keys are 17 slots.)
+struct BlockRuns {
+  int slots;
+  bool waves;
+};
+template <int KT, int VT, int NT>
+int launch_block_tiles(const BlockArgs &k, dim3 grid, BlockRuns runs, cudaStream_t st) {
+  using Three = BlockGeo<KT, VT, NT, 3>;
+  if constexpr (Three::kTeams == 3) {
+    if (runs.slots >= (Three::DK > 1 ? 16 : runs.waves ? 28 : 80)) return launch_block_teams<KT, VT, NT, 3>(k, grid, st);
+  }
+  return launch_block_teams<KT, VT, NT, 2>(k, grid, st);
+}
 template <int KT, int VT>
-int launch_block_chunk(const BlockArgs &k, dim3 grid, cudaStream_t st) {
+int launch_block_chunk(const BlockArgs &k, dim3 grid, BlockRuns runs, cudaStream_t st) {
   switch (block_tiles(k.chunk)) {
-    case 2: return launch_block_tiles<KT, VT, 2>(k, grid, st);
-    case 3: return launch_block_tiles<KT, VT, 3>(k, grid, st);
-    case 4: return launch_block_tiles<KT, VT, 4>(k, grid, st);
-    default: return launch_block_tiles<KT, VT, 6>(k, grid, st);
+    case 2: return launch_block_tiles<KT, VT, 2>(k, grid, runs, st);
+    case 3: return launch_block_tiles<KT, VT, 3>(k, grid, runs, st);
+    case 4: return launch_block_tiles<KT, VT, 4>(k, grid, runs, st);
+    default: return launch_block_tiles<KT, VT, 6>(k, grid, runs, st);
   }
 }
 
@@ -571,7 +601,7 @@ int launch_block_typed(const DecodeArgs &a, int chunk, cudaStream_t st) {
   k.nkv = a.n_head_kv;
   k.qscale = a.scale * 1.4426950408889634f;
   return launch_block_chunk<KT, VT>(
-      k, dim3((unsigned)a.n_splits, (unsigned)a.n_head_kv, (unsigned)((a.n_tok + chunk - 1) / chunk)), st);
+      k, dim3((unsigned)a.n_splits, (unsigned)a.n_head_kv, (unsigned)((a.n_tok + chunk - 1) / chunk)), {0, false}, st);
 }
 
 // Many sequences: grid (work items, n_head_kv).
@@ -587,7 +617,7 @@ int launch_block_multi_typed(const MultiDecodeArgs &a, cudaStream_t st) {
   k.qscale = a.scale * 1.4426950408889634f;
   k.seqs = a.dev_seqs;
   k.items = a.dev_items;
-  return launch_block_chunk<KT, VT>(k, dim3((unsigned)a.n_items, (unsigned)a.n_head_kv), st);
+  return launch_block_chunk<KT, VT>(k, dim3((unsigned)a.n_items, (unsigned)a.n_head_kv), {a.item_slots, a.waves}, st);
 }
 
 }  // namespace rd

@@ -137,6 +137,8 @@ struct MultiDecodeArgs {
   const DecodeSeq *dev_seqs;
   const int4 *dev_items;  // (sequence, first token, split, 0)
   int n_items;
+  int item_slots;         // 64-key slots of an item, on average, and
+  bool waves;             // whether the CTAs are more than a wave (BlockRuns)
   int q_len;
   int n_head;
   int n_head_kv;

@@ -76,3 +76,39 @@ def test_many_sequences_items_and_merges(G, oracle, n_seq, lo, hi, q_len):
         check_attn(G.host(out), want, what=f"sequence {i}, {n} keys")
         assert np.allclose(G.host(dg), sg, atol=1e-6)
     G.status_ok()
+
+
+# the 64-key slots of a run where many sequences go from two teams of warps to three: 16 (several slots in a team's ring),
+# with a single slot 28 in more than a wave of CTAs and 80 in less (four tokens are split again there)
+RUNS = [(3, 3, 37, 15), (3, 3, 37, 16), (4, 5, 37, 16), (2, 1, 64, 27), (2, 1, 64, 28), (1, 1, 64, 28), (2, 1, 37, 79),
+        (2, 1, 37, 80)]
+
+
+@pytest.mark.parametrize("kt,vt,n_seq,slots,q_len", [(*r, q) for r in RUNS for q in (2, 4, 5) if (r[3], q) != (80, 4)])
+def test_teams_of_many_sequences(G, oracle, kt, vt, n_seq, slots, q_len):
+    rd, lib, nkv, nh = G.rd, G.lib, 4, 24
+    lens = [64 * slots - i % 3 for i in range(n_seq)]
+    t, split = (C.c_int32 * n_seq)(*[n - 1 for n in lens]), (C.c_int32 * n_seq)()
+    rd.check(lib.rd_attn_multi_split(C.addressof(t), n_seq, q_len, nkv, kt, vt, 148, C.addressof(split)))
+    assert list(split) == [1] * n_seq
+    g = torch.Generator(device="cuda").manual_seed(slots + q_len)
+    seqs, keep = (rd.AttnSeq * n_seq)(), []
+    for i, n in enumerate(lens):
+        q, out, caches = torch.randn(q_len, nh, HD, device="cuda", generator=g), G.poison((q_len, nh, HD)), []
+        for kind in (kt, vt):
+            c = torch.empty(n, nkv * rd.row_bytes(kind), dtype=torch.uint8, device="cuda")
+            rd.check(lib.rd_kv_store_rows(kind, rd.ptr(torch.randn(n, nkv * HD, device="cuda", generator=g)), rd.ptr(c),
+                                          n * nkv * HD, G.st()))
+            caches.append(c)
+        seqs[i].q, seqs[i].k, seqs[i].v, seqs[i].out = rd.ptr(q), rd.ptr(caches[0]), rd.ptr(caches[1]), rd.ptr(out)
+        seqs[i].gate, seqs[i].t = None, n - 1
+        keep.append((q, *caches, out, n))
+    nb = lib.rd_attn_multi_workspace_bytes(n_seq, q_len, nh, HD)
+    ws = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    rd.check(lib.rd_attn_decode_multi(C.addressof(seqs), n_seq, q_len, nh, nkv, HD, 1 / 16, kt, vt, rd.ptr(ws), nb, G.st()))
+    torch.cuda.synchronize()
+    G.status_ok()
+    for i in (0, 1, n_seq - 1):
+        q, kc, vc, out, n = keep[i]
+        want = oracle.attn(G.host(q), G.host(kc), G.host(vc), np.arange(n - q_len, n, dtype=np.int32), nkv, 1 / 16, kt, vt)
+        check_attn(G.host(out), want, what=f"sequence {i}")
