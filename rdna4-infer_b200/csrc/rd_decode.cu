@@ -101,13 +101,23 @@ int launch_block_multi(int kt, int vt, const MultiDecodeArgs &a, cudaStream_t st
   }
 }
 
-// Where the lines lie, measured (us per layer with its pre-attention stage, 4 KV heads: one cluster per KV
-// head / step_kernel with records + merge / decode_kernel + merge):
-//   keys       3000       4096               8192              16384            32768            65536
-//   f16        11.9 / -   12.2 / 12.8 / 18   16.1 / 15.6 / 22  22.8 / 20.8 / 28 -  / 32 / 39     -
-//   q8_0/f16   12.0 / -   12.9 / 12.4 / 16   16.5 / 15.0 / 18  -  / 18.7 / 22   -  / 28.0 / 30   -  / 44.3 / 45.2
-//   q8_0       12.2 / -   12.7 / 12.0 / 14   16.5 / 14.8 / 17  -  / 19.0 / 20   -  / 26.1 / 24.8 -  / 39.3 / 36.5
-//   q4_0       11.0 / -   11.7 / 11.8 / 14   14.4 / 13.3 / 16  -  / 16.4 / 18   -  / 21.4 / 21.9 -  / 30.9 / 30.5
+// Where the lines lie, measured (us per layer with its pre-attention stage, 4 KV heads: one cluster per KV head /
+// step_kernel with records + merge; the two forms of one build):
+//   keys       2000         3000         3584         4096         4600         5632         6200         8192
+//   f16        10.4 / 11.8  11.3 / 12.7  12.0 / 13.3  12.1 / 13.6  12.7 / 14.0  13.8 / 14.5  15.3 / 14.9  16.6 / 16.3
+//   q8_0/f16   10.4 / 11.7  11.6 / 12.5  12.0 / 13.0  12.8 / 13.3  13.4 / 13.5  14.2 / 14.5  15.6 / 14.7  16.9 / 15.7
+//   q8_0       10.1 / 11.6  11.5 / 12.4  12.5 / 12.6  12.9 / 12.9  13.5 / 12.9  14.5 / 13.8  15.7 / 14.0  16.8 / 15.5
+//   q4_0        9.6 / 11.2  10.4 / 11.7  11.3 / 11.9  11.5 / 12.0  12.1 / 12.1  12.9 / 12.9  14.0 / 12.9  14.8 / 13.8
+//   q5_0/q4_1   9.7 / 11.3  10.8 / 12.0  11.7 / 12.3  12.1 / 12.5  12.9 / 12.6  13.8 / 13.3  14.9 / 13.4  16.0 / 14.3
+//   q8_0/q4_0   9.9 / 11.3  10.8 / 12.2  12.0 / 12.5  12.4 / 12.6  12.9 / 12.8  13.6 / 13.5  14.8 / 13.6  15.6 / 14.7
+// The first line (5632 keys, 3584 for the pairs of three groups) was fitted to slower clusters; today they are the faster
+// form, or as fast, up to 4096 keys for those pairs too (0 to 4 % at 4096).
+// The second line, and decode_kernel (all heads) before it (step_kernel with records / decode_kernel, merges included):
+//   keys       4096         8192         16384        32768        65536
+//   f16        12.8 / 18    15.6 / 22    20.8 / 28    32 / 39      -
+//   q8_0/f16   12.4 / 16    15.0 / 18    18.7 / 22    28.0 / 30    44.3 / 45.2
+//   q8_0       12.0 / 14    14.8 / 17    19.0 / 20    26.1 / 24.8  39.3 / 36.5
+//   q4_0       11.8 / 14    13.3 / 16    16.4 / 18    21.4 / 21.9  30.9 / 30.5
 // The line at 24576 keys for the other three-group pairs (decode and merge alone, records per head / all heads):
 //   keys       4096        16384         24576         32768         65536
 //   q5_0/q4_1  8.4 / 11.5  14.2 / 14.8   17.6 / 17.5   20.1 / 19.5   31.3 / 29.1

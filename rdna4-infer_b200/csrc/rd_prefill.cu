@@ -1111,16 +1111,19 @@ int prefill_splits(int n_q, int keys_total, int n_head, int sms) {
 // Three heads of 42 tokens leave fewer rows empty than one head of 128 where the tokens end soon behind a tile's
 // edge or do not fill a tile, and their smaller launch leaves room for more key ranges. Where both cost the same, the
 // smaller split launch is the faster one, of unsplit ones that with one head (its warps without a row do nothing).
-// us a layer, one head | three heads, best split in brackets:
-//     24 of 24024   58.6 (6) | 34.9 (18)       130 of  4130   33.3 (3) | 30.3 (4)       31 of   31   14.9 | 16.0
-//     60 of  9060   32.0 (6) | 30.1 (8)        200 of 12200   64.0 (3) | 60.4 (3)      450 of 4450   61.9 | 61.1
-//    700 of  5700   82.7     | 77.7            389 of 12346  123.5 (3) | 118.1 (3)    1500 of 4500  128.3 | 134.7
+// us a layer with the chunk's append, one head | three heads, best split in brackets (this table and the next: one GPU,
+// one build, forms forced):
+//     24 of 24024   59.3 (6) | 37.2 (18)       130 of  4130   35.3 (3) | 32.2 (4)       31 of   31   15.4 | 17.4
+//     60 of  9060   34.2 (6) | 32.2 (8)        200 of 12200   64.2 (3) | 62.5 (3)      450 of 4450   62.2 | 60.5
+//    700 of  5700   79.0     | 78.2            389 of 12346  124.7 (3) | 121.2 (3)    1500 of 4500  120.1 | 121.0
 // A balanced launch has no empty SMs in its last wave and a fifth of the records, combined where they are wanted
 // instead of by a launch of their own; but most pairs of CTAs work on two parts, so it costs a run, the prologue (6) and
 // epilogue of both (a record 4, the output 5.5) and 1.5 per record read. It has to win by 5 %: long passes run at
-// the power cap, where idle SMs leave the others a higher clock. Best of the other two forms | balanced, on one GPU:
-//    389 of 12346  131.7 | 108.2     450 of 9450  111.1 | 97.6     1000 of 8000  195.3 | 152.7    512 of 12512 154.5 | 135.5
-//    512 of  8192   94.3 | 93.4      640 of 9640  116.2 | 122.5     260 of 12260  87.4 | 90.5     200 of 12200  62.6 | 74.8
+// the power cap, where idle SMs leave the others a higher clock. Best of the other two forms | balanced with one head |
+// with three:
+//    389 of 12346  121.2 | 121.7 | 112.8      450 of 9450   103.6 |  99.8 | 102.5    1000 of 8000   185.3 | 161.3 | 163.6
+//    512 of 12512  133.7 | 125.9 | 143.2      512 of 8192    98.7 |  91.5 |  96.6     640 of 9640   118.7 | 121.0 | 128.7
+//    260 of 12260   82.8 |  98.3 |  91.0      200 of 12200   62.5 |  77.8 |  75.3     700 of 5700    78.2 |  92.8 |  90.5
 PrefillPlan prefill_plan(int n_q, int keys_total, int n_head, int sms, size_t record_bytes) {
   PrefillPlan best = {1, 1, 0};
   const int tiles = (keys_total + kPfN - 1) / kPfN;
