@@ -694,10 +694,12 @@ static void multi_splits(const int *t, int n_seq, int q_len, int n_head_kv, int 
   // (With one KV head a wave of items of five tokens and more is already beyond that.)
   const int64_t room = 4 * sms / tok_chunk;
   const int most_waves = block ? std::max(1, std::min(8, 4 * sms / tok_chunk / wave)) : 4;
-  // 42 GB/s an SM; a block's tile by its column tiles, one rate for all type pairs. (Measured, us per 64-key tile and CTA
-  // at 2 / 4 / 8 tokens, the rule's 0.66 / 1.32 / 2.64: q4_0 0.92 / 1.06 / 1.56, q8_0/f16 1.18 / 1.33 / 1.80, f16 1.58 / 1.70 /
-  // 2.45. The rate only weighs the tiles against a wave's fixed cost: with the measured ones 9 / 4 / 2 % of random batches
-  // of 2 to 128 sequences would be cut otherwise.)
+  // 42 GB/s an SM; a block's tile by its column tiles, one rate for all type pairs: 0.66 / 1.32 / 1.65 / 2.64 us at 2 / 4 / 5 /
+  // 8 tokens. Measured per 64-key tile and CTA, commit 430ed0c (two teams of warps everywhere), 2 / 4 / 8 tokens: q4_0 0.92 /
+  // 1.06 / 1.56, q8_0/f16 1.18 / 1.33 / 1.80, f16 1.58 / 1.70 / 2.45. Today, prologues and records included, 64 sequences of
+  // 8192 keys, 2 / 4 / 5 tokens: q4_0 1.18 / 1.46 / 1.94, q8_0/f16 1.51 / 1.74 / 2.18, f16 1.65 / 2.23 / 2.99. The rate only
+  // weighs the tiles against a wave's fixed cost: with the rates of 430ed0c 9 / 4 / 2 % of random batches of 2 to 128
+  // sequences would be cut otherwise.
   const double tile_us = block ? 0.11 * tok_chunk * kGroup / 8 * 4
                                : (double)tile * n_head_kv * (row_bytes(k_type) + row_bytes(v_type)) / 42e3;
   std::vector<int> tiles(n_seq);

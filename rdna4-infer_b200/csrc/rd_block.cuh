@@ -35,8 +35,9 @@
 //
 // What bounds it: latency. Two or three warps per scheduler (registers), each a chain of shared-memory loads,
 // dequantization, mma.sync, vote, exponentials, fragment stores, barrier, mma.sync (with two: issue in 35 % of the active
-// cycles, tensor pipe 22 %, DRAM 12 % over 20011 q4_0 keys). Of the 34500 cycles of a CTA there 10200 lie before the
-// first slot, 9700 in it (references, the second part of its weights, cold code), 8600 in the others, 5900 in the records.
+// cycles, tensor pipe 22 %, DRAM 12 % over 20011 q4_0 keys). Of the 33000 cycles of a CTA there (5 tokens, two teams, behind
+// the wait for the launch before it) 7800 lie before the first slot, 7800 in it (references, the second part of its weights,
+// cold code), 13200 in the others, 4200 in the records; with three teams 7800, 10200, 9000 and 5400.
 // A third team, where rings and registers allow it, pays where runs are long (launch_block_tiles); the query rows are
 // requested first and converted under the first slot's copies, since a whole ring's copies take 4400 cycles to issue.
 //   us a layer with its pre-attention, merge and gate launches, commit 430ed0c (two teams, ring first, records by two dims a
